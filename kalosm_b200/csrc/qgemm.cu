@@ -5,7 +5,8 @@
 // (fusor-ml/tile-ir-kernels/src/kernels/qmatmul.rs:237-349) for large M, where the small-batch
 // kernels would re-read W once per 32 rows.
 //
-// One CTA computes a tile of NH x 128 weight rows by BM = 128 or 256 activation rows of
+// This file packs the activations, chooses how a product runs, and holds the kernel of single CTAs, which is left for
+// few rows of wide matrices; most products run on CTA pairs (qgemm_pair.cu). In the kernel here a CTA computes a tile of NH x 128 weight rows by BM = 128 activation rows of
 // Y^T = W . X^T; the fp32 accumulators (NH x BM columns of 128 lanes) live in TMEM. The roles
 // are coupled only by mbarriers, there is no CTA-wide barrier in the main loop:
 //  * weight loader (one thread): W stays quantised in HBM; the raw tile-groups of the CTA's
@@ -28,12 +29,13 @@
 // Every wait is bounded (2^22 polls): on a time-out the status word and a give-up flag in shared
 // memory are set, the other roles leave at their next poll, and the CTA releases its TMEM
 // columns and exits. FB200_TCGEN05=0 switches the kernel off (32-row kernel in chunks);
-// FB200_TC_TILE="BM,NH" forces a tile shape (tests, tuning).
+// FB200_TC_TILE forces a tile shape (tests, tuning).
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 
+#include "qgemm_pair.cuh"
 #include "qgemv_common.cuh"
 
 int fb200_ensure(fb200_device* dev, void** buf, size_t* cur, size_t bytes);
@@ -41,7 +43,7 @@ int fb200_ensure(fb200_device* dev, void** buf, size_t* cur, size_t bytes);
 namespace {
 
 constexpr int BN = 128;  // weight rows per MMA (M of the MMA); a CTA tile holds NH such halves
-// activation rows per CTA tile (N of the MMA): template parameter BM = 128 or 256
+constexpr int SINGLE_BM = 128;  // activation rows per CTA tile (N of the MMA), and of a packed activation tile
 constexpr int BK = 64;   // K elements per operand stage (four K = 16 MMAs)
 constexpr int A_SBO = (BK / 8) * 128 + 64;        // A operand: bytes between 8-row groups, padded by half a
                                                   // core matrix so that rows g and g + 8 fall into different banks
@@ -76,8 +78,6 @@ struct TcArgs {
   int stages, raw_stride;  // operand stages that fit beside the raw buffers; bytes per raw tile-group slot
   int pair_tiles;          // SwiGLU (NH = 2): half 0 = gate rows, half 1 = up rows pair_tiles row-tiles further;
                            // y[M, N / 2] = silu(gate) * up. 0 = plain product
-  int kg_per;              // K groups per split (grid.z splits; = ngroups without split-K). Split z covers the
-                           // K groups z kg_per .. and writes its partial product to y + z M N (no residuals)
   int* status;
 };
 
@@ -294,11 +294,7 @@ qgemm_tc_kernel(const TcArgs a) {
   auto tile_of = [&](int i) { return a.pair_tiles ? tile0 + (i & 7) + (i >> 3) * a.pair_tiles : tile0 + i; };
   auto has_tile = [&](int i) { return a.pair_tiles ? tile0 + (i & 7) < a.pair_tiles : tile0 + i < a.ntiles; };
   constexpr int blocks_per_group = (TYPE == FB200_Q4_K || TYPE == FB200_Q6_K ? 256 : 128) / BK;
-  // this CTA's K groups: kg0 .. kg0 + ngr - 1 (all of them without split-K); the loops below count
-  // from 0 (barrier phases), only addresses use kg0
-  const int kg0 = (int)blockIdx.z * a.kg_per;
-  const int ngr = min(a.kg_per, a.ngroups - kg0);
-  const int nblocks = ngr * blocks_per_group;
+  const int ngr = a.ngroups, nblocks = ngr * blocks_per_group;
 
   if (warp < T::DQ_WARPS) {
     // ---- conversion: warp w turns row-tile w of each K block into fp16 operand rows
@@ -343,13 +339,13 @@ qgemm_tc_kernel(const TcArgs a) {
         for (int i = 0; i < T::DQ_WARPS; ++i)
           if (has_tile(i))
             bulk_g2s(smem_u32(raw + rb * raw_bytes + i * a.raw_stride),
-                     a.w + ((size_t)tile_of(i) * a.ngroups + kg0 + kg) * a.tgb, (uint32_t)a.tgb, bar_raw_full + 8 * rb);
+                     a.w + ((size_t)tile_of(i) * a.ngroups + kg) * a.tgb, (uint32_t)a.tgb, bar_raw_full + 8 * rb);
       }
     }
   } else if (warp == T::DQ_WARPS + 1) {
     // ---- activation loader: one bulk copy per K block (the tile is stored in operand layout)
     if (lane == 0) {
-      const __half* src = a.xh + ((size_t)blockIdx.y * a.ngroups + kg0) * blocks_per_group * (BM * BK);
+      const __half* src = a.xh + (size_t)blockIdx.y * nblocks * (BM * BK);
       int s = 0, round = 0;
       for (int blk = 0; blk < nblocks; ++blk) {
         if (round > 0 && !tc_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status)) break;
@@ -435,7 +431,7 @@ qgemm_tc_kernel(const TcArgs a) {
           float out = __uint_as_float(v[j]) * a.xscale[m];
           if (a.r1) out += a.r1[(size_t)m * a.r1_stride + n];
           if (a.r2) out += a.r2[idx];
-          a.y[(size_t)blockIdx.z * a.M * a.N + idx] = out;
+          a.y[idx] = out;
         }
       }
     }
@@ -446,14 +442,14 @@ qgemm_tc_kernel(const TcArgs a) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(T::TMEM_COLS) : "memory");
 }
 
-// x[M, K] f32 -> fp16 scaled by a power of two per row into (-64, 64), stored as [Mp / bm][K / 64]
-// tiles of bm rows x 64 values in the operand layout of the MMA (8 rows x 16 bytes per core
+// x[M, K] f32 -> fp16 scaled by a power of two per row into (-64, 64), stored as [Mp / 128][K / 64]
+// tiles of 128 rows x 64 values in the operand layout of the MMA (8 rows x 16 bytes per core
 // matrix, core matrices adjacent in K 128 bytes apart, 8-row groups 1024 bytes apart), so that a
 // tile is one contiguous bulk copy. One CTA per PACK_ROWS rows (512 rows give 128 CTAs); two warps
 // find the maximum of a row with independent 16-byte loads; rows >= M are zero.
 constexpr int PACK_ROWS = 4;
 __global__ void __launch_bounds__(256)
-pack_rows16_kernel(const float* __restrict__ x, int M, int K, int bm, __half* __restrict__ xh, float* __restrict__ xscale) {
+pack_rows16_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, float* __restrict__ xscale) {
   __shared__ float part[8];
   __shared__ float inv_s[PACK_ROWS];
   const int m0 = blockIdx.x * PACK_ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -483,6 +479,7 @@ pack_rows16_kernel(const float* __restrict__ x, int M, int K, int bm, __half* __
     xscale[m0 + threadIdx.x] = ldexpf(1.0f, ex - 6);
   }
   __syncthreads();
+  constexpr int bm = SINGLE_BM;
   const int nkb = K / BK;
   uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / bm) * nkb * ((size_t)bm * BK * 2) +
                       ((m0 % bm) >> 3) * CORE_SBO + (m0 & 7) * 16;
@@ -503,45 +500,72 @@ pack_rows16_kernel(const float* __restrict__ x, int M, int K, int bm, __half* __
 }
 
 template <int BM, int NH, int TYPE>
-int launch_tc_type(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, unsigned grid_z, int smem) {
+int launch_tc_type(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, int smem) {
   using T = Tc<BM, NH>;
   static bool configured[64] = {false};
   if (!configured[dev->ordinal & 63]) {
     FB_CUDA(dev, cudaFuncSetAttribute(qgemm_tc_kernel<BM, NH, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET));
     configured[dev->ordinal & 63] = true;
   }
-  return fb200_launch(dev, qgemm_tc_kernel<BM, NH, TYPE>, dim3(grid_n, grid_m, grid_z), dim3(T::THREADS), (size_t)smem, false, a);
+  return fb200_launch(dev, qgemm_tc_kernel<BM, NH, TYPE>, dim3(grid_n, grid_m), dim3(T::THREADS), (size_t)smem, false, a);
 }
 
 template <int BM, int NH>
-int launch_tc(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, unsigned grid_z, int smem) {
+int launch_tc(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, int smem) {
   switch (a.type) {
-    case FB200_Q4_0: return launch_tc_type<BM, NH, FB200_Q4_0>(dev, a, grid_n, grid_m, grid_z, smem);
-    case FB200_Q8_0: return launch_tc_type<BM, NH, FB200_Q8_0>(dev, a, grid_n, grid_m, grid_z, smem);
-    case FB200_Q4_K: return launch_tc_type<BM, NH, FB200_Q4_K>(dev, a, grid_n, grid_m, grid_z, smem);
-    case FB200_Q6_K: return launch_tc_type<BM, NH, FB200_Q6_K>(dev, a, grid_n, grid_m, grid_z, smem);
+    case FB200_Q4_0: return launch_tc_type<BM, NH, FB200_Q4_0>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q8_0: return launch_tc_type<BM, NH, FB200_Q8_0>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q4_K: return launch_tc_type<BM, NH, FB200_Q4_K>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q6_K: return launch_tc_type<BM, NH, FB200_Q6_K>(dev, a, grid_n, grid_m, smem);
   }
   return 1;
 }
 
-// Tile shape of one product: NH x 128 weight rows by bm activation rows, and the operand stages that
-// fit. Returns false when no shape fits.
-struct TcShape { int bm = 0, nh = 0, stages = 0, split = 1; size_t ctas = 0, cost = 0; };
+// How one product runs: on CTA pairs (qgemm_pair.cu, tiles of 256 activation rows by nw = 128 or 256 weight rows), or on
+// single CTAs (nw = 0; 256 weight rows by 128 activation rows, `stages` operand stages); split = K ranges side by side.
+struct TcShape { int nw = 0, stages = 0, split = 1; size_t ctas = 0; double ns = 0; };
 
-// measured time per unit of tile area relative to the 256 x 256 tile, in 1/64ths
-static const int kRelCost[2][2] = {{134, 87}, {96, 64}};  // [nh - 1][bm == 256]
+// Cost model in ns, a fit to 40..2048 rows of Llama-8B-shaped matrices: time of one tile per 256 values of K, and beside its K
+// loop. At 512 rows 28672 x 4096 Q4_K with SwiGLU takes 118 / 121 us on pairs (nw = 256 / 128) and 224 us on single CTAs,
+// 4096 x 14336 Q6_K 124 / 87 / 235 us. Single CTAs win where the pairs need one round more: up to 128 rows of many weight rows
+// (100 rows of 28672 x 4096: 63.6 us, pairs 70.1).
+constexpr int NH = 2;
+double tile_ns(const fb200_qmatrix* w, const TcShape& sh) {
+  const double k256 = (double)w->k / 256.0 / sh.split;
+  return sh.nw == 256 ? k256 * 1700.0 + 2500.0 : sh.nw ? k256 * 1050.0 + 1500.0 : k256 * 3300.0;
+}
 
-bool tc_shape(const fb200_qmatrix* w, const TileGeom& geo, size_t m, int swiglu, int bm, int nh, TcShape* out) {
-  const int raw_stride = (geo.tg_bytes + 127) & ~127;
-  const int stage = nh * A_HALF + bm * BK * 2;
-  const int stages = std::min(MAX_STAGES, (SMEM_BUDGET - TAIL_BYTES - 2 * 8 * nh * raw_stride) / stage);
-  if (stages < 2) return false;
+// Fills in what follows from nw / split; false when the shape does not fit.
+bool tc_shape(const fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, size_t m, int swiglu, TcShape* sh) {
   const size_t n_rows = swiglu ? w->n / 2 : w->n;  // weight rows along the grid
-  const size_t rows_per_cta = swiglu ? BN : BN * nh;
-  out->bm = bm; out->nh = nh; out->stages = stages;
-  out->ctas = ((n_rows + rows_per_cta - 1) / rows_per_cta) * ((m + bm - 1) / bm);
-  out->cost = (size_t)(nh * bm) * kRelCost[nh - 1][bm == 256];  // time of one CTA
+  size_t rows, tiles_m, slots;
+  if (sh->nw) {
+    rows = (size_t)(swiglu ? sh->nw / 2 : sh->nw);
+    tiles_m = (m + 255) / 256;
+    slots = (size_t)dev->sm_count / 2;
+  } else {
+    const int raw_stride = (geo.tg_bytes + 127) & ~127, stage = NH * A_HALF + SINGLE_BM * BK * 2;
+    sh->stages = std::min(MAX_STAGES, (SMEM_BUDGET - TAIL_BYTES - 2 * 8 * NH * raw_stride) / stage);
+    if (sh->stages < 2) return false;
+    rows = (size_t)(swiglu ? BN : BN * NH);
+    tiles_m = (m + SINGLE_BM - 1) / SINGLE_BM;
+    slots = (size_t)dev->sm_count;
+  }
+  sh->ctas = ((n_rows + rows - 1) / rows) * tiles_m * sh->split;
+  sh->ns = 9000.0 + (double)((sh->ctas + slots - 1) / slots) * tile_ns(w, *sh);  // packing, launches, filling the pipeline
+  if (sh->split > 1) {  // the ranges' partial products and the adding kernel
+    const double out_bytes = (double)m * (double)w->n * 4.0;
+    sh->ns += sh->split * out_bytes / 3000.0 + 2000.0 + (sh->split + 1) * out_bytes / 7000.0;
+  }
   return true;
+}
+
+// FB200_TC_TILE="256,2" / "256,1": pairs with 256 / 128 weight rows; "128,..": single CTAs
+bool tc_forced(const TcShape& sh) {
+  int bm = 0, nh = 0;
+  const char* cfg = getenv("FB200_TC_TILE");
+  if (!cfg || sscanf(cfg, "%d,%d", &bm, &nh) != 2) return true;
+  return sh.split == 1 && sh.nw == (bm == 256 ? 128 * nh : 0);
 }
 
 bool tc_covers(const fb200_qmatrix* w, const float* x, size_t m, TileGeom* geo) {
@@ -575,47 +599,66 @@ splitk_add_kernel(const float4* __restrict__ parts, int nsplit, size_t n4, int n
   y[i] = acc;
 }
 
-// Launches the product of packed rows (xh, xscale: pack_rows16_kernel with this bm) on dev->stream.
-// With sh.split > 1 the K groups are cut into sh.split ranges (grid.z), every range writes its
-// partial product into the handle's split-K scratch and a second kernel adds them (+ residuals).
+// Launches the product of packed rows (xh, xscale: pack_rows16_kernel with 128-row tiles) on dev->stream.
+// With sh.split > 1 every K range writes its partial product into the handle's split-K scratch and a second kernel adds
+// them (+ residuals).
 int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, const TcShape& sh, const __half* xh,
               const float* xscale, size_t m, float* y, bool r1_is_bias, const float* r1, const float* r2, int swiglu) {
-  const int bm = sh.bm, nh = sh.nh;
-  const int raw_stride = (geo.tg_bytes + 127) & ~127;
-  const int mp = (int)((m + bm - 1) / bm) * bm;
-  const int split = swiglu ? 1 : sh.split;
-  float* parts = nullptr;
-  if (split > 1) {
-    int rc = fb200_ensure(dev, &dev->splitk, &dev->splitk_bytes, (size_t)split * m * w->n * sizeof(float));
-    if (rc) return rc;
-    parts = reinterpret_cast<float*>(dev->splitk);
+  const int halves = (int)((m + 127) / 128), split = sh.split;
+  const size_t n_rows = swiglu ? w->n / 2 : w->n;
+  int rc;
+  if (sh.nw) {
+    PairArgs a = {};
+    a.w = w->data; a.xh = xh; a.xscale = xscale; a.y = y; a.r1 = r1; a.r2 = r2; a.r1_stride = r1_is_bias ? 0 : (int)w->n;
+    a.M = (int)m; a.N = (int)w->n; a.ngroups = w->ngroups; a.ntiles = w->ntiles; a.pair_tiles = swiglu ? w->ntiles / 2 : 0;
+    const int rows = swiglu ? sh.nw / 2 : sh.nw;
+    a.m_tiles = (halves + 1) / 2; a.n_tiles = (int)((n_rows + rows - 1) / rows);
+    a.kg_per = (w->ngroups + split - 1) / split;
+    a.splits = (w->ngroups + a.kg_per - 1) / a.kg_per;  // every range holds at least one K group
+    a.x_halves = halves; a.status = dev->status;
+    if (split > 1) {
+      rc = fb200_ensure(dev, &dev->splitk, &dev->splitk_bytes, (size_t)split * m * w->n * sizeof(float));
+      if (rc) return rc;
+      a.y = reinterpret_cast<float*>(dev->splitk);
+      a.r1 = a.r2 = nullptr;
+    }
+    a.vec = n_rows % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.r1) | reinterpret_cast<uintptr_t>(a.r2)) & 7) == 0;
+    rc = fb200_qgemm_pair(dev, sh.nw, w->type, a);
+    if (rc || split == 1) return rc;
+    const size_t n4 = m * w->n / 4;
+    splitk_add_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, dev->stream>>>(
+        reinterpret_cast<const float4*>(a.y), a.splits, n4, (int)(w->n / 4), r1, r1_is_bias ? 0 : (int)w->n, r2,
+        reinterpret_cast<float4*>(y));
+    FB_LAUNCH_CHECK(dev);
+    return FB200_OK;
   }
+  const int raw_stride = (geo.tg_bytes + 127) & ~127;
   TcArgs a;
-  a.w = w->data; a.xh = xh; a.xscale = xscale;
-  a.y = split > 1 ? parts : y;
-  a.r1 = split > 1 ? nullptr : r1;
-  a.r2 = split > 1 ? nullptr : r2;
+  a.w = w->data; a.xh = xh; a.xscale = xscale; a.y = y; a.r1 = r1; a.r2 = r2;
   a.r1_stride = r1_is_bias ? 0 : (int)w->n;
   a.M = (int)m; a.N = (int)w->n; a.K = (int)w->k;
   a.ngroups = w->ngroups; a.ntiles = w->ntiles; a.type = (int)w->type; a.tgb = geo.tg_bytes;
   a.group_elems = geo.group_elems; a.status = dev->status;
   a.stages = sh.stages; a.raw_stride = raw_stride;
   a.pair_tiles = swiglu ? w->ntiles / 2 : 0;
-  a.kg_per = (w->ngroups + split - 1) / split;
-  const unsigned gz = (unsigned)((w->ngroups + a.kg_per - 1) / a.kg_per);  // every range holds at least one K group
-  const int smem = sh.stages * (nh * A_HALF + bm * BK * 2) + 2 * 8 * nh * raw_stride + TAIL_BYTES;
-  const size_t n_rows = swiglu ? w->n / 2 : w->n;
-  const size_t rows_per_cta = swiglu ? BN : BN * nh;
-  const unsigned gn = (unsigned)((n_rows + rows_per_cta - 1) / rows_per_cta), gm = (unsigned)(mp / bm);
-  int rc;
-  if (nh == 2) rc = bm == 256 ? launch_tc<256, 2>(dev, a, gn, gm, gz, smem) : launch_tc<128, 2>(dev, a, gn, gm, gz, smem);
-  else rc = bm == 256 ? launch_tc<256, 1>(dev, a, gn, gm, gz, smem) : launch_tc<128, 1>(dev, a, gn, gm, gz, smem);
-  if (rc || split == 1) return rc;
-  const size_t n4 = m * w->n / 4;
-  splitk_add_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, dev->stream>>>(
-      reinterpret_cast<const float4*>(parts), (int)gz, n4, (int)(w->n / 4), r1, r1_is_bias ? 0 : (int)w->n, r2,
-      reinterpret_cast<float4*>(y));
+  const int smem = sh.stages * (NH * A_HALF + SINGLE_BM * BK * 2) + 2 * 8 * NH * raw_stride + TAIL_BYTES;
+  const size_t rows_per_cta = swiglu ? BN : BN * NH;
+  const unsigned gn = (unsigned)((n_rows + rows_per_cta - 1) / rows_per_cta), gm = (unsigned)halves;
+  return launch_tc<SINGLE_BM, NH>(dev, a, gn, gm, smem);
+}
+
+// x -> fp16 tiles and row scales in the handle's scratch
+int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const __half** xh, const float** xscale) {
+  const int mp = (int)((m + 127) / 128) * 128;
+  const size_t xbytes = (size_t)mp * k * 2, need = xbytes + (size_t)mp * sizeof(float);
+  int rc = fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, need);
+  if (rc) return rc;
+  __half* h = reinterpret_cast<__half*>(dev->xpack);
+  float* s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
+  pack_rows16_kernel<<<mp / PACK_ROWS, 256, 0, dev->stream>>>(x, (int)m, (int)k, h, s);
   FB_LAUNCH_CHECK(dev);
+  *xh = h;
+  *xscale = s;
   return FB200_OK;
 }
 
@@ -628,59 +671,30 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
                 const float* r2, int swiglu) {
   TileGeom geo;
   if (!tc_covers(w, x, m, &geo)) return 1;
-  // CTA tile: cost model waves x time of one CTA; among equals the larger tile (fewer re-reads of
-  // the activations through L2).
-  int force_bm = 0, force_nh = 0;
-  if (const char* cfg = getenv("FB200_TC_TILE")) sscanf(cfg, "%d,%d", &force_bm, &force_nh);
-  TcShape best;
-  size_t best_cost = ~(size_t)0;
-  for (int nh = 2; nh >= (swiglu ? 2 : 1); --nh)
-    for (int bm = 256; bm >= 128; bm -= 128) {
-      if ((force_bm && bm != force_bm) || (force_nh && nh != force_nh && !swiglu)) continue;
-      TcShape sh;
-      if (!tc_shape(w, geo, m, swiglu, bm, nh, &sh)) continue;
-      const size_t cost = ((sh.ctas + dev->sm_count - 1) / dev->sm_count) * sh.cost;
-      if (cost < best_cost) { best_cost = cost; best = sh; }
-    }
-  if (!best.bm) return 1;
-  // Split-K (plain and residual epilogues, 16-byte aligned outputs, at least 2048 values of K per range):
-  // the K groups in 2 or 4 ranges side by side (grid.z) when that lets a larger, more efficient tile
-  // fill the SMs. Times in ns, from measurements at 512 rows: a 256 x 256 tile takes 4 us per 256 values
-  // of K (the other shapes in proportion to the table above), a CTA costs 8 us beside its K loop, the
-  // ranges write split x the output at about 3 TB/s and the adding kernel takes 2 us + (split + 1)
-  // passes over the output at 7 TB/s.
+  // A split of K (plain and residual epilogues, 16-byte aligned outputs, at least 2048 values of K per range) fills the
+  // SMs where there are few tiles; it has to promise a tenth less, and the scratch for the partial products has to fit.
   static const bool no_split = getenv("FB200_TC_SPLITK") && getenv("FB200_TC_SPLITK")[0] == '0';
-  const bool may_split = !no_split && !swiglu && !force_bm && !force_nh && w->n % 4 == 0 &&
+  const bool may_split = !no_split && !swiglu && w->n % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(r1) | reinterpret_cast<uintptr_t>(r2)) & 15) == 0;
-  if (may_split) {
-    const double unit_ns = 4000.0 * ((double)w->k / 256.0) / 32768.0, out_bytes = (double)m * (double)w->n * 4.0;
-    auto total_ns = [&](const TcShape& sh, int split) {
-      const double waves = (double)((sh.ctas * split + dev->sm_count - 1) / dev->sm_count);
-      double t = waves * ((double)sh.cost * unit_ns / split + 8000.0);
-      if (split > 1) t += split * out_bytes / 3000.0 + 2000.0 + (split + 1) * out_bytes / 7000.0;
-      return t;
-    };
-    double best_ns = 0.9 * total_ns(best, 1);  // a split has to promise a tenth less
-    for (int split = 2; split <= 4; split *= 2) {
+  TcShape best;
+  for (int split = 1; split <= (may_split ? 4 : 1); split *= 2) {
+    if (split > 1) {
+      const size_t want = (size_t)split * m * w->n * sizeof(float);
       if (w->k / split < 2048 || w->ngroups < 2 * split) break;
-      for (int nh = 2; nh >= 1; --nh)
-        for (int bm = 256; bm >= 128; bm -= 128) {
-          TcShape sh;
-          if (!tc_shape(w, geo, m, 0, bm, nh, &sh)) continue;
-          const double t = total_ns(sh, split);
-          if (t < best_ns) { best_ns = t; best = sh; best.split = split; }
-        }
+      if (want > dev->splitk_bytes && dev->scratch_limit && dev->scratch_total - dev->splitk_bytes + want > dev->scratch_limit) break;
+    }
+    for (int nw = 256; nw >= (split > 1 ? 128 : 0); nw -= 128) {
+      TcShape sh;
+      sh.nw = nw; sh.split = split;
+      if (!tc_forced(sh) || !tc_shape(dev, w, geo, m, swiglu, &sh)) continue;
+      if (!best.ctas || sh.ns < (split > 1 ? 0.9 : 1.0) * best.ns) best = sh;
     }
   }
-  const int mp = (int)((m + best.bm - 1) / best.bm) * best.bm;
-  const size_t xbytes = (size_t)mp * w->k * 2, need = xbytes + (size_t)mp * sizeof(float);
-  int rc = fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, need);
-  if (rc) return rc;
-  __half* xh = reinterpret_cast<__half*>(dev->xpack);
-  float* xscale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
-  pack_rows16_kernel<<<mp / PACK_ROWS, 256, 0, dev->stream>>>(x, (int)m, (int)w->k, best.bm, xh, xscale);
-  FB_LAUNCH_CHECK(dev);
-  return tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu);
+  if (!best.ctas) return 1;
+  const __half* xh;
+  const float* xscale;
+  int rc = tc_pack(dev, x, m, w->k, &xh, &xscale);
+  return rc ? rc : tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu);
 }
 
 // Up to three products of the same rows (the q, k and v projections of a prompt pass):
@@ -695,38 +709,34 @@ int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* 
   TileGeom geo[3];
   for (int i = 0; i < n; ++i)
     if (!ws[i] || !tc_covers(ws[i], x, m, &geo[i]) || ws[i]->k != ws[0]->k) return 1;
-  // one bm for all (they share the packed rows), nh per matrix; cost = waves of all CTAs together x
-  // the time of the slowest CTA
+  // one kind of tile for all; cost = rounds of all CTAs together x the time of the slowest tile
   TcShape best[3];
-  size_t best_cost = ~(size_t)0;
-  for (int bm = 256; bm >= 128; bm -= 128)
-    for (int mask = 0; mask < (1 << n); ++mask) {
-      TcShape sh[3];
-      size_t ctas = 0, slowest = 0;
-      bool ok = true;
-      for (int i = 0; i < n && ok; ++i) {
-        ok = tc_shape(ws[i], geo[i], m, 0, bm, (mask >> i) & 1 ? 2 : 1, &sh[i]);
-        if (ok) { ctas += sh[i].ctas; slowest = std::max(slowest, sh[i].cost); }
-      }
-      if (!ok) continue;
-      const size_t cost = ((ctas + dev->sm_count - 1) / dev->sm_count) * slowest;
-      if (cost < best_cost) { best_cost = cost; for (int i = 0; i < n; ++i) best[i] = sh[i]; }
+  double best_ns = 0;
+  for (int nw = 256; nw >= 128; nw -= 128) {
+    TcShape sh[3];
+    double slowest = 0;
+    size_t ctas = 0;
+    bool ok = true;
+    for (int i = 0; i < n && ok; ++i) {
+      sh[i].nw = nw;
+      ok = tc_shape(dev, ws[i], geo[i], m, 0, &sh[i]);
+      ctas += sh[i].ctas;
+      slowest = std::max(slowest, tile_ns(ws[i], sh[i]));
     }
-  if (best_cost == ~(size_t)0) return 1;
+    const size_t slots = (size_t)dev->sm_count / 2;
+    const double ns = (double)((ctas + slots - 1) / slots) * slowest;
+    if (ok && (best_ns == 0 || ns < best_ns)) { best_ns = ns; for (int i = 0; i < n; ++i) best[i] = sh[i]; }
+  }
+  if (best_ns == 0) return 1;
   for (int i = 0; i < n - 1; ++i) {
     if (!dev->side_stream[i]) FB_CUDA(dev, cudaStreamCreateWithFlags(&dev->side_stream[i], cudaStreamNonBlocking));
     if (!dev->join_ev[i]) FB_CUDA(dev, cudaEventCreateWithFlags(&dev->join_ev[i], cudaEventDisableTiming));
   }
   if (!dev->fork_ev) FB_CUDA(dev, cudaEventCreateWithFlags(&dev->fork_ev, cudaEventDisableTiming));
-  const int bm = best[0].bm;
-  const int mp = (int)((m + bm - 1) / bm) * bm;
-  const size_t xbytes = (size_t)mp * ws[0]->k * 2, need = xbytes + (size_t)mp * sizeof(float);
-  int rc = fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, need);
+  const __half* xh;
+  const float* xscale;
+  int rc = tc_pack(dev, x, m, ws[0]->k, &xh, &xscale);
   if (rc) return rc;
-  __half* xh = reinterpret_cast<__half*>(dev->xpack);
-  float* xscale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
-  pack_rows16_kernel<<<mp / PACK_ROWS, 256, 0, dev->stream>>>(x, (int)m, (int)ws[0]->k, bm, xh, xscale);
-  FB_LAUNCH_CHECK(dev);
   FB_CUDA(dev, cudaEventRecord(dev->fork_ev, dev->stream));
   cudaStream_t main_stream = dev->stream;
   // the largest product stays on the handle's stream

@@ -1,0 +1,25 @@
+// The prefill product on CTA pairs (qgemm_pair.cu), as qgemm.cu calls it.
+#pragma once
+
+#include "common.cuh"
+
+struct PairArgs {
+  const uint8_t* w;      // tiled weights
+  const __half* xh;      // fp16 activations, [x_halves][K / 64] tiles of 128 rows in the operand layout
+  const float* xscale;   // [M] power-of-two scale of each row
+  float* y;              // [M, N]; with splits > 1 the partial product of range z goes to y + z M N
+  const float* r1;       // optional residuals [M, N], or one bias row [N] when r1_stride is 0
+  const float* r2;
+  int r1_stride;
+  int M, N;
+  int ngroups, ntiles;   // K groups per row-tile, 16-row tiles of W
+  int pair_tiles;        // SwiGLU: up rows lie this many row-tiles behind their gate rows, y is [M, N / 2]; 0: plain product
+  int m_tiles, n_tiles;  // tiles of 256 activation rows and of nw weight rows (SwiGLU: nw / 2 outputs)
+  int splits, kg_per;    // K ranges, K groups per range (every range holds at least one)
+  int x_halves;          // 128-row tiles in xh
+  int vec;               // rows of y and of the residuals are 8-byte aligned
+  int* status;
+};
+
+// Launches the product with nw = 128 or 256 weight rows per tile; 1 when the type has no kernel.
+int fb200_qgemm_pair(fb200_device* dev, int nw, uint32_t type, const PairArgs& a);

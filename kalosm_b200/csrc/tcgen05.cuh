@@ -155,4 +155,69 @@ __device__ __forceinline__ void x_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr) : "memory");
 }
 
+// ---- CTA pairs (clusters of two, the even CTA issues)
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrives on the barrier at the same place in CTA `rank` of the cluster. What the arrival announces was written by the async
+// proxy or fenced towards it, so no release at cluster scope is asked for (it takes most of a microsecond and would be paid per stage).
+__device__ __forceinline__ void cluster_arrive(uint32_t bar, uint32_t rank) {
+  asm volatile(
+      "{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %0, %1;\n"
+      "mbarrier.arrive.shared::cluster.b64 _, [r];\n}"
+      ::"r"(bar), "r"(rank) : "memory");
+}
+// One whole warp of either CTA takes and returns the columns; the address goes to `slot` of the own CTA.
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t slot, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_tmem_free(uint32_t tmem, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+// Four MMAs, K steps of 16 values whose operands lie 256 bytes apart (both K-major without swizzle). M = 256 over the pair:
+// either CTA holds 128 rows of A and half of the rows of B at the same shared-memory addresses, and all N columns of its 128 rows
+// of D at the same TMEM address. Called by a converged warp of the even CTA; one elected lane issues them all (an election per
+// instruction took longer than the MMAs).
+__device__ __forceinline__ void pair_mma4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q, t;\n.reg .b64 a1, b1, a2, b2, a3, b3;\n"
+      "add.u64 a1, %1, 16;\nadd.u64 b1, %2, 16;\nadd.u64 a2, %1, 32;\nadd.u64 b2, %2, 32;\nadd.u64 a3, %1, 48;\nadd.u64 b3, %2, 48;\n"
+      "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 t, 0, 0;\nelect.sync _|q, 0xFFFFFFFF;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, t;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, t;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, t;\n}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One poll of a barrier's phase; the answer may be asked for later
+__device__ __forceinline__ uint32_t x_poll(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok;
+}
+// Arrives on the barrier at this address in both CTAs when the MMAs issued so far are done.
+__device__ __forceinline__ void pair_commit(uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xFFFFFFFF;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
+      ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// 16 lanes x 32 columns, laid out as x_ld16x256
+__device__ __forceinline__ void x_ld16x256_32(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr) : "memory");
+}
+
 }  // namespace

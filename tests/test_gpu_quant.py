@@ -119,6 +119,32 @@ def test_prefill_product_tensor_cores(dev, tname, tile, monkeypatch):
     assert np.array_equal(xt.q_mat_mul(gu).as_slice(), xt.q_mat_mul(gu).as_slice())
 
 
+@pytest.mark.parametrize("tname", list(TYPES))
+@pytest.mark.parametrize("tile", ["256,1", "256,2"])
+@pytest.mark.parametrize("m,n,k", [(33, 16, 256), (128, 127, 512), (129, 129, 1280), (256, 257, 256), (257, 4000, 768), (900, 30000, 256)])
+def test_prefill_product_cta_pairs(dev, tname, tile, m, n, k, monkeypatch):
+    # tiles of 256 activation rows by 128 or 256 weight rows, at their edges: odd N (no paired stores), rows of one and of both
+    # CTAs, K of fewer units than conversion sets, more tiles than pairs (accumulators alternate). fp16 operands of 11 bits
+    # and exact products: each of the k terms is off by 2^-11 at most, relative to the sum of the squares far below TOL
+    monkeypatch.setenv("FB200_TC_TILE", tile)
+    ty = TYPES[tname]
+    raw = weights(41, n, k, ty)
+    w = kb.QMatrix.from_raw_bytes(dev, (n, k), raw, ty)
+    x = activations(m + n, m, k)
+    exp = x.astype(np.float64) @ w.dequantize().as_slice().astype(np.float64).T
+    assert F.rel_l2(dev.tensor(x).q_mat_mul(w).as_slice(), exp) < TOL
+    r = activations(m, m, n)
+    y = dev.tensor(x).q_mat_mul(w, epilogue=kb.EPI_RESIDUAL, r1=dev.tensor(r)).as_slice()
+    assert F.rel_l2(y, exp + r) < TOL
+    b = activations(m + 1, 1, n)[0]
+    assert F.rel_l2(dev.tensor(x).q_mat_mul(w, epilogue=kb.EPI_BIAS, r1=dev.tensor(b)).as_slice(), exp + b) < TOL
+    if n % 32 == 0:
+        h = dev.tensor(x).q_mat_mul(w, epilogue=kb.EPI_SWIGLU).as_slice()
+        g, u = exp[:, : n // 2], exp[:, n // 2:]
+        assert F.rel_l2(h, g / (1.0 + np.exp(-g)) * u) < TOL
+    assert dev.status() == 0
+
+
 def _sampled_columns(raw, ty, n, k, cols):
     """Raw GGUF bytes of the rows `cols` of an [n, k] matrix (rows are contiguous block runs)."""
     bs, bb = O.BLOCK[ty]
