@@ -43,6 +43,7 @@ int fb200_dense_product(fb200_device* dev, const fb200_dense_job& j);
 int fb200_dense_gemv(fb200_device* dev, const fb200_dense_job& j);      // m == 1
 int fb200_dense_gemm_f32(fb200_device* dev, const fb200_dense_job& j);  // F32 weights
 int fb200_dense_gemm_tc(fb200_device* dev, const fb200_dense_job& j);   // BF16 weights, tcgen05
+int fb200_dense_gemm_pair(fb200_device* dev, const fb200_dense_job& j, int nw);  // its form on CTA pairs, nw = 128 or 256 weight rows a tile
 // f32 rows (n elements at stride ldx) -> bf16 rows of np elements (zeros from n on), RMS-normalised when w is given.
 // With w2 an output row is 2 np elements: the row under w, then the row under w2.
 int fb200_rows_to_bf16(fb200_device* dev, const float* x, size_t ldx, const float* w, const float* w2, float eps, size_t rows,

@@ -1,6 +1,7 @@
 // Products of many activation rows with BF16 weights on the 5th-generation tensor cores.
 //
 // Bound: tensor cores (2 M N K flops) for prompts, HBM (the matrix is read once) for a few rows.
+// This file chooses the tiles and holds the kernel of single CTAs, for few rows (more: dense_pair.cu).
 // A CTA computes NH x 128 weight rows by BM activation rows of Y^T = W . X^T; the fp32 accumulators
 // (NH x BM columns of 128 lanes) live in tensor memory. Roles, coupled only by mbarriers:
 //  * copy requester (one thread): a stage is the NH weight boxes (64 columns x 128 rows) and the activation
@@ -260,7 +261,10 @@ int fb200_dense_gemm_tc(fb200_device* dev, const fb200_dense_job& j) {
   a.bias = j.bias; a.alpha = j.alpha; a.softcap = j.softcap; a.gelu = j.act == FB200_FFN_GELU; a.ff_col = (int)j.ff_off;
   a.m = j.m; a.kblocks = (j.kx + TC_BK - 1) / TC_BK; a.row0 = j.row0; a.n_plain = j.n_plain; a.gate0 = j.gate0; a.up0 = j.up0; a.ff = j.ff;
   a.status = dev->status;
-  // tile shape by a small cost model: rounds of CTAs over the SMs x time of one tile (relative to 256 x 256)
+  // Tile shape by a small cost model: rounds of tiles over the SMs (pairs: over half as many) x time of one tile, in units of 35 us
+  // per 2048 values of K. Above 128 rows CTA pairs (dense_pair.cu) take part: 8192 rows of 14336 x 2048 take 343 us (nw = 256)
+  // and 476 us (128), single CTAs with 256 x 256 tiles took 486 and those of 128 rows take 609; 512 rows of 2048 x 8192 64.5 us
+  // (128), 72.7 (256), 72.7 (single). Up to 128 rows half of a pair's tile is idle: 100 rows of 14336 x 2048 33.8 us, pairs 35.8.
   auto cost = [&](int bm, int nh, double tile) {
     if (nh == 1 && j.ff && j.act != FB200_FFN_GELU) return 1e30;
     const long tiles = (long)((j.n_plain + TC_BN * nh - 1) / (TC_BN * nh) + tc_ff_tiles(j, nh)) * ((j.m + bm - 1) / bm);
@@ -271,22 +275,28 @@ int fb200_dense_gemm_tc(fb200_device* dev, const fb200_dense_job& j) {
     if (rest) rounds += bm <= 64 ? (rest > dev->sm_count ? 1.0 : 0.5) : 1.0;
     return rounds * tile * (bm <= 64 ? 2.0 : 1.0);
   };
+  auto pair_cost = [&](int nw, double tile) {
+    if (j.m <= 128) return 1e30;
+    const int ff_rows = j.act == FB200_FFN_GELU ? nw : nw / 2, slots = dev->sm_count / 2;
+    const long tiles = (long)((j.n_plain + nw - 1) / nw + (j.ff + ff_rows - 1) / ff_rows) * ((j.m + 255) / 256);
+    return (double)((tiles + slots - 1) / slots) * tile;
+  };
   struct Cand { int bm, nh; double tile; };
-  const Cand cands[] = {{256, 2, 1.0}, {256, 1, 0.62}, {128, 2, 0.62}, {128, 1, 0.38}, {64, 2, 0.42}, {64, 1, 0.24}, {32, 2, 0.36}, {32, 1, 0.19}};
+  const Cand cands[] = {{128, 2, 0.62}, {128, 1, 0.38}, {64, 2, 0.42}, {64, 1, 0.24}, {32, 2, 0.36}, {32, 1, 0.19}};
   int pick = 0;
   double best = 1e31;
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 6; ++i) {
     const double c = cost(cands[i].bm, cands[i].nh, cands[i].tile);
     if (c < best) { best = c; pick = i; }
   }
+  const double c256 = pair_cost(256, 0.36), c128 = pair_cost(128, 0.26);
+  if (std::min(c256, c128) < best) return fb200_dense_gemm_pair(dev, j, c256 <= c128 ? 256 : 128);
   switch (pick) {
-    case 0: return launch_tc<256, 2>(dev, j, a);
-    case 1: return launch_tc<256, 1>(dev, j, a);
-    case 2: return launch_tc<128, 2>(dev, j, a);
-    case 3: return launch_tc<128, 1>(dev, j, a);
-    case 4: return launch_tc<64, 2>(dev, j, a);
-    case 5: return launch_tc<64, 1>(dev, j, a);
-    case 6: return launch_tc<32, 2>(dev, j, a);
+    case 0: return launch_tc<128, 2>(dev, j, a);
+    case 1: return launch_tc<128, 1>(dev, j, a);
+    case 2: return launch_tc<64, 2>(dev, j, a);
+    case 3: return launch_tc<64, 1>(dev, j, a);
+    case 4: return launch_tc<32, 2>(dev, j, a);
     default: return launch_tc<32, 1>(dev, j, a);
   }
 }

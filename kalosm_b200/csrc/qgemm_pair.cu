@@ -416,7 +416,7 @@ qgemm_pair_kernel(const PairArgs a) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int b = 0; b < 2; ++b)
-          pair_mma4(tmem + (uint32_t)(buf * NW), adesc0 + (uint64_t)((now * P::STAGE + b * PAIR_A_BLOCK) >> 4),
+          pair_mma4<16>(tmem + (uint32_t)(buf * NW), adesc0 + (uint64_t)((now * P::STAGE + b * PAIR_A_BLOCK) >> 4),
                     bdesc0 + (uint64_t)((now * P::STAGE + b * P::B_BLOCK) >> 4), P::IDESC, (u | b) ? 1u : 0u);
         pair_commit(stage_free + 8 * now);
       }

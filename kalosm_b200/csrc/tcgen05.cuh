@@ -164,6 +164,17 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// x_tma_box2 into the own CTA, counted on a barrier of either CTA of the pair (`bar`: cluster_addr)
+__device__ __forceinline__ void pair_tma_box2(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
 // Arrives on the barrier at the same place in CTA `rank` of the cluster. What the arrival announces was written by the async
 // proxy or fenced towards it, so no release at cluster scope is asked for (it takes most of a microsecond and would be paid per stage).
 __device__ __forceinline__ void cluster_arrive(uint32_t bar, uint32_t rank) {
@@ -180,20 +191,21 @@ __device__ __forceinline__ void pair_tmem_alloc(uint32_t slot, uint32_t cols) {
 __device__ __forceinline__ void pair_tmem_free(uint32_t tmem, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
-// Four MMAs, K steps of 16 values whose operands lie 256 bytes apart (both K-major without swizzle). M = 256 over the pair:
+// Four MMAs, K steps of 16 values whose operands lie STEP x 16 bytes apart (both K-major). M = 256 over the pair:
 // either CTA holds 128 rows of A and half of the rows of B at the same shared-memory addresses, and all N columns of its 128 rows
 // of D at the same TMEM address. Called by a converged warp of the even CTA; one elected lane issues them all (an election per
 // instruction took longer than the MMAs).
+template <int STEP>
 __device__ __forceinline__ void pair_mma4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p, q, t;\n.reg .b64 a1, b1, a2, b2, a3, b3;\n"
-      "add.u64 a1, %1, 16;\nadd.u64 b1, %2, 16;\nadd.u64 a2, %1, 32;\nadd.u64 b2, %2, 32;\nadd.u64 a3, %1, 48;\nadd.u64 b3, %2, 48;\n"
+      "add.u64 a1, %1, %5;\nadd.u64 b1, %2, %5;\nadd.u64 a2, %1, %6;\nadd.u64 b2, %2, %6;\nadd.u64 a3, %1, %7;\nadd.u64 b3, %2, %7;\n"
       "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 t, 0, 0;\nelect.sync _|q, 0xFFFFFFFF;\n"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, t;\n"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, t;\n"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, t;\n}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(STEP), "n"(2 * STEP), "n"(3 * STEP) : "memory");
 }
 // One poll of a barrier's phase; the answer may be asked for later
 __device__ __forceinline__ uint32_t x_poll(uint32_t bar, uint32_t parity) {

@@ -55,6 +55,20 @@ def test_dense_products(dev, m, n, k, ty):
     assert np.array_equal(q.dequantize().as_slice(), U.from_bf16(w))
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 1, 64), (129, 127, 72), (256, 129, 200), (257, 10001, 64), (600, 9990, 328)])
+def test_dense_products_on_cta_pairs(dev, m, n, k):
+    # tiles of 256 activation rows by 128 or 256 weight rows at their edges: odd N (no paired stores), rows of one CTA only, K of
+    # one block and with a ragged last one, more tiles than pairs. bf16 products are exact, sums are f32: 2^-24 sqrt(k) and less
+    rng = np.random.default_rng(m + n + k)
+    w = U.to_bf16(rng.standard_normal((n, k)))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    q = kb.QMatrix.from_raw_bytes(dev, (n, k), w, kb.BF16)
+    want = U.from_bf16(U.to_bf16(x)).astype(np.float64) @ U.from_bf16(w).astype(np.float64).T
+    got = dev.tensor(x).q_mat_mul(q).as_slice()
+    assert np.linalg.norm(got - want) < 3e-6 * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert dev.status() == 0
+
+
 # ---- each mechanism alone ------------------------------------------------------------------------------------
 
 DELTAS = [dict(), dict(heads=1, kv_heads=1, dim=8, vdim=8, conv=1), dict(heads=6, kv_heads=1, dim=33, vdim=17, conv=2),
