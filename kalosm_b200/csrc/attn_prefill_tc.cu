@@ -10,9 +10,9 @@
 //
 // One CTA = 128 query rows of one head: 128 softmax threads (thread r owns query row r, which is
 // also lane r of the CTA's TMEM columns, so the softmax statistics of a row never leave a thread)
-// one warp whose first lane issues the MMAs and one whose first lane requests the K and V tiles
-// (TMA). The roles meet only at mbarriers (tile landed: the copy's byte count; P written: 128
-// arrivals; product done: tcgen05.commit); there is no CTA-wide barrier in the loop, and neither
+// one warp that issues the MMAs and one whose first lane requests the K and V tiles
+// (TMA). The roles meet only at mbarriers (tile landed: the copy's byte count; P written: an
+// arrival per warp; product done: tcgen05.commit); there is no CTA-wide barrier in the loop, and neither
 // the issue latency of the MMAs nor the copies are on the softmax threads' path.
 // Per tile t of 64 keys:
 //   S_t = Q K_t^T   8 tcgen05.mma (M = 128 queries, N = 64 keys, K = 16 of the head size) into one of
@@ -41,6 +41,7 @@
 #include <cuda.h>
 
 #include "attn_mma.cuh"
+#include "state_columns.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -81,12 +82,13 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // bar_s[2]: S_t complete (one per S buffer); bar_o: O += P V_t complete; bar_kfull[3], bar_vfull[2]: tile
-  // landed (byte count of its two boxes); bar_pfull: P written (128 arrivals)
+  // landed (byte count of its two boxes); bar_pfull: P written (an arrival per softmax warp)
   const uint32_t bar_s = smem_u32(bars), bar_o = smem_u32(bars + 2), bar_kfull = smem_u32(bars + 3),
                  bar_vfull = smem_u32(bars + 6), bar_pfull = smem_u32(bars + 8);
 
-  const int qt = gridDim.x - 1 - blockIdx.x;  // longest key ranges first
-  const int head = blockIdx.y, bi = blockIdx.z, kvh = head / a.groups;
+  // Longest key ranges of all heads first (heads fastest): a long range that starts late is what the last round waits for
+  const int qt = gridDim.y - 1 - blockIdx.y;
+  const int head = blockIdx.x, bi = blockIdx.z, kvh = head / a.groups;
   const int skv = a.skv_dev ? (*a.skv_dev + a.sq) : a.skv;
   const int off = skv - a.sq;  // query i sees keys j <= i + off
   const int q0 = qt * XQ;
@@ -107,7 +109,7 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
     mbar_init(bar_o, 1);
     for (int i = 0; i < X_KBUFS; ++i) mbar_init(bar_kfull + 8 * i, 1);
     for (int i = 0; i < X_VBUFS; ++i) mbar_init(bar_vfull + 8 * i, 1);
-    mbar_init(bar_pfull, X_THREADS);
+    mbar_init(bar_pfull, X_THREADS / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -158,30 +160,32 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
       }
     }
   } else if (warp == X_THREADS / 32) {
-    // ---- MMA issuer: S_0, then per tile S_(t+1) (runs under the softmax of tile t) and O += P V_t
-    if (lane == 0 && ntiles > 0) {
+    // ---- MMA issuer: S_0, then per tile S_(t+1) (runs under the softmax of tile t) and O += P V_t. The whole warp runs the
+    // loop and one elected lane issues four MMAs at a time: issued by a lane of its own, one by one, they were what the
+    // softmax waited for (780 of 1900 cycles per tile)
+    if (ntiles > 0) {
+      const uint64_t qdesc = x_desc(pf_smem(Qs), 128, (XD / 8) * 128);
       auto issue_s = [&](int tile) {  // S buffer tile & 1 = Q . K_tile^T
-        x_wait(bar_kfull + 8 * (tile % X_KBUFS), (uint32_t)((tile / X_KBUFS) & 1), dead, a.status);
+        w_wait(bar_kfull + 8 * (tile % X_KBUFS), (uint32_t)((tile / X_KBUFS) & 1), dead, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ks = pf_smem(Ks + (tile % X_KBUFS) * X_KV_BYTES);
-#pragma unroll
-        for (int s = 0; s < XD / 16; ++s)  // k-step s: box s / 4, 32 bytes further inside the 128-byte rows per step
-          x_mma(tmem + (uint32_t)((tile & 1) * XK), x_desc(pf_smem(Qs) + s * 256, 128, (XD / 8) * 128),
-                x_desc(ks + (s >> 2) * X_BOX_BYTES + (s & 3) * 32, (uint32_t)a.k_lbo, 1024, X_SW128), IDESC_S, s ? 1u : 0u);
-        x_commit(bar_s + 8 * (tile & 1));
+        const uint64_t kdesc = x_desc(pf_smem(Ks + (tile % X_KBUFS) * X_KV_BYTES), (uint32_t)a.k_lbo, 1024, X_SW128);
+        const uint32_t d = tmem + (uint32_t)((tile & 1) * XK);
+        // a K step is 256 bytes of Q and, inside a 128-byte row of the box, 32 bytes of K
+        w_mma4<16, 2>(d, qdesc, kdesc, IDESC_S, 0u);
+        w_mma4<16, 2>(d, qdesc + 64, kdesc + (X_BOX_BYTES >> 4), IDESC_S, 1u);
+        w_commit(bar_s + 8 * (tile & 1));
       };
+      static_assert(XD == 128 && XK == 64, "eight K steps over two boxes, four K steps of 16 keys");
       issue_s(0);
       for (int tile = 0; tile < ntiles; ++tile) {
         if (tile + 1 < ntiles) issue_s(tile + 1);
-        x_wait(bar_pfull, (uint32_t)(tile & 1), dead, a.status);
-        x_wait(bar_vfull + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status);
+        w_wait(bar_vfull + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status);
+        w_wait(bar_pfull, (uint32_t)(tile & 1), dead, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t vs = pf_smem(Vs + (tile % X_VBUFS) * X_KV_BYTES);
-#pragma unroll
-        for (int s = 0; s < XK / 16; ++s)  // k-step s: 16 keys = 16 rows of 128 bytes further
-          x_mma_ta(tmem + 2 * XK, tmem + (uint32_t)((tile & 1) * XK + s * 8),
-                   x_desc(vs + s * 2048, (uint32_t)a.v_lbo, (uint32_t)a.v_sbo, X_SW128), IDESC_O, (tile | s) ? 1u : 0u);
-        x_commit(bar_o);
+        // a K step is 16 keys: 8 columns of P, 16 rows of 128 bytes of V
+        w_mma4_ta<8, 128>(tmem + 2 * XK, tmem + (uint32_t)((tile & 1) * XK),
+                          x_desc(pf_smem(Vs + (tile % X_VBUFS) * X_KV_BYTES), (uint32_t)a.v_lbo, (uint32_t)a.v_sbo, X_SW128), IDESC_O, tile ? 1u : 0u);
+        w_commit(bar_o);
       }
     }
   } else {
@@ -209,24 +213,32 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
           if (col >= skv || (a.causal && col > row + off)) sv[j >> 5][j & 31] = 0xFF800000u;  // -inf
         }
       }
-      float mx = -INFINITY;
+      // eight chains for the maximum and four for the sum: one after the other the 64 steps of either take longer than the
+      // exponentials
+      float m8[8];
 #pragma unroll
-      for (int j = 0; j < XK; ++j) mx = fmaxf(mx, __uint_as_float(sv[j >> 5][j & 31]));
+      for (int j = 0; j < 8; ++j) m8[j] = fmaxf(__uint_as_float(sv[0][j]), __uint_as_float(sv[0][8 + j]));
+#pragma unroll
+      for (int j = 16; j < XK; ++j) m8[j & 7] = fmaxf(m8[j & 7], __uint_as_float(sv[j >> 5][j & 31]));
+      const float mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7])));
       const float m_new = fmaxf(m_ref, mx * a.scale_log2);
       // follow the maximum lazily: rescale when it has outgrown the reference by more than 2^X_RESCALE
       const bool grow = m_new > m_ref + X_RESCALE;  // also true for the first finite maximum (m_ref = -inf)
       const float alpha = grow ? x_ex2(m_ref - m_new) : 1.0f;  // 2^-inf = 0 for a row that had no key yet
       if (grow) m_ref = m_new;
       const float msafe = m_ref == -INFINITY ? 0.f : m_ref;
-      float psum = 0.f;
+      const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), ref2 = make_float2(-msafe, -msafe);
+      float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t pk[XK / 2];  // P as fp16 pairs: column j of the A operand holds keys 2 j, 2 j + 1
 #pragma unroll
       for (int j = 0; j < XK / 2; ++j) {
-        const float p0 = x_ex2(fmaf(__uint_as_float(sv[(2 * j) >> 5][(2 * j) & 31]), a.scale_log2, -msafe));
-        const float p1 = x_ex2(fmaf(__uint_as_float(sv[(2 * j + 1) >> 5][(2 * j + 1) & 31]), a.scale_log2, -msafe));
-        psum += p0 + p1;
-        pk[j] = pf_pack(p0, p1);
+        float2 e = fma2(make_float2(__uint_as_float(sv[(2 * j) >> 5][(2 * j) & 31]), __uint_as_float(sv[(2 * j + 1) >> 5][(2 * j + 1) & 31])), scale2, ref2);
+        e.x = x_ex2(e.x);
+        e.y = x_ex2(e.y);
+        sum2[j & 1] = add2(sum2[j & 1], e);
+        pk[j] = pf_pack(e.x, e.y);
       }
+      const float psum = (sum2[0].x + sum2[1].x) + (sum2[0].y + sum2[1].y);
       l_run = l_run * alpha + psum;
       // P goes into the first half of the S buffer it came from (this thread's lane only; the next
       // product into that buffer, S_(t+2), is issued behind O += P V_t)
@@ -251,7 +263,8 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
       // before the last product can start, the one before it is seen complete: the final wait below then is for the
       // phase in progress (a parity wait must be neither two phases early nor two late)
       if (tile > 0 && tile == ntiles - 1) x_wait(bar_o, (uint32_t)((tile - 1) & 1), dead, a.status);
-      mbar_arrive(bar_pfull);  // phase t
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_pfull);  // phase t
     }
 
     // ---- the last product, then normalise and store (nothing is stored after a wait has given up)
@@ -324,7 +337,7 @@ int fb200_launch_attention_prefill_tc(fb200_device* dev, const float* q, const _
                                       int hkv, int sq, int skv, const int* skv_dev, int cap, int d, float scale,
                                       int causal, float* out, int bshd) {
   static const bool off = getenv("FB200_ATTN_TCGEN05") && getenv("FB200_ATTN_TCGEN05")[0] == '0';
-  if (off || d != XD || h % hkv || b > 65535 || h > 65535 || !(scale > 0.f) || skv <= 0 || skv > cap) return 1;
+  if (off || d != XD || h % hkv || b > 65535 || h > 65535 || (sq + XQ - 1) / XQ > 65535 || !(scale > 0.f) || skv <= 0 || skv > cap) return 1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(k) |
        reinterpret_cast<uintptr_t>(v)) & 15u)
     return 1;
@@ -338,7 +351,7 @@ int fb200_launch_attention_prefill_tc(fb200_device* dev, const float* q, const _
   a.v_lbo = X_BOX_BYTES;  // MN-major V: between the two 64-dim boxes
   a.v_sbo = 1024;         // ... and between groups of 8 keys
   a.status = dev->status;
-  const dim3 grid((unsigned)((sq + XQ - 1) / XQ), (unsigned)h, (unsigned)b);
+  const dim3 grid((unsigned)h, (unsigned)((sq + XQ - 1) / XQ), (unsigned)b);
   static bool configured[64] = {false};
   if (!configured[dev->ordinal & 63]) {
     FB_CUDA(dev, cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM));

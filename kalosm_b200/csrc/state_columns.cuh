@@ -29,6 +29,13 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
   return r;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
 
 // A column's d elements lie over LPC lanes, EPT per lane: element 4 (i LPC + p) + j is float j of piece i of lane p.
 template <int EPT, int LPC>

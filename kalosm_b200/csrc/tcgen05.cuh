@@ -74,6 +74,34 @@ __device__ __forceinline__ void w_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint6
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Four of them, issued by one elected lane: operands of the next K step lie STEP_A and STEP_B descriptor units (16 bytes) further.
+template <int STEP_A, int STEP_B>
+__device__ __forceinline__ void w_mma4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q, t;\n.reg .b64 a1, b1, a2, b2, a3, b3;\n"
+      "add.u64 a1, %1, %5;\nadd.u64 b1, %2, %6;\nadd.u64 a2, %1, %7;\nadd.u64 b2, %2, %8;\nadd.u64 a3, %1, %9;\nadd.u64 b3, %2, %10;\n"
+      "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 t, 0, 0;\nelect.sync _|q, 0xFFFFFFFF;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(STEP_A), "n"(STEP_B), "n"(2 * STEP_A), "n"(2 * STEP_B),
+        "n"(3 * STEP_A), "n"(3 * STEP_B) : "memory");
+}
+// The same with A in tensor memory, COLS_A columns per K step
+template <int COLS_A, int STEP_B>
+__device__ __forceinline__ void w_mma4_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q, t;\n.reg .b64 b1, b2, b3;\n.reg .b32 a1, a2, a3;\n"
+      "add.u32 a1, %1, %5;\nadd.u64 b1, %2, %6;\nadd.u32 a2, %1, %7;\nadd.u64 b2, %2, %8;\nadd.u32 a3, %1, %9;\nadd.u64 b3, %2, %10;\n"
+      "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 t, 0, 0;\nelect.sync _|q, 0xFFFFFFFF;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(COLS_A), "n"(STEP_B), "n"(2 * COLS_A), "n"(2 * STEP_B),
+        "n"(3 * COLS_A), "n"(3 * STEP_B) : "memory");
+}
 __device__ __forceinline__ void w_commit(uint32_t bar) {
   asm volatile(
       "{\n.reg .pred q;\nelect.sync _|q, 0xFFFFFFFF;\n"
