@@ -124,6 +124,7 @@ dense_pair_kernel(const DPairArgs a, const __grid_constant__ CUtensorMap wmap, c
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. of this CTA's 128 activation rows, one half of the columns
     const int quad = warp & 3, ch = warp >> 2;
     int n = 0;
+    pdl_wait();
     for (int item = pair; item < items; item += npairs, ++n) {
       const int buf = n & 1;
       if (!w_wait(acc_full + 8 * buf, (uint32_t)((n >> 1) & 1), dead, a.status)) break;
@@ -216,6 +217,7 @@ dense_pair_kernel(const DPairArgs a, const __grid_constant__ CUtensorMap wmap, c
   } else if (warp == DP_EPI_WARPS) {
     // ---- copy requester
     if (lane == 0) {
+      pdl_wait();
       int k = 0;
       bool alive = true;
       for (int item = pair; item < items && alive; item += npairs) {
@@ -294,7 +296,7 @@ int launch_pair(fb200_device* dev, const fb200_dense_job& j, DPairArgs a) {
     FB_CUDA(dev, cudaFuncSetAttribute(dense_pair_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM));
     configured[dev->ordinal & 63] = true;
   }
-  return fb200_launch(dev, dense_pair_kernel<NW>, dim3((unsigned)(2 * pairs)), dim3(DP_THREADS), (size_t)P::SMEM, false, a, wmap, xmap);
+  return fb200_launch(dev, dense_pair_kernel<NW>, dim3((unsigned)(2 * pairs)), dim3(DP_THREADS), (size_t)P::SMEM, true, a, wmap, xmap);
 }
 
 }  // namespace

@@ -453,6 +453,7 @@ pack_rows16_kernel(const float* __restrict__ x, int M, int K, __half* __restrict
   __shared__ float part[8];
   __shared__ float inv_s[PACK_ROWS];
   const int m0 = blockIdx.x * PACK_ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch_dependents();
   {
     const int row = warp % PACK_ROWS, half = warp / PACK_ROWS;  // 8 warps: two per row, half of K each
     const int m = m0 + row;
@@ -601,9 +602,9 @@ splitk_add_kernel(const float4* __restrict__ parts, int nsplit, size_t n4, int n
 
 // Launches the product of packed rows (xh, xscale: pack_rows16_kernel with 128-row tiles) on dev->stream.
 // With sh.split > 1 every K range writes its partial product into the handle's split-K scratch and a second kernel adds
-// them (+ residuals).
+// them (+ residuals). `early`: the packing kernel is the last work on the stream, and the product may start beside it.
 int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, const TcShape& sh, const __half* xh,
-              const float* xscale, size_t m, float* y, bool r1_is_bias, const float* r1, const float* r2, int swiglu) {
+              const float* xscale, size_t m, float* y, bool r1_is_bias, const float* r1, const float* r2, int swiglu, bool early) {
   const int halves = (int)((m + 127) / 128), split = sh.split;
   const size_t n_rows = swiglu ? w->n / 2 : w->n;
   int rc;
@@ -623,7 +624,7 @@ int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, co
       a.r1 = a.r2 = nullptr;
     }
     a.vec = n_rows % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.r1) | reinterpret_cast<uintptr_t>(a.r2)) & 7) == 0;
-    rc = fb200_qgemm_pair(dev, sh.nw, w->type, a);
+    rc = fb200_qgemm_pair(dev, sh.nw, w->type, a, early);
     if (rc || split == 1) return rc;
     const size_t n4 = m * w->n / 4;
     splitk_add_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, dev->stream>>>(
@@ -694,7 +695,7 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
   const __half* xh;
   const float* xscale;
   int rc = tc_pack(dev, x, m, w->k, &xh, &xscale);
-  return rc ? rc : tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu);
+  return rc ? rc : tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu, true);
 }
 
 // Up to three products of the same rows (the q, k and v projections of a prompt pass):
@@ -748,14 +749,14 @@ int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* 
     cudaStream_t st = dev->side_stream[side];
     FB_CUDA(dev, cudaStreamWaitEvent(st, dev->fork_ev, 0));
     dev->stream = st;  // the launch helpers take the handle's stream
-    rc = tc_launch(dev, ws[i], geo[i], best[i], xh, xscale, m, ys[i], false, nullptr, nullptr, 0);
+    rc = tc_launch(dev, ws[i], geo[i], best[i], xh, xscale, m, ys[i], false, nullptr, nullptr, 0, false);  // (its stream's last work is a wait for an event, not the packing kernel)
     dev->stream = main_stream;
     if (!rc) {
       FB_CUDA(dev, cudaEventRecord(dev->join_ev[side], st));
       ++side;
     }
   }
-  if (!rc) rc = tc_launch(dev, ws[first], geo[first], best[first], xh, xscale, m, ys[first], false, nullptr, nullptr, 0);
+  if (!rc) rc = tc_launch(dev, ws[first], geo[first], best[first], xh, xscale, m, ys[first], false, nullptr, nullptr, 0, false);
   // join whatever was forked, also after a failed launch: the stream must not run ahead of its side streams
   for (int j = 0; j < side; ++j) FB_CUDA(dev, cudaStreamWaitEvent(main_stream, dev->join_ev[j], 0));
   return rc;

@@ -270,6 +270,7 @@ qgemm_pair_kernel(const PairArgs a) {
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. of this CTA's 128 activation rows
     const int quad = warp & 3;
     int n = 0;
+    pdl_wait();
     for (int item = pair; item < items; item += npairs, ++n) {
       const int buf = n & 1;
       if (!w_wait(acc_full + 8 * buf, (uint32_t)((n >> 1) & 1), dead, a.status)) break;
@@ -370,8 +371,10 @@ qgemm_pair_kernel(const PairArgs a) {
       if (lane == 0) cluster_arrive(acc_free + 8 * buf, 0);
     }
   } else if (warp == PAIR_CONV_WARPS + PAIR_EPI_WARPS) {
-    // ---- activation loader: this CTA's 128 rows of the tile, one bulk copy per stage
+    // ---- activation loader: this CTA's 128 rows of the tile, one bulk copy per stage. Only this role and the epilogue wait for
+    // the packing kernel in front: the first stages' weights are loaded and converted beside it
     if (lane == 0) {
+      pdl_wait();
       int n = 0;
       bool alive = true;
       for (int item = pair; item < items && alive; item += npairs) {
@@ -433,7 +436,7 @@ qgemm_pair_kernel(const PairArgs a) {
 }
 
 template <int NW, int TYPE>
-int launch_pair(fb200_device* dev, const PairArgs& a) {
+int launch_pair(fb200_device* dev, const PairArgs& a, bool early) {
   using P = Pair<NW>;
   static bool configured[64] = {false};
   if (!configured[dev->ordinal & 63]) {
@@ -441,18 +444,18 @@ int launch_pair(fb200_device* dev, const PairArgs& a) {
     configured[dev->ordinal & 63] = true;
   }
   const int items = a.m_tiles * a.n_tiles * a.splits, pairs = std::min(items, dev->sm_count / 2);
-  return fb200_launch(dev, qgemm_pair_kernel<NW, TYPE>, dim3((unsigned)(2 * pairs)), dim3(PAIR_THREADS), (size_t)P::SMEM, false, a);
+  return fb200_launch(dev, qgemm_pair_kernel<NW, TYPE>, dim3((unsigned)(2 * pairs)), dim3(PAIR_THREADS), (size_t)P::SMEM, early, a);
 }
 
 }  // namespace
 
-int fb200_qgemm_pair(fb200_device* dev, int nw, uint32_t type, const PairArgs& a) {
+int fb200_qgemm_pair(fb200_device* dev, int nw, uint32_t type, const PairArgs& a, bool early) {
   const bool wide = nw == 256;
   switch (type) {
-    case FB200_Q4_0: return wide ? launch_pair<256, FB200_Q4_0>(dev, a) : launch_pair<128, FB200_Q4_0>(dev, a);
-    case FB200_Q8_0: return wide ? launch_pair<256, FB200_Q8_0>(dev, a) : launch_pair<128, FB200_Q8_0>(dev, a);
-    case FB200_Q4_K: return wide ? launch_pair<256, FB200_Q4_K>(dev, a) : launch_pair<128, FB200_Q4_K>(dev, a);
-    case FB200_Q6_K: return wide ? launch_pair<256, FB200_Q6_K>(dev, a) : launch_pair<128, FB200_Q6_K>(dev, a);
+    case FB200_Q4_0: return wide ? launch_pair<256, FB200_Q4_0>(dev, a, early) : launch_pair<128, FB200_Q4_0>(dev, a, early);
+    case FB200_Q8_0: return wide ? launch_pair<256, FB200_Q8_0>(dev, a, early) : launch_pair<128, FB200_Q8_0>(dev, a, early);
+    case FB200_Q4_K: return wide ? launch_pair<256, FB200_Q4_K>(dev, a, early) : launch_pair<128, FB200_Q4_K>(dev, a, early);
+    case FB200_Q6_K: return wide ? launch_pair<256, FB200_Q6_K>(dev, a, early) : launch_pair<128, FB200_Q6_K>(dev, a, early);
   }
   return 1;
 }

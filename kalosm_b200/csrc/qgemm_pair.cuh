@@ -21,5 +21,6 @@ struct PairArgs {
   int* status;
 };
 
-// Launches the product with nw = 128 or 256 weight rows per tile; 1 when the type has no kernel.
-int fb200_qgemm_pair(fb200_device* dev, int nw, uint32_t type, const PairArgs& a);
+// Launches the product with nw = 128 or 256 weight rows per tile; 1 when the type has no kernel. `early`: it may start while the
+// kernel in front on the stream (which packs its activations) still runs.
+int fb200_qgemm_pair(fb200_device* dev, int nw, uint32_t type, const PairArgs& a, bool early);
