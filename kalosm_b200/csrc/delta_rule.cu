@@ -6,17 +6,17 @@
 // what a group of lanes owns for the whole sequence: it stays in registers, k and q come from shared memory.
 // Both sums over d are formed in one pass from the state BEFORE the token,
 //   S^T k -> g (S^T k),   o = g (S^T q) + u (k . q),
-// and in a prompt four tokens share a pass: with a_i = S^T k_i, c_i = S^T q_i from the state before the four,
+// and in a prompt eight tokens share a pass: with a_i = S^T k_i, c_i = S^T q_i from the state before the eight,
 // G_i = g_0 .. g_i and w_j = (g_(j+1) .. g_i) u_j,
 //   u_i = beta_i (v_i - G_i a_i - sum_(j<i) (k_j . k_i) w_j),   o_i = G_i c_i + sum_(j<=i) (k_j . q_i) w_j,
-//   S <- G_3 S + sum_j k_j w_j,
-// the same recurrence with one reduction over the lanes per four tokens. Everything is f32.
+//   S <- G_7 S + sum_j k_j w_j,
+// the same recurrence with one reduction over the lanes per eight tokens. Everything is f32.
 //
 //  * delta_step_kernel: one new token per sequence. One CTA per (head, sequence): convolution, unit vectors,
 //    decay, state update, read-out, RMSNorm and gate. Bound: HBM on the state (read and written once).
-//  * prompts: delta_prep_kernel (convolution, SiLU, unit vectors, products of the four tokens' k and q, decay and
-//    write strength), delta_scan_kernel (the recurrence; bound: f32 FMA issue, packed two-wide), delta_out_kernel (RMSNorm, gate) and
-//    conv_ring_kernel (the convolution's memory).
+//  * prompts: delta_prep_kernel (convolution, SiLU, unit vectors, decay and write strength), delta_pairs_kernel (products of
+//    eight tokens' k and q), delta_scan_kernel (the recurrence; bound: latency of the pass, a warp per scheduler), delta_out_kernel
+//    (RMSNorm, gate) and conv_ring_kernel (the convolution's memory).
 #include "mixers.cuh"
 #include "qgemv_common.cuh"
 #include "state_columns.cuh"
@@ -196,38 +196,35 @@ __global__ void __launch_bounds__(ST_MAX_THREADS) delta_step_kernel(const fb200_
 }
 
 // ---- prompts ---------------------------------------------------------------------------------------------
-constexpr int CH = 4;  // tokens per pass of the recurrence
+// Tokens per pass of the recurrence: 8192 tokens of 16 heads of 128 take 1.22 ms, 1.36 with four (heads of 64, 256 and 512 gain alike)
+constexpr int CH = 8;
+constexpr int PREP_TOK = 4;  // tokens per warp of the preparation
 constexpr int PREP_WARPS = 4, PREP_VCH = 128;
-constexpr int PAIRS = 16;  // k_j . k_i (j < i): 6 values, then k_j . q_i (j <= i): 10 values, i-major
-// (j, i) of pair p, two bits each
-constexpr uint32_t PAIR_J = 0u | 0u << 2 | 1u << 4 | 0u << 6 | 1u << 8 | 2u << 10 | 0u << 12 | 0u << 14 | 1u << 16 | 0u << 18 | 1u << 20 |
-                            2u << 22 | 0u << 24 | 1u << 26 | 2u << 28 | 3u << 30;
-constexpr uint32_t PAIR_I = 1u | 2u << 2 | 2u << 4 | 3u << 6 | 3u << 8 | 3u << 10 | 0u << 12 | 1u << 14 | 1u << 16 | 2u << 18 | 2u << 20 |
-                            2u << 22 | 3u << 24 | 3u << 26 | 3u << 28 | 3u << 30;
+constexpr int KK = CH * (CH - 1) / 2, PAIRS = CH * CH;  // k_j . k_i (j < i), then k_j . q_i (j <= i), i-major
 
-// convolution + SiLU of channel c for the CH tokens from t0 (zeros from token s on); inputs before this pass come
+// convolution + SiLU of channel c for the PREP_TOK tokens from t0 (zeros from token s on); inputs before this pass come
 // from the ring. Addresses are selected, not branched on, so that a channel's loads go out together.
-__device__ __forceinline__ void conv_chunk(const fb200_delta_args& a, int b, int c, int t0, int pos, float (&out)[CH]) {
+__device__ __forceinline__ void conv_chunk(const fb200_delta_args& a, int b, int c, int t0, int pos, float (&out)[PREP_TOK]) {
 #pragma unroll
-  for (int i = 0; i < CH; ++i) out[i] = 0.f;
+  for (int i = 0; i < PREP_TOK; ++i) out[i] = 0.f;
   for (int j0 = 0; j0 < a.taps; j0 += 4) {  // four taps at a time meet seven inputs
-    float w[4], x[CH + 3];
+    float w[4], x[PREP_TOK + 3];
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = j0 + j < a.taps ? a.conv_w[(size_t)(j0 + j) * a.channels + c] : 0.f;
 #pragma unroll
-    for (int r = 0; r < CH + 3; ++r) {
+    for (int r = 0; r < PREP_TOK + 3; ++r) {
       const int t = t0 - (a.taps - 1) + j0 + r, p = pos + t;
-      const bool valid = j0 + r < a.taps + CH - 1 && t < a.s && p >= 0;
+      const bool valid = j0 + r < a.taps + PREP_TOK - 1 && t < a.s && p >= 0;
       const float* src = t >= 0 ? a.y + ((size_t)b * a.s + t) * a.ldy + c : a.ring + ((size_t)b * a.taps + (valid ? p % a.taps : 0)) * a.channels + c;
       x[r] = valid ? *src : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int i = 0; i < CH; ++i) out[i] = fmaf(w[j], x[i + j], out[i]);
+      for (int i = 0; i < PREP_TOK; ++i) out[i] = fmaf(w[j], x[i + j], out[i]);
   }
 #pragma unroll
-  for (int i = 0; i < CH; ++i) out[i] = t0 + i < a.s ? dr_silu(out[i]) : 0.f;
+  for (int i = 0; i < PREP_TOK; ++i) out[i] = t0 + i < a.s ? dr_silu(out[i]) : 0.f;
 }
 
 // Sums v[0..31] over the lanes of a warp; lane l returns the total of v[l].
@@ -245,46 +242,37 @@ __device__ __forceinline__ float warp_sum32(float (&v)[32]) {
   return v[0];
 }
 
-// A warp per (unit, CH tokens): units 0 .. hk are the q and k vectors of a q/k head, then blocks of 128 v channels, then
+// A warp per (unit, PREP_TOK tokens): units 0 .. hk are the q and k vectors of a q/k head, then blocks of 128 v channels, then
 // the decays and write strengths of all heads. NE = channels of a q/k head per lane.
 template <int NE>
 __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200_delta_args a) {
-  const int lane = threadIdx.x & 31, b = blockIdx.z, t0 = blockIdx.x * CH, n = min(CH, a.s - t0);
+  const int lane = threadIdx.x & 31, b = blockIdx.z, t0 = blockIdx.x * PREP_TOK, n = min(PREP_TOK, a.s - t0);
   const int hv = a.h * a.v, vblocks = (hv + PREP_VCH - 1) / PREP_VCH;
   int unit = blockIdx.y * PREP_WARPS + (threadIdx.x >> 5);
   const int pos = *a.pos_dev;
   if (unit < a.hk) {
-    float q[NE][CH], k[NE][CH], sum[32];
+    float q[NE][PREP_TOK], k[NE][PREP_TOK], sum[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) sum[i] = 0.f;
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
       const int c = lane + 32 * e;
 #pragma unroll
-      for (int i = 0; i < CH; ++i) q[e][i] = k[e][i] = 0.f;
+      for (int i = 0; i < PREP_TOK; ++i) q[e][i] = k[e][i] = 0.f;
       if (c < a.d) {
         conv_chunk(a, b, unit * a.d + c, t0, pos, q[e]);
         conv_chunk(a, b, (a.hk + unit) * a.d + c, t0, pos, k[e]);
       }
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
+      for (int i = 0; i < PREP_TOK; ++i) {
         sum[i] = fmaf(k[e][i], k[e][i], sum[i]);
         sum[4 + i] = fmaf(q[e][i], q[e][i], sum[4 + i]);
-      }
-#pragma unroll
-      for (int p = 0; p < PAIRS; ++p) {
-        const int j = (PAIR_J >> (2 * p)) & 3, i = (PAIR_I >> (2 * p)) & 3;
-        sum[8 + p] = fmaf(k[e][j], p < 6 ? k[e][i] : q[e][i], sum[8 + p]);
       }
     }
     const float total = warp_sum32(sum);
     const float inv = (1.0f / sqrtf(total + UNIT_EPS)) * (lane >= 4 ? 1.0f / sqrtf((float)a.d) : 1.0f);  // lanes 0..3: k, 4..7: q
-    const int p = lane - 8;
-    const float sj = __shfl_sync(0xFFFFFFFFu, inv, (PAIR_J >> (2 * (p & 15))) & 3);
-    const float si = __shfl_sync(0xFFFFFFFFu, inv, ((PAIR_I >> (2 * (p & 15))) & 3) + (p < 6 ? 0 : 4));
-    if (p >= 0 && p < PAIRS) a.kq[(((size_t)b * gridDim.x + blockIdx.x) * a.hk + unit) * PAIRS + p] = total * sj * si;
 #pragma unroll
-    for (int i = 0; i < CH; ++i) {
+    for (int i = 0; i < PREP_TOK; ++i) {
       const float ik = __shfl_sync(0xFFFFFFFFu, inv, i), iq = __shfl_sync(0xFFFFFFFFu, inv, 4 + i);
       if (i >= n) continue;
       const size_t row = ((size_t)b * a.s + t0 + i) * a.hk + unit;
@@ -301,7 +289,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200
   }
   unit -= a.hk;
   if (unit < vblocks) {
-    float v[PREP_VCH / 32][CH];
+    float v[PREP_VCH / 32][PREP_TOK];
 #pragma unroll
     for (int e = 0; e < PREP_VCH / 32; ++e) {
       const int c = unit * PREP_VCH + lane + 32 * e;
@@ -311,7 +299,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200
     for (int e = 0; e < PREP_VCH / 32; ++e) {
       const int c = unit * PREP_VCH + lane + 32 * e;
 #pragma unroll
-      for (int i = 0; i < CH; ++i)
+      for (int i = 0; i < PREP_TOK; ++i)
         if (c < hv && i < n) a.vn[((size_t)b * a.s + t0 + i) * hv + c] = v[e][i];
     }
     return;
@@ -326,17 +314,51 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200
   }
 }
 
+// A warp per (CH tokens, q/k head): k_j . k_i (j < i) and k_j . q_i (j <= i) of the unit vectors; tokens behind the last are zero.
+__global__ void __launch_bounds__(PREP_WARPS * 32) delta_pairs_kernel(const fb200_delta_args a) {
+  const int lane = threadIdx.x & 31, b = blockIdx.z, t0 = blockIdx.x * CH, hk = blockIdx.y * PREP_WARPS + (threadIdx.x >> 5);
+  if (hk >= a.hk) return;
+  float sum[2][32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) sum[0][i] = sum[1][i] = 0.f;
+  for (int c = 4 * lane; c < a.dp; c += 128) {
+    float4 k[CH], q[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const size_t at = (((size_t)b * a.s + min(t0 + i, a.s - 1)) * a.hk + hk) * a.dp + c;
+      const bool in = t0 + i < a.s;
+      k[i] = in ? *reinterpret_cast<const float4*>(a.kn + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      q[i] = in ? *reinterpret_cast<const float4*>(a.qn + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    auto dot = [](float4 x, float4 y, float acc) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, acc)))); };
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        const int kq = KK + i * (i + 1) / 2 + j;
+        sum[kq >> 5][kq & 31] = dot(k[j], q[i], sum[kq >> 5][kq & 31]);
+        if (j < i) {
+          const int kk = i * (i - 1) / 2 + j;
+          sum[kk >> 5][kk & 31] = dot(k[j], k[i], sum[kk >> 5][kk & 31]);
+        }
+      }
+  }
+  float* out = a.kq + (((size_t)b * gridDim.x + blockIdx.x) * a.hk + hk) * PAIRS;
+  out[lane] = warp_sum32(sum[0]);
+  out[32 + lane] = warp_sum32(sum[1]);
+}
+
 constexpr int SC_WARPS = 4, CPT = 4;  // columns per group of lanes
 
 // A group of LPC lanes owns CPT columns of S: k and q read from shared memory serve all of them, and the sums are
-// reduced so that lane p ends up with those of column p % 4, so one pass over the four tokens does all columns.
+// reduced so that lane p ends up with those of column p % 4, so one pass over the eight tokens does all columns.
 // TOK tokens make a shared-memory stage (a multiple of CH).
 template <int EPT, int LPC, int TOK>
 __global__ void __launch_bounds__(SC_WARPS * 32) delta_scan_kernel(const fb200_delta_args a) {
   constexpr int DP = EPT * LPC, GROUPS = SC_WARPS * 32 / LPC, COLS = GROUPS * CPT, THREADS = SC_WARPS * 32, NC = TOK / CH;
   // floats of a stage: k, q [TOK][DP], v [COLS][TOK], pairs [NC][PAIRS], g [TOK], beta [TOK]
   constexpr int OV = 2 * TOK * DP, OP = OV + COLS * TOK, OG = OP + NC * PAIRS, STAGE = OG + 2 * TOK;
-  constexpr bool KEEP = EPT <= 16;  // k of the four tokens stays in registers for the update
+  constexpr bool KEEP = EPT <= 8;  // k of the eight tokens stays in registers for the update
   extern __shared__ __align__(16) float dsm[];
   const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, b = blockIdx.z, group = a.h / a.hk, hk = h / group, hv = a.h * a.v;
   const int p = tid % LPC, cl = tid / LPC, c = blockIdx.x * COLS + cl;  // columns c, c + GROUPS, ..
@@ -444,40 +466,49 @@ __global__ void __launch_bounds__(SC_WARPS * 32) delta_scan_kernel(const fb200_d
         for (int o = 4; o < LPC; o <<= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
         val[0][x] = t;
       }
-      // ---- the four tokens in order
-      float pr[PAIRS];
-#pragma unroll
-      for (int i = 0; i < PAIRS / 4; ++i) {
-        const float4 x = *reinterpret_cast<const float4*>(sb + OP + ch * PAIRS + 4 * i);
-        pr[4 * i] = x.x; pr[4 * i + 1] = x.y; pr[4 * i + 2] = x.z; pr[4 * i + 3] = x.w;
-      }
-      const float4 g4 = *reinterpret_cast<const float4*>(sb + OG + ch * CH), b4 = *reinterpret_cast<const float4*>(sb + OG + TOK + ch * CH);
-      const float gi[CH] = {g4.x, g4.y, g4.z, g4.w}, bi[CH] = {b4.x, b4.y, b4.z, b4.w};
-      const float2 G2 = make_float2(((g4.x * g4.y) * g4.z) * g4.w, ((g4.x * g4.y) * g4.z) * g4.w);
+      // ---- the eight tokens in order
       const int mycol = cl + (p & 3) * GROUPS;
-      const float4 v4 = *reinterpret_cast<const float4*>(sb + OV + mycol * TOK + ch * CH);
-      const float vi[CH] = {v4.x, v4.y, v4.z, v4.w};
+      float gi[CH], bi[CH], vi[CH];
+#pragma unroll
+      for (int i = 0; i < CH; i += 4) {
+        const float4 g4 = *reinterpret_cast<const float4*>(sb + OG + ch * CH + i), b4 = *reinterpret_cast<const float4*>(sb + OG + TOK + ch * CH + i);
+        const float4 v4 = *reinterpret_cast<const float4*>(sb + OV + mycol * TOK + ch * CH + i);
+        gi[i] = g4.x; gi[i + 1] = g4.y; gi[i + 2] = g4.z; gi[i + 3] = g4.w;
+        bi[i] = b4.x; bi[i + 1] = b4.y; bi[i + 2] = b4.z; bi[i + 3] = b4.w;
+        vi[i] = v4.x; vi[i + 1] = v4.y; vi[i + 2] = v4.z; vi[i + 3] = v4.w;
+      }
+      const float* pr = sb + OP + ch * PAIRS;
       float u[CH], out[CH], G = 1.f;
-      int pk = 0, pq = 6;
 #pragma unroll
       for (int i = 0; i < CH; ++i) {
         G *= gi[i];
-        float uk = G * val[0][i], o = G * val[0][CH + i];
+        float uk[2] = {G * val[0][i], 0.f}, o[2] = {G * val[0][CH + i], 0.f};  // two chains each
 #pragma unroll
-        for (int j = 0; j < CH; ++j)
-          if (j < i) {
-            u[j] *= gi[i];
-            uk = fmaf(pr[pk++], u[j], uk);
-            o = fmaf(pr[pq++], u[j], o);
-          }
-        u[i] = bi[i] * (vi[i] - uk);
-        out[i] = fmaf(pr[pq++], u[i], o);
+        for (int j = 0; j < i; ++j) {
+          u[j] *= gi[i];
+          uk[j & 1] = fmaf(pr[i * (i - 1) / 2 + j], u[j], uk[j & 1]);
+          o[j & 1] = fmaf(pr[KK + i * (i + 1) / 2 + j], u[j], o[j & 1]);
+        }
+        u[i] = bi[i] * (vi[i] - (uk[0] + uk[1]));
+        out[i] = fmaf(pr[KK + i * (i + 1) / 2 + i], u[i], o[0] + o[1]);
       }
-      if (p < 8 && blockIdx.x * COLS + mycol < a.v) {  // lanes 0..3 store tokens 0 and 1, lanes 4..7 tokens 2 and 3
-        const int i0 = p < 4 ? 0 : 2;
-        float* dst = a.o + (row0 + t0 + i0) * hv + h * a.v + blockIdx.x * COLS + mycol;
-        if (t0 + i0 < a.s) dst[0] = p < 4 ? out[0] : out[2];
-        if (t0 + i0 + 1 < a.s) dst[hv] = p < 4 ? out[1] : out[3];
+      const float2 G2 = make_float2(G, G);
+      // every four lanes (one per column) store some of the tokens
+      constexpr int QUADS = LPC / 4 < CH ? LPC / 4 : CH, EACH = CH / QUADS;
+      if (blockIdx.x * COLS + mycol < a.v) {
+        const int quad = p >> 2;
+        float* dst = a.o + (row0 + t0 + quad * EACH) * hv + h * a.v + blockIdx.x * COLS + mycol;
+#pragma unroll
+        for (int e = 0; e < EACH; ++e) {
+          float pick[QUADS];  // token quad * EACH + e, by selects (an index would put the array into local memory)
+#pragma unroll
+          for (int i = 0; i < QUADS; ++i) pick[i] = out[i * EACH + e];
+#pragma unroll
+          for (int o = QUADS / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < o; ++i) pick[i] = quad & o ? pick[i + o] : pick[i];
+          if (quad < QUADS && t0 + quad * EACH + e < a.s) dst[(size_t)e * hv] = pick[0];
+        }
       }
       float w[CPT][CH];
 #pragma unroll
@@ -573,8 +604,11 @@ int launch_scan(fb200_device* dev, const fb200_delta_args& a) {
 template <int NE>
 int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
   const int units = a.hk + (a.h * a.v + PREP_VCH - 1) / PREP_VCH + 1;
-  delta_prep_kernel<NE><<<dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
+  delta_prep_kernel<NE><<<dim3((unsigned)((a.s + PREP_TOK - 1) / PREP_TOK), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
                           PREP_WARPS * 32, 0, dev->stream>>>(a);
+  FB_LAUNCH_CHECK(dev);
+  delta_pairs_kernel<<<dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b), PREP_WARPS * 32, 0,
+                       dev->stream>>>(a);
   FB_LAUNCH_CHECK(dev);
   return FB200_OK;
 }

@@ -530,7 +530,7 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
       {(void**)&m->x, rows * hy->ldx * 4}, {(void**)&hy->x2, hy->w_loop ? rows * hy->ldx * 4 : 0}, {(void**)&m->xn, (norm2 ? 2 : 1) * rows * E * 4},
       {(void**)&hy->proj, rows * hy->ldy * 4}, {(void**)&hy->zf, rows * hy->ldz * 4}, {(void**)&hy->hb, rows * hb * 2},
       {(void**)&hy->zb, rows * hy->ldz * 2}, {(void**)&hy->qn, rows * q * 4}, {(void**)&hy->kn, rows * qk * 4}, {(void**)&hy->vn, rows * hv * 4},
-      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 3 * nb) / 4 * kvh * 64 + 64}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
+      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 7 * nb) / 8 * kvh * 256 + 64}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
       {(void**)&hy->qa, qa * 4}, {(void**)&hy->part, part * 4}, {(void**)&hy->done, (done + nb) * 4}};
   for (auto& b : bufs) {
     if (*b.p) { cudaFree(*b.p); *b.p = nullptr; }
