@@ -5,6 +5,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "qgemm_pair.cuh"
 #include "common.cuh"
 
 size_t fb200_xpack_bytes(int mp, uint64_t kp);
@@ -14,8 +15,6 @@ int fb200_q5_mat_mul(fb200_device* dev, const fb200_qmatrix* w, const float* x, 
 int fb200_qgemv_chunk(fb200_device* dev, const fb200_qmatrix* w, const float* x, int mc, float* y,
                       int epi, const float* r1, const float* r2, void* scratch, bool r1_is_bias);
 int fb200_dense_matmul(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_t m, float* y);
-int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_t m, float* y, bool r1_is_bias,
-                const float* r1, const float* r2, int swiglu);
 bool fb200_qgemv1_fits(const fb200_qmatrix* w);
 int fb200_qgemv1(fb200_device* dev, const fb200_qmatrix* w, const float* x, const float* xres,
                  const float* norm_w, float eps, float* y, int epi, const float* r1, const float* r2);

@@ -12,6 +12,7 @@
 #include <cstring>
 #include <memory>
 
+#include "qgemm_pair.cuh"
 #include "decoder.cuh"
 
 void fb200_rope_tables_host(int head_dim, int ctx, float theta, float factor, float low_ff,
@@ -28,7 +29,6 @@ int fb200_launch_attention(fb200_device* dev, const float* q, const __half* k, c
                            float* part, int nsplit, int bshd);
 size_t fb200_xpack_bytes(int mp, uint64_t kp);
 int fb200_pack16_rows(int mc);
-int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* const* ys, int n, const float* x, size_t m);
 uint64_t fb200_qmatrix_kp(const fb200_qmatrix* w);
 int fb200_pack_x16(fb200_device* dev, const float* x, int mc, uint64_t k, uint64_t kp, void* scratch, const void** xh,
                    const float** xscale);
@@ -513,12 +513,14 @@ int run_forward(fb200_llama* m, int batch, int seq, bool commit = true) {
       }
       if (rc) return rc;
     } else {
-      if ((rc = fb200_launch_rms_norm_strided(dev, m->x, E, nullptr, L.attn_norm, c.rms_eps, rows, E, m->xn))) return rc;
-      // a prompt pass: the three projections side by side (each alone fills a fraction of the SMs)
+      // a prompt pass: the three projections side by side (each alone fills a fraction of the SMs), their rows normalised as
+      // they are packed
       const fb200_qmatrix* qkv_w[3] = {L.wq, L.wk, L.wv};
       float* qkv_y[3] = {m->q, m->k, m->v};
-      rc = rows > 32 ? fb200_qgemm_group(dev, qkv_w, qkv_y, 3, m->xn, rows) : 1;
+      const fb200_row_norm norm{nullptr, L.attn_norm, c.rms_eps};
+      rc = rows > 32 ? fb200_qgemm_group(dev, qkv_w, qkv_y, 3, m->x, rows, &norm) : 1;
       if (rc == 1) {
+        if ((rc = fb200_launch_rms_norm_strided(dev, m->x, E, nullptr, L.attn_norm, c.rms_eps, rows, E, m->xn))) return rc;
         if ((rc = fb200_q_mat_mul(dev, m->xn, rows, L.wq, m->q, nullptr))) return rc;
         if ((rc = fb200_q_mat_mul(dev, m->xn, rows, L.wk, m->k, nullptr))) return rc;
         if ((rc = fb200_q_mat_mul(dev, m->xn, rows, L.wv, m->v, nullptr))) return rc;
@@ -571,9 +573,18 @@ int run_forward(fb200_llama* m, int batch, int seq, bool commit = true) {
       if ((rc = fb200_norm_pack_x16(dev, m->attn_out, E, m->x, L.ffn_norm, c.rms_eps, (int)rows, E, kp_e, dev->xpack, &xh, &xs))) return rc;
       if ((rc = fb200_qgemm16_packed(dev, L.gate_up, xh, xs, (int)rows, mp, m->hbuf, FB200_EPI_SWIGLU, nullptr, nullptr, false))) return rc;
     } else if (L.gate_up) {
-      if ((rc = fb200_launch_rms_norm_strided(dev, m->attn_out, E, m->x, L.ffn_norm, c.rms_eps, rows, E, m->xn))) return rc;
-      fb200_epilogue ep{FB200_EPI_SWIGLU, nullptr, nullptr};
-      if ((rc = fb200_q_mat_mul(dev, m->xn, rows, L.gate_up, m->hbuf, &ep))) return rc;
+      const fb200_row_norm norm{m->x, L.ffn_norm, c.rms_eps};
+      rc = 1;
+      if (rows > 32 && L.gate_up->n % 32 == 0) {
+        fb200_op_trace scope(dev, "q_mat_mul (> 32 rows)", (double)L.gate_up->raw_nbytes + 4.0 * (double)rows * (double)(E + L.gate_up->n));
+        rc = fb200_qgemm(dev, L.gate_up, m->attn_out, rows, m->hbuf, false, nullptr, nullptr, 1, &norm);
+      }
+      if (rc == 1) {
+        if ((rc = fb200_launch_rms_norm_strided(dev, m->attn_out, E, m->x, L.ffn_norm, c.rms_eps, rows, E, m->xn))) return rc;
+        fb200_epilogue ep{FB200_EPI_SWIGLU, nullptr, nullptr};
+        rc = fb200_q_mat_mul(dev, m->xn, rows, L.gate_up, m->hbuf, &ep);
+      }
+      if (rc) return rc;
     } else {
       if ((rc = fb200_launch_rms_norm_strided(dev, m->attn_out, E, m->x, L.ffn_norm, c.rms_eps, rows, E, m->xn))) return rc;
       if ((rc = fb200_q_mat_mul(dev, m->xn, rows, L.gate, m->gbuf, nullptr))) return rc;

@@ -445,58 +445,112 @@ qgemm_tc_kernel(const TcArgs a) {
 // x[M, K] f32 -> fp16 scaled by a power of two per row into (-64, 64), stored as [Mp / 128][K / 64]
 // tiles of 128 rows x 64 values in the operand layout of the MMA (8 rows x 16 bytes per core
 // matrix, core matrices adjacent in K 128 bytes apart, 8-row groups 1024 bytes apart), so that a
-// tile is one contiguous bulk copy. One CTA per PACK_ROWS rows (512 rows give 128 CTAs); two warps
-// find the maximum of a row with independent 16-byte loads; rows >= M are zero.
-constexpr int PACK_ROWS = 4;
-__global__ void __launch_bounds__(256)
-pack_rows16_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, float* __restrict__ xscale) {
-  __shared__ float part[8];
-  __shared__ float inv_s[PACK_ROWS];
-  const int m0 = blockIdx.x * PACK_ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// tile is one contiguous bulk copy; rows >= M are zero. With NORM the rows are (x + res) / rms * w (RMSNorm; res may be null).
+// Bound: latency of one read of the rows. A CTA takes two rows and every thread all its values at once into registers (up to
+// PACK_CHUNKS x 8; the rest is read again), so that the maximum, or sum of squares and maximum, cost no second pass; adjacent
+// threads take the same place of the two rows and write one sector.
+constexpr int PACK_ROWS = 2, PACK_THREADS = 512, PACK_CHUNKS = 7, PACK_STEP = PACK_THREADS / PACK_ROWS;
+template <bool NORM>
+__global__ void __launch_bounds__(PACK_THREADS)
+pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, const float* __restrict__ w, float eps, int M, int K,
+                   __half* __restrict__ xh, float* __restrict__ xscale) {
+  __shared__ float part[2][PACK_THREADS / 32][PACK_ROWS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid & 1, c0 = tid >> 1;
+  const int m0 = blockIdx.x * PACK_ROWS, m = m0 + r, chunks = K / 8;
   pdl_launch_dependents();
-  {
-    const int row = warp % PACK_ROWS, half = warp / PACK_ROWS;  // 8 warps: two per row, half of K each
-    const int m = m0 + row;
-    float amax = 0.f;
-    if (m < M) {
-      const float4* xr = reinterpret_cast<const float4*>(x + (size_t)m * K) + (size_t)half * (K / 8);
-      const int n4 = K / 8;  // float4 per half row (K is a multiple of 64)
-#pragma unroll 8
-      for (int i = lane; i < n4; i += 32) {
-        const float4 v = __ldg(xr + i);
-        amax = fmaxf(fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+  const bool in = m < M;
+  const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(in ? m : 0) * K);
+  const float4* rr = NORM && res ? reinterpret_cast<const float4*>(res + (size_t)(in ? m : 0) * K) : nullptr;
+  auto load = [&](int c, float4 (&v)[2]) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      v[e] = in && c < chunks ? __ldg(xr + 2 * c + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (NORM && rr && in && c < chunks) {
+        const float4 q = __ldg(rr + 2 * c + e);
+        v[e] = make_float4(v[e].x + q.x, v[e].y + q.y, v[e].z + q.z, v[e].w + q.w);
       }
     }
+  };
+  // over the threads of the own row: 16 lanes of every warp
+  auto block = [&](float v, int slot, bool sum) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    if (lane == 0) part[warp] = amax;
-  }
-  __syncthreads();
-  if (threadIdx.x < PACK_ROWS) {
-    const float amax = fmaxf(part[threadIdx.x], part[threadIdx.x + PACK_ROWS]);
-    int ex = 0;
-    if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);
-    inv_s[threadIdx.x] = ldexpf(64.0f, -ex);
-    xscale[m0 + threadIdx.x] = ldexpf(1.0f, ex - 6);
-  }
-  __syncthreads();
-  constexpr int bm = SINGLE_BM;
-  const int nkb = K / BK;
-  uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / bm) * nkb * ((size_t)bm * BK * 2) +
-                      ((m0 % bm) >> 3) * CORE_SBO + (m0 & 7) * 16;
-  for (int q = threadIdx.x; q < K / 8 * PACK_ROWS; q += 256) {  // K / 8 chunks of 8 values x PACK_ROWS rows
-    const int r = q % PACK_ROWS, kc = q / PACK_ROWS, m = m0 + r;
-    uint4 out = make_uint4(0u, 0u, 0u, 0u);
-    if (m < M) {
-      const float4* src = reinterpret_cast<const float4*>(x + (size_t)m * K + 8 * kc);
-      const float4 lo = __ldg(src), hi = __ldg(src + 1);
-      const float inv = inv_s[r];
-      out.x = h2u(__floats2half2_rn(lo.x * inv, lo.y * inv));
-      out.y = h2u(__floats2half2_rn(lo.z * inv, lo.w * inv));
-      out.z = h2u(__floats2half2_rn(hi.x * inv, hi.y * inv));
-      out.w = h2u(__floats2half2_rn(hi.z * inv, hi.w * inv));
+    for (int o = 16; o > 1; o >>= 1) {
+      const float other = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+      v = sum ? v + other : fmaxf(v, other);
     }
-    *reinterpret_cast<uint4*>(tile_row + (size_t)(kc >> 3) * ((size_t)bm * BK * 2) + (kc & 7) * CORE_LBO + r * 16) = out;
+    if (lane < PACK_ROWS) part[slot][warp][lane] = v;
+    __syncthreads();
+    v = part[slot][0][r];
+#pragma unroll
+    for (int i = 1; i < PACK_THREADS / 32; ++i) v = sum ? v + part[slot][i][r] : fmaxf(v, part[slot][i][r]);
+    return v;
+  };
+  float4 held[PACK_CHUNKS][2];
+#pragma unroll
+  for (int i = 0; i < PACK_CHUNKS; ++i) load(c0 + i * PACK_STEP, held[i]);
+  float rms = 1.f;
+  if (NORM) {
+    auto squares = [](const float4 (&v)[2], float acc) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) acc = fmaf(v[e].x, v[e].x, fmaf(v[e].y, v[e].y, fmaf(v[e].z, v[e].z, fmaf(v[e].w, v[e].w, acc))));
+      return acc;
+    };
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < PACK_CHUNKS; ++i) ss = squares(held[i], ss);
+    for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+      float4 v[2];
+      load(c, v);
+      ss = squares(v, ss);
+    }
+    rms = sqrtf(block(ss, 0, true) / (float)K + eps);
+  }
+  // a chunk as it is packed
+  auto finish = [&](int c, float4 (&v)[2]) {
+    if (!NORM || c >= chunks) return;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(w) + 2 * c + e);
+      v[e] = make_float4((v[e].x / rms) * q.x, (v[e].y / rms) * q.y, (v[e].z / rms) * q.z, (v[e].w / rms) * q.w);
+    }
+  };
+  auto biggest = [](const float4 (&v)[2], float acc) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) acc = fmaxf(fmaxf(acc, fmaxf(fabsf(v[e].x), fabsf(v[e].y))), fmaxf(fabsf(v[e].z), fabsf(v[e].w)));
+    return acc;
+  };
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < PACK_CHUNKS; ++i) {
+    finish(c0 + i * PACK_STEP, held[i]);
+    amax = biggest(held[i], amax);
+  }
+  for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+    float4 v[2];
+    load(c, v);
+    finish(c, v);
+    amax = biggest(v, amax);
+  }
+  amax = block(amax, 1, false);
+  int ex = 0;
+  if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);
+  const float inv = ldexpf(64.0f, -ex);
+  if (tid < PACK_ROWS) xscale[m] = ldexpf(1.0f, ex - 6);
+  uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / SINGLE_BM) * (K / BK) * ((size_t)SINGLE_BM * BK * 2) +
+                      ((m0 % SINGLE_BM) >> 3) * CORE_SBO + (m & 7) * 16;
+  auto store = [&](int c, const float4 (&v)[2]) {
+    if (c >= chunks) return;
+    *reinterpret_cast<uint4*>(tile_row + (size_t)(c >> 3) * ((size_t)SINGLE_BM * BK * 2) + (c & 7) * CORE_LBO) =
+        make_uint4(h2u(__floats2half2_rn(v[0].x * inv, v[0].y * inv)), h2u(__floats2half2_rn(v[0].z * inv, v[0].w * inv)),
+                   h2u(__floats2half2_rn(v[1].x * inv, v[1].y * inv)), h2u(__floats2half2_rn(v[1].z * inv, v[1].w * inv)));
+  };
+#pragma unroll
+  for (int i = 0; i < PACK_CHUNKS; ++i) store(c0 + i * PACK_STEP, held[i]);
+  for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+    float4 v[2];
+    load(c, v);
+    finish(c, v);
+    store(c, v);
   }
 }
 
@@ -648,19 +702,25 @@ int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, co
   return launch_tc<SINGLE_BM, NH>(dev, a, gn, gm, smem);
 }
 
-// x -> fp16 tiles and row scales in the handle's scratch
-int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const __half** xh, const float** xscale) {
+// x (under `norm`, if given) -> fp16 tiles and row scales in the handle's scratch
+int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const fb200_row_norm* norm, const __half** xh, const float** xscale) {
   const int mp = (int)((m + 127) / 128) * 128;
   const size_t xbytes = (size_t)mp * k * 2, need = xbytes + (size_t)mp * sizeof(float);
   int rc = fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, need);
   if (rc) return rc;
   __half* h = reinterpret_cast<__half*>(dev->xpack);
   float* s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
-  pack_rows16_kernel<<<mp / PACK_ROWS, 256, 0, dev->stream>>>(x, (int)m, (int)k, h, s);
+  if (norm) pack_rows16_kernel<true><<<mp / PACK_ROWS, PACK_THREADS, 0, dev->stream>>>(x, norm->res, norm->w, norm->eps, (int)m, (int)k, h, s);
+  else pack_rows16_kernel<false><<<mp / PACK_ROWS, PACK_THREADS, 0, dev->stream>>>(x, nullptr, nullptr, 0.f, (int)m, (int)k, h, s);
   FB_LAUNCH_CHECK(dev);
   *xh = h;
   *xscale = s;
   return FB200_OK;
+}
+
+// 16-byte loads of the norm's weights and residual
+bool norm_covers(const fb200_row_norm* norm) {
+  return !norm || ((reinterpret_cast<uintptr_t>(norm->w) | reinterpret_cast<uintptr_t>(norm->res)) & 15) == 0;
 }
 
 }  // namespace
@@ -669,9 +729,9 @@ int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const __half*
 // and y[M, N / 2] = silu(gate) * up. Returns 1 when the shape is not covered (the
 // caller falls back to the small-batch kernel in chunks of 32 rows).
 int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_t m, float* y, bool r1_is_bias, const float* r1,
-                const float* r2, int swiglu) {
+                const float* r2, int swiglu, const fb200_row_norm* norm) {
   TileGeom geo;
-  if (!tc_covers(w, x, m, &geo)) return 1;
+  if (!tc_covers(w, x, m, &geo) || !norm_covers(norm)) return 1;
   // A split of K (plain and residual epilogues, 16-byte aligned outputs, at least 2048 values of K per range) fills the
   // SMs where there are few tiles; it has to promise a tenth less, and the scratch for the partial products has to fit.
   static const bool no_split = getenv("FB200_TC_SPLITK") && getenv("FB200_TC_SPLITK")[0] == '0';
@@ -694,7 +754,7 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
   if (!best.ctas) return 1;
   const __half* xh;
   const float* xscale;
-  int rc = tc_pack(dev, x, m, w->k, &xh, &xscale);
+  int rc = tc_pack(dev, x, m, w->k, norm, &xh, &xscale);
   return rc ? rc : tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu, true);
 }
 
@@ -704,9 +764,10 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
 // products run side by side: the first on the handle's stream, the others on side streams forked
 // behind the packing kernel and joined again before the call returns to the stream. Returns 1 when
 // the shapes are not covered (the caller issues the products one after the other).
-int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* const* ys, int n, const float* x, size_t m) {
+int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* const* ys, int n, const float* x, size_t m,
+                      const fb200_row_norm* norm) {
   static const bool off = getenv("FB200_TC_GROUP") && getenv("FB200_TC_GROUP")[0] == '0';
-  if (off || n < 2 || n > 3 || m <= 32 || getenv("FB200_TC_TILE")) return 1;
+  if (off || n < 2 || n > 3 || m <= 32 || getenv("FB200_TC_TILE") || !norm_covers(norm)) return 1;
   TileGeom geo[3];
   for (int i = 0; i < n; ++i)
     if (!ws[i] || !tc_covers(ws[i], x, m, &geo[i]) || ws[i]->k != ws[0]->k) return 1;
@@ -736,7 +797,7 @@ int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* 
   if (!dev->fork_ev) FB_CUDA(dev, cudaEventCreateWithFlags(&dev->fork_ev, cudaEventDisableTiming));
   const __half* xh;
   const float* xscale;
-  int rc = tc_pack(dev, x, m, ws[0]->k, &xh, &xscale);
+  int rc = tc_pack(dev, x, m, ws[0]->k, norm, &xh, &xscale);
   if (rc) return rc;
   FB_CUDA(dev, cudaEventRecord(dev->fork_ev, dev->stream));
   cudaStream_t main_stream = dev->stream;

@@ -1,7 +1,17 @@
-// The prefill product on CTA pairs (qgemm_pair.cu), as qgemm.cu calls it.
+// Prefill products (qgemm.cu) and their kernel on CTA pairs (qgemm_pair.cu).
 #pragma once
 
 #include "common.cuh"
+
+// RMSNorm of the rows in front of a product: (x + res) / rms * w (res may be null; rows contiguous, of the product's K)
+struct fb200_row_norm {
+  const float *res, *w;
+  float eps;
+};
+int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_t m, float* y, bool r1_is_bias, const float* r1,
+                const float* r2, int swiglu, const fb200_row_norm* norm = nullptr);
+int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* const* ys, int n, const float* x, size_t m,
+                      const fb200_row_norm* norm = nullptr);
 
 struct PairArgs {
   const uint8_t* w;      // tiled weights
