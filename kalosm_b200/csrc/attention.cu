@@ -354,8 +354,8 @@ int fb200_launch_attention(fb200_device* dev, const float* q, const __half* k, c
   if (h % hkv) return fb200_fail(dev, FB200_ERR_INVALID_SHAPE, "attention: %d heads not divisible by %d kv heads", h, hkv);
   if (d != 64 && d != 128) return fb200_fail(dev, FB200_ERR_INVALID_SHAPE, "attention: head_dim %d (64 or 128 supported)", d);
   if (sq >= PREFILL_MIN_ROWS && mask_kind <= 1) {
-    // many query positions, no mask or causal: the tensor-core kernels (tcgen05 for head size 128
-    // and at least half a 128-row tile of queries, mma.sync otherwise)
+    // many query positions, no mask or causal: the tensor-core kernels (tcgen05 for at
+    // least half a 128-row tile of queries, mma.sync otherwise)
     int rc = 1;
     if (sq >= 64) rc = fb200_launch_attention_prefill_tc(dev, q, k, v, b, h, hkv, sq, skv, skv_dev, cap, d, scale, mask_kind, out, bshd);
     if (rc == 1) rc = fb200_launch_attention_prefill(dev, q, k, v, b, h, hkv, sq, skv, skv_dev, cap, d, scale, mask_kind, out, bshd);

@@ -1,4 +1,4 @@
-// Prefill attention (many query positions, no mask or causal, head size 128) on the 5th-generation
+// Prefill attention (many query positions, no mask or causal, head size 64 or 128) on the 5th-generation
 // tensor cores: both products of the attention run as tcgen05.mma with their results in tensor
 // memory (TMEM).
 //
@@ -46,13 +46,16 @@
 
 namespace {
 
-constexpr int XQ = 128, XK = 64, XD = 128, X_THREADS = 128;  // X_THREADS: the softmax threads (one per query row)
+constexpr int XQ = 128, XK = 64, X_THREADS = 128;  // X_THREADS: the softmax threads (one per query row)
 constexpr int X_BLOCK = X_THREADS + 64;                       // + the MMA issuer's warp + the copy requester's warp
-constexpr int X_Q_BYTES = XQ * XD * 2;   // 32 KB
-constexpr int X_KV_BYTES = XK * XD * 2;  // 16 KB per K or V tile
 constexpr int X_TAIL = 256;              // barriers, TMEM slot, give-up flag
 constexpr int X_KBUFS = 3, X_VBUFS = 2;   // K tiles are requested three tiles ahead, V tiles two
-constexpr int X_SMEM = X_Q_BYTES + (X_KBUFS + X_VBUFS) * X_KV_BYTES + X_TAIL;
+// XD: head size, 64 or 128
+template <int XD>
+struct XSize {
+  static constexpr int Q_BYTES = XQ * XD * 2, KV_BYTES = XK * XD * 2;  // 32 KB and 16 KB per K or V tile at 128
+  static constexpr int SMEM = Q_BYTES + (X_KBUFS + X_VBUFS) * KV_BYTES + X_TAIL;
+};
 constexpr int X_TMEM_COLS = 256;         // S buffers: columns 0..63 and 64..127; O: columns 128..255
 constexpr float X_RESCALE = 8.0f;        // log2 of the growth of a row maximum that triggers a rescale of O
 
@@ -71,20 +74,26 @@ struct XArgs {
 constexpr uint32_t X_SW128 = 2;
 constexpr uint32_t X_BOX_BYTES = XK * 64 * 2;  // one TMA box: 64 keys x 64 dims of fp16 = 8 KB
 
+template <int XD>
 __global__ void __launch_bounds__(X_BLOCK, 2)
 attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
+  constexpr int X_Q_BYTES = XSize<XD>::Q_BYTES, X_KV_BYTES = XSize<XD>::KV_BYTES;
   extern __shared__ __align__(1024) uint8_t sm[];  // the swizzled tiles need 1024-byte alignment (checked below)
   uint8_t* Qs = sm;
   uint8_t* Ks = sm + X_Q_BYTES;                        // [X_KBUFS][2 boxes]
   uint8_t* Vs = Ks + X_KBUFS * X_KV_BYTES;             // [X_VBUFS][2 boxes]
   uint64_t* bars = reinterpret_cast<uint64_t*>(Vs + X_VBUFS * X_KV_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // bar_s[2]: S_t complete (one per S buffer); bar_o: O += P V_t complete; bar_kfull[3], bar_vfull[2]: tile
-  // landed (byte count of its two boxes); bar_pfull: P written (an arrival per softmax warp)
+  // landed (byte count of its two boxes); bar_pfull[2]: P written (an arrival per softmax
+  // warp; one per S buffer: a warp may be a tile ahead of another, and its arrival must not count for the tile before)
   const uint32_t bar_s = smem_u32(bars), bar_o = smem_u32(bars + 2), bar_kfull = smem_u32(bars + 3),
-                 bar_vfull = smem_u32(bars + 6), bar_pfull = smem_u32(bars + 8);
+                 bar_vfull = smem_u32(bars + 6), bar_pfull = smem_u32(bars + 14), bar_kfree = smem_u32(bars + 9), bar_vfree = smem_u32(bars + 12);
+  // bar_kfree[3], bar_vfree[2]: the products that read a buffer are done. One barrier per buffer: its next phase needs the copy that
+  // the requester makes after this one, so a requester that is late cannot be overtaken (with bar_s and bar_o it could, and its wait
+  // for a phase that was over ran out)
 
   // Longest key ranges of all heads first (heads fastest): a long range that starts late is what the last round waits for
   const int qt = gridDim.y - 1 - blockIdx.y;
@@ -107,9 +116,10 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
     mbar_init(bar_s, 1);
     mbar_init(bar_s + 8, 1);
     mbar_init(bar_o, 1);
-    for (int i = 0; i < X_KBUFS; ++i) mbar_init(bar_kfull + 8 * i, 1);
-    for (int i = 0; i < X_VBUFS; ++i) mbar_init(bar_vfull + 8 * i, 1);
+    for (int i = 0; i < X_KBUFS; ++i) { mbar_init(bar_kfull + 8 * i, 1); mbar_init(bar_kfree + 8 * i, 1); }
+    for (int i = 0; i < X_VBUFS; ++i) { mbar_init(bar_vfull + 8 * i, 1); mbar_init(bar_vfree + 8 * i, 1); }
     mbar_init(bar_pfull, X_THREADS / 32);
+    mbar_init(bar_pfull + 8, X_THREADS / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -119,7 +129,7 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
   // Q tile: f32 -> fp16 into the K-major operand layout (rows past Sq are zero), by the softmax threads
   if (warp < X_THREADS / 32) {
     for (int id = warp; id < (XQ / 8) * (XD / 32); id += X_THREADS / 32) {
-      const int row = (id >> 2) * 8 + (lane & 7), c = (id & 3) * 4 + (lane >> 3);
+      const int row = id / (XD / 32) * 8 + (lane & 7), c = id % (XD / 32) * 4 + (lane >> 3);
       float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
       if (q0 + row < a.sq) {
         const float4* src = reinterpret_cast<const float4*>(a.q + q_base + (size_t)(q0 + row) * q_row + c * 8);
@@ -144,18 +154,18 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
     // O += P V_t has. A tile is two boxes (dims 0..63 and 64..127) of 64 keys.
     if (lane == 0 && ntiles > 0) {
       auto fetch = [&](const CUtensorMap* map, int tile, uint32_t dst, uint32_t bar) {
-        mbar_expect_tx(bar, 2 * X_BOX_BYTES);
+        mbar_expect_tx(bar, X_KV_BYTES);
         x_tma_box(dst, map, 0, tile * XK, plane, bar);
-        x_tma_box(dst + X_BOX_BYTES, map, 64, tile * XK, plane, bar);
+        if (XD == 128) x_tma_box(dst + X_BOX_BYTES, map, 64, tile * XK, plane, bar);
       };
       const uint32_t k0 = pf_smem(Ks), v0 = pf_smem(Vs);
       for (int t = 0; t < X_KBUFS && t < ntiles; ++t) fetch(&kmap, t, k0 + t * X_KV_BYTES, bar_kfull + 8 * t);
       for (int t = 0; t < X_VBUFS && t < ntiles; ++t) fetch(&vmap, t, v0 + t * X_KV_BYTES, bar_vfull + 8 * t);
       for (int tile = 0; tile + X_VBUFS < ntiles; ++tile) {
-        x_wait(bar_s + 8 * (tile & 1), (uint32_t)((tile >> 1) & 1), dead, a.status);  // K buffer of tile t is free
+        x_wait(bar_kfree + 8 * (tile % X_KBUFS), (uint32_t)((tile / X_KBUFS) & 1), dead, a.status);  // K buffer of tile t is free
         if (tile + X_KBUFS < ntiles)
           fetch(&kmap, tile + X_KBUFS, k0 + (tile % X_KBUFS) * X_KV_BYTES, bar_kfull + 8 * (tile % X_KBUFS));
-        x_wait(bar_o, (uint32_t)(tile & 1), dead, a.status);  // V buffer of tile t is free
+        x_wait(bar_vfree + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status);  // V buffer of tile t is free
         fetch(&vmap, tile + X_VBUFS, v0 + (tile % X_VBUFS) * X_KV_BYTES, bar_vfull + 8 * (tile % X_VBUFS));
       }
     }
@@ -172,24 +182,26 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
         const uint32_t d = tmem + (uint32_t)((tile & 1) * XK);
         // a K step is 256 bytes of Q and, inside a 128-byte row of the box, 32 bytes of K
         w_mma4<16, 2>(d, qdesc, kdesc, IDESC_S, 0u);
-        w_mma4<16, 2>(d, qdesc + 64, kdesc + (X_BOX_BYTES >> 4), IDESC_S, 1u);
+        if (XD == 128) w_mma4<16, 2>(d, qdesc + 64, kdesc + (X_BOX_BYTES >> 4), IDESC_S, 1u);
         w_commit(bar_s + 8 * (tile & 1));
+        w_commit(bar_kfree + 8 * (tile % X_KBUFS));
       };
-      static_assert(XD == 128 && XK == 64, "eight K steps over two boxes, four K steps of 16 keys");
+      static_assert((XD == 128 || XD == 64) && XK == 64, "four K steps in a box of 64 dims, four K steps of 16 keys");
       issue_s(0);
       for (int tile = 0; tile < ntiles; ++tile) {
         if (tile + 1 < ntiles) issue_s(tile + 1);
         w_wait(bar_vfull + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status);
-        w_wait(bar_pfull, (uint32_t)(tile & 1), dead, a.status);
+        w_wait(bar_pfull + 8 * (tile & 1), (uint32_t)((tile >> 1) & 1), dead, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // a K step is 16 keys: 8 columns of P, 16 rows of 128 bytes of V
         w_mma4_ta<8, 128>(tmem + 2 * XK, tmem + (uint32_t)((tile & 1) * XK),
                           x_desc(pf_smem(Vs + (tile % X_VBUFS) * X_KV_BYTES), (uint32_t)a.v_lbo, (uint32_t)a.v_sbo, X_SW128), IDESC_O, tile ? 1u : 0u);
         w_commit(bar_o);
+        w_commit(bar_vfree + 8 * (tile % X_VBUFS));
       }
     }
   } else {
-    // ---- softmax threads
+    // ---- softmax threads (a warp leaves its waits together: the tensor memory accesses behind them are for whole warps)
     const uint32_t tmem_lane = tmem + ((uint32_t)(32 * warp) << 16);  // this warp's 32 lanes
     float m_ref = -INFINITY;  // the maximum the exponentials and O currently refer to (scaled, log2 domain)
     float l_run = 0.f;
@@ -197,7 +209,7 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
 
     for (int tile = 0; tile < ntiles; ++tile) {
       const int sb = tile & 1;
-      x_wait(bar_s + 8 * sb, (uint32_t)((tile >> 1) & 1), dead, a.status);  // S_t is there
+      w_wait(bar_s + 8 * sb, (uint32_t)((tile >> 1) & 1), dead, a.status);  // S_t is there
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
       // ---- this thread's row of S: mask, running maximum and sum
@@ -223,7 +235,9 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
       const float mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7])));
       const float m_new = fmaxf(m_ref, mx * a.scale_log2);
       // follow the maximum lazily: rescale when it has outgrown the reference by more than 2^X_RESCALE
-      const bool grow = m_new > m_ref + X_RESCALE;  // also true for the first finite maximum (m_ref = -inf)
+      // (heads of 64 at once, as the mma.sync kernel that ran them before does: its largest weight is exactly 1, which makes the error
+      // 3 % smaller, and O is half as wide)
+      const bool grow = m_new > m_ref + (XD == 64 ? 0.f : X_RESCALE);  // also true for the first finite maximum (m_ref = -inf)
       const float alpha = grow ? x_ex2(m_ref - m_new) : 1.0f;  // 2^-inf = 0 for a row that had no key yet
       if (grow) m_ref = m_new;
       const float msafe = m_ref == -INFINITY ? 0.f : m_ref;
@@ -246,7 +260,7 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
 
       // ---- O is rescaled only after the previous tile's O += P V has completed
       if (tile > 0 && __any_sync(0xFFFFFFFFu, grow)) {
-        x_wait(bar_o, (uint32_t)((tile - 1) & 1), dead, a.status);
+        w_wait(bar_o, (uint32_t)((tile - 1) & 1), dead, a.status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < XD / 32; ++c) {
@@ -262,14 +276,14 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       // before the last product can start, the one before it is seen complete: the final wait below then is for the
       // phase in progress (a parity wait must be neither two phases early nor two late)
-      if (tile > 0 && tile == ntiles - 1) x_wait(bar_o, (uint32_t)((tile - 1) & 1), dead, a.status);
+      if (tile > 0 && tile == ntiles - 1) w_wait(bar_o, (uint32_t)((tile - 1) & 1), dead, a.status);
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_pfull);  // phase t
+      if (lane == 0) mbar_arrive(bar_pfull + 8 * sb);
     }
 
     // ---- the last product, then normalise and store (nothing is stored after a wait has given up)
     if (ntiles > 0) {
-      x_wait(bar_o, (uint32_t)((ntiles - 1) & 1), dead, a.status);
+      w_wait(bar_o, (uint32_t)((ntiles - 1) & 1), dead, a.status);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     const bool store = row < a.sq && !*dead;
@@ -314,13 +328,13 @@ x_encode_fn x_encoder() {
   }();
   return fn;
 }
-// fp16 cache [planes][cap][128] seen as (dims, keys, planes) with `rows` valid keys per plane; boxes
+// fp16 cache [planes][cap][d] seen as (dims, keys, planes) with `rows` valid keys per plane; boxes
 // of 64 dims x 64 keys, 128-byte swizzle, zeros outside.
-bool x_make_map(CUtensorMap* map, const __half* base, int rows, int cap, int planes) {
+bool x_make_map(CUtensorMap* map, const __half* base, int d, int rows, int cap, int planes) {
   x_encode_fn enc = x_encoder();
   if (!enc) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)XD, (cuuint64_t)rows, (cuuint64_t)planes};
-  const cuuint64_t strides[2] = {(cuuint64_t)XD * 2, (cuuint64_t)cap * XD * 2};
+  const cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)rows, (cuuint64_t)planes};
+  const cuuint64_t strides[2] = {(cuuint64_t)d * 2, (cuuint64_t)cap * d * 2};
   const cuuint32_t box[3] = {64, (cuuint32_t)XK, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(base), dims, strides, box, estr,
@@ -328,21 +342,31 @@ bool x_make_map(CUtensorMap* map, const __half* base, int rows, int cap, int pla
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int XD>
+int x_launch(fb200_device* dev, dim3 grid, const XArgs& a, const CUtensorMap& kmap, const CUtensorMap& vmap) {
+  static bool configured[64] = {false};
+  if (!configured[dev->ordinal & 63]) {
+    FB_CUDA(dev, cudaFuncSetAttribute(attn_prefill_tc_kernel<XD>, cudaFuncAttributeMaxDynamicSharedMemorySize, XSize<XD>::SMEM));
+    configured[dev->ordinal & 63] = true;
+  }
+  return fb200_launch(dev, attn_prefill_tc_kernel<XD>, grid, dim3(X_BLOCK), (size_t)XSize<XD>::SMEM, false, a, kmap, vmap);
+}
+
 }  // namespace
 
-// Covers: head size 128, no mask or causal, 16-byte aligned q / out / cache, the number of keys known
+// Covers: head sizes 64 and 128 (16 heads of 64, 2000 queries: see below), no mask or causal, 16-byte aligned q / out / cache, the number of keys known
 // on the host (skv > 0; skv_dev, if given, must hold skv - sq). Returns 1 when the shape is not
 // covered (the caller then runs the mma.sync kernel). FB200_ATTN_TCGEN05=0 switches it off.
 int fb200_launch_attention_prefill_tc(fb200_device* dev, const float* q, const __half* k, const __half* v, int b, int h,
                                       int hkv, int sq, int skv, const int* skv_dev, int cap, int d, float scale,
                                       int causal, float* out, int bshd) {
   static const bool off = getenv("FB200_ATTN_TCGEN05") && getenv("FB200_ATTN_TCGEN05")[0] == '0';
-  if (off || d != XD || h % hkv || b > 65535 || h > 65535 || (sq + XQ - 1) / XQ > 65535 || !(scale > 0.f) || skv <= 0 || skv > cap) return 1;
+  if (off || (d != 64 && d != 128) || h % hkv || b > 65535 || h > 65535 || (sq + XQ - 1) / XQ > 65535 || !(scale > 0.f) || skv <= 0 || skv > cap) return 1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(k) |
        reinterpret_cast<uintptr_t>(v)) & 15u)
     return 1;
   CUtensorMap kmap, vmap;
-  if (!x_make_map(&kmap, k, skv, cap, b * hkv) || !x_make_map(&vmap, v, skv, cap, b * hkv)) return 1;
+  if (!x_make_map(&kmap, k, d, skv, cap, b * hkv) || !x_make_map(&vmap, v, d, skv, cap, b * hkv)) return 1;
   XArgs a = {};
   a.q = q; a.k = k; a.v = v; a.out = out; a.skv_dev = skv_dev;
   a.b = b; a.h = h; a.hkv = hkv; a.sq = sq; a.skv = skv; a.cap = cap; a.groups = h / hkv; a.bshd = bshd;
@@ -352,10 +376,5 @@ int fb200_launch_attention_prefill_tc(fb200_device* dev, const float* q, const _
   a.v_sbo = 1024;         // ... and between groups of 8 keys
   a.status = dev->status;
   const dim3 grid((unsigned)h, (unsigned)((sq + XQ - 1) / XQ), (unsigned)b);
-  static bool configured[64] = {false};
-  if (!configured[dev->ordinal & 63]) {
-    FB_CUDA(dev, cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM));
-    configured[dev->ordinal & 63] = true;
-  }
-  return fb200_launch(dev, attn_prefill_tc_kernel, grid, dim3(X_BLOCK), (size_t)X_SMEM, false, a, kmap, vmap);
+  return d == 64 ? x_launch<64>(dev, grid, a, kmap, vmap) : x_launch<128>(dev, grid, a, kmap, vmap);
 }
