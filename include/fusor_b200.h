@@ -80,7 +80,9 @@ FB200_API int fb200_device_clear_status(fb200_device* dev);
 /* Scratch buffers of the handle (packed activations, normalised rows, host staging) replace the
  * reference's BufferPool (fusor-ml/tile-ir-runtime/src/buffer_pool.rs:74-260). A budget of
  * `bytes` (0 = unlimited; also FB200_SCRATCH_LIMIT in the environment at creation) makes a call
- * that would grow them beyond it fail with FB200_ERR_CAPACITY instead of allocating. */
+ * that would grow them beyond it fail with FB200_ERR_CAPACITY instead of allocating. Partial products
+ * of a prompt product that splits K are held only where there is room for them: without it the product
+ * runs unsplit (other rounding of its last bits), and they are given back to a call that needs the room. */
 FB200_API int fb200_device_set_scratch_limit(fb200_device* dev, size_t bytes);
 /* Poison mode (also FB200_POISON=1 at creation): freshly allocated scratch is filled with 0xFF
  * bytes (NaN as f32 / f16), the analogue of the pool's poison fill (buffer_pool.rs:198-207,

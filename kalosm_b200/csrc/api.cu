@@ -72,7 +72,17 @@ int fb200_bind(fb200_device* dev) {
 int fb200_ensure(fb200_device* dev, void** buf, size_t* cur, size_t bytes) {
   if (*cur >= bytes) return FB200_OK;
   const size_t want = bytes + bytes / 4 + 4096;
-  if (dev->scratch_limit && dev->scratch_total - *cur + want > dev->scratch_limit)
+  auto fits = [&](size_t given_back) { return !dev->scratch_limit || dev->scratch_total - *cur - given_back + want <= dev->scratch_limit; };
+  // The partial products of a split K are scratch that a product can do without: they make room for what a call needs
+  if (!fits(0) && buf != &dev->splitk && dev->splitk && fits(dev->splitk_bytes)) {
+    FB_CUDA(dev, cudaStreamSynchronize(dev->stream));
+    FB_CUDA(dev, cudaFree(dev->splitk));
+    dev->scratch_total -= dev->splitk_bytes;
+    dev->splitk = nullptr;
+    dev->splitk_bytes = 0;
+    dev->scratch_gen++;
+  }
+  if (!fits(0))
     return fb200_fail(dev, FB200_ERR_CAPACITY, "scratch: %zu more bytes would exceed the handle's budget of %zu (in use %zu)",
                       want, dev->scratch_limit, dev->scratch_total);
   if (*buf) {

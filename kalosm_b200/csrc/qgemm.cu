@@ -655,8 +655,8 @@ splitk_add_kernel(const float4* __restrict__ parts, int nsplit, size_t n4, int n
 }
 
 // Launches the product of packed rows (xh, xscale: pack_rows16_kernel with 128-row tiles) on dev->stream.
-// With sh.split > 1 every K range writes its partial product into the handle's split-K scratch and a second kernel adds
-// them (+ residuals). `early`: the packing kernel is the last work on the stream, and the product may start beside it.
+// With sh.split > 1 every K range writes its partial product into the handle's split-K scratch (tc_parts) and a second kernel
+// adds them (+ residuals). `early`: the packing kernel is the last work on the stream, and the product may start beside it.
 int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, const TcShape& sh, const __half* xh,
               const float* xscale, size_t m, float* y, bool r1_is_bias, const float* r1, const float* r2, int swiglu, bool early) {
   const int halves = (int)((m + 127) / 128), split = sh.split;
@@ -672,8 +672,6 @@ int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, co
     a.splits = (w->ngroups + a.kg_per - 1) / a.kg_per;  // every range holds at least one K group
     a.x_halves = halves; a.status = dev->status;
     if (split > 1) {
-      rc = fb200_ensure(dev, &dev->splitk, &dev->splitk_bytes, (size_t)split * m * w->n * sizeof(float));
-      if (rc) return rc;
       a.y = reinterpret_cast<float*>(dev->splitk);
       a.r1 = a.r2 = nullptr;
     }
@@ -702,11 +700,24 @@ int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, co
   return launch_tc<SINGLE_BM, NH>(dev, a, gn, gm, smem);
 }
 
+// Scratch of packed rows: fp16 tiles of 128 rows, then the row scales
+int tc_reserve(fb200_device* dev, size_t m, size_t k) {
+  const size_t mp = (m + 127) / 128 * 128;
+  return fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, mp * k * 2 + mp * sizeof(float));
+}
+
+// Scratch of a split's partial products. A budget or a card without room for them is not an error: the product then runs unsplit.
+bool tc_parts(fb200_device* dev, const fb200_qmatrix* w, size_t m, int split) {
+  if (fb200_ensure(dev, &dev->splitk, &dev->splitk_bytes, (size_t)split * m * w->n * sizeof(float)) == FB200_OK) return true;
+  cudaGetLastError();  // a refused allocation is not the next launch's error
+  return false;
+}
+
 // x (under `norm`, if given) -> fp16 tiles and row scales in the handle's scratch
 int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const fb200_row_norm* norm, const __half** xh, const float** xscale) {
   const int mp = (int)((m + 127) / 128) * 128;
-  const size_t xbytes = (size_t)mp * k * 2, need = xbytes + (size_t)mp * sizeof(float);
-  int rc = fb200_ensure(dev, &dev->xpack, &dev->xpack_bytes, need);
+  const size_t xbytes = (size_t)mp * k * 2;
+  int rc = tc_reserve(dev, m, k);
   if (rc) return rc;
   __half* h = reinterpret_cast<__half*>(dev->xpack);
   float* s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
@@ -733,28 +744,28 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
   TileGeom geo;
   if (!tc_covers(w, x, m, &geo) || !norm_covers(norm)) return 1;
   // A split of K (plain and residual epilogues, 16-byte aligned outputs, at least 2048 values of K per range) fills the
-  // SMs where there are few tiles; it has to promise a tenth less, and the scratch for the partial products has to fit.
+  // SMs where there are few tiles; it has to promise a tenth less, and runs only where the scratch for its partial products fits.
   static const bool no_split = getenv("FB200_TC_SPLITK") && getenv("FB200_TC_SPLITK")[0] == '0';
   const bool may_split = !no_split && !swiglu && w->n % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(r1) | reinterpret_cast<uintptr_t>(r2)) & 15) == 0;
-  TcShape best;
+  TcShape best, whole;  // whole: the best without a split
   for (int split = 1; split <= (may_split ? 4 : 1); split *= 2) {
-    if (split > 1) {
-      const size_t want = (size_t)split * m * w->n * sizeof(float);
-      if (w->k / split < 2048 || w->ngroups < 2 * split) break;
-      if (want > dev->splitk_bytes && dev->scratch_limit && dev->scratch_total - dev->splitk_bytes + want > dev->scratch_limit) break;
-    }
+    if (split > 1 && (w->k / split < 2048 || w->ngroups < 2 * split)) break;
     for (int nw = 256; nw >= (split > 1 ? 128 : 0); nw -= 128) {
       TcShape sh;
       sh.nw = nw; sh.split = split;
       if (!tc_forced(sh) || !tc_shape(dev, w, geo, m, swiglu, &sh)) continue;
       if (!best.ctas || sh.ns < (split > 1 ? 0.9 : 1.0) * best.ns) best = sh;
     }
+    if (split == 1) whole = best;
   }
   if (!best.ctas) return 1;
+  int rc = tc_reserve(dev, m, w->k);  // what the product needs comes before what it can do without
+  if (rc) return rc;
+  if (best.split > 1 && !tc_parts(dev, w, m, best.split)) best = whole;
   const __half* xh;
   const float* xscale;
-  int rc = tc_pack(dev, x, m, w->k, norm, &xh, &xscale);
+  rc = tc_pack(dev, x, m, w->k, norm, &xh, &xscale);
   return rc ? rc : tc_launch(dev, w, geo, best, xh, xscale, m, y, r1_is_bias, r1, r2, swiglu, true);
 }
 

@@ -280,3 +280,30 @@ def test_scratch_budget_and_poison(dev):
     assert F.rel_l2(y, O.q_mat_mul(x, raw, ty, n, k)) < 2e-3
     w.free()
     other.close()
+
+
+def test_split_k_scratch_makes_room(dev):
+    # 200 rows of a 4096 x 4096 matrix run in two ranges of K (2.6 MB of packed rows, 8.2 MB of partial products with the
+    # allocator's margin). A budget without room for both takes the same call unsplit, and partial products that are held are
+    # given back when a later call needs the room (1300 rows: 14.4 MB packed)
+    other = kb.Device(0)
+    ty, n, k = O.Q4K, 4096, 4096
+    raw = weights(13, n, k, ty)
+    w = kb.QMatrix.from_raw_bytes(other, (n, k), raw, ty)
+    deq = w.dequantize().as_slice().astype(np.float64)
+    x = np.random.default_rng(4).standard_normal((1300, k)).astype(np.float32)
+    want = x @ deq.T
+    other.set_scratch_limit(9 << 20)  # room for either, not for both
+    whole = other.tensor(x[:200]).q_mat_mul(w).as_slice()
+    assert F.rel_l2(whole, want[:200]) < 2e-3
+    other.set_scratch_limit(16 << 20)
+    split = other.tensor(x[:200]).q_mat_mul(w).as_slice()
+    assert F.rel_l2(split, want[:200]) < 2e-3
+    assert not np.array_equal(split, whole)  # partial sums are rounded apart: the split did run
+    assert F.rel_l2(other.tensor(x).q_mat_mul(w).as_slice(), want) < 2e-3
+    assert np.array_equal(other.tensor(x[:200]).q_mat_mul(w).as_slice(), whole)  # the packed rows keep the room
+    other.set_scratch_limit(0)
+    assert np.array_equal(other.tensor(x[:200]).q_mat_mul(w).as_slice(), split)
+    assert other.status() == 0
+    w.free()
+    other.close()
