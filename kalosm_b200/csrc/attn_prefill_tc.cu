@@ -362,8 +362,9 @@ int fb200_launch_attention_prefill_tc(fb200_device* dev, const float* q, const _
                                       int causal, float* out, int bshd) {
   static const bool off = getenv("FB200_ATTN_TCGEN05") && getenv("FB200_ATTN_TCGEN05")[0] == '0';
   // Heads of 64: a few short tiles do not pay for the set-up (24 heads, 137 x 137: 16.4 us here, 14.3 on mma.sync; 314 x 314, 40 heads: 18.4
-  // and 20.4; 64 x 1500, 32 heads: 33 and 45; 2000 x 2000, 16 heads: 44 and 76)
-  if (d == 64 && sq < 256 && skv < 512) return 1;
+  // and 20.4; 64 x 1500, 32 heads: 33 and 45; 2000 x 2000, 16 heads: 44 and 76). 256 x 256 still is four by four tiles of 64 there
+  // (back to back, 4 / 16 / 32 heads: 12.2 / 12.5 / 12.5 us here, 10.7 / 11.6 / 11.7), 270 x 270 takes 12.5 us on either
+  if (d == 64 && ((sq < 256 && skv < 512) || (sq <= 256 && skv <= 256))) return 1;
   if (off || (d != 64 && d != 128) || h % hkv || b > 65535 || h > 65535 || (sq + XQ - 1) / XQ > 65535 || !(scale > 0.f) || skv <= 0 || skv > cap) return 1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(k) |
        reinterpret_cast<uintptr_t>(v)) & 15u)

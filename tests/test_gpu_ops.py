@@ -234,6 +234,17 @@ def test_attention_masks_and_cache_capacity(dev):
     assert np.max(np.abs(out - O.attention(q, kf, vf, scale, mask=bk, mask_kind=1))) < 1e-3
 
 
+def test_prefill_attention_short_heads_of_64(dev):
+    # up to 256 queries on 256 keys the mma.sync kernel is the faster one. A causal row's bits do not depend on how many
+    # rows follow it in the same kernel, and they do on the kernel: 192 x 192 has always run there, 257 x 257 does not
+    rng = np.random.default_rng(64)
+    q, k, v = (rng.standard_normal((1, 4, 257, 64)).astype(t) for t in (np.float32, np.float16, np.float16))
+    out = {n: dev.flash_attention(*(dev.tensor(np.ascontiguousarray(a[:, :, :n])) for a in (q, k, v)), 0.125,
+                                  mask_kind=kb.MASK_CAUSAL).as_slice() for n in (192, 256, 257)}
+    assert np.array_equal(out[256][:, :, :192], out[192])
+    assert not np.array_equal(out[257][:, :, :192], out[192])
+
+
 def test_peer_exchange_wait_is_bounded(dev):
     # a peer that never arrives: the wait gives up after its poll limit, the handle's status word
     # says so, and the GPU keeps working (no trap, no hang); a handle of its own keeps the
