@@ -575,8 +575,8 @@ int run_forward(fb200_llama* m, int batch, int seq, bool commit = true) {
     } else if (L.gate_up) {
       const fb200_row_norm norm{m->x, L.ffn_norm, c.rms_eps};
       rc = 1;
-      if (rows > 32 && L.gate_up->n % 32 == 0) {
-        fb200_op_trace scope(dev, "q_mat_mul (> 32 rows)", (double)L.gate_up->raw_nbytes + 4.0 * (double)rows * (double)(E + L.gate_up->n));
+      if (rows > 32 && L.gate_up->n % 32 == 0 && fb200_qgemm_covers(L.gate_up, m->attn_out, rows, &norm)) {
+        fb200_op_trace scope(dev, "rms_norm + q_mat_mul", (double)L.gate_up->raw_nbytes + 4.0 * (double)rows * (double)(2 * E + L.gate_up->n));
         rc = fb200_qgemm(dev, L.gate_up, m->attn_out, rows, m->hbuf, false, nullptr, nullptr, 1, &norm);
       }
       if (rc == 1) {

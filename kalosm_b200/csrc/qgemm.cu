@@ -736,6 +736,11 @@ bool norm_covers(const fb200_row_norm* norm) {
 
 }  // namespace
 
+bool fb200_qgemm_covers(const fb200_qmatrix* w, const float* x, size_t m, const fb200_row_norm* norm) {
+  TileGeom geo;
+  return tc_covers(w, x, m, &geo) && norm_covers(norm);
+}
+
 // y[M, N] = x[M, K] . W^T (+ r1 + r2) for M > 32; with `swiglu`, W stacks gate rows over up rows
 // and y[M, N / 2] = silu(gate) * up. Returns 1 when the shape is not covered (the
 // caller falls back to the small-batch kernel in chunks of 32 rows).

@@ -8,6 +8,8 @@ struct fb200_row_norm {
   const float *res, *w;
   float eps;
 };
+// whether fb200_qgemm takes a product of these rows (the epilogue aside)
+bool fb200_qgemm_covers(const fb200_qmatrix* w, const float* x, size_t m, const fb200_row_norm* norm = nullptr);
 int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_t m, float* y, bool r1_is_bias, const float* r1,
                 const float* r2, int swiglu, const fb200_row_norm* norm = nullptr);
 int fb200_qgemm_group(fb200_device* dev, const fb200_qmatrix* const* ws, float* const* ys, int n, const float* x, size_t m,

@@ -89,6 +89,12 @@ def main(what):
                 err = F.rel_l2(dev.tensor(x).q_mat_mul(w).as_slice(), O.q_mat_mul(x, raw, O.Q5K, n, k))
                 assert err < TOL, (n, k, m, err)
                 print(f"ok Q5_K {n}x{k} rows {m}: {err:.1e}")
+    elif what == "prefill_chunks":   # FB200_TCGEN05=0: products of more than 32 rows in passes of 32
+        products(dev, [33, 70])
+        decoder(dev, 1, prompt_len=48)
+    elif what == "trace":            # one prompt pass of a two-layer decoder, for the lines it prints with FB200_TRACE=1
+        gpu, _ = build_models(dev, tiny_cfg(), batch=1, seed=31)
+        gpu.forward(np.arange(48, dtype=np.uint32)[None])
     elif what == "prefill_sequential":  # FB200_TC_GROUP=0: q, k, v of a prompt pass one after the other
         decoder(dev, 1, prompt_len=48)
     else:
