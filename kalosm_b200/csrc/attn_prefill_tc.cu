@@ -36,8 +36,10 @@
 // it lies in the cache. Two CTAs share an SM (112 KB of shared memory and 256 TMEM columns each). Tiles above the diagonal are never visited; CTAs with the longest key range
 // start first.
 // Every mbarrier wait is bounded: a wait that gives up sets the device status word and a flag in
-// shared memory, every later wait of the CTA then returns at once, the CTA runs through its loop
-// without waiting (results invalid, nothing stored), frees its TMEM columns and exits.
+// shared memory, every later wait of the CTA then returns at once and no further tile is requested; the
+// issuer and the softmax run through their loops without waiting (results invalid, nothing stored). The
+// requester and the issuer then wait, with a limit, for their copies and products in flight, and the CTA
+// frees its TMEM columns and exits.
 #include <cuda.h>
 
 #include "attn_mma.cuh"
@@ -83,14 +85,15 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
   uint8_t* Ks = sm + X_Q_BYTES;                        // [X_KBUFS][2 boxes]
   uint8_t* Vs = Ks + X_KBUFS * X_KV_BYTES;             // [X_VBUFS][2 boxes]
   uint64_t* bars = reinterpret_cast<uint64_t*>(Vs + X_VBUFS * X_KV_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // bar_s[2]: S_t complete (one per S buffer); bar_o: O += P V_t complete; bar_kfull[3], bar_vfull[2]: tile
   // landed (byte count of its two boxes); bar_pfull[2]: P written (an arrival per softmax
   // warp; one per S buffer: a warp may be a tile ahead of another, and its arrival must not count for the tile before)
   const uint32_t bar_s = smem_u32(bars), bar_o = smem_u32(bars + 2), bar_kfull = smem_u32(bars + 3),
-                 bar_vfull = smem_u32(bars + 6), bar_pfull = smem_u32(bars + 14), bar_kfree = smem_u32(bars + 9), bar_vfree = smem_u32(bars + 12);
+                 bar_vfull = smem_u32(bars + 6), bar_pfull = smem_u32(bars + 14), bar_kfree = smem_u32(bars + 9), bar_vfree = smem_u32(bars + 12),
+                 bar_end = smem_u32(bars + 16);  // of a CTA that gave up
   // bar_kfree[3], bar_vfree[2]: the products that read a buffer are done. One barrier per buffer: its next phase needs the copy that
   // the requester makes after this one, so a requester that is late cannot be overtaken (with bar_s and bar_o it could, and its wait
   // for a phase that was over ran out)
@@ -120,6 +123,7 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
     for (int i = 0; i < X_VBUFS; ++i) { mbar_init(bar_vfull + 8 * i, 1); mbar_init(bar_vfree + 8 * i, 1); }
     mbar_init(bar_pfull, X_THREADS / 32);
     mbar_init(bar_pfull + 8, X_THREADS / 32);
+    mbar_init(bar_end, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -159,14 +163,22 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
         if (XD == 128) x_tma_box(dst + X_BOX_BYTES, map, 64, tile * XK, plane, bar);
       };
       const uint32_t k0 = pf_smem(Ks), v0 = pf_smem(Vs);
-      for (int t = 0; t < X_KBUFS && t < ntiles; ++t) fetch(&kmap, t, k0 + t * X_KV_BYTES, bar_kfull + 8 * t);
-      for (int t = 0; t < X_VBUFS && t < ntiles; ++t) fetch(&vmap, t, v0 + t * X_KV_BYTES, bar_vfull + 8 * t);
-      for (int tile = 0; tile + X_VBUFS < ntiles; ++tile) {
-        x_wait(bar_kfree + 8 * (tile % X_KBUFS), (uint32_t)((tile / X_KBUFS) & 1), dead, a.status);  // K buffer of tile t is free
-        if (tile + X_KBUFS < ntiles)
-          fetch(&kmap, tile + X_KBUFS, k0 + (tile % X_KBUFS) * X_KV_BYTES, bar_kfull + 8 * (tile % X_KBUFS));
-        x_wait(bar_vfree + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status);  // V buffer of tile t is free
-        fetch(&vmap, tile + X_VBUFS, v0 + (tile % X_VBUFS) * X_KV_BYTES, bar_vfull + 8 * (tile % X_VBUFS));
+      int nk = 0, nv = 0;
+      for (; nk < X_KBUFS && nk < ntiles; ++nk) fetch(&kmap, nk, k0 + nk * X_KV_BYTES, bar_kfull + 8 * nk);
+      for (; nv < X_VBUFS && nv < ntiles; ++nv) fetch(&vmap, nv, v0 + nv * X_KV_BYTES, bar_vfull + 8 * nv);
+      for (int tile = 0; nv < ntiles; ++tile) {
+        if (!x_wait(bar_kfree + 8 * (tile % X_KBUFS), (uint32_t)((tile / X_KBUFS) & 1), dead, a.status)) break;  // K buffer of tile t is free
+        if (nk < ntiles) {
+          fetch(&kmap, nk, k0 + (tile % X_KBUFS) * X_KV_BYTES, bar_kfull + 8 * (tile % X_KBUFS));
+          ++nk;
+        }
+        if (!x_wait(bar_vfree + 8 * (tile % X_VBUFS), (uint32_t)((tile / X_VBUFS) & 1), dead, a.status)) break;  // V buffer of tile t is free
+        fetch(&vmap, nv, v0 + (tile % X_VBUFS) * X_KV_BYTES, bar_vfull + 8 * (tile % X_VBUFS));
+        ++nv;
+      }
+      if (*dead) {  // before this CTA's shared memory is free
+        for (int u = max(0, nk - X_KBUFS); u < nk; ++u) x_drain(bar_kfull + 8 * (u % X_KBUFS), (uint32_t)((u / X_KBUFS) & 1));
+        for (int u = max(0, nv - X_VBUFS); u < nv; ++u) x_drain(bar_vfull + 8 * (u % X_VBUFS), (uint32_t)((u / X_VBUFS) & 1));
       }
     }
   } else if (warp == X_THREADS / 32) {
@@ -198,6 +210,10 @@ attn_prefill_tc_kernel(const XArgs a, const __grid_constant__ CUtensorMap kmap, 
                           x_desc(pf_smem(Vs + (tile % X_VBUFS) * X_KV_BYTES), (uint32_t)a.v_lbo, (uint32_t)a.v_sbo, X_SW128), IDESC_O, tile ? 1u : 0u);
         w_commit(bar_o);
         w_commit(bar_vfree + 8 * (tile % X_VBUFS));
+      }
+      if (__any_sync(0xFFFFFFFFu, *dead)) {  // before its shared and tensor memory are free
+        w_commit(bar_end);
+        x_drain(bar_end, 0);
       }
     }
   } else {
