@@ -27,8 +27,9 @@
 //    scaled back and written, with the residual adds or SwiGLU (gate and up rows are the two
 //    halves of one CTA, so both values of an output sit in the same TMEM lane).
 // Every wait is bounded (2^22 polls): on a time-out the status word and a give-up flag in shared
-// memory are set, the other roles leave at their next poll, and the CTA releases its TMEM
-// columns and exits. FB200_TCGEN05=0 switches the kernel off (32-row kernel in chunks);
+// memory are set, the other roles leave at their next poll, loaders and issuer wait (with a limit) for
+// their copies and MMAs in flight, and the CTA releases its TMEM columns and exits.
+// FB200_TCGEN05=0 switches the kernel off (32-row kernel in chunks);
 // FB200_TC_TILE forces a tile shape (tests, tuning).
 #include <algorithm>
 #include <cstdint>
@@ -36,7 +37,7 @@
 #include <cstdlib>
 
 #include "qgemm_pair.cuh"
-#include "qgemv_common.cuh"
+#include "tcgen05.cuh"
 
 int fb200_ensure(fb200_device* dev, void** buf, size_t* cur, size_t bytes);
 
@@ -81,25 +82,6 @@ struct TcArgs {
   int* status;
 };
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Bounded wait of the pipeline roles: gives up after 2^22 polls, or as soon as another thread
-// of the CTA has given up (so a broken pipeline drains in one time-out, not one per wait).
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int* dead, int* status) {
-  for (int it = 0; it < (1 << 22); ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (ok) return true;
-    if ((it & 255) == 255 && *dead) return false;
-  }
-  *dead = 1;
-  if (status) atomicExch(status, FB200_ERR_TIMEOUT);
-  return false;
-}
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t lds4(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
@@ -264,7 +246,7 @@ qgemm_tc_kernel(const TcArgs a) {
   const int n0 = blockIdx.x * (a.pair_tiles ? BN : BN * NH), m0 = blockIdx.y * BM;
   const uint32_t bar_raw_full = smem_u32(bars), bar_raw_free = smem_u32(bars + 2), bar_a_full = smem_u32(bars + 4),
                  bar_b_full = smem_u32(bars + 4 + MAX_STAGES), bar_free = smem_u32(bars + 4 + 2 * MAX_STAGES),
-                 bar_done = smem_u32(bars + 4 + 3 * MAX_STAGES);
+                 bar_done = smem_u32(bars + 4 + 3 * MAX_STAGES), bar_end = bar_done + 8;  // bar_end: of a CTA that gave up
 
   if (tid == 0) {
     *dead = 0;
@@ -278,6 +260,7 @@ qgemm_tc_kernel(const TcArgs a) {
       mbar_init(bar_free + 8 * i, 1);
     }
     mbar_init(bar_done, 1);
+    mbar_init(bar_end, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -296,24 +279,23 @@ qgemm_tc_kernel(const TcArgs a) {
   constexpr int blocks_per_group = (TYPE == FB200_Q4_K || TYPE == FB200_Q6_K ? 256 : 128) / BK;
   const int ngr = a.ngroups, nblocks = ngr * blocks_per_group;
 
+  int issued = 0;  // requests of a loader
   if (warp < T::DQ_WARPS) {
     // ---- conversion: warp w turns row-tile w of each K block into fp16 operand rows
     const bool mine = has_tile(warp);
     uint8_t* const a_rows = opnd + (warp >> 3) * A_HALF;
     int s = 0, round = 0;
-    bool alive = true;
-    for (int kg = 0; kg < ngr && alive; ++kg) {
+    for (int kg = 0; kg < ngr; ++kg) {
       const int rb = kg & 1;
-      alive = tc_wait(bar_raw_full + 8 * rb, (uint32_t)((kg >> 1) & 1), dead, a.status);
-      if (!alive) break;
+      // (the warp leaves together: its lanes meet in the shuffles of the conversion)
+      if (!w_wait(bar_raw_full + 8 * rb, (uint32_t)((kg >> 1) & 1), dead, a.status)) break;
       const uint8_t* tg = raw + rb * raw_bytes + warp * a.raw_stride;
       RowScales S;
       if (mine) prepare_scales<TYPE>(tg, lane >> 2, lane & 3, S);
 #pragma unroll
       for (int b = 0; b < blocks_per_group; ++b) {
-        // the stage is free once the MMAs of its previous use have read it
-        if (round > 0) alive = tc_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status);
-        if (!alive) break;
+        // the stage is free once the MMAs of its previous use have read it (or a role gave up, and nothing of this is stored)
+        if (round > 0) x_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status);
         uint8_t* abuf = a_rows + s * T::STAGE;
         if (mine) {
           dequant_chunk<TYPE>(tg, 2 * b, lane, S, abuf, warp & 7, 0);
@@ -332,9 +314,9 @@ qgemm_tc_kernel(const TcArgs a) {
     if (lane == 0) {
       int ntile_here = 0;
       for (int i = 0; i < T::DQ_WARPS; ++i) ntile_here += has_tile(i) ? 1 : 0;
-      for (int kg = 0; kg < ngr; ++kg) {
+      for (int kg = 0; kg < ngr; ++kg, ++issued) {
         const int rb = kg & 1;
-        if (kg >= 2 && !tc_wait(bar_raw_free + 8 * rb, (uint32_t)(((kg >> 1) - 1) & 1), dead, a.status)) break;
+        if (kg >= 2 && !x_wait(bar_raw_free + 8 * rb, (uint32_t)(((kg >> 1) - 1) & 1), dead, a.status)) break;
         mbar_expect_tx(bar_raw_full + 8 * rb, (uint32_t)(ntile_here * a.tgb));
         for (int i = 0; i < T::DQ_WARPS; ++i)
           if (has_tile(i))
@@ -347,8 +329,8 @@ qgemm_tc_kernel(const TcArgs a) {
     if (lane == 0) {
       const __half* src = a.xh + (size_t)blockIdx.y * nblocks * (BM * BK);
       int s = 0, round = 0;
-      for (int blk = 0; blk < nblocks; ++blk) {
-        if (round > 0 && !tc_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status)) break;
+      for (int blk = 0; blk < nblocks; ++blk, ++issued) {
+        if (round > 0 && !x_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status)) break;
         mbar_expect_tx(bar_b_full + 8 * s, (uint32_t)T::B_BYTES);
         bulk_g2s(smem_u32(opnd + s * T::STAGE + T::A_BYTES), src + (size_t)blk * (BM * BK), (uint32_t)T::B_BYTES,
                  bar_b_full + 8 * s);
@@ -361,8 +343,8 @@ qgemm_tc_kernel(const TcArgs a) {
       int s = 0, round = 0;
       bool alive = true;
       for (int blk = 0; blk < nblocks; ++blk) {
-        alive = tc_wait(bar_a_full + 8 * s, (uint32_t)(round & 1), dead, a.status) &&
-                tc_wait(bar_b_full + 8 * s, (uint32_t)(round & 1), dead, a.status);
+        alive = x_wait(bar_a_full + 8 * s, (uint32_t)(round & 1), dead, a.status) &&
+                x_wait(bar_b_full + 8 * s, (uint32_t)(round & 1), dead, a.status);
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t sa = smem_u32(opnd + s * T::STAGE), sb = sa + T::A_BYTES;
@@ -381,9 +363,10 @@ qgemm_tc_kernel(const TcArgs a) {
 
   // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (weight rows) of one half and one
   // half of that half's columns
+  const bool stores = warp < T::DQ_WARPS && __all_sync(0xFFFFFFFFu, x_wait(bar_done, 0u, dead, a.status) && !*dead);
   if (NH == 2 && a.pair_tiles) {
     // SwiGLU: the gate and the up value of an output sit in the same TMEM lane, BM columns apart
-    if (warp < T::DQ_WARPS && tc_wait(bar_done, 0u, dead, a.status)) {
+    if (stores) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int n = n0 + 32 * (warp & 3) + lane, n_out = a.pair_tiles * 16;
       const int cbase = (BM / 4) * (warp >> 2);
@@ -405,7 +388,7 @@ qgemm_tc_kernel(const TcArgs a) {
         }
       }
     }
-  } else if (warp < T::DQ_WARPS && tc_wait(bar_done, 0u, dead, a.status)) {
+  } else if (stores) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int part = warp >> 2, h = part >> 1;
     const int n = n0 + h * BN + 32 * (warp & 3) + lane;
@@ -438,6 +421,17 @@ qgemm_tc_kernel(const TcArgs a) {
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*dead) {  // a role gave up: copies and MMAs in flight are waited for, with a limit, before shared and tensor memory are free
+    if (lane == 0 && warp == T::DQ_WARPS) {
+      for (int i = max(0, issued - 2); i < issued; ++i) x_drain(bar_raw_full + 8 * (i & 1), (uint32_t)((i >> 1) & 1));
+    } else if (lane == 0 && warp == T::DQ_WARPS + 1) {
+      for (int i = max(0, issued - a.stages); i < issued; ++i) x_drain(bar_b_full + 8 * (i % a.stages), (uint32_t)((i / a.stages) & 1));
+    } else if (lane == 0 && warp == T::DQ_WARPS + 2) {
+      tc_commit(bar_end);
+      x_drain(bar_end, 0);
+    }
+    __syncthreads();
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(T::TMEM_COLS) : "memory");
 }
