@@ -121,8 +121,8 @@ dense_tc_kernel(const DenseTcArgs a, const __grid_constant__ CUtensorMap wmap, c
   } else {
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .., columns of one half of the activation rows
     const int quad = warp & 3, ch = warp >> 2;
-    x_wait(done, 0, dead, a.status);
-    if (*dead) x_drain(done, 0);
+    // (by a vote: the tensor memory loads behind it are for whole warps)
+    if (!__all_sync(0xFFFFFFFFu, x_wait(done, 0, dead, a.status) && !*dead)) x_drain(done, 0);
     else {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tl = tmem + ((uint32_t)(32 * quad) << 16);
