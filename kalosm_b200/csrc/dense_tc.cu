@@ -285,9 +285,16 @@ int fb200_dense_gemm_tc(fb200_device* dev, const fb200_dense_job& j) {
   const Cand cands[] = {{128, 2, 0.62}, {128, 1, 0.38}, {64, 2, 0.42}, {64, 1, 0.24}, {32, 2, 0.36}, {32, 1, 0.19}};
   int pick = 0;
   double best = 1e31;
+  // FB200_DENSE_TILE="BM,NH": "256,2" / "256,1" pairs with 256 / 128 weight rows, else single CTAs. What there is not, or what the
+  // product cannot take, leaves the choice to the model
+  int fbm = 0, fnh = 0;
+  if (const char* cfg = getenv("FB200_DENSE_TILE"))
+    if (sscanf(cfg, "%d,%d", &fbm, &fnh) != 2) fbm = 0;
+  if (fbm == 256 && (fnh == 1 || fnh == 2)) return fb200_dense_gemm_pair(dev, j, 128 * fnh);
   for (int i = 0; i < 6; ++i) {
     const double c = cost(cands[i].bm, cands[i].nh, cands[i].tile);
     if (c < best) { best = c; pick = i; }
+    if (c < 1e30 && fbm == cands[i].bm && fnh == cands[i].nh) { best = 0; pick = i; break; }
   }
   const double c256 = pair_cost(256, 0.36), c128 = pair_cost(128, 0.26);
   if (std::min(c256, c128) < best) return fb200_dense_gemm_pair(dev, j, c256 <= c128 ? 256 : 128);

@@ -609,12 +609,17 @@ bool tc_shape(const fb200_device* dev, const fb200_qmatrix* w, const TileGeom& g
   return true;
 }
 
-// FB200_TC_TILE="256,2" / "256,1": pairs with 256 / 128 weight rows; "128,..": single CTAs
-bool tc_forced(const TcShape& sh) {
+// FB200_TC_TILE="BM,NH" or "BM,NH,SPLIT": "256,2" / "256,1" pairs with 256 / 128 weight rows, "128,2" single CTAs, in SPLIT ranges
+// of K (1 if not given). A combination that there is not, or that the product cannot take, leaves the choice to the model.
+struct TcForce { int nw = -1, split = 1; };  // nw < 0: nothing is forced
+TcForce tc_force() {
+  TcForce f;
   int bm = 0, nh = 0;
   const char* cfg = getenv("FB200_TC_TILE");
-  if (!cfg || sscanf(cfg, "%d,%d", &bm, &nh) != 2) return true;
-  return sh.split == 1 && sh.nw == (bm == 256 ? 128 * nh : 0);
+  if (!cfg || sscanf(cfg, "%d,%d,%d", &bm, &nh, &f.split) < 2) return f;
+  if (bm == 256 && (nh == 1 || nh == 2)) f.nw = 128 * nh;
+  else if (bm == SINGLE_BM && nh == NH) f.nw = 0;
+  return f;
 }
 
 bool tc_covers(const fb200_qmatrix* w, const float* x, size_t m, TileGeom* geo) {
@@ -748,15 +753,19 @@ int fb200_qgemm(fb200_device* dev, const fb200_qmatrix* w, const float* x, size_
   const bool may_split = !no_split && !swiglu && w->n % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(r1) | reinterpret_cast<uintptr_t>(r2)) & 15) == 0;
   TcShape best, whole;  // whole: the best without a split
+  const TcForce force = tc_force();
   for (int split = 1; split <= (may_split ? 4 : 1); split *= 2) {
     if (split > 1 && (w->k / split < 2048 || w->ngroups < 2 * split)) break;
-    for (int nw = 256; nw >= (split > 1 ? 128 : 0); nw -= 128) {
+    bool done = false;
+    for (int nw = 256; nw >= (split > 1 ? 128 : 0) && !done; nw -= 128) {
       TcShape sh;
       sh.nw = nw; sh.split = split;
-      if (!tc_forced(sh) || !tc_shape(dev, w, geo, m, swiglu, &sh)) continue;
-      if (!best.ctas || sh.ns < (split > 1 ? 0.9 : 1.0) * best.ns) best = sh;
+      if (!tc_shape(dev, w, geo, m, swiglu, &sh)) continue;
+      done = nw == force.nw && split == force.split;
+      if (done || !best.ctas || sh.ns < (split > 1 ? 0.9 : 1.0) * best.ns) best = sh;
     }
     if (split == 1) whole = best;
+    if (done) break;
   }
   if (!best.ctas) return 1;
   int rc = tc_reserve(dev, m, w->k);  // what the product needs comes before what it can do without

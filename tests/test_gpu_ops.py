@@ -151,7 +151,10 @@ def test_attention_prefill_and_gqa(dev, shape):
 @pytest.mark.parametrize("shape", [(1, 32, 8, 512, 512, 128, True), (2, 8, 2, 100, 100, 64, True),
                                    (1, 8, 8, 96, 300, 128, True), (1, 4, 4, 70, 200, 64, False),
                                    (1, 32, 8, 33, 1000, 128, True), (1, 4, 1, 64, 64, 128, True),
-                                   (1, 2, 2, 65, 129, 64, True), (1, 3, 1, 64, 64, 64, True), (2, 6, 2, 257, 300, 64, True), (1, 40, 8, 700, 641 + 700, 64, False)])
+                                   (1, 2, 2, 65, 129, 64, True), (1, 3, 1, 64, 64, 64, True), (2, 6, 2, 257, 300, 64, True), (1, 40, 8, 700, 641 + 700, 64, False),
+                                   # heads of 64 with fewer than 256 queries: the tcgen05 kernel from 512 keys on
+                                   (1, 3, 1, 64, 513, 64, True), (1, 3, 1, 64, 512, 64, False), (2, 4, 2, 129, 1500, 64, True),
+                                   (1, 5, 5, 255, 511, 64, True), (1, 2, 1, 200, 3000, 64, False)])
 def test_prefill_attention_tensor_cores(dev, shape):
     # 32 or more query positions, no mask or causal: the tensor-core kernel (fp16 operands, fp32
     # accumulation: 2e-3 relative L2 against the f32 oracle). The cache is larger than the valid

@@ -91,9 +91,9 @@ def test_q_mat_mul_batches(dev, tname, m):
 
 
 @pytest.mark.parametrize("tname", list(TYPES))
-@pytest.mark.parametrize("tile", ["128,1", "256,1", "128,2", "256,2", ""])
+@pytest.mark.parametrize("tile", ["256,1", "128,2", "256,2", ""])
 def test_prefill_product_tensor_cores(dev, tname, tile, monkeypatch):
-    # more than 32 rows: the tcgen05 kernel, every CTA tile shape (activation rows, 128-row weight
+    # more than 32 rows: the tcgen05 kernels, every tile shape (activation rows, 128-row weight
     # halves; "" = the cost model's choice), ragged N and M, plain / residual / SwiGLU epilogues
     monkeypatch.setenv("FB200_TC_TILE", tile)
     ty = TYPES[tname]
@@ -142,6 +142,21 @@ def test_prefill_product_cta_pairs(dev, tname, tile, m, n, k, monkeypatch):
         h = dev.tensor(x).q_mat_mul(w, epilogue=kb.EPI_SWIGLU).as_slice()
         g, u = exp[:, : n // 2], exp[:, n // 2:]
         assert F.rel_l2(h, g / (1.0 + np.exp(-g)) * u) < TOL
+    assert dev.status() == 0
+
+
+@pytest.mark.parametrize("tname", ["q4k", "q8_0"])
+@pytest.mark.parametrize("k", [14336, 14592, 20480])
+def test_prefill_product_long_rows(dev, tname, k):
+    # the packing kernel holds 14336 values of a row in registers and reads the rest again
+    ty = TYPES[tname]
+    n, m = 96, 41
+    raw = weights(51, n, k, ty)
+    w = kb.QMatrix.from_raw_bytes(dev, (n, k), raw, ty)
+    x = activations(k, m, k)
+    x[:, -1] *= 50.0  # the largest value of a row decides its scale
+    exp = x.astype(np.float64) @ w.dequantize().as_slice().astype(np.float64).T
+    assert F.rel_l2(dev.tensor(x).q_mat_mul(w).as_slice(), exp) < TOL
     assert dev.status() == 0
 
 
@@ -386,9 +401,11 @@ def test_q5_epilogues(dev):
 
 
 @pytest.mark.parametrize("tname", ["q4k", "q6k", "q8_0"])
-def test_prefill_product_split_k(dev, tname):
-    # long rows, few tiles: the tcgen05 product cuts K into ranges (grid.z) and a second kernel adds the
-    # partial products in range order, together with the residual or bias rows; ragged N and M
+@pytest.mark.parametrize("tile", ["", "256,1,2", "256,2,2", "256,2,4"])
+def test_prefill_product_split_k(dev, tname, tile, monkeypatch):
+    # long rows, few tiles: the tcgen05 product cuts K into ranges side by side and a second kernel adds the partial products
+    # in range order, together with the residual or bias rows; ragged N and M, the cost model's choice and either tile width
+    monkeypatch.setenv("FB200_TC_TILE", tile)
     ty = TYPES[tname]
     n, k = 1000, 8192
     raw = weights(61, n, k, ty)
@@ -400,6 +417,10 @@ def test_prefill_product_split_k(dev, tname):
         y = xt.q_mat_mul(w).as_slice()
         assert F.rel_l2(y, exp) < TOL, (tname, m, F.rel_l2(y, exp))
         assert np.array_equal(y, xt.q_mat_mul(w).as_slice())
+        if tile:  # partial sums are rounded apart: the split did run
+            monkeypatch.setenv("FB200_TC_TILE", tile[:5])
+            assert not np.array_equal(y, xt.q_mat_mul(w).as_slice())
+            monkeypatch.setenv("FB200_TC_TILE", tile)
         r1, r2 = activations(610 + m, m, n), activations(620 + m, m, n)
         y = xt.q_mat_mul(w, epilogue=kb.EPI_RESIDUAL, r1=dev.tensor(r1), r2=dev.tensor(r2)).as_slice()
         assert F.rel_l2(y, (exp + r1) + r2) < TOL

@@ -115,6 +115,25 @@ def test_feed_forward_alone(dev, dtype):
     check(dev, cfg, w, toks(cfg, 300), dtype, [[300], [36, 1, 200, 2]])
 
 
+@pytest.mark.parametrize("tile", ["256,1", "256,2"])
+def test_layers_on_cta_pairs(dev, tile, monkeypatch):
+    # the pair kernel's other forms at odd widths: gelu feed-forward rows with an operand of their own, bias, factor and residual,
+    # the loop's input product, the softcap of several sequences' logits
+    monkeypatch.setenv("FB200_DENSE_TILE", tile)
+    cfg = V.config([V.attention(mlp=201), V.parallel(mlp=41), V.attention(mlp=300)], width=75, vocab=131, loop=(1, 2, 2), cap=2.0)
+    w = V.weights(cfg, 32)
+    check(dev, cfg, w, toks(cfg, 300), "bfloat16", [[300], [130, 20, 150]])
+    m = V.gpu_model(dev, cfg, w, "bfloat16", max_batch=3)
+    tokens = np.stack([toks(cfg, 60, seed) for seed in (1, 2, 3)])
+    want = [V.oracle_logits(cfg, w, t) for t in tokens]
+    tol = max(V.tolerance(cfg, w, t, x, "bfloat16") for t, x in zip(tokens, want))
+    got = m.forward(tokens)[0]
+    for g, x in zip(got, want):
+        assert U.err(g[None], x[-1:]) < tol
+    assert dev.status() == 0
+    m.free()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("loop", [None, (0, 3, 2), (0, 1, 1), (2, 3, 4), (1, 3, 3)], ids=str)
 def test_loops(dev, dtype, loop):
