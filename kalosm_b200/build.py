@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libfusor_b200.so")
 SOURCES = ["api.cu", "repack.cu", "qgemv.cu", "qgemv1.cu", "q5gemv.cu", "dense.cu", "dense_tc.cu", "dense_pair.cu", "qgemm.cu", "qgemm_pair.cu", "ops.cu", "attention.cu", "attn_prefill.cu", "attn_prefill_tc.cu", "attn_decode_tc.cu",
            "fused_step.cu", "llama.cu", "hybrid.cu", "delta_rule.cu", "latent_attn.cu", "latent_prefill.cu", "group_attn.cu", "linear_attn.cu", "linear_prefill.cu", "comm.cu", "sampling.cu"]
-HEADERS = ["common.cuh", "formats.cuh", "qgemv_common.cuh", "qgemv1_groups.cuh", "packed_act.cuh", "qgemm_pair.cuh",
+HEADERS = ["common.cuh", "formats.cuh", "qgemv_common.cuh", "qgemv1_groups.cuh", "packed_act.cuh", "qgemm_pair.cuh", "half_weights.cuh",
            "attn_decode.cuh", "attn_mma.cuh", "qgemv1_groups2.cuh", "fused_step.cuh", "decoder.cuh", "dense.cuh", "mixers.cuh", "state_columns.cuh", "tcgen05.cuh", os.path.join("..", "..", "include", "fusor_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr"]

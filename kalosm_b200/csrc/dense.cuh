@@ -55,6 +55,12 @@ __device__ __forceinline__ float fb_gelu_tanh(float v) {
   return v / (1.0f + expf(-2.0f * u));
 }
 
+// The same with the fast exponential and division, for results that are stored as bf16
+__device__ __forceinline__ float fb_gelu_tanh_fast(float v) {
+  const float u = 0.7978845608028654f * fmaf(0.044715f * v * v, v, v);
+  return __fdividef(v, 1.0f + __expf(-2.0f * u));
+}
+
 // cuTensorMapEncodeTiled of the driver, looked up once (the library does not link against libcuda); a 2-D map of
 // 2-byte elements, 128-byte swizzle, boxes of 64 columns x box_rows rows, zeros outside.
 struct CUtensorMap_st;

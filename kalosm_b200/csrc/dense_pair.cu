@@ -1,9 +1,10 @@
 // Products of many activation rows with BF16 weights on CTA pairs: tcgen05.mma.cta_group::2, 256 activation rows by NW weight rows
 // per pair, persistent, two accumulators per CTA.
 //
-// Bound: tensor cores (2 M N K flops). A single CTA with a tile of 256 x 256 (dense_tc.cu) leaves the tensor cores idle during its epilogue and has
-// half as many operand stages for the same tile; a pair writes one tile while it multiplies the next. The activations are in the M role, so that gate and up rows of an output
-// (halves of the weight tile, one per CTA) meet in one TMEM lane, NW / 2 columns apart.
+// Bound: tensor cores (2 M N K flops). A single CTA with a tile of 256 x 256 left the tensor cores idle during its epilogue and had
+// half as many operand stages for the same tile (8192 rows of 14336 x 2048: 486 us, 343 here); a pair writes one tile while it
+// multiplies the next. The activations are in the M role, so that gate and up rows of an output (halves of the weight tile, one
+// per CTA) meet in one TMEM lane, NW / 2 columns apart.
 //  * copy requester (one thread per CTA): a stage is 64 values of K: boxes of 64 columns by 128 activation rows and by NW / 2
 //    weight rows, by tensor TMA with 128-byte swizzle; rows and columns outside the matrices arrive as zeros. The copies of both CTAs
 //    are counted on the even CTA's barrier (a message from the odd CTA would lengthen every refill);
@@ -38,11 +39,6 @@ struct DPairArgs {
   float alpha, softcap;
   int* status;
 };
-
-// K-major operand with 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart, descriptor version 1
-__device__ __forceinline__ uint64_t dp_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 
 __device__ __forceinline__ void dp_put(float* p, uint32_t v) { *p = __uint_as_float(v); }
 __device__ __forceinline__ void dp_put(__nv_bfloat16* p, uint32_t v) { *p = __float2bfloat16(__uint_as_float(v)); }
@@ -162,10 +158,7 @@ dense_pair_kernel(const DPairArgs a, const __grid_constant__ CUtensorMap wmap, c
               }
             } else {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float t = __uint_as_float(v[i]), w = 0.7978845608028654f * fmaf(0.044715f * t * t, t, t);
-                v[i] = __float_as_uint(__fdividef(t, 1.0f + __expf(-2.0f * w)));
-              }
+              for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(fb_gelu_tanh_fast(__uint_as_float(v[i])));
             }
             dp_store<__nv_bfloat16>(a.z + rows[0] * a.ldz + col0, a.z + rows[1] * a.ldz + col0, v, whole, mrow, a.m, col0, n_out, a.vec_z);
             continue;
@@ -248,7 +241,7 @@ dense_pair_kernel(const DPairArgs a, const __grid_constant__ CUtensorMap wmap, c
     int s = 0, n = 0;
     uint32_t parity = 0, ready = 0;
     bool alive = rank == 0;
-    const uint64_t adesc0 = dp_desc(smem_u32(sm)), bdesc0 = dp_desc(smem_u32(sm) + DP_A_BYTES);
+    const uint64_t adesc0 = x_desc_rows(smem_u32(sm)), bdesc0 = x_desc_rows(smem_u32(sm) + DP_A_BYTES);
     for (int item = pair; item < items && alive; item += npairs, ++n) {
       const int buf = n & 1;
       if (n >= 2) {

@@ -48,10 +48,6 @@ struct DenseTcArgs {
   int* status;
 };
 
-// K-major operand with 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart, descriptor version 1
-__device__ __forceinline__ uint64_t dt_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 template <int BM, int NH>
 __global__ void __launch_bounds__(TC_THREADS, BM <= 64 ? 2 : 1)
 dense_tc_kernel(const DenseTcArgs a, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap) {
@@ -112,7 +108,7 @@ dense_tc_kernel(const DenseTcArgs a, const __grid_constant__ CUtensorMap wmap, c
         for (int k = 0; k < TC_BK / 16; ++k)  // 32 bytes further inside the 128-byte rows per K step
 #pragma unroll
           for (int h = 0; h < NH; ++h)
-            x_mma(tmem + (uint32_t)(h * BM), dt_desc(st + h * TC_BN * TC_BK * 2 + k * 32), dt_desc(st + S::A_BYTES + k * 32), S::IDESC,
+            x_mma(tmem + (uint32_t)(h * BM), x_desc_rows(st + h * TC_BN * TC_BK * 2 + k * 32), x_desc_rows(st + S::A_BYTES + k * 32), S::IDESC,
                    (kb | k) ? 1u : 0u);
         x_commit(empty + 8 * s);
       }
@@ -156,8 +152,7 @@ dense_tc_kernel(const DenseTcArgs a, const __grid_constant__ CUtensorMap wmap, c
 #pragma unroll
               for (int i = 0; i < 16; ++i)
                 if (i < lim) {
-                  const float t = __uint_as_float(v[i]), u = 0.7978845608028654f * fmaf(0.044715f * t * t, t, t);
-                  zp[(size_t)i * a.ldz] = __float2bfloat16(__fdividef(t, 1.0f + __expf(-2.0f * u)));
+                  zp[(size_t)i * a.ldz] = __float2bfloat16(fb_gelu_tanh_fast(__uint_as_float(v[i])));
                 }
               continue;
             }

@@ -6,12 +6,12 @@
 // kernels would re-read W once per 32 rows.
 //
 // This file packs the activations, chooses how a product runs, and holds the kernel of single CTAs, which is left for
-// few rows of wide matrices; most products run on CTA pairs (qgemm_pair.cu). In the kernel here a CTA computes a tile of NH x 128 weight rows by BM = 128 activation rows of
-// Y^T = W . X^T; the fp32 accumulators (NH x BM columns of 128 lanes) live in TMEM. The roles
-// are coupled only by mbarriers, there is no CTA-wide barrier in the main loop:
+// few rows of wide matrices; most products run on CTA pairs (qgemm_pair.cu). In the kernel here a CTA computes a tile of
+// 256 weight rows by 128 activation rows of Y^T = W . X^T; the fp32 accumulators (two halves of 128 lanes x 128 columns)
+// live in TMEM. The roles are coupled only by mbarriers, there is no CTA-wide barrier in the main loop:
 //  * weight loader (one thread): W stays quantised in HBM; the raw tile-groups of the CTA's
-//    8 NH row-tiles for one K group come by 1-D TMA bulk copies, two K groups in flight.
-//  * conversion warps (8 NH, one per row-tile): dequantise to fp16 in registers (byte -> 1024 +
+//    16 row-tiles for one K group come by 1-D TMA bulk copies, two K groups in flight.
+//  * conversion warps (16, one per row-tile): dequantise to fp16 in registers (byte -> 1024 +
 //    byte by a byte permute, exact subtraction, one fused multiply-add with block scale and
 //    offset) and store into the A operand stage in the canonical K-major core-matrix layout of
 //    the MMA (8 rows x 16 bytes per core matrix, no swizzle); a proxy fence, then one arrive per
@@ -19,8 +19,8 @@
 //  * activation loader (one thread): X is converted once per call to fp16 rows scaled by a power
 //    of two and stored tile by tile in the same operand layout, so a B stage is one contiguous
 //    bulk copy.
-//  * MMA issuer (one thread): waits for "A full" and "B full", issues 4 NH tcgen05.mma (M = 128,
-//    N = BM, K = 16, kind::f16, fp32 accumulate) per 64-wide K block; tcgen05.commit on the
+//  * MMA issuer (one thread): waits for "A full" and "B full", issues 8 tcgen05.mma (M = 128,
+//    N = 128, K = 16, kind::f16, fp32 accumulate) per 64-wide K block; tcgen05.commit on the
 //    stage's "free" barrier hands the stage back to both producers (2..4 stages, as many as fit
 //    beside the raw buffers).
 //  * Epilogue: tcgen05.ld brings the accumulator out of TMEM (each warp its 32 lanes), rows are
@@ -36,6 +36,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "half_weights.cuh"
 #include "qgemm_pair.cuh"
 #include "tcgen05.cuh"
 
@@ -43,8 +44,9 @@ int fb200_ensure(fb200_device* dev, void** buf, size_t* cur, size_t bytes);
 
 namespace {
 
-constexpr int BN = 128;  // weight rows per MMA (M of the MMA); a CTA tile holds NH such halves
-constexpr int SINGLE_BM = 128;  // activation rows per CTA tile (N of the MMA), and of a packed activation tile
+constexpr int BN = 128;  // weight rows per MMA (M of the MMA)
+constexpr int NH = 2;    // such halves in a CTA tile
+constexpr int BM = 128;  // activation rows per CTA tile (N of the MMA), and of a packed activation tile
 constexpr int BK = 64;   // K elements per operand stage (four K = 16 MMAs)
 constexpr int A_SBO = (BK / 8) * 128 + 64;        // A operand: bytes between 8-row groups, padded by half a
                                                   // core matrix so that rows g and g + 8 fall into different banks
@@ -54,17 +56,12 @@ constexpr int CORE_SBO = (BK / 8) * 128;          // B operand: bytes between 8-
 constexpr int MAX_STAGES = 4;
 constexpr int TAIL_BYTES = 256;                   // barriers, TMEM slot, give-up flag
 constexpr int SMEM_BUDGET = 227 * 1024;
-template <int BM, int NH>
-struct Tc {
-  static constexpr int A_BYTES = NH * A_HALF;               // one A stage
-  static constexpr int B_BYTES = BM * BK * 2;               // one B stage
-  static constexpr int STAGE = A_BYTES + B_BYTES;
-  static constexpr int TMEM_COLS = NH * BM;                 // fp32 accumulator columns
-  static constexpr int DQ_WARPS = 8 * NH;                   // one warp per 16-row tile
-  static constexpr int THREADS = (DQ_WARPS + 3) * 32;       // + weight loader, activation loader, MMA issuer
-  // instruction descriptor: fp32 accumulator, fp16 A and B, both K-major, N = BM, M = BN
-  static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
-};
+constexpr int A_BYTES = NH * A_HALF, B_BYTES = BM * BK * 2, STAGE = A_BYTES + B_BYTES;  // operands of a stage
+constexpr int TMEM_COLS = NH * BM;            // fp32 accumulator columns
+constexpr int DQ_WARPS = 8 * NH;              // one warp per 16-row tile
+constexpr int THREADS = (DQ_WARPS + 3) * 32;  // + weight loader, activation loader, MMA issuer
+// instruction descriptor: fp32 accumulator, fp16 A and B, both K-major, N = BM, M = BN
+constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
 
 struct TcArgs {
   const uint8_t* w;      // tiled weights
@@ -77,49 +74,13 @@ struct TcArgs {
   int M, N, K;
   int ngroups, ntiles, type, tgb, group_elems;
   int stages, raw_stride;  // operand stages that fit beside the raw buffers; bytes per raw tile-group slot
-  int pair_tiles;          // SwiGLU (NH = 2): half 0 = gate rows, half 1 = up rows pair_tiles row-tiles further;
+  int pair_tiles;          // SwiGLU: half 0 = gate rows, half 1 = up rows pair_tiles row-tiles further;
                            // y[M, N / 2] = silu(gate) * up. 0 = plain product
   int* status;
 };
 
-__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-__device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t lds4(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ uint4 lds16(const uint8_t* p) { return *reinterpret_cast<const uint4*>(p); }
-
-// Four unsigned bytes -> four fp16 values ((1024 + byte) - centre) * scale + offset, as two half2.
-__device__ __forceinline__ uint2 deq4(uint32_t w, __half2 centre, __half2 scale, __half2 offset) {
-  const __half2 v01 = __hsub2(u2h(__byte_perm(w, 0x64646464u, 0x4140)), centre);
-  const __half2 v23 = __hsub2(u2h(__byte_perm(w, 0x64646464u, 0x4342)), centre);
-  return make_uint2(h2u(__hfma2(v01, scale, offset)), h2u(__hfma2(v23, scale, offset)));
-}
-
-// Shared-memory matrix descriptor of a K-major operand without swizzle: start address, leading
-// (K direction) and stride (row-group direction) byte offsets in 16-byte units, descriptor
-// version 1.
-__device__ __forceinline__ uint64_t operand_desc(uint32_t saddr, uint32_t sbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(CORE_LBO >> 4) << 16) |
-         ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr) : "memory");
-}
 
 // Row-tile `tile` of one K group: the four registers of 32-element chunk c for lane (g, t) --
 // bytes of rows g / g + 8, elements 4t.. and 16 + 4t.. -- dequantised and stored into operand
@@ -231,14 +192,13 @@ __device__ __forceinline__ void dequant_chunk(const uint8_t* tg, int c, int lane
   }
 }
 
-template <int BM, int NH, int TYPE>
-__global__ void __launch_bounds__(Tc<BM, NH>::THREADS, 1)
+template <int TYPE>
+__global__ void __launch_bounds__(THREADS, 1)
 qgemm_tc_kernel(const TcArgs a) {
-  using T = Tc<BM, NH>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int raw_bytes = T::DQ_WARPS * a.raw_stride;
+  const int raw_bytes = DQ_WARPS * a.raw_stride;
   uint8_t* opnd = smem;                                   // [stage][A halves | B]
-  uint8_t* raw = smem + a.stages * T::STAGE;              // [2][DQ_WARPS tile-groups]
+  uint8_t* raw = smem + a.stages * STAGE;              // [2][DQ_WARPS tile-groups]
   uint64_t* bars = reinterpret_cast<uint64_t*>(raw + 2 * raw_bytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -252,10 +212,10 @@ qgemm_tc_kernel(const TcArgs a) {
     *dead = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_raw_full + 8 * i, 1);
-      mbar_init(bar_raw_free + 8 * i, T::DQ_WARPS);
+      mbar_init(bar_raw_free + 8 * i, DQ_WARPS);
     }
     for (int i = 0; i < MAX_STAGES; ++i) {
-      mbar_init(bar_a_full + 8 * i, T::DQ_WARPS);
+      mbar_init(bar_a_full + 8 * i, DQ_WARPS);
       mbar_init(bar_b_full + 8 * i, 1);
       mbar_init(bar_free + 8 * i, 1);
     }
@@ -264,7 +224,7 @@ qgemm_tc_kernel(const TcArgs a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(T::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -280,7 +240,7 @@ qgemm_tc_kernel(const TcArgs a) {
   const int ngr = a.ngroups, nblocks = ngr * blocks_per_group;
 
   int issued = 0;  // requests of a loader
-  if (warp < T::DQ_WARPS) {
+  if (warp < DQ_WARPS) {
     // ---- conversion: warp w turns row-tile w of each K block into fp16 operand rows
     const bool mine = has_tile(warp);
     uint8_t* const a_rows = opnd + (warp >> 3) * A_HALF;
@@ -296,7 +256,7 @@ qgemm_tc_kernel(const TcArgs a) {
       for (int b = 0; b < blocks_per_group; ++b) {
         // the stage is free once the MMAs of its previous use have read it (or a role gave up, and nothing of this is stored)
         if (round > 0) x_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status);
-        uint8_t* abuf = a_rows + s * T::STAGE;
+        uint8_t* abuf = a_rows + s * STAGE;
         if (mine) {
           dequant_chunk<TYPE>(tg, 2 * b, lane, S, abuf, warp & 7, 0);
           dequant_chunk<TYPE>(tg, 2 * b + 1, lane, S, abuf, warp & 7, 1);
@@ -309,36 +269,36 @@ qgemm_tc_kernel(const TcArgs a) {
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_raw_free + 8 * rb);
     }
-  } else if (warp == T::DQ_WARPS) {
+  } else if (warp == DQ_WARPS) {
     // ---- weight loader: raw tile-groups of one K group, two groups in flight
     if (lane == 0) {
       int ntile_here = 0;
-      for (int i = 0; i < T::DQ_WARPS; ++i) ntile_here += has_tile(i) ? 1 : 0;
+      for (int i = 0; i < DQ_WARPS; ++i) ntile_here += has_tile(i) ? 1 : 0;
       for (int kg = 0; kg < ngr; ++kg, ++issued) {
         const int rb = kg & 1;
         if (kg >= 2 && !x_wait(bar_raw_free + 8 * rb, (uint32_t)(((kg >> 1) - 1) & 1), dead, a.status)) break;
         mbar_expect_tx(bar_raw_full + 8 * rb, (uint32_t)(ntile_here * a.tgb));
-        for (int i = 0; i < T::DQ_WARPS; ++i)
+        for (int i = 0; i < DQ_WARPS; ++i)
           if (has_tile(i))
             bulk_g2s(smem_u32(raw + rb * raw_bytes + i * a.raw_stride),
                      a.w + ((size_t)tile_of(i) * a.ngroups + kg) * a.tgb, (uint32_t)a.tgb, bar_raw_full + 8 * rb);
       }
     }
-  } else if (warp == T::DQ_WARPS + 1) {
+  } else if (warp == DQ_WARPS + 1) {
     // ---- activation loader: one bulk copy per K block (the tile is stored in operand layout)
     if (lane == 0) {
       const __half* src = a.xh + (size_t)blockIdx.y * nblocks * (BM * BK);
       int s = 0, round = 0;
       for (int blk = 0; blk < nblocks; ++blk, ++issued) {
         if (round > 0 && !x_wait(bar_free + 8 * s, (uint32_t)((round - 1) & 1), dead, a.status)) break;
-        mbar_expect_tx(bar_b_full + 8 * s, (uint32_t)T::B_BYTES);
-        bulk_g2s(smem_u32(opnd + s * T::STAGE + T::A_BYTES), src + (size_t)blk * (BM * BK), (uint32_t)T::B_BYTES,
+        mbar_expect_tx(bar_b_full + 8 * s, (uint32_t)B_BYTES);
+        bulk_g2s(smem_u32(opnd + s * STAGE + A_BYTES), src + (size_t)blk * (BM * BK), (uint32_t)B_BYTES,
                  bar_b_full + 8 * s);
         if (++s == a.stages) { s = 0; ++round; }
       }
     }
   } else {
-    // ---- MMA issuer: 4 NH instructions per K block; the commit frees the stage
+    // ---- MMA issuer: eight instructions per K block; the commit frees the stage
     if (lane == 0) {
       int s = 0, round = 0;
       bool alive = true;
@@ -347,24 +307,24 @@ qgemm_tc_kernel(const TcArgs a) {
                 x_wait(bar_b_full + 8 * s, (uint32_t)(round & 1), dead, a.status);
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sa = smem_u32(opnd + s * T::STAGE), sb = sa + T::A_BYTES;
+        const uint32_t sa = smem_u32(opnd + s * STAGE), sb = sa + A_BYTES;
 #pragma unroll
         for (int h = 0; h < NH; ++h)
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ++ks)
-            tc_mma(tmem_d + (uint32_t)(h * BM), operand_desc(sa + h * A_HALF + ks * 2 * CORE_LBO, A_SBO),
-                   operand_desc(sb + ks * 2 * CORE_LBO, CORE_SBO), T::IDESC, (blk | ks) ? 1u : 0u);
-        tc_commit(bar_free + 8 * s);
+            x_mma(tmem_d + (uint32_t)(h * BM), x_desc(sa + h * A_HALF + ks * 2 * CORE_LBO, CORE_LBO, A_SBO),
+                   x_desc(sb + ks * 2 * CORE_LBO, CORE_LBO, CORE_SBO), IDESC, (blk | ks) ? 1u : 0u);
+        x_commit(bar_free + 8 * s);
         if (++s == a.stages) { s = 0; ++round; }
       }
-      if (alive) tc_commit(bar_done);
+      if (alive) x_commit(bar_done);
     }
   }
 
   // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (weight rows) of one half and one
   // half of that half's columns
-  const bool stores = warp < T::DQ_WARPS && __all_sync(0xFFFFFFFFu, x_wait(bar_done, 0u, dead, a.status) && !*dead);
-  if (NH == 2 && a.pair_tiles) {
+  const bool stores = warp < DQ_WARPS && __all_sync(0xFFFFFFFFu, x_wait(bar_done, 0u, dead, a.status) && !*dead);
+  if (a.pair_tiles) {
     // SwiGLU: the gate and the up value of an output sit in the same TMEM lane, BM columns apart
     if (stores) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -374,8 +334,8 @@ qgemm_tc_kernel(const TcArgs a) {
       for (int i = 0; i < BM / 64; ++i) {
         uint32_t g[16], u[16];
         const uint32_t taddr = tmem_d + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(cbase + 16 * i);
-        tmem_ld16(taddr, g);
-        tmem_ld16(taddr + BM, u);
+        x_ld16(taddr, g);
+        x_ld16(taddr + BM, u);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -397,14 +357,7 @@ qgemm_tc_kernel(const TcArgs a) {
     for (int i = 0; i < BM / 64; ++i) {
       uint32_t v[32];
       const uint32_t taddr = tmem_d + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(h * BM + cbase + 32 * i);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-          "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-            "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-            "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-            "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-          : "r"(taddr) : "memory");
+      x_ld32(taddr, v);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
@@ -422,18 +375,18 @@ qgemm_tc_kernel(const TcArgs a) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (*dead) {  // a role gave up: copies and MMAs in flight are waited for, with a limit, before shared and tensor memory are free
-    if (lane == 0 && warp == T::DQ_WARPS) {
+    if (lane == 0 && warp == DQ_WARPS) {
       for (int i = max(0, issued - 2); i < issued; ++i) x_drain(bar_raw_full + 8 * (i & 1), (uint32_t)((i >> 1) & 1));
-    } else if (lane == 0 && warp == T::DQ_WARPS + 1) {
+    } else if (lane == 0 && warp == DQ_WARPS + 1) {
       for (int i = max(0, issued - a.stages); i < issued; ++i) x_drain(bar_b_full + 8 * (i % a.stages), (uint32_t)((i / a.stages) & 1));
-    } else if (lane == 0 && warp == T::DQ_WARPS + 2) {
-      tc_commit(bar_end);
+    } else if (lane == 0 && warp == DQ_WARPS + 2) {
+      x_commit(bar_end);
       x_drain(bar_end, 0);
     }
     __syncthreads();
   }
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(T::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(TMEM_COLS) : "memory");
 }
 
 // x[M, K] f32 -> fp16 scaled by a power of two per row into (-64, 64), stored as [Mp / 128][K / 64]
@@ -530,11 +483,11 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
   if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);
   const float inv = ldexpf(64.0f, -ex);
   if (tid < PACK_ROWS) xscale[m] = ldexpf(1.0f, ex - 6);
-  uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / SINGLE_BM) * (K / BK) * ((size_t)SINGLE_BM * BK * 2) +
-                      ((m0 % SINGLE_BM) >> 3) * CORE_SBO + (m & 7) * 16;
+  uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / BM) * (K / BK) * ((size_t)BM * BK * 2) +
+                      ((m0 % BM) >> 3) * CORE_SBO + (m & 7) * 16;
   auto store = [&](int c, const float4 (&v)[2]) {
     if (c >= chunks) return;
-    *reinterpret_cast<uint4*>(tile_row + (size_t)(c >> 3) * ((size_t)SINGLE_BM * BK * 2) + (c & 7) * CORE_LBO) =
+    *reinterpret_cast<uint4*>(tile_row + (size_t)(c >> 3) * ((size_t)BM * BK * 2) + (c & 7) * CORE_LBO) =
         make_uint4(h2u(__floats2half2_rn(v[0].x * inv, v[0].y * inv)), h2u(__floats2half2_rn(v[0].z * inv, v[0].w * inv)),
                    h2u(__floats2half2_rn(v[1].x * inv, v[1].y * inv)), h2u(__floats2half2_rn(v[1].z * inv, v[1].w * inv)));
   };
@@ -548,24 +501,22 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
   }
 }
 
-template <int BM, int NH, int TYPE>
+template <int TYPE>
 int launch_tc_type(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, int smem) {
-  using T = Tc<BM, NH>;
   static bool configured[64] = {false};
   if (!configured[dev->ordinal & 63]) {
-    FB_CUDA(dev, cudaFuncSetAttribute(qgemm_tc_kernel<BM, NH, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET));
+    FB_CUDA(dev, cudaFuncSetAttribute(qgemm_tc_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET));
     configured[dev->ordinal & 63] = true;
   }
-  return fb200_launch(dev, qgemm_tc_kernel<BM, NH, TYPE>, dim3(grid_n, grid_m), dim3(T::THREADS), (size_t)smem, false, a);
+  return fb200_launch(dev, qgemm_tc_kernel<TYPE>, dim3(grid_n, grid_m), dim3(THREADS), (size_t)smem, false, a);
 }
 
-template <int BM, int NH>
 int launch_tc(fb200_device* dev, const TcArgs& a, unsigned grid_n, unsigned grid_m, int smem) {
   switch (a.type) {
-    case FB200_Q4_0: return launch_tc_type<BM, NH, FB200_Q4_0>(dev, a, grid_n, grid_m, smem);
-    case FB200_Q8_0: return launch_tc_type<BM, NH, FB200_Q8_0>(dev, a, grid_n, grid_m, smem);
-    case FB200_Q4_K: return launch_tc_type<BM, NH, FB200_Q4_K>(dev, a, grid_n, grid_m, smem);
-    case FB200_Q6_K: return launch_tc_type<BM, NH, FB200_Q6_K>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q4_0: return launch_tc_type<FB200_Q4_0>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q8_0: return launch_tc_type<FB200_Q8_0>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q4_K: return launch_tc_type<FB200_Q4_K>(dev, a, grid_n, grid_m, smem);
+    case FB200_Q6_K: return launch_tc_type<FB200_Q6_K>(dev, a, grid_n, grid_m, smem);
   }
   return 1;
 }
@@ -578,7 +529,6 @@ struct TcShape { int nw = 0, stages = 0, split = 1; size_t ctas = 0; double ns =
 // loop. At 512 rows 28672 x 4096 Q4_K with SwiGLU takes 118 / 121 us on pairs (nw = 256 / 128) and 224 us on single CTAs,
 // 4096 x 14336 Q6_K 124 / 87 / 235 us. Single CTAs win where the pairs need one round more: up to 128 rows of many weight rows
 // (100 rows of 28672 x 4096: 63.6 us, pairs 70.1).
-constexpr int NH = 2;
 double tile_ns(const fb200_qmatrix* w, const TcShape& sh) {
   const double k256 = (double)w->k / 256.0 / sh.split;
   return sh.nw == 256 ? k256 * 1700.0 + 2500.0 : sh.nw ? k256 * 1050.0 + 1500.0 : k256 * 3300.0;
@@ -593,11 +543,11 @@ bool tc_shape(const fb200_device* dev, const fb200_qmatrix* w, const TileGeom& g
     tiles_m = (m + 255) / 256;
     slots = (size_t)dev->sm_count / 2;
   } else {
-    const int raw_stride = (geo.tg_bytes + 127) & ~127, stage = NH * A_HALF + SINGLE_BM * BK * 2;
+    const int raw_stride = (geo.tg_bytes + 127) & ~127, stage = NH * A_HALF + BM * BK * 2;
     sh->stages = std::min(MAX_STAGES, (SMEM_BUDGET - TAIL_BYTES - 2 * 8 * NH * raw_stride) / stage);
     if (sh->stages < 2) return false;
     rows = (size_t)(swiglu ? BN : BN * NH);
-    tiles_m = (m + SINGLE_BM - 1) / SINGLE_BM;
+    tiles_m = (m + BM - 1) / BM;
     slots = (size_t)dev->sm_count;
   }
   sh->ctas = ((n_rows + rows - 1) / rows) * tiles_m * sh->split;
@@ -618,7 +568,7 @@ TcForce tc_force() {
   const char* cfg = getenv("FB200_TC_TILE");
   if (!cfg || sscanf(cfg, "%d,%d,%d", &bm, &nh, &f.split) < 2) return f;
   if (bm == 256 && (nh == 1 || nh == 2)) f.nw = 128 * nh;
-  else if (bm == SINGLE_BM && nh == NH) f.nw = 0;
+  else if (bm == BM && nh == NH) f.nw = 0;
   return f;
 }
 
@@ -693,10 +643,10 @@ int tc_launch(fb200_device* dev, const fb200_qmatrix* w, const TileGeom& geo, co
   a.group_elems = geo.group_elems; a.status = dev->status;
   a.stages = sh.stages; a.raw_stride = raw_stride;
   a.pair_tiles = swiglu ? w->ntiles / 2 : 0;
-  const int smem = sh.stages * (NH * A_HALF + SINGLE_BM * BK * 2) + 2 * 8 * NH * raw_stride + TAIL_BYTES;
+  const int smem = sh.stages * (NH * A_HALF + BM * BK * 2) + 2 * 8 * NH * raw_stride + TAIL_BYTES;
   const size_t rows_per_cta = swiglu ? BN : BN * NH;
   const unsigned gn = (unsigned)((n_rows + rows_per_cta - 1) / rows_per_cta), gm = (unsigned)halves;
-  return launch_tc<SINGLE_BM, NH>(dev, a, gn, gm, smem);
+  return launch_tc(dev, a, gn, gm, smem);
 }
 
 // Scratch of packed rows: fp16 tiles of 128 rows, then the row scales

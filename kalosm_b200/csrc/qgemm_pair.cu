@@ -2,19 +2,19 @@
 // the N role, tcgen05.mma.cta_group::2 with the accumulators in tensor memory.
 //
 // Bound: tensor cores (2 M N K flops). The single-CTA kernel (qgemm.cu) holds W in the M role: a CTA converts 256
-// weight rows for 256 activation rows, its raw buffers leave two operand stages, and every MMA waits for the round trip of
-// one of them. Here a CTA of the pair converts half of the weight rows, and the pair's MMA reads both halves: the same
-// 256 x 256 tile per CTA pair and half costs half of the conversion stores, half of the operand reads of W, and the raw
-// bytes go from global memory straight into the registers of the lane that converts them, so six to eight stages fit.
+// weight rows for 128 activation rows (once 256), its raw buffers leave few operand stages, and every MMA waits for the round
+// trip of one of them. Here a CTA of the pair converts half of the weight rows, and the pair's MMA reads both halves: a tile of
+// 256 x 256 costs a CTA half of the conversion and half of the operand reads of W, and the raw bytes go from global memory
+// straight into the registers of the lane that converts them, so three stages of 128 values of K fit (four with 128 weight rows).
 //
 // The grid is persistent: a pair walks over tiles (activation tiles fastest, so that the pairs that run together share
 // their weight rows in L2), with two accumulators per CTA: the epilogue of a tile runs beside the MMAs of the next.
-//  * conversion (16 warps): a unit is 16 weight rows x 128 values of K, two operand stages. A lane owns one row and 16
+//  * conversion (16 warps): a unit is 16 weight rows x 128 values of K, a warp's part of one stage. A lane owns one row and 16
 //    consecutive values of a 32-value block; it loads its bytes one unit ahead, dequantises (byte -> 1024 + byte by a
 //    byte permute, exact subtraction, one fused multiply-add with block scale and offset), and writes 16-byte core-matrix
 //    rows; eight lanes write 128 consecutive bytes.
-//  * activation loader (one thread): one bulk copy of 16 KB per stage, packed rows in the operand layout.
-//  * issuer (one warp): in the even CTA four MMAs (M = 256, N = NW, K = 16) per stage; in the odd CTA it passes "stage
+//  * activation loader (one thread): one bulk copy of 32 KB per stage, packed rows in the operand layout.
+//  * issuer (one warp): in the even CTA eight MMAs (M = 256, N = NW, K = 16) per stage; in the odd CTA it passes "stage
 //    full" on to the even one. tcgen05.commit frees the stage in both CTAs.
 //  * epilogue (4 warps): tcgen05.ld, row scale, residuals or SwiGLU (gate and up values of an output sit in one lane,
 //    NW / 2 columns apart), whole 32-byte sectors per row.
@@ -23,6 +23,7 @@
 // cluster barrier before the release of the TMEM columns keeps either CTA alive while the other may still reach it.
 #include <algorithm>
 
+#include "half_weights.cuh"
 #include "qgemm_pair.cuh"
 #include "tcgen05.cuh"
 
@@ -48,19 +49,11 @@ struct Pair {
   static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NW >> 3) << 17) | ((uint32_t)(PAIR_M >> 4) << 24);
 };
 
-__device__ __forceinline__ uint32_t p_h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-__device__ __forceinline__ __half2 p_u2h(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint4 p_ldg(const uint8_t* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ uint2 p_ldg8(const uint8_t* p) { return __ldg(reinterpret_cast<const uint2*>(p)); }
 
-// Four unsigned bytes -> four fp16 values ((1024 + byte) - centre) * scale + offset, as two half2.
-__device__ __forceinline__ uint2 p_deq4(uint32_t w, __half2 centre, __half2 scale, __half2 offset) {
-  const __half2 v01 = __hsub2(p_u2h(__byte_perm(w, 0x64646464u, 0x4140)), centre);
-  const __half2 v23 = __hsub2(p_u2h(__byte_perm(w, 0x64646464u, 0x4342)), centre);
-  return make_uint2(p_h2u(__hfma2(v01, scale, offset)), p_h2u(__hfma2(v23, scale, offset)));
-}
 __device__ __forceinline__ void p_store8(uint8_t* dst, uint32_t w0, uint32_t w1, __half2 centre, __half2 scale, __half2 offset) {
-  const uint2 a = p_deq4(w0, centre, scale, offset), b = p_deq4(w1, centre, scale, offset);
+  const uint2 a = deq4(w0, centre, scale, offset), b = deq4(w1, centre, scale, offset);
   *reinterpret_cast<uint4*>(dst) = make_uint4(a.x, a.y, b.x, b.y);
 }
 

@@ -37,6 +37,8 @@ __device__ __forceinline__ uint64_t x_desc(uint32_t saddr, uint32_t lbo, uint32_
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46) |
          ((uint64_t)layout << 61);
 }
+// K-major operand with 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart (the leading offset is not used)
+__device__ __forceinline__ uint64_t x_desc_rows(uint32_t saddr) { return x_desc(saddr, 16, 1024, 2); }
 // One box of a 3-D tensor map (dims, keys, sequence x KV head) into shared memory; completion is
 // counted in bytes on the mbarrier.
 __device__ __forceinline__ void x_tma_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
@@ -50,13 +52,6 @@ __device__ __forceinline__ void x_mma(uint32_t tmem_d, uint64_t adesc, uint64_t 
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The same with the A operand in tensor memory (row i of A in lane i, two fp16 values per column)
-__device__ __forceinline__ void x_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void x_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -68,6 +63,7 @@ __device__ __forceinline__ void w_mma(uint32_t tmem_d, uint64_t adesc, uint64_t 
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// The same with the A operand in tensor memory (row i of A in lane i, two fp16 values per column)
 __device__ __forceinline__ void w_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p, q;\nelect.sync _|q, 0xFFFFFFFF;\nsetp.ne.b32 p, %4, 0;\n"
