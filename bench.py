@@ -805,6 +805,7 @@ def hybrid_work(layers, width, vocab, rows, ctx, n_sm):
             add("delta_step_kernel", "hbm", 8.0 * H * V * mx["dim"])
         elif delta:
             add("delta_prep_kernel", "hbm", 8.0 * rows * (2 * mx["kv_heads"] * mx["dim"] + H * V))
+            add("delta_pairs_kernel", "hbm", 8.0 * rows * mx["kv_heads"] * mx["dim"])
             add("delta_scan_kernel", "f32", 6.0 * rows * H * V * mx["dim"])  # two sums over d and one update
             add("delta_out_kernel", "hbm", 10.0 * rows * H * V)
         elif rows == 1:
@@ -830,6 +831,16 @@ def llama_work(cfg, rows, ctx):
 
 
 def kernel_rows(table, work):
+    """Rows of a pass's kernel table. A pass's products run on CTA pairs, on single CTAs, or on both: their work is given under the
+    single CTAs' name and set against the time of the two together."""
+    table, work = dict(table), dict(work)
+    for pair, single in (("dense_pair_kernel", "dense_tc_kernel"), ("qgemm_pair_kernel", "qgemm_tc_kernel")):
+        if pair in table:
+            name = f"{pair} + {single}" if single in table else pair
+            both = [table.pop(n) for n in (pair, single) if n in table]
+            table[name] = tuple(map(sum, zip(*both)))
+            if single in work:
+                work[name] = work.pop(single)
     rows = []
     for name, (us, n) in sorted(table.items(), key=lambda kv: -kv[1][0]):
         r = {"kernel": name, "us": round(us, 2), "launches": round(n, 2)}
