@@ -35,6 +35,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <type_traits>
 
 #include "half_weights.cuh"
 #include "qgemm_pair.cuh"
@@ -393,17 +394,22 @@ qgemm_tc_kernel(const TcArgs a) {
 // tiles of 128 rows x 64 values in the operand layout of the MMA (8 rows x 16 bytes per core
 // matrix, core matrices adjacent in K 128 bytes apart, 8-row groups 1024 bytes apart), so that a
 // tile is one contiguous bulk copy; rows >= M are zero. With NORM the rows are (x + res) / rms * w (RMSNorm; res may be null).
-// Bound: latency of one read of the rows. A CTA takes two rows and every thread all its values at once into registers (up to
-// PACK_CHUNKS x 8; the rest is read again), so that the maximum, or sum of squares and maximum, cost no second pass; adjacent
-// threads take the same place of the two rows and write one sector.
-constexpr int PACK_ROWS = 2, PACK_THREADS = 512, PACK_CHUNKS = 7, PACK_STEP = PACK_THREADS / PACK_ROWS;
-template <bool NORM>
-__global__ void __launch_bounds__(PACK_THREADS)
+// Bound: latency of one read of the rows, HBM for many of them. A CTA takes ROWS rows and every thread all its values at once into
+// registers (CHUNKS times 8 values; what is behind 14336 of a row is read again), so that the maximum, or sum of squares and
+// maximum, cost no second pass; adjacent threads take the same place of the rows and write whole sectors.
+// With two rows and the registers of 14336 values for every width one CTA fit an SM, and many narrow rows took longer than in two
+// passes (times with a product of 64 columns behind it, two passes / that / now): 16384 rows of 512 values 32 / 91 / 26 us, of 1024
+// 48 / 112 / 38, of 2048 69 / 124 / 61, of 4096 142 / 153 / 94; 512 rows of 4096 37 / 24 / 22.
+constexpr int PACK_THREADS = 512, PACK_CHUNKS = 7;
+template <int N> using PackInt = std::integral_constant<int, N>;
+template <bool NORM, int ROWS, int CHUNKS>
+__global__ void __launch_bounds__(PACK_THREADS, NORM ? (CHUNKS <= 2 ? 2 : 0) : CHUNKS == 1 ? 4 : CHUNKS == PACK_CHUNKS ? 1 : 0)
 pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, const float* __restrict__ w, float eps, int M, int K,
                    __half* __restrict__ xh, float* __restrict__ xscale) {
-  __shared__ float part[2][PACK_THREADS / 32][PACK_ROWS];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid & 1, c0 = tid >> 1;
-  const int m0 = blockIdx.x * PACK_ROWS, m = m0 + r, chunks = K / 8;
+  constexpr int STEP = PACK_THREADS / ROWS;
+  __shared__ float part[2][PACK_THREADS / 32][ROWS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid % ROWS, c0 = tid / ROWS;
+  const int m0 = blockIdx.x * ROWS, m = m0 + r, chunks = K / 8;
   pdl_launch_dependents();
   const bool in = m < M;
   const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(in ? m : 0) * K);
@@ -418,23 +424,23 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
       }
     }
   };
-  // over the threads of the own row: 16 lanes of every warp
+  // over the threads of the own row: 32 / ROWS lanes of every warp
   auto block = [&](float v, int slot, bool sum) {
 #pragma unroll
-    for (int o = 16; o > 1; o >>= 1) {
+    for (int o = 16; o >= ROWS; o >>= 1) {
       const float other = __shfl_xor_sync(0xFFFFFFFFu, v, o);
       v = sum ? v + other : fmaxf(v, other);
     }
-    if (lane < PACK_ROWS) part[slot][warp][lane] = v;
+    if (lane < ROWS) part[slot][warp][lane] = v;
     __syncthreads();
     v = part[slot][0][r];
 #pragma unroll
     for (int i = 1; i < PACK_THREADS / 32; ++i) v = sum ? v + part[slot][i][r] : fmaxf(v, part[slot][i][r]);
     return v;
   };
-  float4 held[PACK_CHUNKS][2];
+  float4 held[CHUNKS][2];
 #pragma unroll
-  for (int i = 0; i < PACK_CHUNKS; ++i) load(c0 + i * PACK_STEP, held[i]);
+  for (int i = 0; i < CHUNKS; ++i) load(c0 + i * STEP, held[i]);
   float rms = 1.f;
   if (NORM) {
     auto squares = [](const float4 (&v)[2], float acc) {
@@ -444,8 +450,8 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
     };
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < PACK_CHUNKS; ++i) ss = squares(held[i], ss);
-    for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+    for (int i = 0; i < CHUNKS; ++i) ss = squares(held[i], ss);
+    for (int c = c0 + CHUNKS * STEP; c < chunks; c += STEP) {
       float4 v[2];
       load(c, v);
       ss = squares(v, ss);
@@ -468,11 +474,11 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
   };
   float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < PACK_CHUNKS; ++i) {
-    finish(c0 + i * PACK_STEP, held[i]);
+  for (int i = 0; i < CHUNKS; ++i) {
+    finish(c0 + i * STEP, held[i]);
     amax = biggest(held[i], amax);
   }
-  for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+  for (int c = c0 + CHUNKS * STEP; c < chunks; c += STEP) {
     float4 v[2];
     load(c, v);
     finish(c, v);
@@ -482,7 +488,7 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
   int ex = 0;
   if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);
   const float inv = ldexpf(64.0f, -ex);
-  if (tid < PACK_ROWS) xscale[m] = ldexpf(1.0f, ex - 6);
+  if (tid < ROWS) xscale[m] = ldexpf(1.0f, ex - 6);
   uint8_t* tile_row = reinterpret_cast<uint8_t*>(xh) + (size_t)(m0 / BM) * (K / BK) * ((size_t)BM * BK * 2) +
                       ((m0 % BM) >> 3) * CORE_SBO + (m & 7) * 16;
   auto store = [&](int c, const float4 (&v)[2]) {
@@ -492,8 +498,8 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
                    h2u(__floats2half2_rn(v[1].x * inv, v[1].y * inv)), h2u(__floats2half2_rn(v[1].z * inv, v[1].w * inv)));
   };
 #pragma unroll
-  for (int i = 0; i < PACK_CHUNKS; ++i) store(c0 + i * PACK_STEP, held[i]);
-  for (int c = c0 + PACK_CHUNKS * PACK_STEP; c < chunks; c += PACK_STEP) {
+  for (int i = 0; i < CHUNKS; ++i) store(c0 + i * STEP, held[i]);
+  for (int c = c0 + CHUNKS * STEP; c < chunks; c += STEP) {
     float4 v[2];
     load(c, v);
     finish(c, v);
@@ -670,8 +676,18 @@ int tc_pack(fb200_device* dev, const float* x, size_t m, size_t k, const fb200_r
   if (rc) return rc;
   __half* h = reinterpret_cast<__half*>(dev->xpack);
   float* s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dev->xpack) + xbytes);
-  if (norm) pack_rows16_kernel<true><<<mp / PACK_ROWS, PACK_THREADS, 0, dev->stream>>>(x, norm->res, norm->w, norm->eps, (int)m, (int)k, h, s);
-  else pack_rows16_kernel<false><<<mp / PACK_ROWS, PACK_THREADS, 0, dev->stream>>>(x, nullptr, nullptr, 0.f, (int)m, (int)k, h, s);
+  auto launch = [&](auto plain_rows, auto chunks) {
+    constexpr int R = decltype(plain_rows)::value, C = decltype(chunks)::value;
+    if (norm) pack_rows16_kernel<true, 2, C><<<mp / 2, PACK_THREADS, 0, dev->stream>>>(x, norm->res, norm->w, norm->eps, (int)m, (int)k, h, s);
+    else pack_rows16_kernel<false, R, C><<<mp / R, PACK_THREADS, 0, dev->stream>>>(x, nullptr, nullptr, 0.f, (int)m, (int)k, h, s);
+  };
+  // as many registers as a thread of this width has values, several narrow rows to a CTA
+  if (k <= 512) launch(PackInt<8>(), PackInt<1>());
+  else if (k <= 1024) launch(PackInt<4>(), PackInt<1>());
+  else if (k <= 2048) launch(PackInt<2>(), PackInt<1>());
+  else if (k <= 4096) launch(PackInt<2>(), PackInt<2>());
+  else if (k <= 8192) launch(PackInt<2>(), PackInt<4>());
+  else launch(PackInt<2>(), PackInt<PACK_CHUNKS>());
   FB_LAUNCH_CHECK(dev);
   *xh = h;
   *xscale = s;

@@ -219,12 +219,12 @@ def test_decoder_at_llama3_8b_widths(dev, flagged_rows, monkeypatch):
     assert gpu.position == 64 + 6 + 32
 
 
-@pytest.mark.parametrize("hidden", [14592, 20480])
-def test_prompt_norm_of_wide_rows(dev, hidden):
-    # more than 32 rows are normalised as they are packed (the second norm with a residual); values behind the 14336 that the
-    # packing kernel holds in registers are read, and normalised, again. Weights as small as it takes for projections with the spread
-    # that they have at a width of 256 (0.3): at 0.02 they spread by 2.9 and the scores by 2.9^2 sqrt(64) = 67, so that 2^-11 of
-    # a score is 3 % of a softmax weight
+@pytest.mark.parametrize("hidden", [2048, 2304, 4352, 8448, 14592, 20480])
+def test_prompt_norm_of_row_lengths(dev, hidden):
+    # more than 32 rows are normalised as they are packed (the second norm with a residual): one to seven pieces of a row per
+    # thread, values behind the 14336 that the packing kernel holds in registers are read, and normalised, again. Weights as small
+    # as it takes for projections with the spread that they have at a width of 256 (0.3): at 0.02 and 20480 they spread by 2.9 and
+    # the scores by 2.9^2 sqrt(64) = 67, so that 2^-11 of a score is 3 % of a softmax weight
     cfg = dict(n_layer=1, hidden=hidden, ffn=256, n_head=4, n_kv_head=2, head_dim=64, vocab=256, ctx=64)
     gpu, cpu = build_models(dev, cfg, batch=1, seed=3, sigma=0.02 * (256 / hidden) ** 0.5)
     prompt = np.random.default_rng(5).integers(0, cfg["vocab"], size=(1, 41), dtype=np.uint32)

@@ -146,11 +146,12 @@ def test_prefill_product_cta_pairs(dev, tname, tile, m, n, k, monkeypatch):
 
 
 @pytest.mark.parametrize("tname", ["q4k", "q8_0"])
-@pytest.mark.parametrize("k", [14336, 14592, 20480])
-def test_prefill_product_long_rows(dev, tname, k):
-    # the packing kernel holds 14336 values of a row in registers and reads the rest again
+@pytest.mark.parametrize("k", [256, 512, 768, 1024, 1280, 2048, 2304, 4096, 4352, 8192, 8448, 14336, 14592, 20480])
+def test_prefill_product_row_lengths(dev, tname, k):
+    # the packing kernel takes eight, four or two rows per CTA and one to seven pieces of a row per thread; it holds 14336 values
+    # of a row in registers and reads the rest again
     ty = TYPES[tname]
-    n, m = 96, 41
+    n, m = 96, 131
     raw = weights(51, n, k, ty)
     w = kb.QMatrix.from_raw_bytes(dev, (n, k), raw, ty)
     x = activations(k, m, k)
