@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256)
 rows_to_bf16_kernel(const float* __restrict__ x, size_t ldx, const float* __restrict__ w, const float* __restrict__ w2, float eps,
                     int n, int np, __nv_bfloat16* __restrict__ y) {
   __shared__ float sh[8];
-  pdl_launch_dependents();  // a product on CTA pairs behind it sets itself up meanwhile
+  pdl_launch_dependents_small();  // a product on CTA pairs behind it sets itself up meanwhile
   const size_t row = blockIdx.x;
   const float* xr = x + row * ldx;
   y += row * (w2 ? 2 : 1) * (size_t)np;

@@ -410,7 +410,7 @@ pack_rows16_kernel(const float* __restrict__ x, const float* __restrict__ res, c
   __shared__ float part[2][PACK_THREADS / 32][ROWS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid % ROWS, c0 = tid / ROWS;
   const int m0 = blockIdx.x * ROWS, m = m0 + r, chunks = K / 8;
-  pdl_launch_dependents();
+  pdl_launch_dependents_small();
   const bool in = m < M;
   const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(in ? m : 0) * K);
   const float4* rr = NORM && res ? reinterpret_cast<const float4*>(res + (size_t)(in ? m : 0) * K) : nullptr;
