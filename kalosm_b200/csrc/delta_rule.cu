@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200
   const int lane = threadIdx.x & 31, b = blockIdx.z, t0 = blockIdx.x * PREP_TOK, n = min(PREP_TOK, a.s - t0);
   const int hv = a.h * a.v, vblocks = (hv + PREP_VCH - 1) / PREP_VCH;
   int unit = blockIdx.y * PREP_WARPS + (threadIdx.x >> 5);
+  pdl_launch_dependents_small();  // delta_pairs_kernel's launch is over when this one's work is
   const int pos = *a.pos_dev;
   if (unit < a.hk) {
     float q[NE][PREP_TOK], k[NE][PREP_TOK], sum[32];
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(const fb200
 __global__ void __launch_bounds__(PREP_WARPS * 32) delta_pairs_kernel(const fb200_delta_args a) {
   const int lane = threadIdx.x & 31, b = blockIdx.z, t0 = blockIdx.x * CH, hk = blockIdx.y * PREP_WARPS + (threadIdx.x >> 5);
   if (hk >= a.hk) return;
+  pdl_wait();
   float sum[2][32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) sum[0][i] = sum[1][i] = 0.f;
@@ -607,10 +609,8 @@ int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
   delta_prep_kernel<NE><<<dim3((unsigned)((a.s + PREP_TOK - 1) / PREP_TOK), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
                           PREP_WARPS * 32, 0, dev->stream>>>(a);
   FB_LAUNCH_CHECK(dev);
-  delta_pairs_kernel<<<dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b), PREP_WARPS * 32, 0,
-                       dev->stream>>>(a);
-  FB_LAUNCH_CHECK(dev);
-  return FB200_OK;
+  return fb200_launch(dev, delta_pairs_kernel, dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
+                      dim3(PREP_WARPS * 32), 0, true, a);
 }
 
 }  // namespace
