@@ -10,12 +10,13 @@
 // G_i = g_0 .. g_i and w_j = (g_(j+1) .. g_i) u_j,
 //   u_i = beta_i (v_i - G_i a_i - sum_(j<i) (k_j . k_i) w_j),   o_i = G_i c_i + sum_(j<=i) (k_j . q_i) w_j,
 //   S <- G_7 S + sum_j k_j w_j,
-// the same recurrence with one reduction over the lanes per eight tokens. Everything is f32.
+// the same recurrence with one reduction over the lanes per eight tokens. Everything is f32 (two tf32 values on tensor cores).
 //
 //  * delta_step_kernel: one new token per sequence. One CTA per (head, sequence): convolution, unit vectors,
 //    decay, state update, read-out, RMSNorm and gate. Bound: HBM on the state (read and written once).
-//  * prompts: delta_prep_kernel (convolution, SiLU, unit vectors, decay and write strength), delta_pairs_kernel (products of
-//    eight tokens' k and q), delta_scan_kernel (the recurrence; bound: latency of the pass, a warp per scheduler), delta_out_kernel
+//  * prompts: delta_prep_kernel (convolution, SiLU, unit vectors, decay and write strength), then delta_pairs_kernel (products of
+//    eight tokens' k and q) and delta_scan_kernel (the recurrence; bound: latency of the pass, a warp per scheduler), or, for long
+//    prompts, delta_chunk_kernel and delta_chunk_scan_kernel (the same over chunks of 32 tokens, on tensor cores), delta_out_kernel
 //    (RMSNorm, gate) and conv_ring_kernel (the convolution's memory).
 #include "mixers.cuh"
 #include "qgemv_common.cuh"
@@ -551,6 +552,436 @@ __global__ void __launch_bounds__(SC_WARPS * 32) delta_scan_kernel(const fb200_d
     if (c + cc * GROUPS < a.v) store_column<EPT, LPC>(state + (size_t)(c + cc * GROUPS) * a.dp, p, s[cc]);
 }
 
+// ---- prompts in chunks of 32 tokens ------------------------------------------------------------------------
+// With r_ij = g_(j+1) .. g_i, A_ij = beta_i (k_i . k_j) r_ij (j < i), P_ij = (q_i . k_j) r_ij (j <= i) and S the state before a
+// chunk, the recurrence above reads
+//   (1 + A) u = beta (v - G K S),   o = G Q S + P u,   S <- G_last S + K^T (r_last u),
+// so u = U - W S and o = O + Z S with W = (1 + A)^-1 beta G K, U = (1 + A)^-1 beta v, Z = G Q - P W, O = P U: all that does not
+// need the state is formed for all chunks side by side (delta_chunk_kernel), and what is left in order is three products with the
+// state per chunk (delta_chunk_scan_kernel). Every decay is a product of decays, never a quotient, and unit k with beta below one
+// keep 1 + A well conditioned: its inverse has entries of at most one.
+//
+// Contractions run on mma.sync with both operands as two tf32 values each (hi, lo; products hi hi, hi lo, lo hi): a product is right
+// to 2^-24.8 of itself in the mean, below what 32-bit sums of that length lose. One layer in f32 against 64 bits, 24 prompts of 200 ..
+// 2400 tokens: 4.30e-7 (passes of eight: 4.29e-7), with decays near one 1.081e-6 (1.079e-6).
+constexpr int CT = 32;        // tokens of a chunk
+constexpr int CDEC = CT + 4;  // decays of a chunk: r_last of every token, then the product of all
+constexpr int CK_THREADS = 128, CS_THREADS = 288, CS_STAGES = 3, SCOLS = 16;
+
+__device__ __forceinline__ float4 lds_v4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float2 lds_v2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+struct Split { uint32_t hi, lo; };
+// hi: x rounded to 11 bits; lo: the rest, rounded to as many (by sums and masks: the conversion takes 4 cycles, these 3)
+__device__ __forceinline__ Split split_tf32(float x) {
+  Split s;
+  s.hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
+  s.lo = (__float_as_uint(x - __uint_as_float(s.hi)) + 0x1000u) & 0xFFFFE000u;
+  return s;
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Operands of m16n8k8 with its k slots t and t + 4 as elements 2t and 2t + 1: a lane's pair lies side by side in memory, and an
+// accumulator tile [16][8] is an A operand of 16 rows over 8 elements as it is.
+struct SplitA { uint32_t hi[4], lo[4]; };
+__device__ __forceinline__ SplitA split_a(float g0, float g1, float h0, float h1) {  // row g: elements 2t, 2t + 1; row g + 8
+  const Split x0 = split_tf32(g0), x1 = split_tf32(h0), x2 = split_tf32(g1), x3 = split_tf32(h1);
+  return {{x0.hi, x1.hi, x2.hi, x3.hi}, {x0.lo, x1.lo, x2.lo, x3.lo}};
+}
+// c += a b; the small products apart, the large ones added with rounding (an accumulator of the tensor cores is cut off)
+__device__ __forceinline__ void mma_split(float (&c)[4], float (&small)[4], const SplitA& a, const Split& b0, const Split& b1) {
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  mma_tf32(small, a.lo, b0.hi, b1.hi);
+  mma_tf32(d, a.hi, b0.hi, b1.hi);
+  mma_tf32(small, a.hi, b0.lo, b1.lo);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] += d[i];
+}
+// A CTA per (chunk, head): the lower tiles of K K^T and Q K^T; the inverse of 1 + A, whose diagonal blocks of 16 are solved by columns, a
+// lane each, and joined by -T22 A21 T11; then 16 columns of [K | V] at a time per warp, transposed: W^T = (beta G K)^T T^T, whose
+// accumulators are the operand of (P W)^T = W^T P^T as they are. Writes W and Z (16-byte piece c of row i at c ^ 2 (i & 3)), U in place
+// of v, O, and the decays. Bound: mma.sync (1540 products of 8.2 cycles a CTA). With a thread per column and the substitution unrolled
+// (no products on tensor cores) 8192 tokens of 16 heads took 225 us a layer, most of it fetching that code.
+template <int DP>
+__global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_delta_args a) {
+  constexpr int LD = DP + 4, LA = CT + 4;
+  extern __shared__ __align__(16) float dsm[];
+  float *ks = dsm, *qs = dsm + CT * LD;
+  __shared__ __align__(16) float A[CT][LA], P[CT][LA], T[CT][LA], M[16][20], gs[CT], bs[CT], Gs[CT];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int t0 = blockIdx.x * CT, h = blockIdx.y, b = blockIdx.z, hk = h / (a.h / a.hk), hv = a.h * a.v;
+  const int n = min(CT, a.s - t0);
+  const size_t row0 = (size_t)b * a.s + t0, chunk = ((size_t)b * a.h + h) * gridDim.x + blockIdx.x;
+  pdl_wait();
+#pragma unroll 4
+  for (int i = tid; i < CT * (DP / 4); i += CK_THREADS) {
+    const int tk = i / (DP / 4), e = (i % (DP / 4)) * 4;
+    const size_t src = ((row0 + min(tk, n - 1)) * a.hk + hk) * (size_t)DP + e;
+    const float4 k = *reinterpret_cast<const float4*>(a.kn + src), q = *reinterpret_cast<const float4*>(a.qn + src);
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(ks + tk * LD + e) = tk < n ? k : z;
+    *reinterpret_cast<float4*>(qs + tk * LD + e) = tk < n ? q : z;
+  }
+  if (tid < CT) {  // tokens behind the last one: decay 1, strength 0
+    const float2 gb = *reinterpret_cast<const float2*>(a.gb + ((row0 + min(tid, n - 1)) * a.h + h) * 2);
+    gs[tid] = tid < n ? gb.x : 1.f;
+    bs[tid] = tid < n ? gb.y : 0.f;
+  }
+  __syncthreads();
+  if (warp == 0) {  // decays from token `lane` on, and from the chunk's start; T holds r_ij until the products are there
+    float r = 1.f, G = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < CT; ++i) {
+      const float gi = gs[i];
+      r = i > lane ? r * gi : 1.f;
+      G *= i <= lane ? gi : 1.f;
+      T[i][lane] = r;
+    }
+    Gs[lane] = G;
+    float* dec = a.dec + chunk * CDEC;
+    dec[lane] = r;
+    if (lane == CT - 1) dec[CT] = G;
+  }
+  // tiles of 16 rows i by 8 rows j with i >= j: (0, 0), (0, 1), (1, 0) .. (1, 3) of K K^T, then of Q K^T; three a warp
+  {
+    float c[3][4], cs[3][4];
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c[x][i] = cs[x][i] = 0.f;
+    const float* rows = (warp & 2 ? qs : ks);
+    // warps 0, 2: (0, 0), (0, 1), (1, 0); warps 1, 3: (1, 1), (1, 2), (1, 3)
+    const int m01 = warp & 1 ? 16 : 0, n0 = warp & 1 ? 8 : 0, n1 = warp & 1 ? 16 : 8, n2 = warp & 1 ? 24 : 0;
+#pragma unroll 2
+    for (int e = 0; e < DP; e += 8) {
+      const float* ra = rows + (m01 + g) * LD + e + 2 * t;
+      const float2 x0 = lds_v2(ra), x1 = lds_v2(ra + 8 * LD);
+      const SplitA f = split_a(x0.x, x0.y, x1.x, x1.y);
+      const float2 y0 = lds_v2(ks + (n0 + g) * LD + e + 2 * t), y1 = lds_v2(ks + (n1 + g) * LD + e + 2 * t);
+      const Split b00 = split_tf32(y0.x), b01 = split_tf32(y0.y);
+      mma_split(c[0], cs[0], f, b00, b01);
+      mma_split(c[1], cs[1], f, split_tf32(y1.x), split_tf32(y1.y));
+      if (warp & 1) {
+        const float2 y2 = lds_v2(ks + (n2 + g) * LD + e + 2 * t);
+        mma_split(c[2], cs[2], f, split_tf32(y2.x), split_tf32(y2.y));
+      } else {
+        const float* rb = rows + (16 + g) * LD + e + 2 * t;
+        const float2 z0 = lds_v2(rb), z1 = lds_v2(rb + 8 * LD);
+        mma_split(c[2], cs[2], split_a(z0.x, z0.y, z1.x, z1.y), b00, b01);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = (x == 2 ? 16 : m01) + g + 8 * (i >> 1), col = (x == 0 ? n0 : x == 1 ? n1 : n2) + 2 * t + (i & 1);
+        const float v = (c[x][i] + cs[x][i]) * T[row][col];
+        if (warp & 2) P[row][col] = col <= row ? v : 0.f;
+        else A[row][col] = col < row ? bs[row] * v : 0.f;
+      }
+  }
+  __syncthreads();
+  if (warp == 0) {  // T = (1 + A)^-1
+    const int o = lane & 16, j = lane & 15;  // block and column
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float s0 = i == j ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+      for (int l = 0; l < i; l += 4) {
+        const float4 v = lds_v4(&A[o + i][o + l]);
+        s0 = fmaf(-v.x, x[l], s0);
+        if (l + 1 < i) s1 = fmaf(-v.y, x[l + 1], s1);
+        if (l + 2 < i) s0 = fmaf(-v.z, x[l + 2], s0);
+        if (l + 3 < i) s1 = fmaf(-v.w, x[l + 3], s1);
+      }
+      x[i] = s0 + s1;
+      T[o + i][o + j] = x[i];
+      if (o == 0) T[i][16 + j] = 0.f;
+    }
+    __syncwarp();
+    const int i = lane & 15, c8 = lane >> 4 << 3;
+#pragma unroll
+    for (int step = 0; step < 2; ++step) {  // M = A21 T11, then T21 = -T22 M
+      float m[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) m[e] = 0.f;
+#pragma unroll 4
+      for (int l = 0; l < 16; ++l) {
+        const float w = step ? -T[16 + i][16 + l] : A[16 + i][l];
+        const float4 u = lds_v4(step ? &M[l][c8] : &T[l][c8]), v = lds_v4(step ? &M[l][c8 + 4] : &T[l][c8 + 4]);
+        m[0] = fmaf(w, u.x, m[0]); m[1] = fmaf(w, u.y, m[1]); m[2] = fmaf(w, u.z, m[2]); m[3] = fmaf(w, u.w, m[3]);
+        m[4] = fmaf(w, v.x, m[4]); m[5] = fmaf(w, v.y, m[5]); m[6] = fmaf(w, v.z, m[6]); m[7] = fmaf(w, v.w, m[7]);
+      }
+      float* d = step ? &T[16 + i][c8] : &M[i][c8];
+      *reinterpret_cast<float4*>(d) = make_float4(m[0], m[1], m[2], m[3]);
+      *reinterpret_cast<float4*>(d + 4) = make_float4(m[4], m[5], m[6], m[7]);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  float* wq = a.wq + chunk * (size_t)(2 * CT * DP);
+  for (int c0 = 16 * warp; c0 < DP + a.v; c0 += 64) {
+    const bool key = c0 < DP;
+    const int col = c0 - DP + g;
+    const size_t at = row0 * hv + h * a.v + col;
+    float d1[4][4], e1[4][4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d1[x][i] = e1[x][i] = 0.f;
+    float in[4][4];  // [eight tokens][token 2 t, 2 t + 1; column g, g + 8]
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int tk = 8 * k + 2 * t + (i & 1);
+        if (key) in[k][i] = ks[tk * LD + c0 + g + 8 * (i >> 1)];
+        else in[k][i] = tk < n && col + 8 * (i >> 1) < a.v ? a.vn[at + (size_t)tk * hv + 8 * (i >> 1)] : 0.f;
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float f[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) f[i] = bs[8 * k + 2 * t + i] * (key ? Gs[8 * k + 2 * t + i] : 1.f);
+      const SplitA x = split_a(f[0] * in[k][0], f[1] * in[k][1], f[0] * in[k][2], f[1] * in[k][3]);
+#pragma unroll
+      for (int r = k; r < 4; ++r) {
+        const float2 y = lds_v2(&T[8 * r + g][8 * k + 2 * t]);
+        mma_split(d1[r], e1[r], x, split_tf32(y.x), split_tf32(y.y));
+      }
+    }
+    float d2[4][4], e2[4][4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        d1[x][i] += e1[x][i];
+        d2[x][i] = e2[x][i] = 0.f;
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const SplitA x = split_a(d1[k][0], d1[k][1], d1[k][2], d1[k][3]);
+#pragma unroll
+      for (int r = k; r < 4; ++r) {
+        const float2 y = lds_v2(&P[8 * r + g][8 * k + 2 * t]);
+        mma_split(d2[r], e2[r], x, split_tf32(y.x), split_tf32(y.y));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int tk = 8 * r + 2 * t + (i & 1), c = c0 + g + 8 * (i >> 1);
+        const float pw = d2[r][i] + e2[r][i];
+        if (key) {
+          float* w = wq + tk * DP + (((c >> 2) ^ ((tk & 3) << 1)) << 2) + (c & 3);
+          w[0] = d1[r][i];
+          w[CT * DP] = fmaf(Gs[tk], qs[tk * LD + c], -pw);
+        } else if (tk < n && c < DP + a.v) {
+          const size_t to = at + (size_t)tk * hv + 8 * (i >> 1);
+          a.vn[to] = d1[r][i];
+          a.o[to] = pw;
+        }
+      }
+  }
+}
+
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// A CTA per (16 columns of S, head). Warps 0 .. 3 carry the recurrence: each holds a quarter of d of S^T [16][d] as accumulator tiles,
+// which are the A operands of S^T W^T as they are; the quarters' sums meet in shared memory, become w = r_last (U - W S), again an A
+// operand, and S^T <- G S^T + w^T K. Warps 4 .. 7 follow with the read-out O + Z S from a copy of S, a chunk behind at most. Warp 8
+// fetches the matrices two chunks ahead (what 128 CTAs have in flight a chunk ahead is too little for HBM). The update is summed from zero and added to S in one rounding, so S drifts no more than
+// with 32-bit sums. Bound: issue (144 products of 8.2 cycles and 1500 other instructions per chunk and scheduler) and the chain of a chunk:
+// 3300 cycles. 8192 tokens of 16 heads of 128: 0.47 ms and 0.18 ms of preparation (delta_scan_kernel: 1.22 ms and 0.03).
+template <int DP>
+__global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const fb200_delta_args a) {
+  constexpr int KS = DP / 4, KT = KS / 8, MAT = CT * DP, KLD = DP + 4;  // a warp's part of d, in tiles of 8; floats of a matrix, of a row of K
+  extern __shared__ __align__(16) float dsm[];  // STAGES x (W, K); STAGES x Z; two copies of S [4][KT][32 lanes] float4
+  __shared__ uint64_t full[2][CS_STAGES], empty[2][CS_STAGES];
+  __shared__ __align__(16) float4 part[2][4][4][32], ws[2][4][32];  // [half][warp][tile of 8 rows][lane]; w: (hi, lo) per tile
+  const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, half = threadIdx.x >> 7, g = lane >> 2, t = lane & 3;
+  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.h / a.hk), hv = a.h * a.v, c0 = blockIdx.x * SCOLS, nch = (a.s + CT - 1) / CT;
+  const size_t row0 = (size_t)b * a.s, chunk0 = ((size_t)b * a.h + h) * nch;
+  const int STAGE = half ? MAT : MAT + CT * KLD;
+  float* stages = dsm + (half ? CS_STAGES * (MAT + CT * KLD) : 0);
+  float4* copies = reinterpret_cast<float4*>(dsm + CS_STAGES * (2 * MAT + CT * KLD));
+  constexpr int COPY = 4 * KT * 32;
+  const int FULL = 3, EMPTY = 5;  // barriers of the copies (1, 2: the halves' own)
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2 * CS_STAGES; ++i) {
+      mbar_init(smem_u32(&full[i / CS_STAGES][i % CS_STAGES]), 1);
+      mbar_init(smem_u32(&empty[i / CS_STAGES][i % CS_STAGES]), 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_wait();
+  if (threadIdx.x >= 256) {  // the last warp fetches: a matrix in one copy, a row of K per lane (rows behind the last token are zero)
+    for (int ch = 0; ch < nch; ++ch) {
+      const int st = ch % CS_STAGES;
+      const uint32_t round = (uint32_t)(ch / CS_STAGES);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float* dst = dsm + (x ? CS_STAGES * (MAT + CT * KLD) + st * MAT : st * (MAT + CT * KLD));
+        const uint32_t bar = smem_u32(&full[x][st]);
+        const int rows = x ? 0 : min(CT, a.s - ch * CT);
+        if (round > 0) mbar_wait(smem_u32(&empty[x][st]), (round - 1) & 1, a.status);
+        if (!x && lane >= rows)
+          for (int e = 0; e < DP; e += 4) *reinterpret_cast<float4*>(dst + MAT + lane * KLD + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        if (lane == 0) {
+          mbar_expect_tx(bar, (uint32_t)(MAT + rows * DP) * 4);
+          bulk_g2s(smem_u32(dst), a.wq + ((chunk0 + ch) * 2 + x) * (size_t)MAT, MAT * 4, bar);
+        }
+        __syncwarp();
+        if (lane < rows) bulk_g2s(smem_u32(dst + MAT + lane * KLD), a.kn + ((row0 + ch * CT + lane) * a.hk + hk) * (size_t)DP, DP * 4, bar);
+      }
+    }
+    return;
+  }
+  auto release = [&](int ch) {  // this warp is through with its half's stage
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[half][ch % CS_STAGES])) : "memory");
+  };
+  // what the sums of a chunk are added to (rows 8 warp + 2 t + i % 2, columns c0 + g + 8 (i / 2)), and its decays
+  struct Ahead { float base[4], rl[2], G; };
+  auto look = [&](int ch, Ahead& n) {
+    const float* add = half ? a.o : a.vn;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int tk = ch * CT + 8 * warp + 2 * t + (i & 1), col = c0 + g + 8 * (i >> 1);
+      n.base[i] = tk < a.s && col < a.v ? add[(row0 + tk) * hv + h * a.v + col] : 0.f;
+    }
+    if (half || ch >= nch) return;
+    const float* dec = a.dec + (chunk0 + ch) * CDEC;
+    n.rl[0] = dec[8 * warp + 2 * t];
+    n.rl[1] = dec[8 * warp + 2 * t + 1];
+    n.G = dec[CT];
+  };
+  Ahead next = {};
+  look(0, next);
+  const int pos = *a.pos_dev;
+  float* state = a.state + ((size_t)b * a.h + h) * (size_t)a.v * DP;
+  // entry i of tile x: column c0 + g + 8 (i / 2), element warp KS + 8 x + 2 t + i % 2
+  float s[KT][4];
+  if (!half) {
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; i += 2) {
+        const int col = c0 + g + 4 * i;
+        const float2 v = col < a.v && pos > 0 ? *reinterpret_cast<const float2*>(state + (size_t)col * DP + warp * KS + 8 * x + 2 * t) : make_float2(0.f, 0.f);
+        s[x][i] = v.x;
+        s[x][i + 1] = v.y;
+      }
+  }
+  for (int ch = 0; ch < nch; ++ch) {
+    if (half) bar_sync(2, 128);  // the sums of the chunk before have been read
+    const float* st = stages + ch % CS_STAGES * STAGE;
+    float4* copy = copies + (ch & 1) * COPY + warp * KT * 32 + lane;
+    const Ahead now = next;
+    look(ch + 1, next);
+    if (half) {
+      bar_sync(FULL + (ch & 1), 256);
+#pragma unroll
+      for (int x = 0; x < KT; ++x) {
+        const float4 v = copy[x * 32];
+        s[x][0] = v.x; s[x][1] = v.y; s[x][2] = v.z; s[x][3] = v.w;
+      }
+      if (ch + 2 < nch) bar_arrive(EMPTY + (ch & 1), 256);
+    } else {
+      if (ch >= 2) bar_sync(EMPTY + (ch & 1), 256);
+#pragma unroll
+      for (int x = 0; x < KT; ++x) copy[x * 32] = make_float4(s[x][0], s[x][1], s[x][2], s[x][3]);
+      bar_arrive(FULL + (ch & 1), 256);
+    }
+    mbar_wait(smem_u32(&full[half][ch % CS_STAGES]), (uint32_t)(ch / CS_STAGES) & 1, a.status);
+    // ---- this warp's part of S^T (W or Z)^T: 16 columns by four tiles of 8 rows
+    float c[4][4], cs[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c[j][i] = cs[j][i] = 0.f;
+#pragma unroll
+    for (int x = 0; x < KT; ++x) {
+      const SplitA f = split_a(s[x][0], s[x][1], s[x][2], s[x][3]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int piece = (warp * KS + 8 * x) / 4 + (t >> 1);
+        const float2 v = lds_v2(st + (8 * j + g) * DP + ((piece ^ ((g & 3) << 1)) << 2) + 2 * (t & 1));
+        mma_split(c[j], cs[j], f, split_tf32(v.x), split_tf32(v.y));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) part[half][warp][j][lane] = make_float4(c[j][0] + cs[j][0], c[j][1] + cs[j][1], c[j][2] + cs[j][2], c[j][3] + cs[j][3]);
+    bar_sync(1 + half, 128);
+    float sum[4];
+    {
+      const float4 p0 = part[half][0][warp][lane], p1 = part[half][1][warp][lane], p2 = part[half][2][warp][lane], p3 = part[half][3][warp][lane];
+      sum[0] = (p0.x + p1.x) + (p2.x + p3.x);
+      sum[1] = (p0.y + p1.y) + (p2.y + p3.y);
+      sum[2] = (p0.z + p1.z) + (p2.z + p3.z);
+      sum[3] = (p0.w + p1.w) + (p2.w + p3.w);
+    }
+    if (half) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int tk = ch * CT + 8 * warp + 2 * t + (i & 1), col = c0 + g + 8 * (i >> 1);
+        if (tk < a.s && col < a.v) a.o[(row0 + tk) * hv + h * a.v + col] = now.base[i] + sum[i];
+      }
+      release(ch);
+      continue;
+    }
+    {
+      float w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = ch * CT + 8 * warp + 2 * t + (i & 1) < a.s ? now.rl[i & 1] * (now.base[i] - sum[i]) : 0.f;
+      const SplitA f = split_a(w[0], w[1], w[2], w[3]);
+      ws[0][warp][lane] = make_float4(__uint_as_float(f.hi[0]), __uint_as_float(f.hi[1]), __uint_as_float(f.hi[2]), __uint_as_float(f.hi[3]));
+      ws[1][warp][lane] = make_float4(__uint_as_float(f.lo[0]), __uint_as_float(f.lo[1]), __uint_as_float(f.lo[2]), __uint_as_float(f.lo[3]));
+    }
+    bar_sync(1, 128);
+    // ---- S^T <- G S^T + w^T K
+    const float* kb = st + MAT;
+    float up[KT][4], us[KT][4];
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) up[x][i] = us[x][i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {  // tokens 8 j ..
+      const float4 whi = ws[0][j][lane], wlo = ws[1][j][lane];
+      const SplitA f = {{__float_as_uint(whi.x), __float_as_uint(whi.y), __float_as_uint(whi.z), __float_as_uint(whi.w)},
+                        {__float_as_uint(wlo.x), __float_as_uint(wlo.y), __float_as_uint(wlo.z), __float_as_uint(wlo.w)}};
+#pragma unroll
+      for (int x = 0; x < KT; ++x) {
+        const float* p = kb + (8 * j + 2 * t) * KLD + warp * KS + 8 * x + g;
+        mma_split(up[x], us[x], f, split_tf32(p[0]), split_tf32(p[KLD]));
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[x][i] = fmaf(now.G, s[x][i], up[x][i] + us[x][i]);
+    release(ch);
+  }
+  if (!half) {
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
+#pragma unroll
+      for (int i = 0; i < 4; i += 2) {
+        const int col = c0 + g + 4 * i;
+        if (col < a.v) *reinterpret_cast<float2*>(state + (size_t)col * DP + warp * KS + 8 * x + 2 * t) = make_float2(s[x][i], s[x][i + 1]);
+      }
+  }
+}
+
 // A warp per (row, head): RMSNorm over v, the plain weight, the SiLU gate.
 __global__ void __launch_bounds__(256) delta_out_kernel(const fb200_delta_args a) {
   const int lane = threadIdx.x & 31;
@@ -603,14 +1034,36 @@ int launch_scan(fb200_device* dev, const fb200_delta_args& a) {
   return FB200_OK;
 }
 
+template <int DP>
+int launch_chunks(fb200_device* dev, const fb200_delta_args& a) {
+  const unsigned nch = (unsigned)((a.s + CT - 1) / CT);
+  constexpr int ck_smem = 2 * CT * (DP + 4) * 4, cs_smem = (CS_STAGES * CT * (3 * DP + 4) + 2 * SCOLS * DP) * 4;
+  static bool configured[64] = {false};
+  if (!configured[dev->ordinal & 63]) {
+    FB_CUDA(dev, cudaFuncSetAttribute(delta_chunk_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ck_smem));
+    FB_CUDA(dev, cudaFuncSetAttribute(delta_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs_smem));
+    configured[dev->ordinal & 63] = true;
+  }
+  if (int rc = fb200_launch(dev, delta_chunk_kernel<DP>, dim3(nch, (unsigned)a.h, (unsigned)a.b), dim3(CK_THREADS), ck_smem, true, a)) return rc;
+  return fb200_launch(dev, delta_chunk_scan_kernel<DP>, dim3((unsigned)((a.v + SCOLS - 1) / SCOLS), (unsigned)a.h, (unsigned)a.b),
+                      dim3(CS_THREADS), cs_smem, true, a);
+}
+
 template <int NE>
 int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
   const int units = a.hk + (a.h * a.v + PREP_VCH - 1) / PREP_VCH + 1;
   delta_prep_kernel<NE><<<dim3((unsigned)((a.s + PREP_TOK - 1) / PREP_TOK), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
                           PREP_WARPS * 32, 0, dev->stream>>>(a);
   FB_LAUNCH_CHECK(dev);
-  return fb200_launch(dev, delta_pairs_kernel, dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
-                      dim3(PREP_WARPS * 32), 0, true, a);
+  return FB200_OK;
+}
+
+// Chunks of 32 tokens or passes of eight. Four layers of 16 heads of 128, passes / chunks: 100 tokens 426 / 452 us, 200 tokens 482 / 481,
+// 512 tokens 690 / 579, 4096 tokens 3398 / 2217 (heads of 64: 393 / 406, 448 / 423, 659 / 512, 3269 / 1860): a chunk's preparation
+// has a longer chain than a few passes. Heads of more than 128 do not fit: three stages of their matrices need 250 KB.
+constexpr int CHUNKS_FROM = 192;
+bool delta_in_chunks(const fb200_delta_args& a) {
+  return fb200_delta_chunks(a.dp) && a.s >= CHUNKS_FROM;
 }
 
 }  // namespace
@@ -620,6 +1073,8 @@ int fb200_delta_dp(int d) {
     if (d <= dp) return dp;
   return 0;
 }
+
+bool fb200_delta_chunks(int dp) { return dp == 64 || dp == 128; }
 
 int fb200_delta_step(fb200_device* dev, const fb200_delta_args& a) {
   switch (a.dp) {
@@ -643,16 +1098,23 @@ int fb200_delta_prompt(fb200_device* dev, const fb200_delta_args& a) {
     default: return fb200_fail(dev, FB200_ERR_INVALID_SHAPE, "delta rule: head size %d", a.d);
   }
   if (rc) return rc;
-  switch (a.dp) {
-    case 32: rc = launch_scan<4, 8, 16>(dev, a); break;
-    case 64: rc = launch_scan<4, 16, 16>(dev, a); break;
-    case 128:
-      // 16 lanes per column group do less per token (fewer shuffles); 32 lanes make more CTAs where there are few heads
-      if ((a.v + 15) / 16 * a.h * a.b <= dev->sm_count) rc = launch_scan<4, 32, 16>(dev, a);
-      else rc = launch_scan<8, 16, 16>(dev, a);
-      break;
-    case 256: rc = launch_scan<8, 32, 16>(dev, a); break;
-    default: rc = launch_scan<16, 32, 8>(dev, a); break;
+  if (delta_in_chunks(a)) {
+    rc = a.dp == 64 ? launch_chunks<64>(dev, a) : launch_chunks<128>(dev, a);
+  } else {
+    rc = fb200_launch(dev, delta_pairs_kernel, dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),
+                      dim3(PREP_WARPS * 32), 0, true, a);
+    if (rc) return rc;
+    switch (a.dp) {
+      case 32: rc = launch_scan<4, 8, 16>(dev, a); break;
+      case 64: rc = launch_scan<4, 16, 16>(dev, a); break;
+      case 128:
+        // 16 lanes per column group do less per token (fewer shuffles); 32 lanes make more CTAs where there are few heads
+        if ((a.v + 15) / 16 * a.h * a.b <= dev->sm_count) rc = launch_scan<4, 32, 16>(dev, a);
+        else rc = launch_scan<8, 16, 16>(dev, a);
+        break;
+      case 256: rc = launch_scan<8, 32, 16>(dev, a); break;
+      default: rc = launch_scan<16, 32, 8>(dev, a); break;
+    }
   }
   if (rc) return rc;
   const size_t warps = (size_t)a.b * a.s * a.h;

@@ -80,7 +80,7 @@ struct fb200_hybrid {
   float* xend = nullptr;    // where a pass leaves the residual stream
   float *proj = nullptr, *zf = nullptr;
   __nv_bfloat16 *hb = nullptr, *zb = nullptr;
-  float *qn = nullptr, *kn = nullptr, *vn = nullptr, *gb = nullptr, *kq = nullptr, *o = nullptr, *seg = nullptr;
+  float *qn = nullptr, *kn = nullptr, *vn = nullptr, *gb = nullptr, *kq = nullptr, *wq = nullptr, *dec = nullptr, *o = nullptr, *seg = nullptr;
   float *qa = nullptr, *part = nullptr;
   int* done = nullptr;      // arrival counters, zero between launches
   size_t done_linear = 0;   // first counter of the linear attention
@@ -370,7 +370,7 @@ int run_mixer(fb200_llama* m, const Mixer& M, int pass, int batch, int seq, bool
     a.state = M.state + pass * M.pass_state; a.ring = M.ring + pass * M.pass_ring; a.b = batch; a.s = seq; a.h = c.heads; a.hk = c.kv_heads;
     a.d = c.dim; a.v = c.vdim; a.dp = M.dp; a.taps = c.conv; a.channels = M.channels; a.pos_dev = m->pos_dev; a.z = z; a.ldz = hy->ldz;
     a.z_bf16 = !wide; a.commit = commit;
-    a.qn = hy->qn; a.kn = hy->kn; a.vn = hy->vn; a.gb = hy->gb; a.kq = hy->kq; a.o = hy->o;
+    a.qn = hy->qn; a.kn = hy->kn; a.vn = hy->vn; a.gb = hy->gb; a.kq = hy->kq; a.wq = hy->wq; a.dec = hy->dec; a.o = hy->o; a.status = dev->status;
     return seq == 1 ? fb200_delta_step(dev, a) : fb200_delta_prompt(dev, a);
   }
   if (c.mixer == FB200_MIX_LINEAR) {
@@ -492,7 +492,7 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
   fb200_device* dev = m->dev;
   fb200_hybrid* hy = m->hybrid;
   const size_t E = m->cfg.hidden, nb = m->cfg.max_batch;
-  size_t q = 0, qk = 0, hv = 0, o = 0, heads = 0, kvh = 0, qa = 0, part = 0, done = 0, seg = 0;
+  size_t q = 0, qk = 0, hv = 0, o = 0, heads = 0, kvh = 0, qa = 0, part = 0, done = 0, seg = 0, wq = 0;
   for (const auto& M : hy->mixers) {
     const auto& c = M.c;
     if (c.mixer == FB200_MIX_DELTA) {
@@ -500,6 +500,7 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
       hv = std::max(hv, (size_t)M.ko);
       heads = std::max(heads, (size_t)c.heads);
       kvh = std::max(kvh, (size_t)c.kv_heads);
+      if (fb200_delta_chunks(M.dp)) wq = std::max(wq, (size_t)c.heads * M.dp * 64);
     } else if (c.mixer == FB200_MIX_LINEAR) {
       o = std::max(o, (size_t)M.ko);
       if (!hy->f32) {
@@ -523,6 +524,7 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
   for (const auto& M : hy->mixers)
     if (M.c.mixer == FB200_MIX_DELTA) o = std::max(o, hv);
   hy->done_linear = done;
+  const size_t chunks = (rows + 31 * nb) / 32;
   bool norm2 = false;
   for (const auto& L : hy->layers) norm2 = norm2 || L.norm2;
   const size_t hb = std::max((norm2 ? 2 : 1) * up_to(E, 64), hy->w_loop ? (size_t)hy->w_loop->k : 0);
@@ -530,7 +532,8 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
       {(void**)&m->x, rows * hy->ldx * 4}, {(void**)&hy->x2, hy->w_loop ? rows * hy->ldx * 4 : 0}, {(void**)&m->xn, (norm2 ? 2 : 1) * rows * E * 4},
       {(void**)&hy->proj, rows * hy->ldy * 4}, {(void**)&hy->zf, rows * hy->ldz * 4}, {(void**)&hy->hb, rows * hb * 2},
       {(void**)&hy->zb, rows * hy->ldz * 2}, {(void**)&hy->qn, rows * q * 4}, {(void**)&hy->kn, rows * qk * 4}, {(void**)&hy->vn, rows * hv * 4},
-      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 7 * nb) / 8 * kvh * 256 + 64}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
+      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 7 * nb) / 8 * kvh * 256 + 64}, {(void**)&hy->wq, wq * chunks * 4},
+      {(void**)&hy->dec, wq ? chunks * heads * 36 * 4 : 0}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
       {(void**)&hy->qa, qa * 4}, {(void**)&hy->part, part * 4}, {(void**)&hy->done, (done + nb) * 4}};
   for (auto& b : bufs) {
     if (*b.p) { cudaFree(*b.p); *b.p = nullptr; }
@@ -640,7 +643,7 @@ void fb200_hybrid_free(fb200_llama* m) {
     for (void* b : bufs) if (b) cudaFree(b);
   }
   if (hy->w_loop) fb200_qmatrix_free(hy->w_loop);
-  void* bufs[] = {hy->proj, hy->zf, hy->hb, hy->zb, hy->qn, hy->kn, hy->vn, hy->gb, hy->kq, hy->o, hy->seg, hy->qa, hy->part, hy->done, hy->x2, hy->kvx};
+  void* bufs[] = {hy->proj, hy->zf, hy->hb, hy->zb, hy->qn, hy->kn, hy->vn, hy->gb, hy->kq, hy->wq, hy->dec, hy->o, hy->seg, hy->qa, hy->part, hy->done, hy->x2, hy->kvx};
   for (void* b : bufs) if (b) cudaFree(b);
   delete hy;
   m->hybrid = nullptr;

@@ -27,7 +27,11 @@ struct fb200_delta_args {
   // prompt pass scratch: unit q and k [rows][hk][dp], v [rows][h v], (decay, write strength) [rows][h][2],
   // products of eight tokens' k and q [b][ceil(s / 8)][hk][64], read-out [rows][h v]
   float *qn, *kn, *vn, *gb, *kq, *o;
+  // chunks of 32 tokens: [b][h][ceil(s / 32)] of two matrices [32][dp], and of 36 decays
+  float *wq, *dec;
+  int* status;
 };
+bool fb200_delta_chunks(int dp);                                   // whether prompts of this head size may use wq and dec
 int fb200_delta_dp(int d);                                         // padded head size, 0 when d is not covered
 int fb200_delta_step(fb200_device* dev, const fb200_delta_args& a);    // s == 1: one kernel
 int fb200_delta_prompt(fb200_device* dev, const fb200_delta_args& a);  // s > 1

@@ -102,6 +102,18 @@ def test_delta_layer(dev, dtype, shape):
     check(dev, cfg, w, t, dtype, [17, 1])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=3, kv_heads=3, dim=33, vdim=17, conv=2), dict(heads=2, kv_heads=1, dim=128, vdim=128),
+                                   dict(heads=2, kv_heads=2, dim=100, vdim=130, conv=5)], ids=str)
+@pytest.mark.parametrize("sizes", [[192], [223, 1], [193, 200], [5, 256, 3]], ids=str)
+def test_delta_prompts_in_chunks(dev, dtype, shape, sizes):
+    # prompts of 192 tokens and more go in chunks of 32: whole ones, one token in the last, all but one, a state of an earlier pass in
+    # front and a pass of another form behind; columns that do not fill a group of 16
+    cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
+    w = U.weights(cfg, 50 + sum(sizes), U.identity_head(cfg))
+    check(dev, cfg, w, toks(cfg, sum(sizes)), dtype, sizes)
+
+
 LATENTS = [dict(), dict(heads=1, dim=8, rot=2, vdim=8, rank=8, window=1), dict(heads=5, dim=24, rot=8, vdim=48, rank=72, window=33, base=50.0),
            dict(heads=2, dim=20, rot=6, vdim=12, rank=30, window=7), dict(heads=4, dim=128, rot=64, vdim=128, rank=512, window=50),
            dict(heads=2, dim=64, rot=32, vdim=200, rank=136, window=64), dict(heads=3, dim=192, rot=72, vdim=72, rank=200, window=40, scale=0.2),
