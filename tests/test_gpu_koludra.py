@@ -103,6 +103,16 @@ def test_delta_layer(dev, dtype, shape):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [dict(heads=2, kv_heads=2, dim=132, vdim=132, conv=5), dict(heads=3, kv_heads=1, dim=64, vdim=260, conv=1), dict(heads=1, kv_heads=1, dim=4, vdim=4, conv=7)], ids=str)
+def test_delta_rows_in_pieces_of_four(dev, dtype, shape):
+    # the preparation and the read-out in 16-byte pieces: a head of two 128-channel blocks, three blocks of values, taps of more than
+    # four, passes of one to seventeen tokens (eight a warp) with the convolution's memory between them
+    cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
+    w = U.weights(cfg, 70, U.identity_head(cfg))
+    check(dev, cfg, w, toks(cfg, 45), dtype, [2, 17, 1, 8, 9])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=3, kv_heads=3, dim=33, vdim=17, conv=2), dict(heads=2, kv_heads=1, dim=128, vdim=128),
                                    dict(heads=2, kv_heads=2, dim=100, vdim=130, conv=5)], ids=str)
 @pytest.mark.parametrize("sizes", [[192], [223, 1], [193, 200], [5, 256, 3]], ids=str)
