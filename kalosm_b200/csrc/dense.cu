@@ -46,6 +46,7 @@ struct GemvArgs {
   float* z;
   int k, kx, row0, n_plain, gate0, up0, ff, act, ks, whole, units;
   float eps, alpha, softcap;
+  int beside;  // the kernel in front is waited for at the end, for those that wait for this one
 };
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(GV_THREADS, 2) dense_gemv_kernel(const GemvArg
       }
     }
   }
-  pdl_wait();
+  if (!a.beside) pdl_wait();
   // ---- the activation row: (RMS-normalised) f32, zero padding beyond kx
   auto root = [&](float ss) {  // of the mean square, over the CTA
 #pragma unroll
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(GV_THREADS, 2) dense_gemv_kernel(const GemvArg
     }
   }
   if (rest < a.units && part == 0 && lane == 0) store(rest, s0, s1);
+  if (a.beside) pdl_wait();
 }
 
 // ---- F32 weights, many rows: 64 output rows x 64 activation rows per CTA, 4 x 4 per thread
@@ -384,7 +386,7 @@ int fb200_dense_gemv(fb200_device* dev, const fb200_dense_job& j) {
   GemvArgs a = {};
   a.w = j.w->data; a.x = (const float*)j.x; a.norm_w = j.norm_w; a.ff_norm_w = j.ff ? j.ff_norm_w : nullptr; a.add = j.add; a.bias = j.bias;
   a.y = (float*)j.y; a.z = (float*)j.z; a.alpha = j.alpha; a.softcap = j.softcap; a.act = j.act;
-  a.k = (int)j.w->k; a.kx = j.kx; a.row0 = j.row0; a.n_plain = j.n_plain; a.gate0 = j.gate0; a.up0 = j.up0; a.ff = j.ff; a.eps = j.eps;
+  a.k = (int)j.w->k; a.kx = j.kx; a.row0 = j.row0; a.n_plain = j.n_plain; a.gate0 = j.gate0; a.up0 = j.up0; a.ff = j.ff; a.eps = j.eps; a.beside = j.beside;
   a.units = (j.n_plain + 1) / 2 + (j.act == FB200_FFN_GELU ? (j.ff + 1) / 2 : j.ff);
   if (a.units == 0) return FB200_OK;
   const size_t smem = (size_t)j.w->k * (a.ff_norm_w ? 8 : 4);

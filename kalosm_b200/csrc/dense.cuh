@@ -37,6 +37,9 @@ struct fb200_dense_job {
   size_t ff_off = 0;
   void* z = nullptr;
   size_t ldz = 0;
+  // one row: nothing that this product reads comes from the kernel in front, and that kernel let this one in behind a wait of its
+  // own for everything before it (a layer's mixer, with the layer's feed-forward rows behind it): it is waited for at the end only
+  bool beside = false;
 };
 
 int fb200_dense_product(fb200_device* dev, const fb200_dense_job& j);

@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_kernel(const fb200_lin
 #pragma unroll
     for (int i = 0; i < EPT / 2; ++i) s[i] = make_float2(0.f, 0.f);
   }
-  pdl_wait();
+  // beside an attention the projections are there; that kernel is waited for at the end, for those that wait for this one
+  if (!a.beside) pdl_wait();
   pdl_launch_dependents();
   const float2 g2 = make_float2(decay, decay);
   for (int t0 = 0; t0 < a.s; t0 += TOK) {
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_kernel(const fb200_lin
     __syncthreads();
   }
   if (c < a.v && a.commit) store_column<EPT, LS_LPC>(st, p, s);
+  if (a.beside) pdl_wait();
   if (a.s > 1) return;
   // one token: the last CTA of the sequence finishes its row
   __threadfence();

@@ -122,6 +122,7 @@ struct fb200_linear_args {
   size_t ldz;
   int z_bf16;
   int commit;  // 0: a dry run of a decode step, the state stays as it is
+  int beside;  // s == 1: the kernel in front is a softmax attention over the same projections, which let this one in behind its own wait
   int bf16;    // prompt operands may be bf16
   float* o;    // read-out [rows][h v]
   int* done;   // [b] arrival counters, zero between launches
