@@ -20,7 +20,7 @@
 
 namespace {
 
-constexpr int LQ_THREADS = 256, LA_WARPS = 4, LO_THREADS = 256;
+constexpr int LQ_THREADS = 256, LQ_AHEAD = 8, LA_WARPS = 4, LO_THREADS = 256;
 
 __device__ __forceinline__ float la_warp_sum(float v) {
 #pragma unroll
@@ -48,6 +48,22 @@ __global__ void __launch_bounds__(LQ_THREADS) latent_query_kernel(const fb200_la
   extern __shared__ __align__(16) float lsm[];  // query head [d + r], or partial sums [LQ_THREADS][E]
   __shared__ float red[LQ_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, b = row / a.s;
+  const int h = blockIdx.x / csplit, cs_i = blockIdx.x % csplit;
+  // W_uk^T q: a thread owns one 16-byte piece of the latent, groups of threads share the sum over d. The first pieces of W_uk do not
+  // depend on the kernel in front
+  const int np = a.rkp / E;
+  const T* w = reinterpret_cast<const T*>(a.w_ukv) + (size_t)h * a.d * a.rkp;
+  const int cper = (np + csplit - 1) / csplit, cend = min(np, (cs_i + 1) * cper);
+  uint4 pre[LQ_AHEAD];
+  if (h < heads) {
+    const int nc = min(cend - cs_i * cper, LQ_THREADS), groups = LQ_THREADS / max(nc, 1), c = tid % max(nc, 1), gr = tid / max(nc, 1);
+#pragma unroll
+    for (int k = 0; k < LQ_AHEAD; ++k) {
+      const int i = gr + k * groups;
+      pre[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (nc > 0 && gr < groups && i < a.d) pre[k] = *reinterpret_cast<const uint4*>(w + (size_t)i * a.rkp + (cs_i * cper + c) * E);
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
   const int pos = *a.pos_dev + row % a.s;
@@ -73,7 +89,6 @@ __global__ void __launch_bounds__(LQ_THREADS) latent_query_kernel(const fb200_la
     }
     return;
   }
-  const int h = blockIdx.x / csplit, cs_i = blockIdx.x % csplit;
   float* qs = lsm;
   float* part = lsm + ((a.d + 3) & ~3);
   const float* q = yr + (size_t)h * (a.d + a.r);
@@ -85,18 +100,25 @@ __global__ void __launch_bounds__(LQ_THREADS) latent_query_kernel(const fb200_la
     out[a.rk + half + i] = (v * cs[i] + u * sn[i]) * a.scale;
   }
   __syncthreads();
-  // W_uk^T q: a thread owns one 16-byte piece of the latent, groups of threads share the sum over d
-  const int np = a.rkp / E;
-  const T* w = reinterpret_cast<const T*>(a.w_ukv) + (size_t)h * a.d * a.rkp;
-  const int cper = (np + csplit - 1) / csplit, cend = min(np, (cs_i + 1) * cper);
   for (int c0 = cs_i * cper; c0 < cend; c0 += LQ_THREADS) {
     const int nc = min(cend - c0, LQ_THREADS), groups = LQ_THREADS / nc, c = tid % nc, gr = tid / nc;
     float acc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = 0.f;
     if (gr < groups) {
+      int i0 = gr;
+      if (c0 == cs_i * cper) {
+#pragma unroll
+        for (int k = 0; k < LQ_AHEAD; ++k, i0 += groups) {
+          float f[E];
+          unpack(pre[k], f, T());
+          const float q = i0 < a.d ? qs[i0] : 0.f;
+#pragma unroll
+          for (int e = 0; e < E; ++e) acc[e] = fmaf(f[e], q, acc[e]);
+        }
+      }
 #pragma unroll 8
-      for (int i = gr; i < a.d; i += groups) {
+      for (int i = i0; i < a.d; i += groups) {
         float f[E];
         unpack(*reinterpret_cast<const uint4*>(w + (size_t)i * a.rkp + (c0 + c) * E), f, T());
 #pragma unroll
@@ -299,7 +321,8 @@ __global__ void __launch_bounds__(LO_THREADS) latent_out_kernel(const fb200_late
 // position is read once for all of them. Tiles of 64 positions come by cp.async. S = Q K^T: a warp takes 16 positions; the queries
 // are split into a bf16 value and a bf16 remainder, so the scores keep them in (nearly) 32 bits. The row maxima meet in
 // shared memory, P is rounded to bf16, and O += P C runs with the latent columns cut over the four warps. NT: 8-column
-// tiles of the latent per warp at most. Positions before this pass are requested before the kernel in front has finished.
+// tiles of the latent per warp at most. Bound in a step: the chain of one or two CTAs (queries and cached rows by element with a division
+// each took 12 us of a layer's 22; in 16-byte pieces, a row per warp, 6). Positions before this pass are requested before the kernel in front has finished.
 constexpr int LM_KEYS = 64, LM_THREADS = 128, LM_PS = LM_KEYS + 8;
 
 template <int NT>
@@ -321,11 +344,13 @@ __global__ void __launch_bounds__(LM_THREADS) latent_attn_mma_kernel(const fb200
   const int chunks = n / 8;
   // rows of tile kt with old (position < base) == want, zeros beyond the split
   auto fetch = [&](int kt, bool old) {
-    for (int i = tid; i < LM_KEYS * chunks; i += LM_THREADS) {
-      const int kr = i / chunks, c = i % chunks, key = kt + kr;
+    for (int kr = warp; kr < LM_KEYS; kr += LM_THREADS / 32) {
+      const int key = kt + kr;
       const bool valid = key < k1;
       if ((!valid || key < base) != old) continue;
-      pf_cp16(pf_smem(Ks + (size_t)kr * stride + c * 8), cache + (size_t)(valid ? key : 0) * a.ldc + c * 8, valid);
+      const __nv_bfloat16* src = cache + (size_t)(valid ? key : 0) * a.ldc;
+      const uint32_t dst = pf_smem(Ks + (size_t)kr * stride);
+      for (int c = lane; c < chunks; c += 32) pf_cp16(dst + c * 16, src + c * 8, valid);
     }
   };
   if (k0 < k1) fetch(k0, true);
@@ -340,12 +365,30 @@ __global__ void __launch_bounds__(LM_THREADS) latent_attn_mma_kernel(const fb200
   if (k0 < k1) {
     fetch(k0, false);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int i = tid; i < 16 * n; i += LM_THREADS) {
-      const int hr = i / n, e = i % n;
-      const float q = h0 + hr < a.h ? a.qa[((size_t)row * a.h + h0 + hr) * n + e] : 0.f;
-      const __nv_bfloat16 hi = __float2bfloat16(q);
-      Qh[hr * stride + e] = hi;
-      Ql[hr * stride + e] = __float2bfloat16(q - __bfloat162float(hi));
+    // queries: four rows a warp, 16-byte pieces (n is a multiple of 16), three loads of all four rows before the first use
+    constexpr int QP = 3, ROWS = 16 / (LM_THREADS / 32);
+    for (int c0 = lane; c0 < n / 4; c0 += 32 * QP) {
+      float4 q[ROWS][QP];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int k = 0; k < QP; ++k) {
+          const int hr = warp + i * (LM_THREADS / 32), c = c0 + 32 * k;
+          q[i][k] = h0 + hr < a.h && c < n / 4 ? *reinterpret_cast<const float4*>(a.qa + ((size_t)row * a.h + h0 + hr) * n + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int k = 0; k < QP; ++k) {
+          const int hr = warp + i * (LM_THREADS / 32), c = c0 + 32 * k;
+          if (c >= n / 4) continue;
+          const float4 v = q[i][k];
+          const __nv_bfloat162 h01 = __floats2bfloat162_rn(v.x, v.y), h23 = __floats2bfloat162_rn(v.z, v.w);
+          const __nv_bfloat162 l01 = __floats2bfloat162_rn(v.x - __low2float(h01), v.y - __high2float(h01));
+          const __nv_bfloat162 l23 = __floats2bfloat162_rn(v.z - __low2float(h23), v.w - __high2float(h23));
+          *reinterpret_cast<uint2*>(Qh + hr * stride + 4 * c) = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+          *reinterpret_cast<uint2*>(Ql + hr * stride + 4 * c) = make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
+        }
     }
   }
   constexpr float LOG2E = 1.4426950408889634f;
