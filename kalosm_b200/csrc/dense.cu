@@ -391,7 +391,8 @@ int fb200_dense_gemv(fb200_device* dev, const fb200_dense_job& j) {
   if (a.units == 0) return FB200_OK;
   const size_t smem = (size_t)j.w->k * (a.ff_norm_w ? 8 : 4);
   const int per_sm = smem <= 100 * 1024 ? 2 : 1;
-  const int ctas = dev->sm_count * per_sm;
+  // all CTAs should run at once: one that waits for the place of a kernel beside starts its share when the others end theirs
+  const int ctas = std::max(dev->sm_count, dev->sm_count * per_sm - j.held);
   // whole rounds, and for the units that are left the split of K that one round has warps for
   a.whole = a.units / (ctas * GV_WARPS);
   const int left = a.units - a.whole * ctas * GV_WARPS;

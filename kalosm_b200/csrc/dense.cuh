@@ -40,6 +40,7 @@ struct fb200_dense_job {
   // one row: nothing that this product reads comes from the kernel in front, and that kernel let this one in behind a wait of its
   // own for everything before it (a layer's mixer, with the layer's feed-forward rows behind it): it is waited for at the end only
   bool beside = false;
+  int held = 0;  // places for its CTAs (two per SM) that the kernels beside it hold
 };
 
 int fb200_dense_product(fb200_device* dev, const fb200_dense_job& j);

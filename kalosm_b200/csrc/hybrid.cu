@@ -408,6 +408,17 @@ int run_mixer(fb200_llama* m, const Mixer& M, int pass, int batch, int seq, bool
   return fb200_latent_rows(dev, a);
 }
 
+// Places for two CTAs per SM of a product of one row that a mixer's kernels hold while they run, by their registers
+int held_places(const fb200_device* dev, const Mixer& M, int cap) {
+  const auto& c = M.c;
+  switch (c.mixer) {
+    case FB200_MIX_DELTA: return 2 * c.heads;                                     // 512 threads a head
+    case FB200_MIX_LINEAR: return c.heads * ((c.vdim + 15) / 16);                  // 256 threads a head and 16 columns
+    case FB200_MIX_LATENT: return c.heads * ((c.vdim + 31) / 32) + (c.heads + 15) / 16 * fb200_latent_nsplit(dev, 1, c.heads, c.window, cap);
+    default: return 0;
+  }
+}
+
 // x: the residual rows, updated in place
 int run_layer(fb200_llama* m, const MixerLayer& L, int pass, float* x, int batch, int seq, bool commit) {
   fb200_device* dev = m->dev;
@@ -448,6 +459,7 @@ int run_layer(fb200_llama* m, const MixerLayer& L, int pass, float* x, int batch
     if (ffn.ff_norm_w) ffn.norm_w = ffn.ff_norm_w;
     ffn.ff_norm_w = nullptr;
     ffn.beside = true;
+    for (int k = 0; k < L.count; ++k) ffn.held += held_places(dev, hy->mixers[L.first + k], m->cfg.max_seq_len);
   }
   if ((rc = fb200_dense_product(dev, in))) return rc;
 
