@@ -438,6 +438,7 @@ __device__ __noinline__ float load_act_ll(const fb200_ll_act& row, int K, int Kp
 
 struct Smem {
   uint8_t* xl;
+  const uint8_t* zeros;       // ZERO_BYTES of zeros
   float* xsc;
   float* xss;
   float* pieces;              // [FW][2][32]
@@ -551,7 +552,8 @@ __device__ __forceinline__ void gemv_phase(const FusedArgs& A, const fb200_fused
         if (cc.type == FB200_Q4_K) run([&](const uint8_t* tg, const Group2Ptrs& G2) { group2_q4k(G2.xq, G2.xsp, tg, L, acc_g, acc_g8); });
         else run([&](const uint8_t* tg, const Group2Ptrs& G2) { group2_q6k(G2.xq, G2.xsp, tg, L, acc_g, acc_g8); });
       } else {
-      GroupPtrs G = group_ptrs(L, S.xl, S.xsc, S.xss, cc.kg, blocks16);
+      FeedZeros B;
+      GroupPtrs G = group_ptrs(L, S.xl, S.zeros, S.xsc, S.xss, cc.kg, blocks16);
       auto run = [&](auto group_fn) {
         for (int kg = cc.kg; kg < kend; ++kg) {
           mbar_wait(R.bar0 + 8 * slot, (R.par >> slot) & 1u, A.status);
@@ -564,7 +566,7 @@ __device__ __forceinline__ void gemv_phase(const FusedArgs& A, const fb200_fused
       if (cc.type == FB200_Q4_K) {
         run([&](const uint8_t* tg) { group1_q4k(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8); });
       } else if (cc.type == FB200_Q6_K) {
-        run([&](const uint8_t* tg) { group1_q6k(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8); });
+        run([&](const uint8_t* tg) { group1_q6k(B, G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8); });
       } else if (LEGACY) {
         if (cc.type == FB200_Q8_0) run([&](const uint8_t* tg) { group1_q8_0(G.xq, G.xscp, tg, L, acc_g, acc_g8); });
         else run([&](const uint8_t* tg) { group1_q4_0(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8); });
@@ -819,8 +821,11 @@ fused_step_kernel(const FusedArgs A) {
   constexpr int MS = LL ? MAX_STAGES_LL : MAX_STAGES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FW * RB);
   uint8_t* xreg = smem + FW * RB + FW * MS * 8;
+  __shared__ __align__(128) uint8_t zeros[LL ? 128 : ZERO_BYTES];
+  if (!LL && tid < ZERO_BYTES / 16) reinterpret_cast<uint4*>(zeros)[tid] = make_uint4(0u, 0u, 0u, 0u);
   Smem S;
   S.xl = xreg;
+  S.zeros = zeros;
   S.pieces = reinterpret_cast<float*>(xreg + A.xregion);
   S.tmp = S.pieces + FW * 2 * 32;
   S.keys = reinterpret_cast<unsigned long long*>(S.tmp + 32);

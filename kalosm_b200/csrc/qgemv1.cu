@@ -11,8 +11,8 @@
 //  * one launch may carry up to three matrices that share the activation row (the q, k and v
 //    projections), of different quant types;
 //  * the prologue turns x into int8 MMA B operands in shared memory once per CTA: optional
-//    residual add and RMSNorm (so the norm needs no kernel of its own), a power-of-two row
-//    scale, then FOUR 7-bit limbs per element, the bit fields of q = rint(x/scale * 2^27)
+//    residual add and RMSNorm (so the norm needs no kernel of its own), a power-of-two scale
+//    per 16 elements, then FOUR 7-bit limbs per element, the bit fields of q = rint(x/scale * 2^27)
 //    (x/scale = (l0 + u1/2^7 + u2/2^14 + u3/2^21) / 64 to 2^-28, l0 signed, u 0..127), plus the
 //    per-16 sums the offsets of Q4_K/Q4_0/Q6_K need;
 //  * quants stay in the byte domain: one logic op turns four packed nibbles into four u8
@@ -59,10 +59,11 @@ qgemv1_kernel(const Gemv1Args a) {
   constexpr int THREADS = W * 32;
   extern __shared__ __align__(128) uint8_t smem[];
   const int S = a.stages;
-  uint8_t* ring = smem;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + W * S * a.stride);
-  uint8_t* xl = smem + W * S * a.stride + W * S * 8;  // first raw f32 x, then limbs (4 B / element)
-  float* xf = reinterpret_cast<float*>(xl);
+  uint8_t* zeros = smem;  // written before the prologue's barrier
+  for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(zeros)[i] = make_uint4(0u, 0u, 0u, 0u);
+  uint8_t* ring = smem + ZERO_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + W * S * a.stride);
+  uint8_t* xl = ring + W * S * a.stride + W * S * 8;  // limbs (4 B / element)
   float* xsc = reinterpret_cast<float*>(xl + (size_t)a.Kp * 4);  // per-16 scale of the limbs
   float* xss = xsc + a.Kp / 16;    // per-16 sum of the activations
   float* red = xss + a.Kp / 16;    // [NP][W][16]
@@ -104,63 +105,61 @@ qgemv1_kernel(const Gemv1Args a) {
   pdl_wait();
 
   // ---- activation prologue ------------------------------------------------------------------
-  const float final_scale = 1.0f;  // the scale of the limbs travels in xsc
+  // One trip: every thread turns blocks of 8 elements into limbs as they arrive, under the power of two of their 16 elements
+  // (q = rint(v / scale 2^27); l0 = q >> 21 signed, u1, u2, u3 = the next three 7-bit fields), and adds up the squares; 1 / rms
+  // goes to the outputs. One scale for the whole row took a second pass behind a block reduction. Together with the operand
+  // loads of qgemv1_groups.cuh, before -> now, back to back on weights that are not in L2: 6144 x 4096 Q4_K 9.4 -> 7.5 us,
+  // 4096 x 4096 Q4_0 8.2 -> 7.6 and Q8_0 9.3 -> 7.9, 28672 x 4096 Q4_K with SwiGLU 22.5 -> 20.4, 4096 x 14336 Q6_K 19.9 -> 17.3,
+  // 128256 x 4096 Q6_K 80.5 -> 75.8 (5.7 TB/s) and Q4_K 62.9 -> 54.5 (5.4 TB/s).
   {
-  // pass 1: v = x (+ residual) -> shared memory as f32;
-    //         sum of squares and max |v * norm_w| in one block reduction
-    float ss = 0.f, amax = 0.f;
-    {
-      for (int k = threadIdx.x; k < a.Kp; k += THREADS) {
-        float v = 0.f;
-        if (k < a.K) {
-          v = a.x[k];
-          if (a.xres) v += a.xres[k];
-          ss = fmaf(v, v, ss);
-          amax = fmaxf(amax, fabsf(a.norm_w ? v * a.norm_w[k] : v));
-        }
-        xf[k] = v;
-      }
-    }
+    const bool vec = !((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.xres) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15);
+    float ss = 0.f;
+    auto get = [&](const float* p, int k, float (&v)[8]) {
+      if (vec && k + 8 <= a.K) {
+        const float4 u = *reinterpret_cast<const float4*>(p + k), w = *reinterpret_cast<const float4*>(p + k + 4);
+        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
+      } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-      amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    }
-    if (lane == 0) { tmp[warp] = ss; tmp[W + warp] = amax; }
-    __syncthreads();
-    ss = 0.f; amax = 0.f;
-    for (int i = 0; i < W; ++i) { ss += tmp[i]; amax = fmaxf(amax, tmp[W + i]); }
-    float rms = 1.f;
-    if (a.norm_w) {
-      // rms_norm_fused_cpu_impl, fusor-ml/fusor/src/composite/normalization.rs:404-461
-      rms = sqrtf(ss / (float)a.K + a.eps);
-      amax = amax / rms * 1.0000005f;  // bound of |(v / rms) * w| with rounding slack
-    }
-    int ex = 0;
-    if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);  // amax = f * 2^ex, f in [0.5, 1)
-    const float inv64 = ldexpf(64.0f, -ex);               // x * inv64 in (-64, 64)
-    const float out_scale = ldexpf(1.0f, ex - 13);        // 2^ex / (64 * 128)
-    // pass 2: each thread turns whole 8-element blocks, in place, into four int8 limbs per element:
-    // q = rint(v * 2^21) (|q| <= 2^27), l0 = q >> 21 (signed), u1, u2, u3 = the next three 7-bit
-    // fields (0..127), so v = (l0 + u1/2^7 + u2/2^14 + u3/2^21) up to 2^-22.
-    const float qscale = inv64 * 2097152.0f;
-    const float inv_rms = 1.0f / rms;  // v * (1/rms) instead of v / rms: within 1.5 ulp of the division
+        for (int i = 0; i < 8; ++i) v[i] = k + i < a.K ? p[k + i] : 0.f;
+      }
+    };
     const int nblk = a.Kp >> 3;
     for (int b0 = 0; b0 < nblk; b0 += THREADS) {
-      const int kb = b0 + threadIdx.x;
-      float sum = 0.f;
-      uint32_t wl[2][4];  // [half of the block][limb 3, 2, 1, 0] four elements per word
-      if (kb < nblk) {
-        const float4 va = *reinterpret_cast<const float4*>(xf + kb * 8);
-        const float4 vb = *reinterpret_cast<const float4*>(xf + kb * 8 + 4);
-        const float vin[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-        uint32_t r[8];
+      const int kb = b0 + (int)threadIdx.x;
+      const bool in = kb < nblk;  // (blocks come in pairs of lanes)
+      float v[8], w[8], amax = 0.f;
+      if (kb * 8 < a.Kp) {
+        get(a.x, kb * 8, v);
+        if (a.norm_w) get(a.norm_w, kb * 8, w);
+        if (a.xres) {
+          float r[8];
+          get(a.xres, kb * 8, r);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] += r[i];
+        }
+      }
+      if (in) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int k = kb * 8 + i;
-          float v = vin[i];
-          if (a.norm_w && k < a.K) v = (v * inv_rms) * a.norm_w[k];
-          const int q = __float2int_rn(v * qscale);
+          if (a.norm_w) {
+            ss = fmaf(v[i], v[i], ss);
+            v[i] *= w[i];
+          }
+          amax = fmaxf(amax, fabsf(v[i]));
+        }
+      }
+      amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+      int ex = 0;
+      if (amax > 0.f && amax < 3.0e38f) frexpf(amax, &ex);  // amax = f * 2^ex, f in [0.5, 1)
+      ex = max(ex, -110);                                   // 2^(6 - ex) and 2^(ex - 13) stay in range
+      const float inv64 = ldexpf(64.0f, -ex);               // v * inv64 in (-64, 64)
+      const float out_scale = ldexpf(1.0f, ex - 13);        // 2^ex / (64 * 128)
+      float sum = 0.f;
+      if (in) {
+        uint32_t r[8], wl[2][4];  // [half of the block][limb 3, 2, 1, 0] four elements per word
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int q = __float2int_rn((v[i] * inv64) * 2097152.0f);
           sum += (float)q;
           // fields at bits 0, 7, 14, 21 -> bytes 0..3 (byte 3 = bits 21..28 = l0 as s8)
           r[i] = ((uint32_t)q & 0x7Fu) | (((uint32_t)q << 1) & 0x7F00u) | (((uint32_t)q << 2) & 0x7F0000u) |
@@ -176,28 +175,40 @@ qgemv1_kernel(const Gemv1Args a) {
           wl[hb][2] = __byte_perm(t01h, t23h, 0x5410);  // u1
           wl[hb][3] = __byte_perm(t01h, t23h, 0x7632);  // l0
         }
-      }
-      // per-16 sums in the units of the integer dot products (128 * sum(v) = sum(q) / 2^14);
-      // the shuffle also orders the reads above before the writes below: a block's limbs go to
-      // the place of another block of the same aligned group of four (limb_block)
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-      __syncwarp();
-      if (kb < nblk) {
         uint4* dst = reinterpret_cast<uint4*>(xl + (size_t)limb_block(kb) * 32);
         dst[0] = make_uint4(wl[0][3], wl[1][3], wl[0][1], wl[1][1]);  // limb 0, limb 2
         dst[1] = make_uint4(wl[0][2], wl[1][2], wl[0][0], wl[1][0]);  // limb 1, limb 3
-        if ((threadIdx.x & 1) == 0) {
-          xsc[kb >> 1] = out_scale;
-          xss[kb >> 1] = sum * (1.0f / 16384.0f) * out_scale;
-        }
+      }
+      // per-16 sums in the units of the integer dot products (128 * sum(v) = sum(q) / 2^14)
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+      if (in && (threadIdx.x & 1) == 0) {
+        xsc[kb >> 1] = out_scale;
+        xss[kb >> 1] = sum * (1.0f / 16384.0f) * out_scale;
       }
     }
+    if (a.norm_w) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+      if (lane == 0) tmp[warp] = ss;
+    }
     __syncthreads();
+    if (threadIdx.x < 16) {  // the half warp that forms the outputs
+      float fs = 1.f;
+      if (a.norm_w) {
+        ss = 0.f;
+        for (int i = 0; i < W; ++i) ss += tmp[i];
+        // rms_norm_fused_cpu_impl, fusor-ml/fusor/src/composite/normalization.rs:404-461
+        fs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
+      }
+      __syncwarp(0xFFFFu);
+      if (threadIdx.x == 0) tmp[0] = fs;
+      __syncwarp(0xFFFFu);
+    }
   }
-  __syncthreads();
 
   int item = 0, st = 0;
   uint32_t phase = 0;
+  FeedB B(L);
   constexpr int BLOCKS16 = (TYPE == FB200_Q4_K || TYPE == FB200_Q6_K) ? 16 : 8;  // 16-element blocks per K group
   for (int j = 0; j < my_units; ++j) {
     const int tile = (int)blockIdx.x + j * (int)gridDim.x;
@@ -205,11 +216,11 @@ qgemv1_kernel(const Gemv1Args a) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       float acc_g = 0.f, acc_g8 = 0.f;
-      GroupPtrs G = group_ptrs(L, xl, xsc, xss, warp, BLOCKS16);
+      GroupPtrs G = group_ptrs(L, xl, zeros, xsc, xss, warp, BLOCKS16);
       for (int kk = 0; kk < gw; ++kk, ++item) {
         mbar_wait(my_bar + 8 * st, phase, a.status);
         const uint8_t* tg = my_ring + st * a.stride;
-        group1_any(TYPE, G, tg, L, acc_g, acc_g8);
+        group1_any(TYPE, B, G, tg, L, acc_g, acc_g8);
         // Every lane has read the stage (its loads precede this barrier in program order and
         // shared loads complete long before a refill from global memory can land).
         __syncwarp();
@@ -236,7 +247,7 @@ qgemv1_kernel(const Gemv1Args a) {
       for (int p = 0; p < NP; ++p) {
         float s = 0.f;
         for (int w = 0; w < W; ++w) s += red[(p * W + w) * 16 + r];
-        v[p] = s * final_scale;
+        v[p] = s * tmp[0];
       }
       if (n < a.n_out) {
         float out;
@@ -261,7 +272,7 @@ constexpr int SMEM_LIMIT = 227 * 1024;
 template <int EPI, int W>
 size_t gemv1_smem(int stages, int stride, int kp) {
   constexpr int NP = EPI == 2 ? 2 : 1;
-  return (size_t)W * stages * stride + (size_t)W * stages * 8 + (size_t)kp * 4 + (size_t)kp / 16 * 4 +
+  return (size_t)ZERO_BYTES + (size_t)W * stages * stride + (size_t)W * stages * 8 + (size_t)kp * 4 + (size_t)kp / 16 * 4 +
          (size_t)kp / 16 * 4 + (size_t)NP * W * 16 * 4 + (size_t)2 * W * 4 + 64;
 }
 
@@ -307,7 +318,8 @@ int launch_cfg(fb200_device* dev, Gemv1Args& a) {
   for (int s = 3; s >= 2; --s)
     if (fits(gemv1_smem<EPI, 16>(s, a.stride, a.Kp), 2)) { a.stages = s; return launch_w<TYPE, EPI, 16, 2>(dev, a); }
   for (int s = 2; s >= 1; --s)
-    if (fits(gemv1_smem<EPI, 32>(s, a.stride, a.Kp), 1)) { a.stages = s; return launch_w<TYPE, EPI, 32, 1>(dev, a); }
+    // (the zeros come out of the 2 KB that are left free: no row length is refused for them)
+    if (fits(gemv1_smem<EPI, 32>(s, a.stride, a.Kp) - ZERO_BYTES, 1)) { a.stages = s; return launch_w<TYPE, EPI, 32, 1>(dev, a); }
   return fb200_fail(dev, FB200_ERR_CAPACITY, "qgemv1: K = %d does not fit in shared memory", a.K);
 }
 

@@ -17,7 +17,12 @@
 // index kb ^ ((kb >> 2) & 3) (limb_block()), i.e. byte bits 5-6 are XOR-ed with bits 7-8. The
 // lanes that feed B in one load differ exactly in bits 7-8 (their scale group t), so the swizzle
 // spreads them over all 32 banks and a B load is a single conflict-free wavefront. Lanes that do
-// not feed B skip the load (their operand is zero).
+// not feed B have a zero operand. A load that only some lanes take, written as a branch around it, costs the
+// branch and four moves of zeros, so these lanes read zeros from shared memory, in other banks than the feeding
+// lanes. In the stand-alone Q6_K product, where shared memory is the bound, they keep registers that are zero from
+// the start instead and load under a predicate (FeedB): 128256 x 4096 took 80 us with branches, 88 with zeros and
+// 78 with predicates. 16 steps of a Llama-8B decoder, one persistent kernel: 32.7 ms with branches, 32.5 with
+// predicates, 32.2 with zeros.
 //
 // Pointer arguments are already advanced to the K group `kg`:
 //   xq[o] = limbs + (g & 1) * 16 + t * 128 + ((o ^ t) << 5) + kg * 4 * group_elems, o = 0..3
@@ -46,18 +51,32 @@ __device__ __forceinline__ Lane make_lane(int lane) {
 // Block index in shared memory of the limbs of 8-element group kb.
 __device__ __forceinline__ int limb_block(int kb) { return kb ^ ((kb >> 2) & 3); }
 
-// The four limb pointers of a lane for K group 0.
-__device__ __forceinline__ void lane_limb_ptrs(const Lane& L, const uint8_t* xl, const uint8_t* (&xq)[4]) {
-#pragma unroll
-  for (int o = 0; o < 4; ++o) xq[o] = xl + (L.g & 1) * 16 + L.t * 128 + ((o ^ L.t) << 5);
-}
+// Zeros for the lanes that do not feed B: the largest offset of a load inside a K group, and the place among the banks.
+constexpr int ZERO_BYTES = 512 + 128;
 
-// 16 limb bytes of a lane that feeds B, zero otherwise.
-__device__ __forceinline__ uint4 ldb(const Lane& L, const uint8_t* p) {
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (L.feeds) v = *reinterpret_cast<const uint4*>(p);
+// 16 limb bytes of a lane that feeds B, zeros otherwise; p: shared address.
+__device__ __forceinline__ uint4 ldb(uint32_t p) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(p));
   return v;
 }
+struct FeedZeros {
+  __device__ __forceinline__ uint4 load(int, uint32_t p) const { return ldb(p); }
+};
+struct FeedB {
+  uint4 v[2];
+  uint32_t feeds;
+  __device__ __forceinline__ explicit FeedB(const Lane& L) : feeds(L.feeds) {
+#pragma unroll
+    for (auto& x : v) x = make_uint4(0u, 0u, 0u, 0u);
+  }
+  __device__ __forceinline__ const uint4& load(int i, uint32_t p) {
+    asm volatile("{\n.reg .pred f;\nsetp.ne.u32 f, %5, 0;\n@f ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n}"
+                 : "+r"(v[i].x), "+r"(v[i].y), "+r"(v[i].z), "+r"(v[i].w)
+                 : "r"(p), "r"(feeds));
+    return v[i];
+  }
+};
 
 __device__ __forceinline__ uint4 lds16(const uint8_t* p) { return *reinterpret_cast<const uint4*>(p); }
 
@@ -77,7 +96,7 @@ __device__ __forceinline__ float limbs_to_float(int c_l0, int c_l1, int c_l2, in
 
 __device__ __forceinline__ float2 lds_f2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
-__device__ __forceinline__ void group1_q4_0(const uint8_t* const (&xq)[4], const float* xscp, const float* xssp,
+__device__ __forceinline__ void group1_q4_0(const uint32_t (&xq)[4], const float* xscp, const float* xssp,
                                             const uint8_t* tg, const Lane& L, float& acc_g, float& acc_g8) {
   const uint4 qa = lds16(tg + L.g * 64 + L.t * 16);
   const uint4 qb = lds16(tg + 512 + L.g * 64 + L.t * 16);
@@ -92,7 +111,7 @@ __device__ __forceinline__ void group1_q4_0(const uint8_t* const (&xq)[4], const
     int c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int sw = 0; sw < 2; ++sw) {
-      const uint4 v = ldb(L, xq[hf * 2 + sw]);
+      const uint4 v = ldb(xq[hf * 2 + sw]);
       const int w0 = sw * 2;
       if (hf == 0)
         step<false>(c1, c2, wa[w0] & 0x0F0F0F0Fu, wb[w0] & 0x0F0F0F0Fu, wa[w0 + 1] & 0x0F0F0F0Fu,
@@ -110,7 +129,7 @@ __device__ __forceinline__ void group1_q4_0(const uint8_t* const (&xq)[4], const
   acc_g8 = fmaf(d_g8, f_g8 - sx8, acc_g8);
 }
 
-__device__ __forceinline__ void group1_q8_0(const uint8_t* const (&xq)[4], const float* xscp, const uint8_t* tg,
+__device__ __forceinline__ void group1_q8_0(const uint32_t (&xq)[4], const float* xscp, const uint8_t* tg,
                                             const Lane& L, float& acc_g, float& acc_g8) {
   uint4 q[2][2];  // [h][half]
 #pragma unroll
@@ -125,8 +144,8 @@ __device__ __forceinline__ void group1_q8_0(const uint8_t* const (&xq)[4], const
   for (int hf = 0; hf < 2; ++hf) {
     int c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0};
     const uint4 a = q[0][hf], b = q[1][hf];
-    step<true>(c1, c2, a.x, b.x, a.y, b.y, ldb(L, xq[hf * 2]));
-    step<true>(c1, c2, a.z, b.z, a.w, b.w, ldb(L, xq[hf * 2 + 1]));
+    step<true>(c1, c2, a.x, b.x, a.y, b.y, ldb(xq[hf * 2]));
+    step<true>(c1, c2, a.z, b.z, a.w, b.w, ldb(xq[hf * 2 + 1]));
     const float xs = hf ? xs2.y : xs2.x;
     f_g = fmaf(limbs_to_float(c1[0], c1[1], c2[0], c2[1]), xs, f_g);
     f_g8 = fmaf(limbs_to_float(c1[2], c1[3], c2[2], c2[3]), xs, f_g8);
@@ -138,7 +157,7 @@ __device__ __forceinline__ void group1_q8_0(const uint8_t* const (&xq)[4], const
 // Q4_K: chain ch covers sub-blocks 4ch .. 4ch+3; lane t owns sub-block 4ch + t, whose quants
 // are the low (t even) or high (t odd) nibbles of qs bytes 32 * (2ch + t/2) .. +32. High
 // nibbles are used in place as 16 * q and the factor goes into the scale.
-__device__ __forceinline__ void group1_q4k(const uint8_t* const (&xq)[4], const float* xscp, const float* xssp,
+__device__ __forceinline__ void group1_q4k(const uint32_t (&xq)[4], const float* xscp, const float* xssp,
                                            const uint8_t* tg, const Lane& L, float& acc_g, float& acc_g8) {
   const uint32_t mask = (L.t & 1) ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
   const float nib_scale = (L.t & 1) ? 0.0625f : 1.0f;
@@ -166,8 +185,8 @@ __device__ __forceinline__ void group1_q4k(const uint8_t* const (&xq)[4], const 
       int c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0};
       const uint4 qa = lds16(tg + ((ch * 2 + 0) * 2 + half) * 256 + slot);
       const uint4 qb = lds16(tg + ((ch * 2 + 1) * 2 + half) * 256 + slot);
-      const uint4 v0 = ldb(L, xq[half * 2] + ch * 512);
-      const uint4 v1 = ldb(L, xq[half * 2 + 1] + ch * 512);
+      const uint4 v0 = ldb(xq[half * 2] + ch * 512);
+      const uint4 v1 = ldb(xq[half * 2 + 1] + ch * 512);
       step<false>(c1, c2, qa.x & mask, qb.x & mask, qa.y & mask, qb.y & mask, v0);
       step<false>(c1, c2, qa.z & mask, qb.z & mask, qa.w & mask, qb.w & mask, v1);
       const float xs = half ? xs2.y : xs2.x;
@@ -182,7 +201,8 @@ __device__ __forceinline__ void group1_q4k(const uint8_t* const (&xq)[4], const 
 
 // Q6_K: chain (c, u) covers the 16-element groups 8c + 2q + u, q = 0..3; lane t owns q = t:
 // nibble t/2 of ql plane slot t%2 and bits 2t, 2t+1 of qh, merged per byte into a u8 in 0..63.
-__device__ __forceinline__ void group1_q6k(const uint8_t* const (&xq)[4], const float* xscp, const float* xssp,
+template <class FEED>
+__device__ __forceinline__ void group1_q6k(FEED& B, const uint32_t (&xq)[4], const float* xscp, const float* xssp,
                                            const uint8_t* tg, const Lane& L, float& acc_g, float& acc_g8) {
   const int sh4 = 4 * (L.t >> 1);
   const int rot = (4 - 2 * L.t) & 31;  // rotate-left that brings bits 2t, 2t+1 of each byte to 4, 5
@@ -207,8 +227,8 @@ __device__ __forceinline__ void group1_q6k(const uint8_t* const (&xq)[4], const 
       const uint4 ha = lds16(tg + 2048 + (cu * 2 + 0) * 128 + L.g * 16);
       const uint4 hb = lds16(tg + 2048 + (cu * 2 + 1) * 128 + L.g * 16);
       // this lane's scale group in the super-block is 8c + 2t + u: steps o = 2u, 2u + 1
-      const uint4 v0 = ldb(L, xq[2 * u] + c * 512);
-      const uint4 v1 = ldb(L, xq[2 * u + 1] + c * 512);
+      const uint4 v0 = B.load(0, xq[2 * u] + c * 512);
+      const uint4 v1 = B.load(1, xq[2 * u + 1] + c * 512);
       int c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0};
       step<false>(c1, c2, merge(la.x, ha.x), merge(lb.x, hb.x), merge(la.y, ha.y), merge(lb.y, hb.y), v0);
       step<false>(c1, c2, merge(la.z, ha.z), merge(lb.z, hb.z), merge(la.w, ha.w), merge(lb.w, hb.w), v1);
@@ -225,32 +245,37 @@ __device__ __forceinline__ void group1_q6k(const uint8_t* const (&xq)[4], const 
 
 // Pointers of a lane for K group kg. group_elems = 128 (Q4_0, Q8_0) or 256 (Q4_K, Q6_K).
 struct GroupPtrs {
-  const uint8_t* xq[4];
+  uint32_t xq[4];  // shared addresses
   const float* xscp;
   const float* xssp;
+  uint32_t moves;  // 64 in a lane that feeds B: bytes of limbs per 16-element block; 0 otherwise
 };
-__device__ __forceinline__ GroupPtrs group_ptrs(const Lane& L, const uint8_t* xl, const float* xsc,
+// zeros: ZERO_BYTES, 128-byte aligned
+__device__ __forceinline__ GroupPtrs group_ptrs(const Lane& L, const uint8_t* xl, const uint8_t* zeros, const float* xsc,
                                                 const float* xss, int kg, int blocks16) {
   GroupPtrs G;
-  lane_limb_ptrs(L, xl, G.xq);
+  G.moves = L.feeds ? 64u : 0u;
 #pragma unroll
-  for (int o = 0; o < 4; ++o) G.xq[o] += kg * blocks16 * 64;
+  for (int o = 0; o < 4; ++o)
+    G.xq[o] = L.feeds ? smem_u32(xl) + (L.g & 1) * 16 + L.t * 128 + ((o ^ L.t) << 5) + kg * blocks16 * 64
+                      : smem_u32(zeros) + ((o ^ (L.g >> 1) ^ 1) << 5);
   G.xscp = xsc + kg * blocks16 + 2 * L.t;
   G.xssp = xss + kg * blocks16 + 2 * L.t;
   return G;
 }
 __device__ __forceinline__ void group_ptrs_next(GroupPtrs& G, int blocks16) {
 #pragma unroll
-  for (int o = 0; o < 4; ++o) G.xq[o] += blocks16 * 64;
+  for (int o = 0; o < 4; ++o) G.xq[o] += blocks16 * G.moves;
   G.xscp += blocks16;
   G.xssp += blocks16;
 }
 
 // One tile-group of any tiled type.
-__device__ __forceinline__ void group1_any(int type, const GroupPtrs& G, const uint8_t* tg, const Lane& L,
+template <class FEED>
+__device__ __forceinline__ void group1_any(int type, FEED& B, const GroupPtrs& G, const uint8_t* tg, const Lane& L,
                                            float& acc_g, float& acc_g8) {
   if (type == FB200_Q4_K) group1_q4k(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8);
-  else if (type == FB200_Q6_K) group1_q6k(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8);
+  else if (type == FB200_Q6_K) group1_q6k(B, G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8);
   else if (type == FB200_Q8_0) group1_q8_0(G.xq, G.xscp, tg, L, acc_g, acc_g8);
   else group1_q4_0(G.xq, G.xscp, G.xssp, tg, L, acc_g, acc_g8);
 }

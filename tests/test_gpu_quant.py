@@ -333,6 +333,38 @@ def test_single_row_large_k_and_tail_tiles(dev):
     assert dev.status() == 0
 
 
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("ty,n,k", [(O.Q4_0, 17, 32), (O.Q4_0, 40, 544), (O.Q8_0, 33, 96), (O.Q4K, 48, 256),
+                                    (O.Q6K, 40, 768), (O.Q6K, 24, 14336)])
+def test_single_row_scales_of_16(dev, ty, n, k, off):
+    # The limbs of the row carry one power of two per 16 elements. The blocks of x differ by up to 2^60, in a row that starts
+    # on a 16-byte boundary or 4 bytes behind one, with and without a norm, which goes to the outputs. Bound for an
+    # output: a limb is within 2^-27 of its block's largest |x|; eight float32 roundings per block at 2^-24, on terms up to
+    # eight times the weight (offset formats subtract): 2^-18 of sum over blocks 16 max|x| max|w|.
+    raw = weights(k + n, n, k, ty)
+    w = kb.QMatrix.from_raw_bytes(dev, (n, k), raw, ty)
+    w64 = O.dequantize(raw, ty, n * k).reshape(n, k).astype(np.float64)
+    rng = np.random.default_rng(k)
+    held = []
+
+    def put(v):
+        held.append(dev.tensor(np.concatenate([np.zeros(off, np.float32), v.ravel()])))
+        return kb.Tensor(dev, (1, k), np.float32, ptr=held[-1].ptr + 4 * off)
+
+    x = (rng.standard_normal((k // 16, 16)) * 2.0 ** rng.integers(-30, 31, (k // 16, 1))).astype(np.float32).reshape(1, k)
+    x[0, 16:32] = 0.0
+    for norm in (None, (1.0 + 0.1 * rng.standard_normal(k)).astype(np.float32)):
+        v = x.astype(np.float64)
+        if norm is None:
+            y = put(x).q_mat_mul(w).as_slice()
+        else:
+            y = put(x).rms_norm_q_mat_mul(put(norm), 1e-5, w).as_slice()
+            v = v / np.sqrt((v * v).mean() + 1e-5) * norm
+        tops = np.abs(v).reshape(-1, 16).max(1).sum() * 16
+        err = np.abs(y[0] - (w64 @ v[0]))
+        assert (err <= 2.0 ** -18 * tops * np.abs(w64).max(1)).all(), (norm is None, err.max())
+
+
 Q5_TYPES = {"q5_0": O.Q5_0, "q5k": O.Q5K}
 
 
