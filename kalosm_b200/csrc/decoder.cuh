@@ -35,6 +35,8 @@ struct fb200_llama {
   float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr,
         *attn_out = nullptr, *hbuf = nullptr, *gbuf = nullptr, *last = nullptr, *logits = nullptr;
   float* att_part = nullptr;
+  uint2* part_ll = nullptr;        // persistent step: partial rows of the attention's splits (in ll_slab)
+  unsigned* part_epoch = nullptr;  // and the epoch of the next launch's first phase
   size_t att_part_bytes = 0;
   uint32_t *ids = nullptr, *next = nullptr, *hist = nullptr;
   int hist_cap = 0;

@@ -69,6 +69,8 @@ struct FusedArgs {
   unsigned long long* trace;  // optional [nphases][8] time stamps of CTA 0 in the last step (ns)
   fb200_fused_xchg x;         // tensor-parallel exchange (world <= 1: none)
   unsigned epoch_base;        // flagged rows: epoch of phase 0 of this launch
+  const int* pos_dev;         // attention: position of a step (null: no attention phase)
+  unsigned* part_epoch;       // attention: epoch of the partial rows of phase 0 of this launch
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -789,11 +791,12 @@ __device__ __noinline__ void advance_phase(const FusedArgs& A, const fb200_fused
 // run time is mostly fixed latencies, so many small items finish sooner than few large ones, and
 // very short contexts run a single item per KV head with nothing to merge.
 template <int D, int ROWS, bool LL>
-__device__ __noinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm, unsigned lep, int* status) {
+__device__ __noinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm, unsigned lep, unsigned ep_part, int pos, int* status) {
   const int tid = threadIdx.x;
   if (tid >= DEC_THREADS) return;
   fb200_dec_args a = P.att;
-  a.pos_plus1 = __ldcg(a.pos_dev) + 1;
+  a.pos_plus1 = pos + 1;
+  a.ep_part = ep_part;
   const int skv = a.pos_plus1;
   a.nsplit = max(1, min(a.nsplit, (skv + FUSED_SPLIT_KEYS - 1) / FUSED_SPLIT_KEYS));
   a.ep_in = lep - 1u;
@@ -801,9 +804,14 @@ __device__ __noinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm
   a.status = status;
   const int nitems = a.b * a.hkv * a.nsplit;
   for (int item = (int)blockIdx.x; item < nitems; item += (int)gridDim.x) {
-    attn_decode_item<D, FUSED_DEC_CH, ROWS, 1, false, LL>(a, item, dsm, tid);
+    attn_decode_item<D, FUSED_DEC_CH, ROWS, 1, false, LL, 1, true>(a, item, dsm, tid);
     dec_sync<1>();
   }
+  if (a.nsplit > 1)
+    for (int blk = (int)blockIdx.x; blk < a.h * D / 32; blk += (int)gridDim.x) {
+      attn_merge_block<D, 1, LL>(a, blk, reinterpret_cast<float (*)[32]>(dsm), tid);
+      dec_sync<1>();
+    }
 }
 
 // One kernel variant per attention shape (head size D, query rows per KV head ROWS) and per
@@ -854,6 +862,13 @@ fused_step_kernel(const FusedArgs A) {
     uint4* dst = reinterpret_cast<uint4*>(sdesc + (g % DESC_SLOTS) * DESC_WORDS);
     for (int i = tid; i < DESC_WORDS / 4; i += FT) cp_async16(dst + i, src + i);
   };
+  // What the attention phases need, in shared memory because the product loop has no registers to spare: the step's position, and
+  // the epoch of the launch's partial rows. The epochs go on from launch to launch in the model's memory (a captured
+  // launch may be replayed): CTA 0 stores the next one at the end, when every CTA has passed a meeting. Without meetings
+  // the launch brings its own.
+  __shared__ int att_pos;
+  __shared__ unsigned att_ep;
+  if (tid == 0) att_ep = LL ? A.epoch_base : A.part_epoch ? ld_relaxed_u32(A.part_epoch) : 0u;
   for (int g = 0; g < DESC_SLOTS - 1; ++g) load_desc(g);
   cp_async_wait_all();
   __syncthreads();
@@ -882,6 +897,7 @@ fused_step_kernel(const FusedArgs A) {
       const unsigned lep = A.epoch_base + (unsigned)g;  // flagged rows: this phase's epoch
       unsigned long long* tr = A.trace && blockIdx.x == 0 && tid == 0 && step == A.nsteps - 1 ? A.trace + ph * 8 : nullptr;
       if (tr) tr[0] = global_ns();
+      if (ph == 0 && tid == 0 && A.pos_dev) att_pos = __ldcg(A.pos_dev);  // (a step moves it in its last phase)
       switch (P.kind) {
         case FB200_PH_GEMV: {
           S.xsc = reinterpret_cast<float*>(S.xl + (LL ? ((size_t)P.Kp / 8 * 18 + 63) / 64 * 64 : (size_t)P.Kp * 4));
@@ -896,7 +912,7 @@ fused_step_kernel(const FusedArgs A) {
           break;
         }
         case FB200_PH_ATTN:
-          attn_phase<D, ROWS, LL>(P, xreg, lep, A.status);
+          attn_phase<D, ROWS, LL>(P, xreg, lep, att_ep + (unsigned)g, att_pos, A.status);
           break;
         case FB200_PH_PACK:
         case FB200_PH_EMBED:
@@ -913,6 +929,7 @@ fused_step_kernel(const FusedArgs A) {
       cp_async_wait_all();  // this thread's part of the descriptor fetched during the phase (the meeting above publishes it)
     }
   }
+  if (!LL && A.part_epoch && blockIdx.x == 0 && tid == 0) *A.part_epoch = att_ep + (unsigned)(A.nsteps * A.nphases);
 }
 
 size_t x_region_need(const fb200_fused_phase* prog, int nphases, bool flagged) {
@@ -1125,6 +1142,8 @@ int fb200_fused_launch(fb200_device* dev, const fb200_fused_phase* prog_dev, con
   a.gp = reinterpret_cast<float*>((uint8_t*)dev->fused + gp_off);
   a.counters = reinterpret_cast<int*>((uint8_t*)dev->fused + cnt_off);
   a.status = dev->status;
+  for (int i = 0; i < nphases; ++i)
+    if (prog_host[i].kind == FB200_PH_ATTN) { a.pos_dev = prog_host[i].att.pos_dev; a.part_epoch = prog_host[i].att.part_epoch; }
   if (xchg) a.x = *xchg;
   if (flagged) {
     // one epoch per phase executed; 0 is the value of cleared buffers and is skipped when the

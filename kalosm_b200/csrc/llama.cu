@@ -281,7 +281,6 @@ int build_fused_program(fb200_llama* m) {
   int nsplit = grid / HK;
   if (nsplit > 32) nsplit = 32;
   if (nsplit < 1) nsplit = 1;
-  if ((size_t)nsplit * H * (D + 2) * sizeof(float) > m->att_part_bytes) return FB200_OK;
   auto gemv = [&](const fb200_qmatrix* const* ws, float* const* ys, int nw, int epi, fb200_fused_phase& p) {
     p = blank();
     p.eps = c.rms_eps;
@@ -303,7 +302,7 @@ int build_fused_program(fb200_llama* m) {
     p.att_d = D;
     p.att.q = m->q; p.att.k_new = m->k; p.att.v_new = m->v; p.att.kc = L.kc; p.att.vc = L.vc;
     p.att.rope_cos = m->rope_cos; p.att.rope_sin = m->rope_sin; p.att.pos_dev = m->pos_dev;
-    p.att.part = m->att_part; p.att.out = nullptr; p.att.done = m->att_done; p.att.out_packed = m->patt;
+    p.att.part_ll = m->part_ll; p.att.part_epoch = m->part_epoch; p.att.out = nullptr; p.att.out_packed = m->patt;
     p.att.b = 1; p.att.h = H; p.att.hkv = HK; p.att.groups = H / HK; p.att.cap = c.max_seq_len;
     p.att.nsplit = nsplit; p.att.scale = (float)(1.0 / sqrt((double)D));
     p.att.q_ll = m->q_ll; p.att.k_ll = m->k_ll; p.att.v_ll = m->v_ll; p.att.out_ll = m->patt_ll;
@@ -771,6 +770,9 @@ int fb200_llama_create(fb200_device* dev, const fb200_llama_config* cfg, fb200_l
     size_t bytes = 0;
     for (size_t n : packed_n) bytes += n / 16 * FB200_LL_GRANULES * sizeof(uint2);
     for (size_t n : f32_n) bytes += n * sizeof(uint2);
+    // the partial rows of up to 32 splits of an attention phase, and their epoch
+    const size_t part_n = (size_t)32 * c.n_head * (c.head_dim + 2);
+    bytes += 256 + part_n * sizeof(uint2);
     FB_CUDA(dev, cudaMalloc(&m->ll_slab, bytes));
     FB_CUDA(dev, cudaMemset(m->ll_slab, 0, bytes));
     uint8_t* p = m->ll_slab;
@@ -778,6 +780,10 @@ int fb200_llama_create(fb200_device* dev, const fb200_llama_config* cfg, fb200_l
     for (int i = 0; i < 4; ++i) { rows[i]->g = reinterpret_cast<uint2*>(p); p += packed_n[i] / 16 * FB200_LL_GRANULES * sizeof(uint2); }
     uint2** f32s[5] = {&m->q_ll, &m->k_ll, &m->v_ll, &m->x_ll, &m->attn_ll};
     for (int i = 0; i < 5; ++i) { *f32s[i] = reinterpret_cast<uint2*>(p); p += f32_n[i] * sizeof(uint2); }
+    m->part_ll = reinterpret_cast<uint2*>(p);
+    m->part_epoch = reinterpret_cast<unsigned*>(p + part_n * sizeof(uint2));
+    const unsigned first = 1;  // 0 is what cleared rows carry
+    FB_CUDA(dev, cudaMemcpy(m->part_epoch, &first, sizeof first, cudaMemcpyHostToDevice));
     if (const char* e = getenv("FB200_FUSED_LL")) m->fused_flagged = e[0] == '1' && e[1] == 0;
   }
   // attention split scratch: the largest a forward pass can ask for is bounded by 64 splits of

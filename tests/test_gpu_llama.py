@@ -140,6 +140,34 @@ def test_decode_over_a_long_context(dev, head_dim, n_head, n_kv_head, flagged_ro
     assert gpu.position == 291 + 5 + 6
 
 
+@pytest.mark.parametrize("flagged_rows", [False, True], ids=["grid-barriers", "flagged-rows"])
+@pytest.mark.parametrize("n_head,n_kv_head,prompt", [(48, 8, 30), (6, 2, 62)])
+def test_decode_across_split_counts(dev, n_head, n_kv_head, prompt, flagged_rows, monkeypatch):
+    # The merge of an attention phase: from one split to two and on (a split per 32 keys), more 32-element blocks of the row
+    # than CTAs (48 heads of 128) and fewer, launches of one step and of several, whose partial rows carry growing
+    # epochs in the same memory. Tolerance of the other decode tests: 2e-3 of the oracle's logits (fp16 cache).
+    monkeypatch.setenv("FB200_FUSED_LL", "1" if flagged_rows else "0")
+    cfg = dict(tiny_cfg(), ctx=128, head_dim=128, n_head=n_head, n_kv_head=n_kv_head)
+    gpu, cpu = build_models(dev, cfg, batch=1, seed=21)
+    rng = np.random.default_rng(prompt)
+    toks = rng.integers(0, cfg["vocab"], size=(1, prompt + 6), dtype=np.uint32)
+    gpu.forward(toks[:, :prompt])
+    cpu.forward(toks[:, :prompt])
+    for i in range(prompt, prompt + 6):
+        lg, _ = gpu.forward(toks[:, i:i + 1])
+        lo = cpu.forward(toks[:, i:i + 1])
+        assert F.rel_l2(lg, lo) < 2e-3, (i, F.rel_l2(lg, lo))
+    first = np.array([O.top_k(lo[0], 1)[0][0]], dtype=np.uint32)
+    run = gpu.generate_greedy(first, 34)[0]
+    t = first
+    for step in range(34):
+        lo = cpu.forward(t[:, None])
+        if run[step] != O.top_k(lo[0], 1)[0][0]:
+            assert _margin(lo)[0] < 1e-3, (step, _margin(lo)[0])
+            break
+        t = run[step:step + 1].astype(np.uint32)
+
+
 def test_model_loaded_from_a_gguf_file_equals_the_directly_built_one(dev, tmp_path):
     # checkpoint -> GGUF file -> kalosm_b200.gguf.load_llama: same bytes on the device as setting
     # the tensors one by one, so logits and greedy ids agree bit for bit
