@@ -43,7 +43,6 @@ struct fb200_dec_args {
   // persistent decode kernel: the splits' partial rows as granules {value, epoch}, and the epoch of the model's next launch
   uint2* part_ll;       // [nsplit][H][D + 2]
   unsigned* part_epoch;
-  unsigned ep_part;     // epoch of this phase
 };
 
 namespace {
@@ -84,27 +83,25 @@ __device__ __forceinline__ void dec_sync() {
 // One (batch, kv head, split) item, executed by DEC_THREADS threads (tid = 0 .. DEC_THREADS - 1).
 // DEC_CH = keys per shared-memory chunk; ROWS = query rows computed per KV head (>= H / Hkv). PDL: the caller is a kernel launched with programmatic
 // stream serialization, whose predecessor produced q, k_new and v_new.
-// Two neighbouring f32 granules (elements 2p, 2p + 1) of a flagged row, polled until both carry
-// `epoch` (bounded, like every wait).
-__device__ __forceinline__ float2 ld_ll_pair(const uint2* p, uint32_t epoch, int* status) {
-  const uint4* line = reinterpret_cast<const uint4*>(p);
-  uint4 v = ld_ll_line(line);
+// Polls the 16-byte line p (two neighbouring f32 granules, already read once into v) until both carry `epoch` (bounded,
+// like every wait).
+__device__ __forceinline__ float2 settle_ll_pair(uint4 v, const uint4* p, uint32_t epoch, int* status) {
   int polls = 0;
   while (v.y != epoch || v.w != epoch) {
     if (++polls > FB200_LL_POLL_LIMIT || ((polls & 63) == 0 && __ldcg(status) != 0)) {
       atomicExch(status, FB200_ERR_TIMEOUT);
       break;
     }
-    v = ld_ll_line(line);
+    v = ld_ll_line(p);
   }
   return make_float2(__uint_as_float(v.x), __uint_as_float(v.z));
 }
 
-// LLIO: q / k_new / v_new come in and the merged row goes out as flagged rows (see DecArgs).
+// LLIN: q / k_new / v_new come in as flagged rows, LLOUT: the merged row goes out as one (see DecArgs).
 // NB = 2: two staging buffers; the copy of chunk i + 1 runs while chunk i is being used, so a long
 // key range streams at the memory system's pace instead of paying its latency once per chunk.
 // SPREAD: the partial rows of more than one split leave as granules for attn_merge_block.
-template <int D, int DEC_CH, int ROWS, int BAR, bool PDL, bool LLIO = false, int NB = 1, bool SPREAD = false>
+template <int D, int DEC_CH, int ROWS, int BAR, bool PDL, bool LLIN = false, int NB = 1, bool SPREAD = false, bool LLOUT = false>
 __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int tid) {
   constexpr int ATT_THREADS = DEC_THREADS;
   constexpr int KSTR = D * 2 + 64;   // bytes per staged row: consecutive keys land 64 B apart mod 128
@@ -161,13 +158,16 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
   const bool has_new = kbeg <= pos && pos < kend;
   constexpr int QN = (ROWS * D + ATT_THREADS - 1) / ATT_THREADS;
   float qself[QN], qother[QN], qc[QN], qsn[QN];
+  uint4 ql[LLIN ? QN : 1], kl, vl;
 #pragma unroll
   for (int u = 0; u < QN; ++u) {
     const int i = tid + u * ATT_THREADS, r = i / D, e = i % D;
     qself[u] = qother[u] = qc[u] = qsn[u] = 0.f;
     if (i < ROWS * D && r < nrows) {
       const size_t qoff = ((size_t)bi * a.h + kvh * a.groups + r) * D;
-      if constexpr (!LLIO) {
+      if constexpr (LLIN) {
+        ql[u] = ld_ll_line(reinterpret_cast<const uint4*>(a.q_ll + qoff + (e & ~1)));
+      } else {
         qself[u] = __ldcg(a.q + qoff + e);
         if (pos >= 0) qother[u] = __ldcg(a.q + qoff + (e ^ 1));
       }
@@ -177,10 +177,13 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
       }
     }
   }
+  const size_t koff = ((size_t)bi * a.hkv + kvh) * D + 2 * tid;
   float x0 = 0.f, x1 = 0.f, v0 = 0.f, v1 = 0.f, c = 0.f, sn = 0.f;
   if (has_new && tid < D / 2) {
-    const size_t koff = ((size_t)bi * a.hkv + kvh) * D + 2 * tid;
-    if constexpr (!LLIO) {
+    if constexpr (LLIN) {
+      kl = ld_ll_line(reinterpret_cast<const uint4*>(a.k_ll + koff));
+      vl = ld_ll_line(reinterpret_cast<const uint4*>(a.v_ll + koff));
+    } else {
       x0 = __ldcg(a.k_new + koff); x1 = __ldcg(a.k_new + koff + 1);
       v0 = __ldcg(a.v_new + koff); v1 = __ldcg(a.v_new + koff + 1);
     }
@@ -194,9 +197,9 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
     float v = 0.f;
     if (r < nrows) {
       // interleaved RoPE at the new position (fusor-ml/fusor/src/composite/rope.rs:77-108)
-      if constexpr (LLIO) {
+      if constexpr (LLIN) {
         const size_t qoff = ((size_t)bi * a.h + kvh * a.groups + r) * D;
-        const float2 pr = ld_ll_pair(a.q_ll + qoff + (e & ~1), a.ep_in, a.status);
+        const float2 pr = settle_ll_pair(ql[u], reinterpret_cast<const uint4*>(a.q_ll + qoff + (e & ~1)), a.ep_in, a.status);
         qself[u] = (e & 1) ? pr.y : pr.x;
         qother[u] = (e & 1) ? pr.x : pr.y;
       }
@@ -210,10 +213,9 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
   if (has_new && tid < D / 2) {
     // append the new position (KvCache::append, fusor-ml/fusor/src/cache/kv_cache.rs:50-62)
     const int p = tid;
-    if constexpr (LLIO) {
-      const size_t koff = ((size_t)bi * a.hkv + kvh) * D + 2 * p;
-      const float2 kp = ld_ll_pair(a.k_ll + koff, a.ep_in, a.status);
-      const float2 vp = ld_ll_pair(a.v_ll + koff, a.ep_in, a.status);
+    if constexpr (LLIN) {
+      const float2 kp = settle_ll_pair(kl, reinterpret_cast<const uint4*>(a.k_ll + koff), a.ep_in, a.status);
+      const float2 vp = settle_ll_pair(vl, reinterpret_cast<const uint4*>(a.v_ll + koff), a.ep_in, a.status);
       x0 = kp.x; x1 = kp.y; v0 = vp.x; v1 = vp.y;
     }
     const __half2 kh = __floats2half2_rn(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn)),
@@ -375,7 +377,7 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
         acc *= l > 0.f ? 1.0f / l : 0.f;
         if (a.out) a.out[grow * D + e] = acc;
       }
-      if constexpr (LLIO) {
+      if constexpr (LLOUT) {
         if (bi == 0 && valid) emit_ll16(a.out_ll, (int)(grow * D) + e, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
       } else {
         if (a.out_packed.limbs && bi == 0 && valid)
@@ -392,8 +394,8 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
     const size_t grow = (size_t)bi * a.h + kvh * a.groups + r;
     if constexpr (SPREAD) {
       uint2* pp = a.part_ll + ((size_t)split * rows_all + grow) * (D + 2);
-      st_ll(pp + e, __float_as_uint(s), a.ep_part);
-      if (e < 2) st_ll(pp + D + e, __float_as_uint(e == 0 ? row_m[r] : row_l[r]), a.ep_part);
+      st_ll(pp + e, __float_as_uint(s), a.ep_out);
+      if (e < 2) st_ll(pp + D + e, __float_as_uint(e == 0 ? row_m[r] : row_l[r]), a.ep_out);
     } else {
       float* pp = a.part + ((size_t)split * rows_all + grow) * (D + 2);
       pp[e] = s;
@@ -445,7 +447,7 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
       if (a.out) a.out[grow * D + e] = acc;
     }
     // packed rows are single-sequence; nrows * D is a multiple of 32, so `valid` is warp-uniform
-    if constexpr (LLIO) {
+    if constexpr (LLOUT) {
       if (bi == 0 && valid) emit_ll16(a.out_ll, (int)(grow * D) + e, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
     } else {
       if (a.out_packed.limbs && bi == 0 && valid)
@@ -461,7 +463,7 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
 // fence. With that gone and the loads of an item requested together, an attention phase with 520 cached keys (Llama 8B, 17
 // splits) takes 8.1 us instead of 11.5, and 16 steps 30.6 ms instead of 32.4. The caller's CTAs are all resident, and
 // none of them waits before its items are out. Waits are bounded as every wait.
-template <int D, int BAR, bool LLIO>
+template <int D, int BAR, bool LLOUT>
 __device__ __forceinline__ void attn_merge_block(const DecArgs& a, int blk, float (*pv)[32], int tid) {
   constexpr int W = DEC_THREADS / 32, MAXS = 32;
   const int warp = tid >> 5, lane = tid & 31;
@@ -474,25 +476,25 @@ __device__ __forceinline__ void attn_merge_block(const DecArgs& a, int blk, floa
     atomicExch(a.status, FB200_ERR_TIMEOUT);
     return true;
   };
-  uint4 ml = make_uint4(0xFF800000u, a.ep_part, 0u, a.ep_part);  // lane s: maximum (-inf) and normaliser of split s
+  uint4 ml = make_uint4(0xFF800000u, a.ep_out, 0u, a.ep_out);  // lane s: maximum (-inf) and normaliser of split s
   const uint4* pml = reinterpret_cast<const uint4*>(base + (lane < a.nsplit ? lane : 0) * sstride + D);
   if (warp == 0 && lane < a.nsplit) ml = ld_ll_line(pml);
   uint2 v[MAXS / W];
 #pragma unroll
   for (int j = 0; j < MAXS / W; ++j) {
-    v[j] = make_uint2(0u, a.ep_part);
+    v[j] = make_uint2(0u, a.ep_out);
     if (warp + W * j < a.nsplit) v[j] = ld_ll_granule(base + (warp + W * j) * sstride + e);
   }
 #pragma unroll
   for (int j = 0; j < MAXS / W; ++j) {
-    while (v[j].y != a.ep_part) {
+    while (v[j].y != a.ep_out) {
       if (give_up()) break;
       v[j] = ld_ll_granule(base + (warp + W * j) * sstride + e);
     }
     if (warp + W * j < a.nsplit) pv[warp + W * j][lane] = __uint_as_float(v[j].x);
   }
   if (warp == 0)
-    while (ml.y != a.ep_part || ml.w != a.ep_part) {
+    while (ml.y != a.ep_out || ml.w != a.ep_out) {
       if (give_up()) break;
       ml = ld_ll_line(pml);
     }
@@ -510,7 +512,7 @@ __device__ __forceinline__ void attn_merge_block(const DecArgs& a, int blk, floa
 #pragma unroll 8
     for (int s = 0; s < a.nsplit; ++s) acc = fmaf(pv[s][lane], __shfl_sync(0xFFFFFFFFu, wgt, s), acc);
     acc *= l > 0.f ? 1.0f / l : 0.f;
-    if constexpr (LLIO) emit_ll16(a.out_ll, n, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
+    if constexpr (LLOUT) emit_ll16(a.out_ll, n, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
     else emit_packed16(a.out_packed, n, acc, acc, true, 0xFFFFFFFFu);
   }
 }

@@ -70,7 +70,7 @@ struct FusedArgs {
   fb200_fused_xchg x;         // tensor-parallel exchange (world <= 1: none)
   unsigned epoch_base;        // flagged rows: epoch of phase 0 of this launch
   const int* pos_dev;         // attention: position of a step (null: no attention phase)
-  unsigned* part_epoch;       // attention: epoch of the partial rows of phase 0 of this launch
+  unsigned* part_epoch;       // attention: epoch of phase 0 of this launch, unless epoch_base gives it
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -353,7 +353,7 @@ __device__ __noinline__ void unit_epilogue(const fb200_fused_phase& P, int unit,
       out = v0;
     }
     if (yout) yout[n] = out;
-    if (LL && P.seg[sidx].yl) st_ll(P.seg[sidx].yl + n, __float_as_uint(out), E.ep);
+    if (P.seg[sidx].yl) st_ll(P.seg[sidx].yl + n, __float_as_uint(out), LL ? E.ep : P.epoch);
     if (XS && E.xs && sidx == 0) {
       // partial row of a tensor-parallel projection: straight into every rank's buffer (P2P stores)
       for (int r = 0; r < E.xs->world; ++r) E.xs->data[r][E.xs_off + n] = out;
@@ -464,7 +464,7 @@ __device__ __forceinline__ void gemv_phase(const FusedArgs& A, const fb200_fused
   E.best_key = 0ull;
   E.xs = XS && P.xs_index >= 0 && A.x.world > 1 ? &A.x : nullptr;
   E.xs_off = XS ? (int)((epoch & 1u) * (unsigned)A.x.world + (unsigned)A.x.me) * A.x.stride : 0;
-  E.ep = lep;
+  E.ep = LL ? lep : 0u;
   if constexpr (LL) {
     // ---- activation row: poll the producers' flagged row straight into shared memory. A CTA
     // without items in this phase needs no activations and goes on to the next phase.
@@ -639,12 +639,15 @@ __device__ __forceinline__ void gemv_phase(const FusedArgs& A, const fb200_fused
       if (lane < 16) {
         // warp wlo holds its piece of unit m in slot 0 if its share starts inside m, else in
         // slot 1; every later warp starts inside m
-        int slot = r.c0 + wlo * r.per >= m * q.ipu ? 0 : 1;
-        for (int w = wlo; w <= whi; ++w) {
-          const float* pc = S.pieces + (w * 2 + slot) * 32;
-          s0 += pc[lane];
-          s1 += pc[16 + lane];
-          slot = 0;
+        const float* pc = S.pieces + (wlo * 2 + (r.c0 + wlo * r.per >= m * q.ipu ? 0 : 1)) * 32 + lane;
+        s0 = pc[0];
+        s1 = pc[16];
+        pc = S.pieces + wlo * 64 + lane;
+#pragma unroll 4
+        for (int w = whi - wlo; w > 0; --w) {
+          pc += 64;
+          s0 += pc[0];
+          s1 += pc[16];
         }
       }
       if (tr && m == ua) tr[6] = global_ns();
@@ -790,13 +793,14 @@ __device__ __noinline__ void advance_phase(const FusedArgs& A, const fb200_fused
 // The context is cut into at most att.nsplit splits of at least FUSED_SPLIT_KEYS keys: an item's
 // run time is mostly fixed latencies, so many small items finish sooner than few large ones, and
 // very short contexts run a single item per KV head with nothing to merge.
+// (Inlined on purpose: as a separate function it takes all registers, and what the caller then keeps on the stack around
+// the call, 184 bytes a thread instead of 96, no longer fits the L1 beside the shared memory: 31.9 ms instead of 30.5.)
 template <int D, int ROWS, bool LL>
-__device__ __noinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm, unsigned lep, unsigned ep_part, int pos, int* status) {
+__device__ __forceinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm, unsigned lep, int pos, int* status) {
   const int tid = threadIdx.x;
   if (tid >= DEC_THREADS) return;
   fb200_dec_args a = P.att;
   a.pos_plus1 = pos + 1;
-  a.ep_part = ep_part;
   const int skv = a.pos_plus1;
   a.nsplit = max(1, min(a.nsplit, (skv + FUSED_SPLIT_KEYS - 1) / FUSED_SPLIT_KEYS));
   a.ep_in = lep - 1u;
@@ -804,7 +808,7 @@ __device__ __noinline__ void attn_phase(const fb200_fused_phase& P, uint8_t* dsm
   a.status = status;
   const int nitems = a.b * a.hkv * a.nsplit;
   for (int item = (int)blockIdx.x; item < nitems; item += (int)gridDim.x) {
-    attn_decode_item<D, FUSED_DEC_CH, ROWS, 1, false, LL, 1, true>(a, item, dsm, tid);
+    attn_decode_item<D, FUSED_DEC_CH, ROWS, 1, false, true, 1, true, LL>(a, item, dsm, tid);
     dec_sync<1>();
   }
   if (a.nsplit > 1)
@@ -863,7 +867,7 @@ fused_step_kernel(const FusedArgs A) {
     for (int i = tid; i < DESC_WORDS / 4; i += FT) cp_async16(dst + i, src + i);
   };
   // What the attention phases need, in shared memory because the product loop has no registers to spare: the step's position, and
-  // the epoch of the launch's partial rows. The epochs go on from launch to launch in the model's memory (a captured
+  // the launch's first epoch. The epochs of the flagged rows go on from launch to launch in the model's memory (a captured
   // launch may be replayed): CTA 0 stores the next one at the end, when every CTA has passed a meeting. Without meetings
   // the launch brings its own.
   __shared__ int att_pos;
@@ -884,8 +888,11 @@ fused_step_kernel(const FusedArgs A) {
       const fb200_fused_phase& P = *desc_of(g);
       if (g) {
         // Flagged rows carry their own readiness, so a barrier-free variant meets only where plain
-        // memory changes hands: the greedy-token hand-over (argmax key -> ADVANCE -> next EMBED).
-        const bool meet = !LL || P.kind == FB200_PH_ADVANCE || prev_kind == FB200_PH_ADVANCE;
+        // memory changes hands: the greedy-token hand-over (argmax key -> ADVANCE -> next EMBED). In the others q, k and v
+        // are flagged: an attention item starts when its own heads are there, not 3 us after the last CTA is done (16 steps
+        // of a Llama-8B decoder 30.8 -> 30.5 ms). All else that passes between these two phases is behind the
+        // meeting that follows.
+        const bool meet = LL ? P.kind == FB200_PH_ADVANCE || prev_kind == FB200_PH_ADVANCE : P.kind != FB200_PH_ATTN || prev_kind != FB200_PH_GEMV;
         if (meet)
           grid_barrier(A, target, A.trace && step == A.nsteps - 1 ? A.trace + (size_t)A.nphases * 8 + ph : nullptr);
         else
@@ -894,8 +901,9 @@ fused_step_kernel(const FusedArgs A) {
       load_desc(g + DESC_SLOTS - 1);  // into the slot of the phase that has just ended; waited for below
       prev_kind = P.kind;
       const unsigned epoch = XS ? A.x.epoch_base + (unsigned)(step * A.x.per_step + (P.xs_index >= 0 ? P.xs_index : 0)) : 0u;
-      const unsigned lep = A.epoch_base + (unsigned)g;  // flagged rows: this phase's epoch
+      const unsigned lep = att_ep + (unsigned)g;  // flagged rows: this phase's epoch
       unsigned long long* tr = A.trace && blockIdx.x == 0 && tid == 0 && step == A.nsteps - 1 ? A.trace + ph * 8 : nullptr;
+      if (!LL && tid == 0) const_cast<fb200_fused_phase&>(P).epoch = lep;  // (an epilogue lies behind the barrier of the activation row)
       if (tr) tr[0] = global_ns();
       if (ph == 0 && tid == 0 && A.pos_dev) att_pos = __ldcg(A.pos_dev);  // (a step moves it in its last phase)
       switch (P.kind) {
@@ -912,7 +920,7 @@ fused_step_kernel(const FusedArgs A) {
           break;
         }
         case FB200_PH_ATTN:
-          attn_phase<D, ROWS, LL>(P, xreg, lep, att_ep + (unsigned)g, att_pos, A.status);
+          attn_phase<D, ROWS, LL>(P, xreg, lep, att_pos, A.status);
           break;
         case FB200_PH_PACK:
         case FB200_PH_EMBED:

@@ -68,6 +68,7 @@ struct fb200_fused_seg {
 
 struct alignas(16) fb200_fused_phase {  // 16-byte multiples: descriptors are copied with 16-byte asynchronous copies
   int kind;
+  unsigned epoch;    // of the running phase (written into the copy in shared memory)
   int next_gemv;  // index of the next product phase in execution order (may wrap to the next step), -1: none
   // ---- FB200_PH_GEMV: up to three matrices that share the activation row
   fb200_fused_seg seg[3];

@@ -294,7 +294,7 @@ int build_fused_program(fb200_llama* m) {
     if (!gemv(qkv, qkv_out, 3, FB200_EPI_NONE, p)) return FB200_OK;
     p.xp = m->px; p.xp_norm = 1;
     p.xll = m->px_ll; p.seg[0].yl = m->q_ll; p.seg[1].yl = m->k_ll; p.seg[2].yl = m->v_ll;
-    if (flagged) p.seg[0].y = p.seg[1].y = p.seg[2].y = nullptr;  // the flagged rows are the only copy
+    p.seg[0].y = p.seg[1].y = p.seg[2].y = nullptr;  // the flagged rows are the only copy
     prog.push_back(p);
 
     p = blank();
@@ -316,6 +316,7 @@ int build_fused_program(fb200_llama* m) {
     // published three phases earlier (the previous layer's down projection, or the embedding)
     p.xll = m->patt_ll; p.seg[0].yl = m->attn_ll; p.yll = m->pv_ll; p.addl = m->x_ll; p.add_back = 3;
     if (flagged) p.seg[0].y = nullptr;
+    else p.seg[0].yl = nullptr;
     if (tp) {
       p.xs_index = 2 * li;
       prog.push_back(p);
@@ -342,6 +343,7 @@ int build_fused_program(fb200_llama* m) {
     p.xll = m->ph_ll; p.seg[0].yl = m->x_ll; p.yll = m->px_ll;
     p.r1l = m->attn_ll; p.r1_back = 2; p.r2l = m->x_ll; p.r2_back = 5;
     if (flagged) p.seg[0].y = nullptr;
+    else p.seg[0].yl = nullptr;
     if (tp) {
       p.xs_index = 2 * li + 1;
       prog.push_back(p);
