@@ -85,6 +85,12 @@ __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
   return v;
 }
 
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Grid-wide barrier: every CTA adds one to a counter that only grows; generation n is complete
 // when the counter reaches n * gridDim.x. Bounded: after ~2^24 polls (seconds) or as soon as
 // another wait has given up, the CTA records the timeout and carries on.
@@ -96,15 +102,15 @@ __device__ __forceinline__ void grid_barrier(const FusedArgs& A, unsigned& targe
     // arrival = one fire-and-forget reduction with release semantics (orders this CTA's writes,
     // made visible to thread 0 by the barrier above, before the count)
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.bar) : "memory");
-    // polls are relaxed loads (no ordering work per poll); one acquire fence after the last one
-    // orders everything this CTA reads next behind the arrivals it has seen
+    // polls are acquire loads: the last one orders everything this CTA reads next behind the arrivals it has seen.
+    // (Relaxed polls with one acquire-release fence after the last cost more: that fence is a full barrier. 160 meetings a
+    // step; 16 steps of a Llama-8B decoder 30.1 -> 29.2 ms.)
     unsigned polls = 0;
-    while ((int)(ld_relaxed_u32(A.bar) - target) < 0) {
+    while ((int)(ld_acquire_u32(A.bar) - target) < 0) {
       ++polls;
       if ((polls & 1023u) == 0u && __ldcg(A.status) != 0) break;
       if (polls > (1u << 24)) { atomicExch(A.status, FB200_ERR_TIMEOUT); break; }
     }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
   }
   __syncthreads();
 }
