@@ -1,5 +1,6 @@
 // Fused decode step: one persistent cooperative kernel, one CTA per SM, runs a whole single-token
-// forward pass (or several in a row) as a program of phases separated by grid-wide barriers.
+// forward pass (or several in a row) as a program of phases separated by grid-wide barriers (except
+// between the q/k/v product and the attention, see the meetings in the kernel).
 //
 // Replaces, for one new position of one sequence, the reference's per-operation graph execution
 // (fusor-ml/core/src/compute_graph/resolve/run.rs:29-135) of the Llama decoder
