@@ -1,6 +1,7 @@
 // Decode-time attention for one new position per sequence, as a device function shared by the
 // stand-alone kernel and the fused decode-step kernel: RoPE(q), RoPE(k) + fp16 append,
-// split-KV online softmax over the cache, partials merged by the split that arrives last.
+// split-KV online softmax over the cache, partials merged by the split that arrives last, or, in the
+// persistent kernel, by all CTAs (attn_merge_block).
 // Attention math as fusor-ml/fusor/src/composite/attention.rs (scaled q.k, softmax, .v) with
 // interleaved RoPE (fusor-ml/fusor/src/composite/rope.rs:77-108) and the KV append of
 // fusor-ml/fusor/src/cache/kv_cache.rs:50-62. Everything another CTA may have written during
@@ -31,9 +32,9 @@ struct fb200_dec_args {
   int pos_plus1;        // > 0: *pos_dev + 1, already read by the caller (saves a dependent load); 0: not known
   int min_keys;         // stand-alone kernel: a split takes at least this many keys (0: 64), so short
                         // contexts run fewer splits than the launch provided
-  // flagged rows (persistent decode kernel without grid barriers between its phases): q, k_new
-  // and v_new arrive as f32 granules {value, epoch} that the item polls, and the merged output
-  // leaves as a flagged packed row
+  // flagged rows (persistent decode kernel): q, k_new and v_new arrive as f32 granules {value, epoch}
+  // that the item polls; without grid barriers between its phases the merged output leaves as a flagged
+  // packed row too
   const uint2* q_ll;
   const uint2* k_ll;
   const uint2* v_ll;
