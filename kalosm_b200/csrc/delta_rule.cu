@@ -10,7 +10,7 @@
 // G_i = g_0 .. g_i and w_j = (g_(j+1) .. g_i) u_j,
 //   u_i = beta_i (v_i - G_i a_i - sum_(j<i) (k_j . k_i) w_j),   o_i = G_i c_i + sum_(j<=i) (k_j . q_i) w_j,
 //   S <- G_7 S + sum_j k_j w_j,
-// the same recurrence with one reduction over the lanes per eight tokens. Everything is f32 (two tf32 values on tensor cores).
+// the same recurrence with one reduction over the lanes per eight tokens. Everything is f32 (on tensor cores as three bf16 values).
 //
 //  * delta_step_kernel: one new token per sequence. One CTA per (head, sequence): convolution, unit vectors,
 //    decay, state update, read-out, RMSNorm and gate. Bound: HBM on the state (read and written once).
@@ -665,48 +665,59 @@ __global__ void __launch_bounds__(SC_WARPS * 32) delta_scan_kernel(const fb200_d
 // state per chunk (delta_chunk_scan_kernel). Every decay is a product of decays, never a quotient, and unit k with beta below one
 // keep 1 + A well conditioned: its inverse has entries of at most one.
 //
-// Contractions run on mma.sync with both operands as two tf32 values each (hi, lo; products hi hi, hi lo, lo hi): a product is right
-// to 2^-24.8 of itself in the mean, below what 32-bit sums of that length lose. One layer in f32 against 64 bits, 24 prompts of 200 ..
-// 2400 tokens: 4.30e-7 (passes of eight: 4.29e-7), with decays near one 1.081e-6 (1.079e-6).
+// Contractions run on mma.sync with both operands as three bf16 values each, which hold all 24 bits; of the nine products the three
+// below 2^-23 of the whole are left out (2^-26 of it in the mean, less than the rounding of a 32-bit sum). Two tf32 values, three products, take the
+// same tensor time (four layers of 16 heads of 128, 2048 tokens: 1122 us, now 1141), but they drop bits, and their rounding made
+// zero of a NaN. One layer with f32 products around it against 64 bits, 24 prompts of 200 .. 2400 tokens: 4.159e-7 (two tf32 4.198e-7,
+// passes of eight 4.151e-7), with decays near one 8.494e-7 (8.524e-7, 8.453e-7).
 constexpr int CT = 32;        // tokens of a chunk
 constexpr int CDEC = CT + 4;  // decays of a chunk: r_last of every token, then the product of all
 constexpr int CK_THREADS = 128, CS_THREADS = 288, CS_STAGES = 3, SCOLS = 16;
 
 __device__ __forceinline__ float4 lds_v4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float2 lds_v2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-struct Split { uint32_t hi, lo; };
-// hi: x rounded to 11 bits; lo: the rest, rounded to as many (by sums and masks: the conversion takes 4 cycles, these 3)
-__device__ __forceinline__ Split split_tf32(float x) {
-  Split s;
-  s.hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
-  s.lo = (__float_as_uint(x - __uint_as_float(s.hi)) + 0x1000u) & 0xFFFFE000u;
+// Two neighbouring elements as three bf16 each (x in the lower half): 8 bits by a cut, 8 of the rest rounded, and what is left, which
+// fits 8 bits: together all 24. A NaN stays one in `hi` (or, by its last bits, in `mid`), an infinite value brings a NaN in `mid`
+struct Parts { uint32_t hi, mid, lo; };
+__device__ __forceinline__ Parts split_pair(float x, float y) {
+  Parts s;
+  s.hi = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+  x -= __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+  y -= __uint_as_float(__float_as_uint(y) & 0xFFFF0000u);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
+  s.mid = *reinterpret_cast<const uint32_t*>(&m);
+  x -= __uint_as_float(s.mid << 16);
+  y -= __uint_as_float(s.mid & 0xFFFF0000u);
+  s.lo = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
   return s;
 }
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Operands of m16n8k8 with its k slots t and t + 4 as elements 2t and 2t + 1: a lane's pair lies side by side in memory, and an
-// accumulator tile [16][8] is an A operand of 16 rows over 8 elements as it is.
-struct SplitA { uint32_t hi[4], lo[4]; };
-__device__ __forceinline__ SplitA split_a(float g0, float g1, float h0, float h1) {  // row g: elements 2t, 2t + 1; row g + 8
-  const Split x0 = split_tf32(g0), x1 = split_tf32(h0), x2 = split_tf32(g1), x3 = split_tf32(h1);
-  return {{x0.hi, x1.hi, x2.hi, x3.hi}, {x0.lo, x1.lo, x2.lo, x3.lo}};
+// Operand A of m16n8k16 from two accumulator tiles [16][8], side by side along K
+struct PartsA { uint32_t hi[4], mid[4], lo[4]; };
+__device__ __forceinline__ PartsA split_a(const float (&p)[4], const float (&q)[4]) {
+  const Parts x0 = split_pair(p[0], p[1]), x1 = split_pair(p[2], p[3]), x2 = split_pair(q[0], q[1]), x3 = split_pair(q[2], q[3]);
+  return {{x0.hi, x1.hi, x2.hi, x3.hi}, {x0.mid, x1.mid, x2.mid, x3.mid}, {x0.lo, x1.lo, x2.lo, x3.lo}};
 }
 // c += a b; the small products apart, the large ones added with rounding (an accumulator of the tensor cores is cut off)
-__device__ __forceinline__ void mma_split(float (&c)[4], float (&small)[4], const SplitA& a, const Split& b0, const Split& b1) {
+__device__ __forceinline__ void mma_split(float (&c)[4], float (&small)[4], const PartsA& a, const Parts& b0, const Parts& b1) {
   float d[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_tf32(small, a.lo, b0.hi, b1.hi);
-  mma_tf32(d, a.hi, b0.hi, b1.hi);
-  mma_tf32(small, a.hi, b0.lo, b1.lo);
+  mma_bf16(small, a.lo, b0.hi, b1.hi);
+  mma_bf16(small, a.hi, b0.lo, b1.lo);
+  mma_bf16(d, a.hi, b0.hi, b1.hi);
+  mma_bf16(small, a.mid, b0.mid, b1.mid);
+  mma_bf16(small, a.mid, b0.hi, b1.hi);
+  mma_bf16(small, a.hi, b0.mid, b1.mid);
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[i] += d[i];
 }
 // A CTA per (chunk, head): the lower tiles of K K^T and Q K^T; the inverse of 1 + A, whose diagonal blocks of 16 are solved by columns, a
 // lane each, and joined by -T22 A21 T11; then 16 columns of [K | V] at a time per warp, transposed: W^T = (beta G K)^T T^T, whose
 // accumulators are the operand of (P W)^T = W^T P^T as they are. Writes W and Z (16-byte piece c of row i at c ^ 2 (i & 3)), U in place
-// of v, O, and the decays. Bound: mma.sync (1540 products of 8.2 cycles a CTA). With a thread per column and the substitution unrolled
+// of v, O, and the decays. Bound: mma.sync (1728 products of 8.2 cycles a CTA). With a thread per column and the substitution unrolled
 // (no products on tensor cores) 8192 tokens of 16 heads took 225 us a layer, most of it fetching that code.
 template <int DP>
 __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_delta_args a) {
@@ -758,23 +769,22 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
     const float* rows = (warp & 2 ? qs : ks);
     // warps 0, 2: (0, 0), (0, 1), (1, 0); warps 1, 3: (1, 1), (1, 2), (1, 3)
     const int m01 = warp & 1 ? 16 : 0, n0 = warp & 1 ? 8 : 0, n1 = warp & 1 ? 16 : 8, n2 = warp & 1 ? 24 : 0;
-#pragma unroll 2
-    for (int e = 0; e < DP; e += 8) {
-      const float* ra = rows + (m01 + g) * LD + e + 2 * t;
-      const float2 x0 = lds_v2(ra), x1 = lds_v2(ra + 8 * LD);
-      const SplitA f = split_a(x0.x, x0.y, x1.x, x1.y);
-      const float2 y0 = lds_v2(ks + (n0 + g) * LD + e + 2 * t), y1 = lds_v2(ks + (n1 + g) * LD + e + 2 * t);
-      const Split b00 = split_tf32(y0.x), b01 = split_tf32(y0.y);
-      mma_split(c[0], cs[0], f, b00, b01);
-      mma_split(c[1], cs[1], f, split_tf32(y1.x), split_tf32(y1.y));
-      if (warp & 1) {
-        const float2 y2 = lds_v2(ks + (n2 + g) * LD + e + 2 * t);
-        mma_split(c[2], cs[2], f, split_tf32(y2.x), split_tf32(y2.y));
-      } else {
-        const float* rb = rows + (16 + g) * LD + e + 2 * t;
-        const float2 z0 = lds_v2(rb), z1 = lds_v2(rb + 8 * LD);
-        mma_split(c[2], cs[2], split_a(z0.x, z0.y, z1.x, z1.y), b00, b01);
-      }
+#pragma unroll 1
+    for (int e = 2 * t; e < DP; e += 16) {
+      auto rows_a = [&](const float* r) {
+        const float2 x0 = lds_v2(r + e), x1 = lds_v2(r + 8 * LD + e), y0 = lds_v2(r + e + 8), y1 = lds_v2(r + 8 * LD + e + 8);
+        return split_a({x0.x, x0.y, x1.x, x1.y}, {y0.x, y0.y, y1.x, y1.y});
+      };
+      auto rows_b = [&](int n, int half) {
+        const float2 x = lds_v2(ks + (n + g) * LD + e + 8 * half);
+        return split_pair(x.x, x.y);
+      };
+      const PartsA f = rows_a(rows + (m01 + g) * LD);
+      const Parts b0 = rows_b(n0, 0), b1 = rows_b(n0, 1);
+      mma_split(c[0], cs[0], f, b0, b1);
+      mma_split(c[1], cs[1], f, rows_b(n1, 0), rows_b(n1, 1));
+      if (warp & 1) mma_split(c[2], cs[2], f, rows_b(n2, 0), rows_b(n2, 1));
+      else mma_split(c[2], cs[2], rows_a(rows + (16 + g) * LD), b0, b1);
     }
     __syncthreads();
 #pragma unroll
@@ -847,15 +857,19 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
         else in[k][i] = tk < n && col + 8 * (i >> 1) < a.v ? a.vn[at + (size_t)tk * hv + 8 * (i >> 1)] : 0.f;
       }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float f[2];
+    for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) f[i] = bs[8 * k + 2 * t + i] * (key ? Gs[8 * k + 2 * t + i] : 1.f);
-      const SplitA x = split_a(f[0] * in[k][0], f[1] * in[k][1], f[0] * in[k][2], f[1] * in[k][3]);
+      for (int i = 0; i < 4; ++i) {
+        const int tk = 8 * k + 2 * t + (i & 1);
+        in[k][i] *= bs[tk] * (key ? Gs[tk] : 1.f);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+      const PartsA x = split_a(in[k], in[k + 1]);
 #pragma unroll
       for (int r = k; r < 4; ++r) {
-        const float2 y = lds_v2(&T[8 * r + g][8 * k + 2 * t]);
-        mma_split(d1[r], e1[r], x, split_tf32(y.x), split_tf32(y.y));
+        const float2 y0 = lds_v2(&T[8 * r + g][8 * k + 2 * t]), y1 = lds_v2(&T[8 * r + g][8 * k + 8 + 2 * t]);
+        mma_split(d1[r], e1[r], x, split_pair(y0.x, y0.y), split_pair(y1.x, y1.y));
       }
     }
     float d2[4][4], e2[4][4];
@@ -867,12 +881,12 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
         d2[x][i] = e2[x][i] = 0.f;
       }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const SplitA x = split_a(d1[k][0], d1[k][1], d1[k][2], d1[k][3]);
+    for (int k = 0; k < 4; k += 2) {
+      const PartsA x = split_a(d1[k], d1[k + 1]);
 #pragma unroll
       for (int r = k; r < 4; ++r) {
-        const float2 y = lds_v2(&P[8 * r + g][8 * k + 2 * t]);
-        mma_split(d2[r], e2[r], x, split_tf32(y.x), split_tf32(y.y));
+        const float2 y0 = lds_v2(&P[8 * r + g][8 * k + 2 * t]), y1 = lds_v2(&P[8 * r + g][8 * k + 8 + 2 * t]);
+        mma_split(d2[r], e2[r], x, split_pair(y0.x, y0.y), split_pair(y1.x, y1.y));
       }
     }
 #pragma unroll
@@ -908,7 +922,8 @@ __global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const f
   constexpr int KS = DP / 4, KT = KS / 8, MAT = CT * DP, KLD = DP + 4;  // a warp's part of d, in tiles of 8; floats of a matrix, of a row of K
   extern __shared__ __align__(16) float dsm[];  // STAGES x (W, K); STAGES x Z; two copies of S [4][KT][32 lanes] float4
   __shared__ uint64_t full[2][CS_STAGES], empty[2][CS_STAGES];
-  __shared__ __align__(16) float4 part[2][4][4][32], ws[2][4][32];  // [half][warp][tile of 8 rows][lane]; w: (hi, lo) per tile
+  __shared__ __align__(16) float4 part[2][4][4][32];  // [half][warp][tile of 8 rows][lane]
+  __shared__ uint2 ws[3][4][32];                      // w: hi, mid, lo; tile of 8 rows; a pair of column g, a pair of column g + 8
   const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, half = threadIdx.x >> 7, g = lane >> 2, t = lane & 3;
   const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.h / a.hk), hv = a.h * a.v, c0 = blockIdx.x * SCOLS, nch = (a.s + CT - 1) / CT;
   const size_t row0 = (size_t)b * a.s, chunk0 = ((size_t)b * a.h + h) * nch;
@@ -1013,13 +1028,16 @@ __global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const f
 #pragma unroll
       for (int i = 0; i < 4; ++i) c[j][i] = cs[j][i] = 0.f;
 #pragma unroll
-    for (int x = 0; x < KT; ++x) {
-      const SplitA f = split_a(s[x][0], s[x][1], s[x][2], s[x][3]);
+    for (int x = 0; x < KT; x += 2) {
+      const PartsA f = split_a(s[x], s[x + 1]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int piece = (warp * KS + 8 * x) / 4 + (t >> 1);
-        const float2 v = lds_v2(st + (8 * j + g) * DP + ((piece ^ ((g & 3) << 1)) << 2) + 2 * (t & 1));
-        mma_split(c[j], cs[j], f, split_tf32(v.x), split_tf32(v.y));
+        auto part_b = [&](int tile) {
+          const int piece = (warp * KS + 8 * tile) / 4 + (t >> 1);
+          const float2 v = lds_v2(st + (8 * j + g) * DP + ((piece ^ ((g & 3) << 1)) << 2) + 2 * (t & 1));
+          return split_pair(v.x, v.y);
+        };
+        mma_split(c[j], cs[j], f, part_b(x), part_b(x + 1));
       }
     }
 #pragma unroll
@@ -1046,9 +1064,10 @@ __global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const f
       float w[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) w[i] = ch * CT + 8 * warp + 2 * t + (i & 1) < a.s ? now.rl[i & 1] * (now.base[i] - sum[i]) : 0.f;
-      const SplitA f = split_a(w[0], w[1], w[2], w[3]);
-      ws[0][warp][lane] = make_float4(__uint_as_float(f.hi[0]), __uint_as_float(f.hi[1]), __uint_as_float(f.hi[2]), __uint_as_float(f.hi[3]));
-      ws[1][warp][lane] = make_float4(__uint_as_float(f.lo[0]), __uint_as_float(f.lo[1]), __uint_as_float(f.lo[2]), __uint_as_float(f.lo[3]));
+      const Parts p0 = split_pair(w[0], w[1]), p1 = split_pair(w[2], w[3]);
+      ws[0][warp][lane] = make_uint2(p0.hi, p1.hi);
+      ws[1][warp][lane] = make_uint2(p0.mid, p1.mid);
+      ws[2][warp][lane] = make_uint2(p0.lo, p1.lo);
     }
     bar_sync(1, 128);
     // ---- S^T <- G S^T + w^T K
@@ -1059,14 +1078,13 @@ __global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const f
 #pragma unroll
       for (int i = 0; i < 4; ++i) up[x][i] = us[x][i] = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {  // tokens 8 j ..
-      const float4 whi = ws[0][j][lane], wlo = ws[1][j][lane];
-      const SplitA f = {{__float_as_uint(whi.x), __float_as_uint(whi.y), __float_as_uint(whi.z), __float_as_uint(whi.w)},
-                        {__float_as_uint(wlo.x), __float_as_uint(wlo.y), __float_as_uint(wlo.z), __float_as_uint(wlo.w)}};
+    for (int j = 0; j < 4; j += 2) {  // tokens 8 j ..
+      const uint2 h0 = ws[0][j][lane], h1 = ws[0][j + 1][lane], m0 = ws[1][j][lane], m1 = ws[1][j + 1][lane], l0 = ws[2][j][lane], l1 = ws[2][j + 1][lane];
+      const PartsA f = {{h0.x, h0.y, h1.x, h1.y}, {m0.x, m0.y, m1.x, m1.y}, {l0.x, l0.y, l1.x, l1.y}};
 #pragma unroll
       for (int x = 0; x < KT; ++x) {
         const float* p = kb + (8 * j + 2 * t) * KLD + warp * KS + 8 * x + g;
-        mma_split(up[x], us[x], f, split_tf32(p[0]), split_tf32(p[KLD]));
+        mma_split(up[x], us[x], f, split_pair(p[0], p[KLD]), split_pair(p[8 * KLD], p[9 * KLD]));
       }
     }
 #pragma unroll

@@ -124,6 +124,35 @@ def test_delta_prompts_in_chunks(dev, dtype, shape, sizes):
     check(dev, cfg, w, toks(cfg, sum(sizes)), dtype, sizes)
 
 
+BAD_ROW = 7  # a token whose embedding the tests below replace
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=2, kv_heads=1, dim=128, vdim=128)], ids=str)
+@pytest.mark.parametrize("at", [0, 70, 191, 255])
+def test_delta_prompt_behind_a_nan(dev, dtype, shape, at):
+    # A token that is not a number in a prompt that goes in chunks: all that follows it is none either, in the prompt and behind
+    # it; the sequence beside it does not notice.
+    cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
+    w = U.weights(cfg, 60, U.identity_head(cfg))
+    t = np.random.default_rng(at).integers(BAD_ROW + 1, cfg["vocab"], (2, 256))
+    m = U.gpu_model(dev, cfg, w, dtype, max_batch=2)
+    m.forward(t, want_logits=False)
+    clean = m.logits_at(range(512))
+    m.free()
+    w["embed"].reshape(cfg["vocab"], -1)[BAD_ROW] = 0x7FC0
+    t[0, at] = BAD_ROW
+    m = U.gpu_model(dev, cfg, w, dtype, max_batch=2)
+    m.forward(t, want_logits=False)
+    got = m.logits_at(range(512))
+    after, _ = m.forward(t[:, :1] * 0 + 50)
+    m.free()
+    assert np.isnan(got[at:256]).all()
+    assert np.array_equal(got[256:].view(np.uint32), clean[256:].view(np.uint32))
+    assert np.isnan(after[0]).all() and np.isfinite(after[1]).all()
+    assert dev.status() == 0
+
+
 LATENTS = [dict(), dict(heads=1, dim=8, rot=2, vdim=8, rank=8, window=1), dict(heads=5, dim=24, rot=8, vdim=48, rank=72, window=33, base=50.0),
            dict(heads=2, dim=20, rot=6, vdim=12, rank=30, window=7), dict(heads=4, dim=128, rot=64, vdim=128, rank=512, window=50),
            dict(heads=2, dim=64, rot=32, vdim=200, rank=136, window=64), dict(heads=3, dim=192, rot=72, vdim=72, rank=200, window=40, scale=0.2),
