@@ -22,6 +22,8 @@
 #include "qgemv_common.cuh"
 #include "state_columns.cuh"
 
+#include <cstdlib>
+
 namespace {
 
 constexpr float UNIT_EPS = 1e-6f;  // inside the root of the unit vectors
@@ -1226,9 +1228,13 @@ int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
 // Chunks of 32 tokens or passes of eight. Four layers of 16 heads of 128, passes / chunks: 100 tokens 426 / 452 us, 200 tokens 482 / 481,
 // 512 tokens 690 / 579, 4096 tokens 3398 / 2217 (heads of 64: 393 / 406, 448 / 423, 659 / 512, 3269 / 1860): a chunk's preparation
 // has a longer chain than a few passes. Heads of more than 128 do not fit: three stages of their matrices need 250 KB.
+// Models in float32 keep the passes of eight, whose error is the smaller one (by 0.2 %, see above): there a chunk rounds W, U and Z
+// between its products. FB200_DELTA_CHUNKS=1 takes chunks wherever the head size allows, 0 never.
 constexpr int CHUNKS_FROM = 192;
 bool delta_in_chunks(const fb200_delta_args& a) {
-  return fb200_delta_chunks(a.dp) && a.s >= CHUNKS_FROM;
+  if (!fb200_delta_chunks(a.dp)) return false;
+  if (const char* e = getenv("FB200_DELTA_CHUNKS")) return e[0] == '1';
+  return a.z_bf16 && a.s >= CHUNKS_FROM;
 }
 
 }  // namespace

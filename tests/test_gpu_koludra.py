@@ -116,12 +116,25 @@ def test_delta_rows_in_pieces_of_four(dev, dtype, shape):
 @pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=3, kv_heads=3, dim=33, vdim=17, conv=2), dict(heads=2, kv_heads=1, dim=128, vdim=128),
                                    dict(heads=2, kv_heads=2, dim=100, vdim=130, conv=5)], ids=str)
 @pytest.mark.parametrize("sizes", [[192], [223, 1], [193, 200], [5, 256, 3]], ids=str)
-def test_delta_prompts_in_chunks(dev, dtype, shape, sizes):
+def test_delta_prompts_in_chunks(dev, dtype, shape, sizes, monkeypatch):
     # prompts of 192 tokens and more go in chunks of 32: whole ones, one token in the last, all but one, a state of an earlier pass in
     # front and a pass of another form behind; columns that do not fill a group of 16
+    # (float32 does so on request only)
+    monkeypatch.setenv("FB200_DELTA_CHUNKS", "1")
     cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
     w = U.weights(cfg, 50 + sum(sizes), U.identity_head(cfg))
     check(dev, cfg, w, toks(cfg, sum(sizes)), dtype, sizes)
+
+
+def test_delta_prompts_of_float32_models(dev):
+    # A prompt of any length goes in passes of eight tokens there: in one piece or in pieces of multiples of eight, the same bits.
+    cfg = U.config([U.delta(ff=0, heads=2, kv_heads=1, dim=64, vdim=64)], width=88, vocab=88)
+    w = U.weights(cfg, 61, U.identity_head(cfg))
+    t = toks(cfg, 400)
+    m = U.gpu_model(dev, cfg, w, "float32")
+    whole, pieces = U.run_portions(m, t, [400]), U.run_portions(m, t, [96, 160, 144])
+    m.free()
+    assert np.array_equal(whole.view(np.uint32), pieces.view(np.uint32))
 
 
 BAD_ROW = 7  # a token whose embedding the tests below replace
@@ -130,9 +143,10 @@ BAD_ROW = 7  # a token whose embedding the tests below replace
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=2, kv_heads=1, dim=128, vdim=128)], ids=str)
 @pytest.mark.parametrize("at", [0, 70, 191, 255])
-def test_delta_prompt_behind_a_nan(dev, dtype, shape, at):
+def test_delta_prompt_behind_a_nan(dev, dtype, shape, at, monkeypatch):
     # A token that is not a number in a prompt that goes in chunks: all that follows it is none either, in the prompt and behind
     # it; the sequence beside it does not notice.
+    monkeypatch.setenv("FB200_DELTA_CHUNKS", "1")
     cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
     w = U.weights(cfg, 60, U.identity_head(cfg))
     t = np.random.default_rng(at).integers(BAD_ROW + 1, cfg["vocab"], (2, 256))
