@@ -716,10 +716,38 @@ __device__ __forceinline__ void mma_split(float (&c)[4], float (&small)[4], cons
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[i] += d[i];
 }
+__device__ __forceinline__ bool not_finite(float4 v) { return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) != 0.f; }
+// v: [eight tokens][token 2 t, 2 t + 1; column g, g + 8]. Where a column has values that are not finite, the tokens from the first on become
+// zeros and `cut` goes down to it; whether any lane's column has
+__device__ __forceinline__ bool zero_from_bad(float (&v)[4][4], int (&cut)[2], int t) {
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) any |= not_finite(make_float4(v[k][0], v[k][1], v[k][2], v[k][3]));
+  if (!__any_sync(0xFFFFFFFFu, any)) return false;
+  auto token = [&](int k, int i) { return 8 * k + 2 * t + (i & 1); };
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (v[k][i] * 0.f != 0.f) cut[i >> 1] = min(cut[i >> 1], token(k, i));
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    cut[j] = min(cut[j], __shfl_xor_sync(0xFFFFFFFFu, cut[j], 1));
+    cut[j] = min(cut[j], __shfl_xor_sync(0xFFFFFFFFu, cut[j], 2));
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (token(k, i) >= cut[i >> 1]) v[k][i] = 0.f;
+  return true;
+}
 // A CTA per (chunk, head): the lower tiles of K K^T and Q K^T; the inverse of 1 + A, whose diagonal blocks of 16 are solved by columns, a
 // lane each, and joined by -T22 A21 T11; then 16 columns of [K | V] at a time per warp, transposed: W^T = (beta G K)^T T^T, whose
 // accumulators are the operand of (P W)^T = W^T P^T as they are. Writes W and Z (16-byte piece c of row i at c ^ 2 (i & 3)), U in place
-// of v, O, and the decays. Bound: mma.sync (1728 products of 8.2 cycles a CTA). With a thread per column and the substitution unrolled
+// of v, O, and the decays. Zeros that the products meet above the diagonals of T and P keep no value out that is not finite, so tokens from the
+// first such k, decay or strength on (values: per column) take part as zeros, and their rows are written as NaN: the rows in front of
+// them stay what they are without them. Bound: mma.sync (1728 products of 8.2 cycles a CTA). With a thread per column and the substitution unrolled
 // (no products on tensor cores) 8192 tokens of 16 heads took 225 us a layer, most of it fetching that code.
 template <int DP>
 __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_delta_args a) {
@@ -727,11 +755,13 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
   extern __shared__ __align__(16) float dsm[];
   float *ks = dsm, *qs = dsm + CT * LD;
   __shared__ __align__(16) float A[CT][LA], P[CT][LA], T[CT][LA], M[16][20], gs[CT], bs[CT], Gs[CT];
+  __shared__ int bad[CK_THREADS / 32];  // first token whose k, decay or strength is not finite, as the warps see it
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int t0 = blockIdx.x * CT, h = blockIdx.y, b = blockIdx.z, hk = h / (a.h / a.hk), hv = a.h * a.v;
   const int n = min(CT, a.s - t0);
   const size_t row0 = (size_t)b * a.s + t0, chunk = ((size_t)b * a.h + h) * gridDim.x + blockIdx.x;
   pdl_wait();
+  int first = CT;
 #pragma unroll 4
   for (int i = tid; i < CT * (DP / 4); i += CK_THREADS) {
     const int tk = i / (DP / 4), e = (i % (DP / 4)) * 4;
@@ -740,13 +770,26 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     *reinterpret_cast<float4*>(ks + tk * LD + e) = tk < n ? k : z;
     *reinterpret_cast<float4*>(qs + tk * LD + e) = tk < n ? q : z;
+    if (not_finite(k) && tk < n) first = min(first, tk);
   }
   if (tid < CT) {  // tokens behind the last one: decay 1, strength 0
     const float2 gb = *reinterpret_cast<const float2*>(a.gb + ((row0 + min(tid, n - 1)) * a.h + h) * 2);
     gs[tid] = tid < n ? gb.x : 1.f;
     bs[tid] = tid < n ? gb.y : 0.f;
+    if (not_finite(make_float4(gb.x, gb.y, 0.f, 0.f)) && tid < n) first = min(first, tid);
   }
+  first = __reduce_min_sync(0xFFFFFFFFu, first);
+  if (lane == 0) bad[warp] = first;
   __syncthreads();
+  first = min(min(bad[0], bad[1]), min(bad[2], bad[3]));
+  if (first < CT) {
+    for (int i = tid; i < (CT - first) * DP; i += CK_THREADS) ks[(first + i / DP) * LD + i % DP] = 0.f;
+    if (tid >= first && tid < CT) {
+      gs[tid] = 1.f;
+      bs[tid] = 0.f;
+    }
+    __syncthreads();
+  }
   if (warp == 0) {  // decays from token `lane` on, and from the chunk's start; T holds r_ij until the products are there
     float r = 1.f, G = 1.f;
 #pragma unroll 8
@@ -858,6 +901,9 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
         if (key) in[k][i] = ks[tk * LD + c0 + g + 8 * (i >> 1)];
         else in[k][i] = tk < n && col + 8 * (i >> 1) < a.v ? a.vn[at + (size_t)tk * hv + 8 * (i >> 1)] : 0.f;
       }
+    int cut[2] = {first, first};  // tokens of column g and g + 8 from which on rows are NaN
+    bool cuts = first < CT;
+    cuts |= zero_from_bad(in, cut, t);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -882,6 +928,7 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
         d1[x][i] += e1[x][i];
         d2[x][i] = e2[x][i] = 0.f;
       }
+    cuts |= zero_from_bad(d1, cut, t);
 #pragma unroll
     for (int k = 0; k < 4; k += 2) {
       const PartsA x = split_a(d1[k], d1[k + 1]);
@@ -891,6 +938,12 @@ __global__ void __launch_bounds__(CK_THREADS, 4) delta_chunk_kernel(const fb200_
         mma_split(d2[r], e2[r], x, split_pair(y0.x, y0.y), split_pair(y1.x, y1.y));
       }
     }
+    if (cuts)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (8 * r + 2 * t + (i & 1) >= cut[i >> 1]) d1[r][i] = d2[r][i] = __uint_as_float(0x7FC00000u);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll

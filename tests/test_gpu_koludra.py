@@ -142,19 +142,26 @@ BAD_ROW = 7  # a token whose embedding the tests below replace
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [dict(heads=4, kv_heads=2, dim=64, vdim=40), dict(heads=2, kv_heads=1, dim=128, vdim=128)], ids=str)
+@pytest.mark.parametrize("what", ["row", "value"])
 @pytest.mark.parametrize("at", [0, 70, 191, 255])
-def test_delta_prompt_behind_a_nan(dev, dtype, shape, at, monkeypatch):
-    # A token that is not a number in a prompt that goes in chunks: all that follows it is none either, in the prompt and behind
-    # it; the sequence beside it does not notice.
+def test_delta_prompt_around_a_value_that_is_not_finite(dev, dtype, shape, what, at, monkeypatch):
+    # A token whose row is NaN, or one of whose values is infinite, in a prompt that goes in chunks: all that follows it is NaN, in
+    # the prompt and behind it; what precedes it, and the sequence beside it, stay bit for bit what they are without it.
     monkeypatch.setenv("FB200_DELTA_CHUNKS", "1")
     cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
     w = U.weights(cfg, 60, U.identity_head(cfg))
+    embed, wv = w["embed"].reshape(cfg["vocab"], -1), w["l0.mix.v"].reshape(-1, cfg["width"])
+    embed[:, 5] = 0
+    wv[9, 5] = 0x7F61  # 3e38: only a token whose embedding has this element sees it
     t = np.random.default_rng(at).integers(BAD_ROW + 1, cfg["vocab"], (2, 256))
     m = U.gpu_model(dev, cfg, w, dtype, max_batch=2)
     m.forward(t, want_logits=False)
     clean = m.logits_at(range(512))
     m.free()
-    w["embed"].reshape(cfg["vocab"], -1)[BAD_ROW] = 0x7FC0
+    if what == "row":
+        embed[BAD_ROW] = 0x7FC0
+    else:
+        embed[BAD_ROW, 5] = 0x4248  # 50
     t[0, at] = BAD_ROW
     m = U.gpu_model(dev, cfg, w, dtype, max_batch=2)
     m.forward(t, want_logits=False)
@@ -162,6 +169,7 @@ def test_delta_prompt_behind_a_nan(dev, dtype, shape, at, monkeypatch):
     after, _ = m.forward(t[:, :1] * 0 + 50)
     m.free()
     assert np.isnan(got[at:256]).all()
+    assert np.array_equal(got[:at].view(np.uint32), clean[:at].view(np.uint32))
     assert np.array_equal(got[256:].view(np.uint32), clean[256:].view(np.uint32))
     assert np.isnan(after[0]).all() and np.isfinite(after[1]).all()
     assert dev.status() == 0
