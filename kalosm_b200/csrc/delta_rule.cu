@@ -223,8 +223,10 @@ __device__ __forceinline__ void conv_chunk(const fb200_delta_args& a, int b, int
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
+      if (j0 + j < a.taps) {  // (what a tap too many would meet are later tokens, which may not be numbers)
 #pragma unroll
-      for (int i = 0; i < PREP_TOK; ++i) out[i] = fmaf(w[j], x[i + j], out[i]);
+        for (int i = 0; i < PREP_TOK; ++i) out[i] = fmaf(w[j], x[i + j], out[i]);
+      }
   }
 #pragma unroll
   for (int i = 0; i < PREP_TOK; ++i) out[i] = t0 + i < a.s ? dr_silu(out[i]) : 0.f;
@@ -339,12 +341,14 @@ __device__ __forceinline__ void conv_chunk4(const fb200_delta_args& a, int b, in
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
+      if (j0 + j < a.taps) {
 #pragma unroll
-      for (int i = 0; i < PREP4_TOK; ++i) {
-        out[i].x = fmaf(w[j].x, x[i + j].x, out[i].x);
-        out[i].y = fmaf(w[j].y, x[i + j].y, out[i].y);
-        out[i].z = fmaf(w[j].z, x[i + j].z, out[i].z);
-        out[i].w = fmaf(w[j].w, x[i + j].w, out[i].w);
+        for (int i = 0; i < PREP4_TOK; ++i) {
+          out[i].x = fmaf(w[j].x, x[i + j].x, out[i].x);
+          out[i].y = fmaf(w[j].y, x[i + j].y, out[i].y);
+          out[i].z = fmaf(w[j].z, x[i + j].z, out[i].z);
+          out[i].w = fmaf(w[j].w, x[i + j].w, out[i].w);
+        }
       }
   }
 #pragma unroll

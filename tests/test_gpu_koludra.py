@@ -175,6 +175,25 @@ def test_delta_prompt_around_a_value_that_is_not_finite(dev, dtype, shape, what,
     assert dev.status() == 0
 
 
+@pytest.mark.parametrize("dim", [33, 36])
+@pytest.mark.parametrize("conv", [1, 2, 3, 4, 5, 6])
+def test_convolution_in_front_of_a_nan(dev, dim, conv):
+    # Tokens in front of one whose row is NaN, any number of taps, channels by element (33) and in pieces of four
+    cfg = U.config([U.delta(ff=0, heads=2, kv_heads=1, dim=dim, vdim=dim, conv=conv)], width=88, vocab=88)
+    w = U.weights(cfg, 62, U.identity_head(cfg))
+    t = np.random.default_rng(conv).integers(BAD_ROW + 1, cfg["vocab"], 24)
+    m = U.gpu_model(dev, cfg, w, "float32")
+    clean = U.run_portions(m, t, [24])
+    m.free()
+    w["embed"].reshape(cfg["vocab"], -1)[BAD_ROW] = 0x7FC0
+    m = U.gpu_model(dev, cfg, w, "float32")
+    for at in range(8, 16):
+        got = U.run_portions(m, np.where(np.arange(24) == at, BAD_ROW, t), [24])
+        assert np.array_equal(got[:at].view(np.uint32), clean[:at].view(np.uint32)), at
+        assert np.isnan(got[at:]).all()
+    m.free()
+
+
 LATENTS = [dict(), dict(heads=1, dim=8, rot=2, vdim=8, rank=8, window=1), dict(heads=5, dim=24, rot=8, vdim=48, rank=72, window=33, base=50.0),
            dict(heads=2, dim=20, rot=6, vdim=12, rank=30, window=7), dict(heads=4, dim=128, rot=64, vdim=128, rank=512, window=50),
            dict(heads=2, dim=64, rot=32, vdim=200, rank=136, window=64), dict(heads=3, dim=192, rot=72, vdim=72, rank=200, window=40, scale=0.2),
