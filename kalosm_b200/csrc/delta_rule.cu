@@ -1288,21 +1288,22 @@ int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
 // Models in float32 keep the passes of eight, whose error is the smaller one (by 0.2 %, see above): there a chunk rounds W, U and Z
 // between its products. FB200_DELTA_CHUNKS=1 takes chunks wherever the head size allows, 0 never.
 constexpr int CHUNKS_FROM = 192;
-bool delta_in_chunks(const fb200_delta_args& a) {
-  if (!fb200_delta_chunks(a.dp)) return false;
-  if (const char* e = getenv("FB200_DELTA_CHUNKS")) return e[0] == '1';
-  return a.z_bf16 && a.s >= CHUNKS_FROM;
-}
 
 }  // namespace
+
+bool fb200_delta_in_chunks(int dp, int s, bool bf16) {
+  if (s == 1 || (dp != 64 && dp != 128)) return false;
+  if (const char* e = getenv("FB200_DELTA_CHUNKS")) return e[0] == '1';
+  return bf16 && s >= CHUNKS_FROM;
+}
+size_t fb200_delta_wq_floats(int b, int s, int h, int dp) { return (size_t)b * h * ((s + CT - 1) / CT) * 2 * CT * dp; }
+size_t fb200_delta_dec_floats(int b, int s, int h) { return (size_t)b * h * ((s + CT - 1) / CT) * CDEC; }
 
 int fb200_delta_dp(int d) {
   for (int dp : {32, 64, 128, 256, 512})
     if (d <= dp) return dp;
   return 0;
 }
-
-bool fb200_delta_chunks(int dp) { return dp == 64 || dp == 128; }
 
 int fb200_delta_step(fb200_device* dev, const fb200_delta_args& a) {
   switch (a.dp) {
@@ -1326,7 +1327,7 @@ int fb200_delta_prompt(fb200_device* dev, const fb200_delta_args& a) {
     default: return fb200_fail(dev, FB200_ERR_INVALID_SHAPE, "delta rule: head size %d", a.d);
   }
   if (rc) return rc;
-  if (delta_in_chunks(a)) {
+  if (a.wq && fb200_delta_in_chunks(a.dp, a.s, a.z_bf16)) {
     rc = a.dp == 64 ? launch_chunks<64>(dev, a) : launch_chunks<128>(dev, a);
   } else {
     rc = fb200_launch(dev, delta_pairs_kernel, dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),

@@ -86,6 +86,7 @@ struct fb200_hybrid {
   size_t done_linear = 0;   // first counter of the linear attention
   __nv_bfloat16* kvx = nullptr;
   size_t kvx_elems = 0;
+  size_t chunk_floats = 0;  // of wq, which dec lies behind
 };
 
 namespace {
@@ -515,13 +516,49 @@ embed_rows_kernel(const T* __restrict__ table, const uint32_t* __restrict__ ids,
   }
 }
 
+void drop_chunks(fb200_hybrid* hy) {
+  if (hy->wq) cudaFree(hy->wq);
+  hy->wq = hy->dec = nullptr;
+  hy->chunk_floats = 0;
+}
+
+// What a pass's delta rules in chunks hand on (16 KB a token at 16 heads of 128). They can do without: a pass that finds no room, on the device
+// or in the handle's budget, goes in passes of eight tokens, and every other buffer of the model has precedence.
+int ensure_chunks(fb200_llama* m, int batch, int seq) {
+  fb200_device* dev = m->dev;
+  fb200_hybrid* hy = m->hybrid;
+  size_t wq = 0, dec = 0;
+  for (const auto& M : hy->mixers)
+    if (M.c.mixer == FB200_MIX_DELTA && fb200_delta_in_chunks(M.dp, seq, !hy->f32)) {
+      wq = std::max(wq, fb200_delta_wq_floats(batch, seq, M.c.heads, M.dp));
+      dec = std::max(dec, fb200_delta_dec_floats(batch, seq, M.c.heads));
+    }
+  if (wq + dec <= hy->chunk_floats) {
+    hy->dec = hy->wq + wq;
+    return FB200_OK;
+  }
+  FB_CUDA(dev, cudaStreamSynchronize(dev->stream));
+  drop_chunks(hy);
+  const size_t bytes = (wq + dec) * 4;
+  if (dev->scratch_limit && dev->scratch_total + bytes > dev->scratch_limit) return FB200_OK;
+  if (cudaMalloc(&hy->wq, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    hy->wq = nullptr;
+    return FB200_OK;
+  }
+  if (dev->poison) FB_CUDA(dev, cudaMemsetAsync(hy->wq, 0xFF, bytes, dev->stream));
+  hy->chunk_floats = wq + dec;
+  hy->dec = hy->wq + wq;
+  return FB200_OK;
+}
+
 }  // namespace
 
 int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
   fb200_device* dev = m->dev;
   fb200_hybrid* hy = m->hybrid;
   const size_t E = m->cfg.hidden, nb = m->cfg.max_batch;
-  size_t q = 0, qk = 0, hv = 0, o = 0, heads = 0, kvh = 0, qa = 0, part = 0, done = 0, seg = 0, wq = 0;
+  size_t q = 0, qk = 0, hv = 0, o = 0, heads = 0, kvh = 0, qa = 0, part = 0, done = 0, seg = 0;
   for (const auto& M : hy->mixers) {
     const auto& c = M.c;
     if (c.mixer == FB200_MIX_DELTA) {
@@ -529,7 +566,6 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
       hv = std::max(hv, (size_t)M.ko);
       heads = std::max(heads, (size_t)c.heads);
       kvh = std::max(kvh, (size_t)c.kv_heads);
-      if (fb200_delta_chunks(M.dp)) wq = std::max(wq, (size_t)c.heads * M.dp * 64);
     } else if (c.mixer == FB200_MIX_LINEAR) {
       o = std::max(o, (size_t)M.ko);
       if (!hy->f32) {
@@ -553,7 +589,6 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
   for (const auto& M : hy->mixers)
     if (M.c.mixer == FB200_MIX_DELTA) o = std::max(o, hv);
   hy->done_linear = done;
-  const size_t chunks = (rows + 31 * nb) / 32;
   bool norm2 = false;
   for (const auto& L : hy->layers) norm2 = norm2 || L.norm2;
   const size_t hb = std::max((norm2 ? 2 : 1) * up_to(E, 64), hy->w_loop ? (size_t)hy->w_loop->k : 0);
@@ -561,9 +596,9 @@ int fb200_hybrid_ensure_rows(fb200_llama* m, size_t rows) {
       {(void**)&m->x, rows * hy->ldx * 4}, {(void**)&hy->x2, hy->w_loop ? rows * hy->ldx * 4 : 0}, {(void**)&m->xn, (norm2 ? 2 : 1) * rows * E * 4},
       {(void**)&hy->proj, rows * hy->ldy * 4}, {(void**)&hy->zf, rows * hy->ldz * 4}, {(void**)&hy->hb, rows * hb * 2},
       {(void**)&hy->zb, rows * hy->ldz * 2}, {(void**)&hy->qn, rows * q * 4}, {(void**)&hy->kn, rows * qk * 4}, {(void**)&hy->vn, rows * hv * 4},
-      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 7 * nb) / 8 * kvh * 256 + 64}, {(void**)&hy->wq, wq * chunks * 4},
-      {(void**)&hy->dec, wq ? chunks * heads * 36 * 4 : 0}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
+      {(void**)&hy->gb, rows * heads * 8}, {(void**)&hy->kq, (rows + 7 * nb) / 8 * kvh * 256 + 64}, {(void**)&hy->o, rows * o * 4}, {(void**)&hy->seg, seg * 4},
       {(void**)&hy->qa, qa * 4}, {(void**)&hy->part, part * 4}, {(void**)&hy->done, (done + nb) * 4}};
+  drop_chunks(hy);
   for (auto& b : bufs) {
     if (*b.p) { cudaFree(*b.p); *b.p = nullptr; }
     FB_CUDA(dev, cudaMalloc(b.p, b.bytes ? b.bytes : 16));
@@ -609,9 +644,16 @@ int fb200_hybrid_forward(fb200_llama* m, int batch, int seq, bool commit) {
     if (hy->kvx) cudaFree(hy->kvx);
     hy->kvx = nullptr;
     hy->kvx_elems = 0;
-    FB_CUDA(dev, cudaMalloc(&hy->kvx, kvx * 2));
+    cudaError_t e = cudaMalloc(&hy->kvx, kvx * 2);
+    if (e == cudaErrorMemoryAllocation && hy->wq) {
+      cudaGetLastError();
+      drop_chunks(hy);
+      e = cudaMalloc(&hy->kvx, kvx * 2);
+    }
+    FB_CUDA(dev, e);
     hy->kvx_elems = kvx;
   }
+  if ((rc = ensure_chunks(m, batch, seq))) return rc;
   const int E = m->cfg.hidden, rows = batch * seq;
   float *x = m->x, *other = hy->w_loop ? hy->x2 : nullptr;
   const auto& emb = *m->token_embd;
@@ -672,7 +714,7 @@ void fb200_hybrid_free(fb200_llama* m) {
     for (void* b : bufs) if (b) cudaFree(b);
   }
   if (hy->w_loop) fb200_qmatrix_free(hy->w_loop);
-  void* bufs[] = {hy->proj, hy->zf, hy->hb, hy->zb, hy->qn, hy->kn, hy->vn, hy->gb, hy->kq, hy->wq, hy->dec, hy->o, hy->seg, hy->qa, hy->part, hy->done, hy->x2, hy->kvx};
+  void* bufs[] = {hy->proj, hy->zf, hy->hb, hy->zb, hy->qn, hy->kn, hy->vn, hy->gb, hy->kq, hy->wq, hy->o, hy->seg, hy->qa, hy->part, hy->done, hy->x2, hy->kvx};
   for (void* b : bufs) if (b) cudaFree(b);
   delete hy;
   m->hybrid = nullptr;

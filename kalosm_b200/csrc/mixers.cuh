@@ -27,11 +27,13 @@ struct fb200_delta_args {
   // prompt pass scratch: unit q and k [rows][hk][dp], v [rows][h v], (decay, write strength) [rows][h][2],
   // products of eight tokens' k and q [b][ceil(s / 8)][hk][64], read-out [rows][h v]
   float *qn, *kn, *vn, *gb, *kq, *o;
-  // chunks of 32 tokens: [b][h][ceil(s / 32)] of two matrices [32][dp], and of 36 decays
+  // chunks of 32 tokens: [b][h][ceil(s / 32)] of two matrices [32][dp], and of 36 decays (null: passes of eight tokens)
   float *wq, *dec;
   int* status;
 };
-bool fb200_delta_chunks(int dp);                                   // whether prompts of this head size may use wq and dec
+bool fb200_delta_in_chunks(int dp, int s, bool bf16);                 // whether a pass takes chunks where it has wq and dec
+size_t fb200_delta_wq_floats(int b, int s, int h, int dp);
+size_t fb200_delta_dec_floats(int b, int s, int h);
 int fb200_delta_dp(int d);                                         // padded head size, 0 when d is not covered
 int fb200_delta_step(fb200_device* dev, const fb200_delta_args& a);    // s == 1: one kernel
 int fb200_delta_prompt(fb200_device* dev, const fb200_delta_args& a);  // s > 1

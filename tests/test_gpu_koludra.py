@@ -137,6 +137,34 @@ def test_delta_prompts_of_float32_models(dev):
     assert np.array_equal(whole.view(np.uint32), pieces.view(np.uint32))
 
 
+def test_delta_prompt_without_room_for_chunks(monkeypatch):
+    # What chunks hand on counts against the handle's budget; a pass that it has no room for goes in passes of eight, as one told to
+    own = kb.Device(0)
+    cfg = U.config([U.delta(ff=0, heads=2, kv_heads=1, dim=64, vdim=64)], width=88, vocab=88)
+    w = U.weights(cfg, 63, U.identity_head(cfg))
+    t = toks(cfg, 400)
+
+    def run(m):
+        return U.run_portions(m, t, [400]).view(np.uint32)
+    m = U.gpu_model(own, cfg, w, "bfloat16")
+    chunks = run(m)
+    m.free()
+    monkeypatch.setenv("FB200_DELTA_CHUNKS", "0")
+    m = U.gpu_model(own, cfg, w, "bfloat16")
+    eights = run(m)
+    m.free()
+    monkeypatch.delenv("FB200_DELTA_CHUNKS")
+    assert not np.array_equal(chunks, eights)
+    own.set_scratch_limit(1)
+    m = U.gpu_model(own, cfg, w, "bfloat16")
+    assert np.array_equal(run(m), eights)
+    own.set_scratch_limit(0)
+    assert np.array_equal(run(m), chunks)
+    m.free()
+    assert own.status() == 0
+    own.close()
+
+
 BAD_ROW = 7  # a token whose embedding the tests below replace
 
 
