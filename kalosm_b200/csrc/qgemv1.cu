@@ -154,13 +154,13 @@ qgemv1_kernel(const Gemv1Args a) {
       ex = max(ex, -110);                                   // 2^(6 - ex) and 2^(ex - 13) stay in range
       const float inv64 = ldexpf(64.0f, -ex);               // v * inv64 in (-64, 64)
       const float out_scale = ldexpf(1.0f, ex - 13);        // 2^ex / (64 * 128)
-      float sum = 0.f;
+      uint32_t sum = 0;  // of the q, as int: 16 of them stay below 2^31 (floats in their place: 2.15e-7 of error at 4096 x 4096 Q4_0, not 1.7e-7)
       if (in) {
         uint32_t r[8], wl[2][4];  // [half of the block][limb 3, 2, 1, 0] four elements per word
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int q = __float2int_rn((v[i] * inv64) * 2097152.0f);
-          sum += (float)q;
+          sum += (uint32_t)q;
           // fields at bits 0, 7, 14, 21 -> bytes 0..3 (byte 3 = bits 21..28 = l0 as s8)
           r[i] = ((uint32_t)q & 0x7Fu) | (((uint32_t)q << 1) & 0x7F00u) | (((uint32_t)q << 2) & 0x7F0000u) |
                  (((uint32_t)q << 3) & 0xFF000000u);
@@ -183,7 +183,7 @@ qgemv1_kernel(const Gemv1Args a) {
       sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
       if (in && (threadIdx.x & 1) == 0) {
         xsc[kb >> 1] = out_scale;
-        xss[kb >> 1] = sum * (1.0f / 16384.0f) * out_scale;
+        xss[kb >> 1] = (float)(int)sum * (1.0f / 16384.0f) * out_scale;
       }
     }
     if (a.norm_w) {
