@@ -198,7 +198,8 @@ qgemv1_kernel(const Gemv1Args a) {
         ss = 0.f;
         for (int i = 0; i < W; ++i) ss += tmp[i];
         // rms_norm_fused_cpu_impl, fusor-ml/fusor/src/composite/normalization.rs:404-461
-        fs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
+        const float rms = sqrtf(ss / (float)a.K + a.eps);
+        fs = rms == 0.f ? 0.f : 1.0f / rms;  // a row of zeros without an eps stays zero
       }
       __syncwarp(0xFFFFu);
       if (threadIdx.x == 0) tmp[0] = fs;

@@ -365,6 +365,15 @@ def test_single_row_scales_of_16(dev, ty, n, k, off):
         assert (err <= 2.0 ** -18 * tops * np.abs(w64).max(1)).all(), (norm is None, err.max())
 
 
+@pytest.mark.parametrize("ty", list(TYPES.values()), ids=list(TYPES))
+def test_norm_of_a_zero_row(dev, ty):
+    # without an eps to hold it up, the root mean square of the row is zero: the products are zero, not 0 / 0
+    raw = weights(5, 40, 512, ty)
+    w = kb.QMatrix.from_raw_bytes(dev, (40, 512), raw, ty)
+    x, norm = dev.tensor(np.zeros((1, 512), np.float32)), dev.tensor(np.ones(512, np.float32))
+    assert np.array_equal(x.rms_norm_q_mat_mul(norm, 0.0, w).as_slice(), np.zeros((1, 40), np.float32))
+
+
 def test_single_row_sums_of_offset_formats(dev):
     # Q4_0 subtracts eight times the sum of 16 activations, which is formed in integers. Error against 64 bits: 1.7e-7 in that
     # way, 2.15e-7 with sums in floats; the seeds differ by 2 %.
