@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_kernel(const fb200_lin
 #pragma unroll
     for (int i = 0; i < EPT / 2; ++i) s[i] = make_float2(0.f, 0.f);
   }
-  // beside an attention the projections are there; that kernel is waited for at the end, for those that wait for this one
+  // beside an attention the projections are there; that kernel is waited for at the end, for those that wait for this one. (They are read
+  // in L2: without a wait of its own the kernel does not count on an L1 without an earlier layer's)
   if (!a.beside) pdl_wait();
   pdl_launch_dependents();
   const float2 g2 = make_float2(decay, decay);
@@ -95,12 +96,12 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_kernel(const fb200_lin
     for (int i = tid; i < n * DP; i += LS_THREADS) {
       const int t = i / DP, e = i % DP;
       const float* yr = a.y + ((size_t)b * a.s + t0 + t) * a.ldy + (size_t)h * a.d + e;
-      qs[t][e] = e < a.d ? dr_silu(yr[0]) : 0.f;
-      ks[t][e] = e < a.d ? dr_silu(yr[a.off_k]) : 0.f;
+      qs[t][e] = e < a.d ? dr_silu(__ldcg(yr)) : 0.f;
+      ks[t][e] = e < a.d ? dr_silu(__ldcg(yr + a.off_k)) : 0.f;
     }
     for (int i = tid; i < n * LS_COLS; i += LS_THREADS) {
       const int t = i / LS_COLS, cc = c0 + i % LS_COLS;
-      vs[t][i % LS_COLS] = cc < a.v ? dr_silu(a.y[((size_t)b * a.s + t0 + t) * a.ldy + a.off_v + (size_t)h * a.v + cc]) : 0.f;
+      vs[t][i % LS_COLS] = cc < a.v ? dr_silu(__ldcg(a.y + ((size_t)b * a.s + t0 + t) * a.ldy + a.off_v + (size_t)h * a.v + cc)) : 0.f;
     }
     __syncthreads();
 #pragma unroll 4

@@ -205,6 +205,38 @@ def test_state_of_an_earlier_request_is_gone(dev, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kind", ["delta", "latent", "parallel", "all"])
+def test_kernels_side_by_side_change_nothing(kind, dtype, monkeypatch):
+    # One sequence: the feed-forward rows run beside the mixer, and a linear attention beside a softmax attention. The same kernels one
+    # after the other give the same bits, step by step and through the captured step. Wide layers, so that the
+    # rows beside outlast the mixers in some and not in others.
+    if kind == "parallel":
+        util, layers = V, [V.parallel(a=V.left(heads=8, kv_heads=2, dim=64, vdim=64), b=V.right(heads=8, dim=64, vdim=64), mlp=n) for n in (2048, 64, 1000)]
+    else:
+        util, layers = U, [U.delta(heads=8, kv_heads=4, dim=64, vdim=64, ff=n) for n in (2048, 64)] if kind != "latent" else []
+        if kind != "delta":
+            layers = layers + [U.latent(heads=8, dim=64, rot=32, vdim=64, rank=128, window=40, ff=n) for n in (64, 2048)]
+    cfg = util.config(layers * 2, width=512, vocab=600)
+    w = util.weights(cfg, 80)
+    t = np.random.default_rng(80).integers(0, 600, 60)
+    out = []
+    for pdl in ("1", "0"):
+        monkeypatch.setenv("FB200_PDL", pdl)
+        own = kb.Device(0)
+        m = util.gpu_model(own, cfg, w, dtype)
+        m.forward(t[:5], want_logits=False)
+        logits = [m.forward(t[i:i + 1])[0] for i in range(5, 60)]
+        ids = m.generate_greedy(t[:1], 60)
+        logits.append(m.forward(t[:1])[0])
+        out.append((np.stack(logits), ids))
+        assert own.status() == 0
+        m.free()
+        own.close()
+    assert np.array_equal(out[0][0].view(np.uint32), out[1][0].view(np.uint32))
+    assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_batch_equals_each_sequence_alone(dev, dtype):
     cfg = mixed()
     w = V.weights(cfg, 11)
