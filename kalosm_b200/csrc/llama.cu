@@ -784,7 +784,8 @@ int fb200_llama_create(fb200_device* dev, const fb200_llama_config* cfg, fb200_l
     for (int i = 0; i < 5; ++i) { *f32s[i] = reinterpret_cast<uint2*>(p); p += f32_n[i] * sizeof(uint2); }
     m->part_ll = reinterpret_cast<uint2*>(p);
     m->part_epoch = reinterpret_cast<unsigned*>(p + part_n * sizeof(uint2));
-    const unsigned first = 1;  // 0 is what cleared rows carry
+    unsigned first = 1;  // 0 is what cleared rows carry
+    if (const char* e = getenv("FB200_FUSED_EPOCH")) first = (unsigned)strtoul(e, nullptr, 10);
     FB_CUDA(dev, cudaMemcpy(m->part_epoch, &first, sizeof first, cudaMemcpyHostToDevice));
     if (const char* e = getenv("FB200_FUSED_LL")) m->fused_flagged = e[0] == '1' && e[1] == 0;
   }

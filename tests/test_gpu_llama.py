@@ -168,6 +168,26 @@ def test_decode_across_split_counts(dev, n_head, n_kv_head, prompt, flagged_rows
         t = run[step:step + 1].astype(np.uint32)
 
 
+def test_decode_across_the_wrap_of_the_epochs(dev, monkeypatch):
+    # The granules of q, k, v and of the partial rows carry a 32-bit epoch that grows from launch to launch. 0 is what cleared rows carry:
+    # a count that would run over it, in a launch of one step or of several, starts again at 1.
+    cfg = dict(tiny_cfg(), ctx=128, head_dim=128, n_head=6, n_kv_head=2)
+    toks = np.random.default_rng(9).integers(0, cfg["vocab"], size=(1, 46), dtype=np.uint32)
+    want = None
+    for first in (1, 2**32 - 1, 2**32 - 2, 2**32 - 7, 2**32 - 40, 2**32 - 100, 0):
+        monkeypatch.setenv("FB200_FUSED_EPOCH", str(first))
+        gpu, _ = build_models(dev, cfg, batch=1, seed=22)
+        gpu.forward(toks[:, :40])
+        logits = [gpu.forward(toks[:, i:i + 1])[0] for i in range(40, 46)]
+        ids = gpu.generate_greedy(toks[0, :1], 30)
+        logits.append(gpu.forward(toks[:, :1])[0])
+        got = np.stack(logits).view(np.uint32)
+        want = want or (got, ids)
+        assert np.array_equal(got, want[0]) and np.array_equal(ids, want[1]), first
+        gpu.free()
+    assert dev.status() == 0
+
+
 def test_model_loaded_from_a_gguf_file_equals_the_directly_built_one(dev, tmp_path):
     # checkpoint -> GGUF file -> kalosm_b200.gguf.load_llama: same bytes on the device as setting
     # the tensors one by one, so logits and greedy ids agree bit for bit
