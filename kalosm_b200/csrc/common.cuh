@@ -82,9 +82,11 @@ int fb200_fail(fb200_device* dev, int code, const char* fmt, ...);
 #define FB_CUDA(dev, expr)                                                              \
   do {                                                                                  \
     cudaError_t e__ = (expr);                                                           \
-    if (e__ != cudaSuccess)                                                             \
+    if (e__ != cudaSuccess) {                                                           \
+      cudaGetLastError(); /* reported here, not by the check of a later launch */       \
       return fb200_fail((dev), FB200_ERR_CUDA, "%s: %s (%s:%d)", #expr,                 \
                         cudaGetErrorString(e__), __FILE__, __LINE__);                   \
+    }                                                                                   \
   } while (0)
 
 #define FB_LAUNCH_CHECK(dev)                                                            \

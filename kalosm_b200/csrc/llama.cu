@@ -143,6 +143,8 @@ int ensure_rows(fb200_llama* m, size_t rows) {
   FB_CUDA(dev, cudaStreamSynchronize(dev->stream));
   if (m->graph_exec) { cudaGraphExecDestroy(m->graph_exec); m->graph_exec = nullptr; }
   m->fused_valid = false;  // the program holds pointers into these buffers
+  m->rows_cap = 0;         // where there is no room for the new ones, the next call starts over
+  m->last_batch = m->last_seq = 0;
   int rc;
   if (m->hybrid) {
     if ((rc = fb200_hybrid_ensure_rows(m, rows))) return rc;
@@ -162,6 +164,7 @@ int ensure_rows(fb200_llama* m, size_t rows) {
   if ((rc = alloc_f(dev, &m->hbuf, rows * c.ffn))) return rc;
   if ((rc = alloc_f(dev, &m->gbuf, rows * c.ffn))) return rc;
   if (m->ids) cudaFree(m->ids);
+  m->ids = nullptr;
   FB_CUDA(dev, cudaMalloc(&m->ids, rows * sizeof(uint32_t)));
   m->rows_cap = rows;
   return FB200_OK;

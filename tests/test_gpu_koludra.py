@@ -165,6 +165,26 @@ def test_delta_prompt_without_room_for_chunks(monkeypatch):
     own.close()
 
 
+def test_a_pass_without_room_leaves_the_model_usable(dev):
+    # A million rows of 132 thousand projections (520 GB) are refused by the allocation of their buffers. The buffers of the
+    # pass before are gone by then: its rows cannot be asked for any more, and the next pass makes its own.
+    cfg = U.config([U.delta(ff=0, heads=512, kv_heads=512, dim=64, vdim=64)], width=16, vocab=16)
+    w = U.weights(cfg, 64, U.identity_head(cfg))
+    m = U.gpu_model(dev, cfg, w, "bfloat16", max_seq_len=1 << 20)
+    t = toks(cfg, 5)
+    want = U.run_portions(m, t, [5])
+    m.reset()
+    with pytest.raises(kb.FusorError) as e:
+        m.forward(np.zeros((1 << 20) - 1, np.uint32), want_logits=False)
+    assert "memory" in str(e.value)
+    with pytest.raises(kb.FusorError):
+        m.logits_at([0])
+    assert m.position == 0
+    assert np.array_equal(U.run_portions(m, t, [5]).view(np.uint32), want.view(np.uint32))
+    m.free()
+    assert dev.status() == 0
+
+
 BAD_ROW = 7  # a token whose embedding the tests below replace
 
 
