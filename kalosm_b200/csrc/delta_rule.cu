@@ -973,9 +973,10 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("
 // A CTA per (16 columns of S, head). Warps 0 .. 3 carry the recurrence: each holds a quarter of d of S^T [16][d] as accumulator tiles,
 // which are the A operands of S^T W^T as they are; the quarters' sums meet in shared memory, become w = r_last (U - W S), again an A
 // operand, and S^T <- G S^T + w^T K. Warps 4 .. 7 follow with the read-out O + Z S from a copy of S, a chunk behind at most. Warp 8
-// fetches the matrices two chunks ahead (what 128 CTAs have in flight a chunk ahead is too little for HBM). The update is summed from zero and added to S in one rounding, so S drifts no more than
-// with 32-bit sums. Bound: issue (144 products of 8.2 cycles and 1500 other instructions per chunk and scheduler) and the chain of a chunk:
-// 3300 cycles. 8192 tokens of 16 heads of 128: 0.47 ms and 0.18 ms of preparation (delta_scan_kernel: 1.22 ms and 0.03).
+// fetches the matrices two chunks ahead (what 128 CTAs have in flight a chunk ahead is too little for HBM). The update is summed
+// from zero and added to S in one rounding, so S drifts no more than with 32-bit sums. Bound: issue (144 products of 8.2 cycles and
+// 1500 other instructions per chunk and scheduler) and the chain of a chunk: 3500 cycles. 8192 tokens of 16 heads of 128: 0.51 ms and 0.19
+// ms of preparation (with two tf32 values 0.49 and 0.18; delta_scan_kernel: 1.22 ms and 0.03).
 template <int DP>
 __global__ void __launch_bounds__(CS_THREADS, 1) delta_chunk_scan_kernel(const fb200_delta_args a) {
   constexpr int KS = DP / 4, KT = KS / 8, MAT = CT * DP, KLD = DP + 4;  // a warp's part of d, in tiles of 8; floats of a matrix, of a row of K
@@ -1282,19 +1283,36 @@ int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
   return FB200_OK;
 }
 
-// Chunks of 32 tokens or passes of eight. Four layers of 16 heads of 128, passes / chunks: 100 tokens 426 / 452 us, 200 tokens 482 / 481,
-// 512 tokens 690 / 579, 4096 tokens 3398 / 2217 (heads of 64: 393 / 406, 448 / 423, 659 / 512, 3269 / 1860): a chunk's preparation
-// has a longer chain than a few passes. Heads of more than 128 do not fit: three stages of their matrices need 250 KB.
-// Models in float32 keep the passes of eight, whose error is the smaller one (by 0.2 %, see above): there a chunk rounds W, U and Z
-// between its products. FB200_DELTA_CHUNKS=1 takes chunks wherever the head size allows, 0 never.
-constexpr int CHUNKS_FROM = 192;
-
 }  // namespace
 
-bool fb200_delta_in_chunks(int dp, int s, bool bf16) {
+// Chunks of 32 tokens or passes of eight. A chunk's preparation has a longer chain than a few passes, and the scan over chunks takes 16 columns
+// a CTA and one CTA per SM, where the passes take 32 columns and two CTAs share an SM. Four layers, b = 1, passes / chunks in us:
+//   heads of 128, v 128         192 tokens    256          512          2048
+//    8  ( 64 CTAs of 148 SMs)   356 /  349   402 /  386   554 /  453   1540 /  914
+//   16  (128)                   391 /  398   418 /  413   605 /  518   1686 / 1141
+//   24  (192)                               498 /  518   733 /  681   2208 / 1821
+//   32  (256)                   481 /  525   542 /  557   802 /  751   2376 / 2092
+//   40  (320)                               681 /  665  1060 /  965   3310 / 2729
+//   54  (432)                               760 /  751  1166 / 1080   3528 / 3071
+//   64  (512)                   707 /  777   816 /  872  1243 / 1309   3706 / 3840
+//   heads of 64, v 64           192           256          512          1024          4096
+//   16  ( 64)                   349 /  324   392 /  332   563 /  406
+//   32  (128)                   391 /  359   432 /  375   622 /  470
+//   38  (152)                                            648 /  628   1049 /  995   3452 / 3069
+//   48  (192)                                            672 /  674   1096 / 1053   3634 / 3352
+//   64  (256)                   449 /  466   532 /  532   761 /  791   1230 / 1243   3951 / 3841
+// (384 tokens of 20, 32, 36, 40 and 54 heads of 128: 610 / 581, 683 / 675, 698 / 683, 872 / 804, 962 / 936.)
+// What counts is columns, not heads: 8 heads of four sequences or of four times the columns lie where 32 heads do (16 heads of 128, four sequences:
+// 512 tokens 1130 / 1201, as 64 heads). Heads of more than 128 do not fit: three stages of their matrices take 290 KB.
+// Models in float32 keep the passes of eight, whose error is the smaller one (by 0.2 %, see above): there a chunk rounds W, U and Z
+// between its products. FB200_DELTA_CHUNKS=1 takes chunks wherever the head size allows, 0 never.
+bool fb200_delta_in_chunks(const fb200_device* dev, int dp, int h, int v, int b, int s, bool bf16) {
   if (s == 1 || (dp != 64 && dp != 128)) return false;
   if (const char* e = getenv("FB200_DELTA_CHUNKS")) return e[0] == '1';
-  return bf16 && s >= CHUNKS_FROM;
+  const long ctas = (long)b * h * ((v + SCOLS - 1) / SCOLS), sms = dev->sm_count;
+  if (!bf16) return false;
+  if (dp == 64) return ctas <= sms ? s >= 192 : 2 * ctas <= 3 * sms && s >= 512;
+  return 2 * ctas <= sms ? s >= 192 : ctas <= sms ? s >= 256 : ctas <= 3 * sms && s >= 384;
 }
 size_t fb200_delta_wq_floats(int b, int s, int h, int dp) { return (size_t)b * h * ((s + CT - 1) / CT) * 2 * CT * dp; }
 size_t fb200_delta_dec_floats(int b, int s, int h) { return (size_t)b * h * ((s + CT - 1) / CT) * CDEC; }
@@ -1327,7 +1345,7 @@ int fb200_delta_prompt(fb200_device* dev, const fb200_delta_args& a) {
     default: return fb200_fail(dev, FB200_ERR_INVALID_SHAPE, "delta rule: head size %d", a.d);
   }
   if (rc) return rc;
-  if (a.wq && fb200_delta_in_chunks(a.dp, a.s, a.z_bf16)) {
+  if (a.wq && fb200_delta_in_chunks(dev, a.dp, a.h, a.v, a.b, a.s, a.z_bf16)) {
     rc = a.dp == 64 ? launch_chunks<64>(dev, a) : launch_chunks<128>(dev, a);
   } else {
     rc = fb200_launch(dev, delta_pairs_kernel, dim3((unsigned)((a.s + CH - 1) / CH), (unsigned)((a.hk + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b),

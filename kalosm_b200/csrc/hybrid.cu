@@ -529,7 +529,7 @@ int ensure_chunks(fb200_llama* m, int batch, int seq) {
   fb200_hybrid* hy = m->hybrid;
   size_t wq = 0, dec = 0;
   for (const auto& M : hy->mixers)
-    if (M.c.mixer == FB200_MIX_DELTA && fb200_delta_in_chunks(M.dp, seq, !hy->f32)) {
+    if (M.c.mixer == FB200_MIX_DELTA && fb200_delta_in_chunks(dev, M.dp, M.c.heads, M.c.vdim, batch, seq, !hy->f32)) {
       wq = std::max(wq, fb200_delta_wq_floats(batch, seq, M.c.heads, M.dp));
       dec = std::max(dec, fb200_delta_dec_floats(batch, seq, M.c.heads));
     }

@@ -31,7 +31,7 @@ struct fb200_delta_args {
   float *wq, *dec;
   int* status;
 };
-bool fb200_delta_in_chunks(int dp, int s, bool bf16);                 // whether a pass takes chunks where it has wq and dec
+bool fb200_delta_in_chunks(const fb200_device* dev, int dp, int h, int v, int b, int s, bool bf16);  // whether a pass takes chunks where it has wq and dec
 size_t fb200_delta_wq_floats(int b, int s, int h, int dp);
 size_t fb200_delta_dec_floats(int b, int s, int h);
 int fb200_delta_dp(int d);                                         // padded head size, 0 when d is not covered

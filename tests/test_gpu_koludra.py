@@ -6,6 +6,7 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 import hybrid_util as U
 import kalosm_b200 as kb
@@ -124,6 +125,35 @@ def test_delta_prompts_in_chunks(dev, dtype, shape, sizes, monkeypatch):
     cfg = U.config([U.delta(ff=0, **shape)], width=88, vocab=88)
     w = U.weights(cfg, 50 + sum(sizes), U.identity_head(cfg))
     check(dev, cfg, w, toks(cfg, sum(sizes)), dtype, sizes)
+
+
+@pytest.mark.parametrize("heads,dim,vdim,batch,lengths", [(9, 128, 128, 1, (191, 192)), (4, 128, 300, 1, (255, 256)), (6, 128, 40, 8, (255, 256)),
+                                                          (19, 128, 128, 1, (383, 384)), (3, 128, 128, 18, (383, 384)), (56, 128, 128, 1, (400,)),
+                                                          (37, 64, 64, 1, (191, 192)), (38, 64, 64, 1, (511, 512)), (28, 64, 64, 2, (512,))])
+def test_delta_prompts_take_chunks_by_their_columns(dev, heads, dim, vdim, batch, lengths, monkeypatch):
+    # Both sides of every line of the rule on 148 SMs (16 columns a CTA): the pass is the one that the rule names, bit for bit, and the
+    # two forms agree within the rounding that they do apart. Their read-outs differ in the last bits of 32, so a row differs where
+    # that moves a bf16 operand by a step, 2^-7 of it at most: one of four times the mean size among heads x vdim of them.
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lengths are those of 148 SMs")
+    cfg = U.config([U.delta(ff=0, heads=heads, kv_heads=1, dim=dim, vdim=vdim)], width=88, vocab=88)
+    w = U.weights(cfg, 65, U.identity_head(cfg))
+    for n in lengths:
+        t = np.random.default_rng(n).integers(0, 88, (batch, n))
+        got = []
+        for form in (None, "0", "1"):
+            if form is None:
+                monkeypatch.delenv("FB200_DELTA_CHUNKS", raising=False)
+            else:
+                monkeypatch.setenv("FB200_DELTA_CHUNKS", form)
+            m = U.gpu_model(dev, cfg, w, "bfloat16", max_batch=batch)
+            m.forward(t, want_logits=False)
+            got.append(m.logits_at(range(batch * n)))
+            m.free()
+        chunks = len(lengths) == 2 and n == lengths[1]
+        assert np.array_equal(got[0], got[2 if chunks else 1]) and not np.array_equal(got[1], got[2]), n
+        assert U.err(got[2], got[1]) < 4 * 2.0 ** -7 / (heads * vdim) ** 0.5
+    assert dev.status() == 0
 
 
 def test_delta_prompts_of_float32_models(dev):
