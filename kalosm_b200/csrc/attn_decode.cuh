@@ -378,6 +378,7 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
         acc *= l > 0.f ? 1.0f / l : 0.f;
         if (a.out) a.out[grow * D + e] = acc;
       }
+      // packed rows are single-sequence; nrows * D is a multiple of 32, so `valid` is warp-uniform
       if constexpr (LLOUT) {
         if (bi == 0 && valid) emit_ll16(a.out_ll, (int)(grow * D) + e, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
       } else {
@@ -403,56 +404,50 @@ __device__ void attn_decode_item(const DecArgs& a, int item, uint8_t* dsm, int t
       if (e == 0) { pp[D] = row_m[r]; pp[D + 1] = row_l[r]; }
     }
   }
-  if constexpr (SPREAD) return;
-  // ---- the split that arrives last merges all partials of this (batch, kv head) in split order
-  __threadfence();
-  dec_sync<BAR>();
-  if (tid == 0) {
-    const int old = atomicAdd(a.done + bi * a.hkv + kvh, 1);
-    is_last = (old == a.nsplit - 1);
-    if (is_last) a.done[bi * a.hkv + kvh] = 0;
-  }
-  dec_sync<BAR>();
-  if (!is_last) return;
-  __threadfence();
-  // Merge in split order. Every thread owns one output element (r, e) per pass and needs, for its
-  // row, all splits' maxima and normalisers and its own column of all partial rows: all of these
-  // loads are issued before the first use, so the merge costs one trip to L2, not one per step.
-  // Lane s of a warp holds split s's maximum and normaliser; the weights travel by shuffle.
-  constexpr int MAXS = 32;
-  for (int i0 = 0; i0 < nrows * D; i0 += ATT_THREADS) {
-    const int i = i0 + tid;
-    const bool valid = i < nrows * D;
-    const int r = valid ? i / D : 0, e = i % D;
-    const size_t grow = (size_t)bi * a.h + kvh * a.groups + r;
-    float acc = 0.f;
-    if (valid) {
-      // (a warp's 32 consecutive elements share the row r: D is a multiple of 32)
-      const float* base = a.part + grow * (D + 2);
-      const size_t sstride = rows_all * (D + 2);
-      const float pm = lane < a.nsplit ? __ldcg(base + lane * sstride + D) : -INFINITY;  // lane s: split s
-      const float pl = lane < a.nsplit ? __ldcg(base + lane * sstride + D + 1) : 0.f;
-      float pv[MAXS];
-#pragma unroll
-      for (int s0 = 0; s0 < MAXS; ++s0) pv[s0] = s0 < a.nsplit ? __ldcg(base + s0 * sstride + e) : 0.f;
-      float mx = pm;
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o2));
-      const float wgt = (pm == -INFINITY) ? 0.f : __expf(pm - mx);
-      float l = pl * wgt;
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o2);
-#pragma unroll
-      for (int s0 = 0; s0 < MAXS; ++s0) acc = fmaf(pv[s0], __shfl_sync(0xFFFFFFFFu, wgt, s0), acc);
-      acc *= l > 0.f ? 1.0f / l : 0.f;
-      if (a.out) a.out[grow * D + e] = acc;
+  if constexpr (!SPREAD) {
+    // ---- the split that arrives last merges all partials of this (batch, kv head) in split order
+    __threadfence();
+    dec_sync<BAR>();
+    if (tid == 0) {
+      const int old = atomicAdd(a.done + bi * a.hkv + kvh, 1);
+      is_last = (old == a.nsplit - 1);
+      if (is_last) a.done[bi * a.hkv + kvh] = 0;
     }
-    // packed rows are single-sequence; nrows * D is a multiple of 32, so `valid` is warp-uniform
-    if constexpr (LLOUT) {
-      if (bi == 0 && valid) emit_ll16(a.out_ll, (int)(grow * D) + e, acc, acc, true, 0xFFFFFFFFu, a.ep_out);
-    } else {
-      if (a.out_packed.limbs && bi == 0 && valid)
-        emit_packed16(a.out_packed, (int)(grow * D) + e, acc, acc, true, 0xFFFFFFFFu);
+    dec_sync<BAR>();
+    if (!is_last) return;
+    __threadfence();
+    // Merge in split order. Every thread owns one output element (r, e) per pass and needs, for its
+    // row, all splits' maxima and normalisers and its own column of all partial rows: all of these
+    // loads are issued before the first use, so the merge costs one trip to L2, not one per step.
+    // Lane s of a warp holds split s's maximum and normaliser; the weights travel by shuffle.
+    constexpr int MAXS = 32;
+    for (int i0 = 0; i0 < nrows * D; i0 += ATT_THREADS) {
+      const int i = i0 + tid;
+      const bool valid = i < nrows * D;
+      const int r = valid ? i / D : 0, e = i % D;
+      const size_t grow = (size_t)bi * a.h + kvh * a.groups + r;
+      float acc = 0.f;
+      if (valid) {
+        // (a warp's 32 consecutive elements share the row r: D is a multiple of 32)
+        const float* base = a.part + grow * (D + 2);
+        const size_t sstride = rows_all * (D + 2);
+        const float pm = lane < a.nsplit ? __ldcg(base + lane * sstride + D) : -INFINITY;  // lane s: split s
+        const float pl = lane < a.nsplit ? __ldcg(base + lane * sstride + D + 1) : 0.f;
+        float pv[MAXS];
+#pragma unroll
+        for (int s0 = 0; s0 < MAXS; ++s0) pv[s0] = s0 < a.nsplit ? __ldcg(base + s0 * sstride + e) : 0.f;
+        float mx = pm;
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o2));
+        const float wgt = (pm == -INFINITY) ? 0.f : __expf(pm - mx);
+        float l = pl * wgt;
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o2);
+#pragma unroll
+        for (int s0 = 0; s0 < MAXS; ++s0) acc = fmaf(pv[s0], __shfl_sync(0xFFFFFFFFu, wgt, s0), acc);
+        acc *= l > 0.f ? 1.0f / l : 0.f;
+        a.out[grow * D + e] = acc;
+      }
     }
   }
 }

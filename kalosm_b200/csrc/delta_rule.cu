@@ -1275,10 +1275,14 @@ int launch_prep(fb200_device* dev, const fb200_delta_args& a) {
   const int units = a.hk + (a.h * a.v + PREP_VCH - 1) / PREP_VCH + 1;
   const bool by4 = !((a.d | a.v | a.off_v | (int)(a.ldy & 3)) & 3) &&
                    !((reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.conv_w) | reinterpret_cast<uintptr_t>(a.ring)) & 15);
-  const int tok = by4 && NE <= 8 ? PREP4_TOK : PREP_TOK;
-  const dim3 grid((unsigned)((a.s + tok - 1) / tok), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b);
-  if (tok == PREP4_TOK) delta_prep4_kernel<(NE + 3) / 4><<<grid, PREP_WARPS * 32, 0, dev->stream>>>(a);
-  else delta_prep_kernel<NE><<<grid, PREP_WARPS * 32, 0, dev->stream>>>(a);
+  auto launch = [&](auto kernel, int tok) {
+    kernel<<<dim3((unsigned)((a.s + tok - 1) / tok), (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), (unsigned)a.b), PREP_WARPS * 32, 0, dev->stream>>>(a);
+  };
+  bool pieces = false;
+  if constexpr (NE <= 8) {  // (heads of 512 need more registers than there are)
+    if ((pieces = by4)) launch(delta_prep4_kernel<(NE + 3) / 4>, PREP4_TOK);
+  }
+  if (!pieces) launch(delta_prep_kernel<NE>, PREP_TOK);
   FB_LAUNCH_CHECK(dev);
   return FB200_OK;
 }
