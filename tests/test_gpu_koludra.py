@@ -127,6 +127,28 @@ def test_delta_prompts_in_chunks(dev, dtype, shape, sizes, monkeypatch):
     check(dev, cfg, w, toks(cfg, sum(sizes)), dtype, sizes)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [dict(heads=16, kv_heads=4, dim=64, vdim=24), dict(heads=6, kv_heads=3, dim=128, vdim=80)], ids=str)
+def test_delta_chunks_of_several_sequences(dev, dtype, shape, monkeypatch):
+    # Three sequences and more than four heads: each sequence has its own rows, chunks (the last one ragged), state and
+    # convolution memory, in a first pass, in one on top of it and in a step
+    monkeypatch.setenv("FB200_DELTA_CHUNKS", "1")
+    cfg = U.config([U.delta(ff=24, **shape), U.delta(ff=0, **shape)], width=88, vocab=88)
+    w = U.weights(cfg, 66, U.identity_head(cfg))
+    t = np.random.default_rng(66).integers(0, 88, (3, 272))
+    m = U.gpu_model(dev, cfg, w, dtype, max_batch=3)
+    parts = []
+    for a, b in ((0, 201), (201, 271), (271, 272)):
+        m.forward(t[:, a:b], want_logits=False)
+        parts.append(m.logits_at(range(3 * (b - a))).reshape(3, b - a, -1))
+    m.free()
+    got = np.concatenate(parts, 1)
+    for b in range(3):
+        want = U.oracle_logits(cfg, w, t[b])
+        assert U.err(got[b], want) < U.tolerance(cfg, w, t[b], want, dtype), b
+    assert dev.status() == 0
+
+
 @pytest.mark.parametrize("heads,dim,vdim,batch,lengths", [(9, 128, 128, 1, (191, 192)), (4, 128, 300, 1, (255, 256)), (6, 128, 40, 8, (255, 256)),
                                                           (19, 128, 128, 1, (383, 384)), (3, 128, 128, 18, (383, 384)), (56, 128, 128, 1, (400,)),
                                                           (37, 64, 64, 1, (191, 192)), (38, 64, 64, 1, (511, 512)), (28, 64, 64, 2, (512,))])
