@@ -36,7 +36,8 @@ struct fb200_llama {
         *attn_out = nullptr, *hbuf = nullptr, *gbuf = nullptr, *last = nullptr, *logits = nullptr;
   float* att_part = nullptr;
   uint2* part_ll = nullptr;        // persistent step: partial rows of the attention's splits (in ll_slab)
-  unsigned* part_epoch = nullptr;  // and the epoch of the next launch's first phase
+  unsigned* part_epoch = nullptr;  // and the epoch of the next launch's first phase, which next_epoch follows
+  uint32_t next_epoch = 1;
   size_t att_part_bytes = 0;
   uint32_t *ids = nullptr, *next = nullptr, *hist = nullptr;
   int hist_cap = 0;
@@ -49,14 +50,15 @@ struct fb200_llama {
   int* att_done = nullptr;  // arrival counters of the attention splits, one per (batch, kv head)
   // single-row step: activation rows travel between kernels in the products' operand form
   fb200_packed_act px, patt, pv, ph;  // residual stream, attention output, attn_out + x, SwiGLU output
-  // the same rows (and q / k / v, the residual stream and the attention projection as f32) as flagged
-  // rows for the barrier-free variants of the persistent kernel: one slab, zero at creation
+  // the same rows (and the residual stream and the attention projection as f32) as flagged rows for the barrier-free
+  // variants of the persistent kernel; q, k and v are flagged in all its variants: one slab, zero at creation
   uint8_t* ll_slab = nullptr;
+  size_t ll_slab_bytes = 0;
   fb200_ll_act px_ll, patt_ll, pv_ll, ph_ll;
   uint2 *q_ll = nullptr, *k_ll = nullptr, *v_ll = nullptr, *x_ll = nullptr, *attn_ll = nullptr;
   // FB200_FUSED_LL=1 selects the barrier-free variants. Off by default: they are correct (parity
-  // tests run both forms) but measured slower so far (2.2 - 2.6 ms per step of the 8B-shaped model
-  // against 2.03 ms with grid barriers): the trip a flagged row saves at each phase boundary is
+  // tests run both forms) but measured slower so far (2.2 - 2.7 ms per step of the 8B-shaped model
+  // against 1.83 ms with grid barriers): the trip a flagged row saves at each phase boundary is
   // outweighed by slower epilogues (8-byte flagged stores), the 86 KB polled row in front of the
   // down projection and a product loop that gets fewer registers.
   bool fused_flagged = false;

@@ -876,14 +876,10 @@ fused_step_kernel(const FusedArgs A) {
   // What the attention phases need, in shared memory because the product loop has no registers to spare: the step's position, and
   // the launch's first epoch. The epochs of the flagged rows go on from launch to launch in the model's memory (a captured
   // launch may be replayed): CTA 0 stores the next one at the end, when every CTA has passed a meeting. Without meetings
-  // the launch brings its own. 0 is what cleared rows carry: a launch whose epochs would run over it starts at 1.
+  // the launch brings its own.
   __shared__ int att_pos;
   __shared__ unsigned att_ep;
-  const unsigned epochs = (unsigned)(A.nsteps * A.nphases);
-  if (tid == 0) {
-    att_ep = LL ? A.epoch_base : A.part_epoch ? ld_relaxed_u32(A.part_epoch) : 0u;
-    if (!LL && (att_ep == 0u || att_ep + epochs < att_ep)) att_ep = 1u;
-  }
+  if (tid == 0) att_ep = LL ? A.epoch_base : A.part_epoch ? ld_relaxed_u32(A.part_epoch) : 0u;
   for (int g = 0; g < DESC_SLOTS - 1; ++g) load_desc(g);
   cp_async_wait_all();
   __syncthreads();
@@ -948,7 +944,7 @@ fused_step_kernel(const FusedArgs A) {
       cp_async_wait_all();  // this thread's part of the descriptor fetched during the phase (the meeting above publishes it)
     }
   }
-  if (!LL && A.part_epoch && blockIdx.x == 0 && tid == 0) *A.part_epoch = att_ep + epochs;
+  if (!LL && A.part_epoch && blockIdx.x == 0 && tid == 0) *A.part_epoch = att_ep + (unsigned)(A.nsteps * A.nphases);
 }
 
 size_t x_region_need(const fb200_fused_phase* prog, int nphases, bool flagged) {
