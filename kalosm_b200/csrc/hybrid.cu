@@ -410,12 +410,11 @@ int run_mixer(fb200_llama* m, const Mixer& M, int pass, int batch, int seq, bool
 }
 
 // Places for two CTAs per SM of a product of one row that a mixer's kernels hold while they run, by their registers
-int held_places(const fb200_device* dev, const Mixer& M, int cap) {
+int held_places(const Mixer& M) {
   const auto& c = M.c;
   switch (c.mixer) {
     case FB200_MIX_DELTA: return 2 * c.heads;                                     // 512 threads a head
     case FB200_MIX_LINEAR: return c.heads * ((c.vdim + 15) / 16);                  // 256 threads a head and 16 columns
-    case FB200_MIX_LATENT: return c.heads * ((c.vdim + 31) / 32) + (c.heads + 15) / 16 * fb200_latent_nsplit(dev, 1, c.heads, c.window, cap);
     default: return 0;
   }
 }
@@ -448,10 +447,11 @@ int run_layer(fb200_llama* m, const MixerLayer& L, int pass, float* x, int batch
   in.act = L.act; in.ff = L.ffn; in.gate0 = L.n_plain; in.up0 = L.n_plain + (L.act == FB200_FFN_SWIGLU ? L.ffn : 0);
   in.z = wide ? (void*)(hy->zf + L.ko) : (void*)(hy->zb + L.ko); in.ldz = hy->ldz;
   // One row: the mixer's latency leaves HBM idle, so the feed-forward rows, which need nothing of it, go behind it in the stream and
-  // run beside it (10 layers of 2048 with 8192 feed-forward rows, a step: delta rules and latent attentions 485 -> 456 us, softmax and
-  // linear attentions 455 -> 428 us)
+  // run beside it (10 layers, a step, width 2048 / 4096 with 8192 / 14336 feed-forward rows: 6 of them delta rules 446 -> 380 us /
+  // 1062 -> 955, softmax and linear attentions 453 -> 417 / 968 -> 891). Not beside a latent attention: its three kernels have CTAs on
+  // most SMs one after the other, and the rows are in their way (the other 4 of the 10 layers too: 397 / 1085)
   fb200_dense_job ffn = in;
-  const bool split = rows == 1 && L.count > 0 && in.n_plain && in.ff;
+  const bool split = rows == 1 && L.count > 0 && in.n_plain && in.ff && hy->mixers[L.first].c.mixer != FB200_MIX_LATENT;
   if (split) {
     in.ff = 0;
     in.ff_norm_w = nullptr;
@@ -460,7 +460,7 @@ int run_layer(fb200_llama* m, const MixerLayer& L, int pass, float* x, int batch
     if (ffn.ff_norm_w) ffn.norm_w = ffn.ff_norm_w;
     ffn.ff_norm_w = nullptr;
     ffn.beside = true;
-    for (int k = 0; k < L.count; ++k) ffn.held += held_places(dev, hy->mixers[L.first + k], m->cfg.max_seq_len);
+    for (int k = 0; k < L.count; ++k) ffn.held += held_places(hy->mixers[L.first + k]);
   }
   if ((rc = fb200_dense_product(dev, in))) return rc;
 

@@ -150,9 +150,8 @@ __global__ void __launch_bounds__(LA_WARPS * 32) latent_attn_kernel(const fb200_
   extern __shared__ __align__(16) float lsm[];  // [LA_WARPS][rk]
   __shared__ float wm[LA_WARPS], wl[LA_WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, row = blockIdx.z, b = row / a.s;
-  // the kernel in front was let in behind the projections: what follows the mixer and needs no more than them may start
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int pos = *a.pos_dev + row % a.s, n = a.rk + a.r;
   const int lo = a.window ? max(0, pos - a.window + 1) : 0, keys = pos + 1 - lo;
   const int per = (keys + a.nsplit - 1) / a.nsplit, k0 = lo + min(keys, (int)blockIdx.x * per), k1 = min(pos + 1, k0 + per);
@@ -247,9 +246,8 @@ __global__ void __launch_bounds__(LO_THREADS) latent_out_kernel(const fb200_late
       pre[i][k] = make_uint4(0u, 0u, 0u, 0u);
       if (v0 + i < a.v && lane + 32 * k < np) pre[i][k] = *reinterpret_cast<const uint4*>(w + (size_t)(v0 + i) * a.rkp + (lane + 32 * k) * E);
     }
-  // the kernel in front was let in behind the projections: what follows the mixer and needs no more than them may start
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const float* part = a.part + ((size_t)row * a.h + h) * a.nsplit * (a.rk + 2);
   float* wt = lsm + a.rkp;
   if (warp == 0) {  // weights of the splits, normalised
@@ -354,9 +352,8 @@ __global__ void __launch_bounds__(LM_THREADS) latent_attn_mma_kernel(const fb200
     }
   };
   if (k0 < k1) fetch(k0, true);
-  // the kernel in front was let in behind the projections: what follows the mixer and needs no more than them may start
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float o[NT][4];
 #pragma unroll
