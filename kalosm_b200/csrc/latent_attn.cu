@@ -41,21 +41,22 @@ __device__ __forceinline__ void store_elem(__nv_bfloat16* p, float v) { *p = __f
 __device__ __forceinline__ void store_elem(float* p, float v) { *p = v; }
 
 // T: element type of the expansion matrices and of the cache. A row's CTAs take `csplit` column ranges of
-// each query head, the last one the new position.
-template <typename T>
+// each query head, the last one the new position. AHEAD: the first pieces of W_uk, which do not depend on the kernel in front, are
+// requested before its wait: for few rows, where a CTA's chain counts. Over many rows the registers that hold them cost more (the new
+// positions of 8192 rows: 89 us a layer with them, 35 without).
+template <typename T, bool AHEAD>
 __global__ void __launch_bounds__(LQ_THREADS) latent_query_kernel(const fb200_latent_args a, int heads, int csplit) {
   constexpr int E = 16 / (int)sizeof(T);
   extern __shared__ __align__(16) float lsm[];  // query head [d + r], or partial sums [LQ_THREADS][E]
   __shared__ float red[LQ_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, b = row / a.s;
   const int h = blockIdx.x / csplit, cs_i = blockIdx.x % csplit;
-  // W_uk^T q: a thread owns one 16-byte piece of the latent, groups of threads share the sum over d. The first pieces of W_uk do not
-  // depend on the kernel in front
+  // W_uk^T q: a thread owns one 16-byte piece of the latent, groups of threads share the sum over d
   const int np = a.rkp / E;
   const T* w = reinterpret_cast<const T*>(a.w_ukv) + (size_t)h * a.d * a.rkp;
   const int cper = (np + csplit - 1) / csplit, cend = min(np, (cs_i + 1) * cper);
-  uint4 pre[LQ_AHEAD];
-  if (h < heads) {
+  uint4 pre[AHEAD ? LQ_AHEAD : 1];
+  if constexpr (AHEAD) if (h < heads) {
     const int nc = min(cend - cs_i * cper, LQ_THREADS), groups = LQ_THREADS / max(nc, 1), c = tid % max(nc, 1), gr = tid / max(nc, 1);
 #pragma unroll
     for (int k = 0; k < LQ_AHEAD; ++k) {
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(LQ_THREADS) latent_query_kernel(const fb200_la
     for (int e = 0; e < E; ++e) acc[e] = 0.f;
     if (gr < groups) {
       int i0 = gr;
-      if (c0 == cs_i * cper) {
+      if constexpr (AHEAD) if (c0 == cs_i * cper) {
 #pragma unroll
         for (int k = 0; k < LQ_AHEAD; ++k, i0 += groups) {
           float f[E];
@@ -517,9 +518,10 @@ int latent_rows(fb200_device* dev, const fb200_latent_args& a) {
   int rc;
   const int csplit = (a.rkp / E + 15) / 16;
   const size_t smem_q = (size_t)(((a.d + 3) & ~3) + LQ_THREADS * E) * 4;
-  if ((rc = fb200_launch(dev, latent_query_kernel<T>, dim3((unsigned)(a.h * csplit + (a.off_dkv >= 0 ? 1 : 0)), rows), dim3(LQ_THREADS), smem_q, true,
-                         a, a.h, csplit)))
-    return rc;
+  const dim3 grid_q((unsigned)(a.h * csplit + (a.off_dkv >= 0 ? 1 : 0)), rows);
+  if (rows <= 16) rc = fb200_launch(dev, latent_query_kernel<T, true>, grid_q, dim3(LQ_THREADS), smem_q, true, a, a.h, csplit);
+  else rc = fb200_launch(dev, latent_query_kernel<T, false>, grid_q, dim3(LQ_THREADS), smem_q, true, a, a.h, csplit);
+  if (rc) return rc;
   if (latent_mma_covers(a)) {
     rc = a.rk <= 128 ? launch_attn_mma<4>(dev, a) : a.rk <= 256 ? launch_attn_mma<8>(dev, a) : launch_attn_mma<16>(dev, a);
   } else {
@@ -554,8 +556,8 @@ int fb200_latent_append(fb200_device* dev, const fb200_latent_args& a) {
   if (a.off_dkv < 0) return FB200_OK;
   const dim3 grid(1, (unsigned)(a.b * a.s));
   if (a.b * a.s > 65535) return fb200_fail(dev, FB200_ERR_CAPACITY, "latent attention: at most 65535 rows per pass");
-  if (a.cache_f32) return fb200_launch(dev, latent_query_kernel<float>, grid, dim3(LQ_THREADS), 16, true, a, 0, 1);
-  return fb200_launch(dev, latent_query_kernel<__nv_bfloat16>, grid, dim3(LQ_THREADS), 16, true, a, 0, 1);
+  if (a.cache_f32) return fb200_launch(dev, latent_query_kernel<float, false>, grid, dim3(LQ_THREADS), 16, true, a, 0, 1);
+  return fb200_launch(dev, latent_query_kernel<__nv_bfloat16, false>, grid, dim3(LQ_THREADS), 16, true, a, 0, 1);
 }
 
 int fb200_latent_rows(fb200_device* dev, const fb200_latent_args& a) {
