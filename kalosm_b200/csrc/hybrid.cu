@@ -449,9 +449,14 @@ int run_layer(fb200_llama* m, const MixerLayer& L, int pass, float* x, int batch
   // One row: the mixer's latency leaves HBM idle, so the feed-forward rows, which need nothing of it, go behind it in the stream and
   // run beside it (10 layers, a step, width 2048 / 4096 with 8192 / 14336 feed-forward rows: 6 of them delta rules 446 -> 380 us /
   // 1062 -> 955, softmax and linear attentions 453 -> 417 / 968 -> 891). Not beside a latent attention: its three kernels have CTAs on
-  // most SMs one after the other, and the rows are in their way (the other 4 of the 10 layers too: 397 / 1085)
+  // most SMs one after the other, and the rows are in their way (the other 4 of the 10 layers too: 397 / 1085). And not where the rows'
+  // weights are few, for the launch: behind it / beside, 6 layers, us a step, by MB of these weights (bf16, then f32):
+  //   delta rules           8.4: 104 / 114, 105 / 114   16.8: 123 / 118, 121 / 130   33.6: 153 / 140, 207 / 190   67: 314 / 291, 237 / 221
+  //   softmax attentions    8.4: 146 / 156, 143 / 149   16.8: 171 / 179, 192 / 192   33.6: 268 / 251, 341 / 331   101: 383 / 380
+  //   softmax and linear    8.4: 231 / 235, 182 / 191   16.8: 237 / 241, 308 / 305   33.6: 457 / 448, 340 / 326   101: 582 / 558
   fb200_dense_job ffn = in;
-  const bool split = rows == 1 && L.count > 0 && in.n_plain && in.ff && hy->mixers[L.first].c.mixer != FB200_MIX_LATENT;
+  const size_t ff_bytes = (size_t)(L.act == FB200_FFN_SWIGLU ? 2 : 1) * L.ffn * E * (hy->f32 ? 4 : 2);
+  const bool split = rows == 1 && L.count > 0 && in.n_plain && hy->mixers[L.first].c.mixer != FB200_MIX_LATENT && ff_bytes >= (size_t)30 << 20;
   if (split) {
     in.ff = 0;
     in.ff_norm_w = nullptr;

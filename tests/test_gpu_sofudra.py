@@ -205,35 +205,48 @@ def test_state_of_an_earlier_request_is_gone(dev, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("kind", ["delta", "latent", "parallel", "all"])
+@pytest.mark.parametrize("kind", ["delta", "parallel", "attention", "latent"])
 def test_kernels_side_by_side_change_nothing(kind, dtype, monkeypatch):
-    # One sequence: the feed-forward rows run beside the mixer, and a linear attention beside a softmax attention. The same kernels one
-    # after the other give the same bits, step by step and through the captured step. Wide layers, so that the
-    # rows beside outlast the mixers in some and not in others.
-    if kind == "parallel":
-        util, layers = V, [V.parallel(a=V.left(heads=8, kv_heads=2, dim=64, vdim=64), b=V.right(heads=8, dim=64, vdim=64), mlp=n) for n in (2048, 64, 1000)]
-    else:
-        util, layers = U, [U.delta(heads=8, kv_heads=4, dim=64, vdim=64, ff=n) for n in (2048, 64)] if kind != "latent" else []
-        if kind != "delta":
-            layers = layers + [U.latent(heads=8, dim=64, rot=32, vdim=64, rank=128, window=40, ff=n) for n in (64, 2048)]
-    cfg = util.config(layers * 2, width=512, vocab=600)
-    w = util.weights(cfg, 80)
-    t = np.random.default_rng(80).integers(0, 600, 60)
-    out = []
-    for pdl in ("1", "0"):
-        monkeypatch.setenv("FB200_PDL", pdl)
+    # One sequence: feed-forward rows of 32 MB and more run beside the mixer (a launch of their own; not beside a latent attention), and a
+    # linear attention beside a softmax attention. The same kernels one after the other give the same bits, step by step and
+    # through the captured step.
+    big = 16384 if kind in ("delta", "latent") else 32768
+
+    def layer(n):
+        if kind == "delta":
+            return U.delta(heads=8, kv_heads=4, dim=64, vdim=64, ff=n)
+        if kind == "latent":
+            return U.latent(heads=8, dim=64, rot=32, vdim=64, rank=128, window=40, ff=n)
+        if kind == "attention":
+            return V.attention(heads=8, kv_heads=2, dim=64, vdim=64, mlp=n)
+        return V.parallel(a=V.left(heads=8, kv_heads=2, dim=64, vdim=64), b=V.right(heads=8, dim=64, vdim=64), mlp=n)
+    util = U if kind in ("delta", "latent") else V
+    t = np.random.default_rng(80).integers(0, 300, 40)
+
+    def run(cfg, w):
         own = kb.Device(0)
         m = util.gpu_model(own, cfg, w, dtype)
         m.forward(t[:5], want_logits=False)
-        logits = [m.forward(t[i:i + 1])[0] for i in range(5, 60)]
-        ids = m.generate_greedy(t[:1], 60)
+        logits = [m.forward(t[i:i + 1])[0] for i in range(5, 40)]
+        before = own.launch_count
         logits.append(m.forward(t[:1])[0])
-        out.append((np.stack(logits), ids))
+        step = own.launch_count - before
+        ids = m.generate_greedy(t[:1], 40)
+        logits.append(m.forward(t[:1])[0])
         assert own.status() == 0
         m.free()
         own.close()
-    assert np.array_equal(out[0][0].view(np.uint32), out[1][0].view(np.uint32))
-    assert np.array_equal(out[0][1], out[1][1])
+        return np.stack(logits).view(np.uint32), ids, step
+    small = util.config([layer(64), layer(64)], width=512, vocab=300)
+    plain = run(small, util.weights(small, 80))[2]
+    cfg = util.config([layer(big), layer(64)], width=512, vocab=300)
+    w = util.weights(cfg, 80)
+    out = []
+    for pdl in ("1", "0"):
+        monkeypatch.setenv("FB200_PDL", pdl)
+        out.append(run(cfg, w))
+    assert out[0][2] == plain + (kind != "latent")
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
