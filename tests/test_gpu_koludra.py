@@ -631,6 +631,11 @@ def test_poisoned_scratch(dev, monkeypatch):
     w = U.weights(cfg, 21)
     for dtype in DTYPES:
         check(own, cfg, w, toks(cfg, 60), dtype, [40, 3, 1])
+    # and what the chunks of a delta rule hand on, the last one of nine tokens
+    monkeypatch.setenv("FB200_DELTA_CHUNKS", "1")
+    cfg = U.config([U.delta(heads=4, kv_heads=2, dim=100, vdim=40, ff=24), U.delta(heads=4, kv_heads=2, dim=64, vdim=130, ff=0)])
+    for dtype in DTYPES:
+        check(own, cfg, U.weights(cfg, 22), toks(cfg, 201), dtype, [201])
     own.close()
 
 
