@@ -804,10 +804,15 @@ def hybrid_work(layers, width, vocab, rows, ctx, n_sm):
         if delta and rows == 1:
             add("delta_step_kernel", "hbm", 8.0 * H * V * mx["dim"])
         elif delta:
-            add("delta_prep_kernel", "hbm", 8.0 * rows * (2 * mx["kv_heads"] * mx["dim"] + H * V))
+            for name in ("delta_prep_kernel", "delta_prep4_kernel"):
+                add(name, "hbm", 8.0 * rows * (2 * mx["kv_heads"] * mx["dim"] + H * V))
             add("delta_pairs_kernel", "hbm", 8.0 * rows * mx["kv_heads"] * mx["dim"])
             add("delta_scan_kernel", "f32", 6.0 * rows * H * V * mx["dim"])  # two sums over d and one update
-            add("delta_out_kernel", "hbm", 10.0 * rows * H * V)
+            # in chunks of 32: k, q, v in, W, Z, U, O out; then the two sums and the update in six bf16 products each
+            add("delta_chunk_kernel", "hbm", 4.0 * rows * (2 * mx["kv_heads"] * mx["dim"] + 2 * H * mx["dim"] + 3 * H * V))
+            add("delta_chunk_scan_kernel", "tensor", 6 * 6.0 * rows * H * V * mx["dim"])
+            for name in ("delta_out_kernel", "delta_out4_kernel"):
+                add(name, "hbm", 10.0 * rows * H * V)
         elif rows == 1:
             add("latent_query_kernel", "hbm", 2.0 * H * mx["dim"] * mx["kv_rank"])
             add("latent_attn_mma_kernel", "hbm", 2.0 * min(mx["mask"]["size"], ctx + 1) * (mx["kv_rank"] + mx["rot_dim"]))
